@@ -33,6 +33,7 @@ SOURCES = [
     "stream_forms.cu",
     "experts.cu",
     "gemm_simt.cu",
+    "gemm_f32.cu",
     "attention_plain.cu",
     "sampling.cu",
     "gemm_tcgen05.cu",

@@ -1713,6 +1713,23 @@ def linear_plain(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torc
     return out
 
 
+def linear_f32_rows_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``linear_f32_rows`` runs for these operands: 1 to 8 rows of float32 on 16-byte boundaries."""
+    return (x.dtype == torch.float32 and 1 <= x.shape[0] <= 8 and x.shape[1] > 0 and x.shape[1] % 4 == 0 and x.stride(0) % 4 == 0
+            and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def linear_f32_rows(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """float32 ``x`` [M, K] times ``weight`` [N, K] transposed for up to 8 rows, with 32-bit FMAs: the weights are streamed."""
+    _need_cuda(x, weight)
+    assert x.dim() == 2 and weight.dim() == 2 and weight.is_contiguous() and weight.dtype == torch.float32
+    assert x.shape[1] == weight.shape[1] and linear_f32_rows_takes(x, weight)
+    m, k, n = x.shape[0], x.shape[1], weight.shape[0]
+    out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    _call("kirai_gemm_f32_rows", _ptr(x), _ptr(weight), _ptr(out), _i(m), _i(n), _i(k), _l(x.stride(0)), _l(n), _stream())
+    return out
+
+
 class TiledWeight:
     """A bf16 weight matrix [N, K] in the layout that the tensor-core product streams fastest: boxes of 128 rows
     x 64 columns, each stored as the 16 KB image that the 128-byte swizzle leaves in shared memory (the 16-byte
@@ -1978,12 +1995,15 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """The linear layer of the product path: 32-bit FMAs for float32; for bfloat16 the tcgen05
-    kernel, or the CUDA-core kernel when K is not a multiple of 8 (TMA cannot read such rows)."""
+    """The linear layer of the product path: 32-bit FMAs for float32 (a kernel that streams the weights for up to 8
+    rows whose rows it can read 16 bytes at a time, else the plain kernel); for bfloat16 the tcgen05 kernel, or the
+    CUDA-core kernel when K is not a multiple of 8 (TMA cannot read such rows)."""
     if isinstance(weight, TiledWeight):
         return linear_tcgen05(x if tcgen05_takes(x) else x.contiguous(), weight, out_dtype)
     if tcgen05_takes(x):
         return linear_tcgen05(x, weight, out_dtype)
+    if weight.dtype == torch.float32 and out_dtype in (None, torch.float32) and linear_f32_rows_takes(x, weight):
+        return linear_f32_rows(x, weight)
     return linear_plain(x, weight, out_dtype)
 
 

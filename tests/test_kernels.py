@@ -119,6 +119,24 @@ def test_linear_plain_float32_is_exact_enough(ops, m, n, k):
     assert float((out - expected).abs().max()) <= 1e-5 * math.sqrt(k)
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("n,k", [(1, 4), (33, 124), (31, 128), (40, 512), (9, 516), (130, 1000), (7, 4100), (1003, 2560)])
+def test_linear_float32_of_few_rows(ops, m, n, k):
+    """Edges of the 128-column pieces, of four warps' shares of K and of a block's rows; rows of a wider matrix."""
+    x, w = rand(m, k + 8)[:, 4 : 4 + k], rand(n, k, seed=3)
+    expected = x.double() @ w.double().T
+    out = ops.linear(x, w)
+    # every rounding of a sum of k products is at most 2^-24 of the running sum of sizes, and no sum is longer than
+    # k / 32 + 16 steps (a lane's share of K, the butterfly, the warps)
+    bound = (k / 32 + 16) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T)
+    assert bool(((out.double() - expected).abs() <= bound).all())
+    assert torch.equal(out, ops.linear_f32_rows(x, w))
+    plain = ops.linear(rand(m, k + 9)[:, 1 : 1 + k], w)  # rows that are not on 16-byte boundaries: the plain kernel
+    assert torch.equal(plain, ops.linear_plain(rand(m, k + 9)[:, 1 : 1 + k], w))
+    x[0, 0] = float("inf")
+    assert torch.equal(ops.linear(x, w)[0].isinf(), w[:, 0] != 0)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 128, 64), (3, 200, 136), (16, 1000, 512), (48, 520, 1032), (64, 4096, 264),
                                    (65, 264, 192), (100, 1000, 2080), (128, 4096, 4096), (129, 520, 1032),
                                    (200, 96, 64), (256, 4096, 2112), (257, 264, 192), (300, 1000, 520), (1024, 768, 2048)])
