@@ -34,6 +34,7 @@ SOURCES = [
     "experts.cu",
     "gemm_simt.cu",
     "gemm_f32.cu",
+    "gemm_f32_tc.cu",
     "attention_plain.cu",
     "sampling.cu",
     "gemm_tcgen05.cu",

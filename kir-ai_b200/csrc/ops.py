@@ -1730,6 +1730,27 @@ def linear_f32_rows(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def linear_f32_tc_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``linear_f32_tc`` runs for these operands: rows of float32 on 16-byte boundaries."""
+    return (x.dtype == torch.float32 and x.shape[0] > 0 and x.shape[1] > 0 and x.shape[1] % 4 == 0 and x.stride(0) % 4 == 0
+            and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
+
+
+def linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, tile_rows: int = 0, splits: int = 0) -> torch.Tensor:
+    """float32 ``x`` [M, K] times ``weight`` [N, K] transposed on the tensor cores, every float as three bf16 values: at
+    least as exact as 32-bit FMAs.  ``tile_rows`` (32, 64, 128 or 192) and ``splits`` (1 to 8) force how the product is
+    cut into CTAs; 0 leaves it to the kernel's rule."""
+    _need_cuda(x, weight)
+    assert x.dim() == 2 and weight.dim() == 2 and weight.is_contiguous() and weight.dtype == torch.float32
+    assert x.shape[1] == weight.shape[1] and linear_f32_tc_takes(x, weight)
+    m, k, n = x.shape[0], x.shape[1], weight.shape[0]
+    out = torch.empty((m, n), dtype=torch.float32, device=x.device)
+    planes = torch.empty((3, m, (k + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
+    _call("kirai_gemm_f32_tc", _ptr(x), _ptr(weight), _ptr(planes), _ptr(out), _i(m), _i(n), _i(k), _l(x.stride(0)), _l(n),
+          _i(tile_rows), _i(splits), _ptr(error_flag(x.device)), _stream())
+    return out
+
+
 class TiledWeight:
     """A bf16 weight matrix [N, K] in the layout that the tensor-core product streams fastest: boxes of 128 rows
     x 64 columns, each stored as the 16 KB image that the 128-byte swizzle leaves in shared memory (the 16-byte
@@ -1995,15 +2016,18 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """The linear layer of the product path: 32-bit FMAs for float32 (a kernel that streams the weights for up to 8
-    rows whose rows it can read 16 bytes at a time, else the plain kernel); for bfloat16 the tcgen05 kernel, or the
+    """The linear layer of the product path: for float32, where rows can be read 16 bytes at a time, a kernel that streams
+    the weights (up to 8 rows) or products of values cut in three on the tensor cores, else the plain kernel; for bfloat16 the tcgen05 kernel, or the
     CUDA-core kernel when K is not a multiple of 8 (TMA cannot read such rows)."""
     if isinstance(weight, TiledWeight):
         return linear_tcgen05(x if tcgen05_takes(x) else x.contiguous(), weight, out_dtype)
     if tcgen05_takes(x):
         return linear_tcgen05(x, weight, out_dtype)
-    if weight.dtype == torch.float32 and out_dtype in (None, torch.float32) and linear_f32_rows_takes(x, weight):
-        return linear_f32_rows(x, weight)
+    if weight.dtype == torch.float32 and out_dtype in (None, torch.float32):
+        if linear_f32_rows_takes(x, weight):
+            return linear_f32_rows(x, weight)
+        if linear_f32_tc_takes(x, weight):
+            return linear_f32_tc(x, weight)
     return linear_plain(x, weight, out_dtype)
 
 

@@ -84,6 +84,40 @@ inline bool bf16_2d_sw128(CUtensorMap* out, const void* ptr, uint64_t rows, uint
     return true;
 }
 
+// The same for any element type and swizzle: FORM 0 is float32 read in boxes of 32 columns with the 128-byte swizzle,
+// FORM 1 bf16 in boxes of 32 columns with the 64-byte swizzle.
+template <int FORM>
+inline bool matrix_boxes(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t cols, uint64_t row_stride, uint32_t box_rows) {
+    static std::unordered_map<Key, CUtensorMap, KeyHash> cache;
+    static std::mutex mutex;
+    constexpr uint64_t element = FORM == 0 ? 4 : 2;
+    const Key key{ptr, rows, cols, row_stride, box_rows, 32};
+    std::lock_guard<std::mutex> lock(mutex);
+    auto found = cache.find(key);
+    if (found != cache.end()) {
+        *out = found->second;
+        return true;
+    }
+    EncodeTiledFn encode = encode_fn();
+    if (!encode) return false;
+    if (((uintptr_t)ptr & 15) || (row_stride * element) % 16 != 0) return false;
+    cuuint64_t dims[2] = {cols, rows};
+    cuuint64_t strides[1] = {row_stride * element};
+    cuuint32_t box[2] = {32, box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    CUtensorMap map;
+    const CUresult status =
+        encode(&map, FORM == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims,
+               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               FORM == 0 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (status != CUDA_SUCCESS) return false;
+    if (cache.size() > 8192) cache.clear();
+    cache.emplace(key, map);
+    *out = map;
+    return true;
+}
+
 // The rows of a paged key/value cache, [rows, head_dim] bf16 with head_dim a multiple of 64, read in boxes of
 // `box_rows` whole rows (a multiple of 8) by ONE request each: the map has the dimensions (64 columns, 8 rows,
 // head_dim / 64 panels, rows / 8 groups), in that order, so that a box lands in shared memory as

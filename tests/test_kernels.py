@@ -137,6 +137,32 @@ def test_linear_float32_of_few_rows(ops, m, n, k):
     assert torch.equal(ops.linear(x, w)[0].isinf(), w[:, 0] != 0)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 4), (9, 130, 36), (32, 128, 32), (33, 127, 64), (64, 256, 96), (65, 129, 100),
+                                   (128, 130, 516), (193, 300, 1028), (400, 257, 2600)])
+def test_linear_float32_on_tensor_cores(ops, m, n, k):
+    """Edges of the tiles (32 to 192 rows, 128 columns, 32 values of K), every cut; rows of a wider matrix."""
+    x, w = rand(m, k + 8)[:, 4 : 4 + k], rand(n, k, seed=3)
+    expected = x.double() @ w.double().T
+    # a product leaves out what lies 2^-24 below it; sums of 32 values drop at most 2^-23 at each of 12 additions, and the
+    # k / 32 sums and up to 8 shares of K are added with 2^-24 each
+    bound = (14 * 2.0 ** -23 + (k / 32 + 8) * 2.0 ** -24) * (x.abs().double() @ w.abs().double().T)
+    for tile_rows in (0, 32, 64, 128, 192):
+        for splits in (1, 2, 3, 8):
+            out = ops.linear_f32_tc(x, w, tile_rows, splits)
+            assert bool(((out.double() - expected).abs() <= bound).all()), (tile_rows, splits)
+    ops.check_device_errors(torch.device(DEV))
+    if m > 8:
+        assert torch.equal(ops.linear(x, w), ops.linear_f32_tc(x, w))
+    # values that are not finite, and such as the sum of two overflows, come out as the chain of FMAs has them
+    x[0, 0], x[-1, -1], w[0, k // 2] = float("inf"), float("nan"), 3e38
+    plain = ops.linear_plain(x, w)
+    for splits in (1, 2):
+        out = ops.linear_f32_tc(x, w, 32, splits)
+        assert torch.equal(out.isnan(), plain.isnan()) and torch.equal(out[out.isinf()], plain[plain.isinf()])
+    with pytest.raises(AssertionError):
+        ops.linear_f32_tc(rand(m, k + 9)[:, 1 : 1 + k], w)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 128, 64), (3, 200, 136), (16, 1000, 512), (48, 520, 1032), (64, 4096, 264),
                                    (65, 264, 192), (100, 1000, 2080), (128, 4096, 4096), (129, 520, 1032),
                                    (200, 96, 64), (256, 4096, 2112), (257, 264, 192), (300, 1000, 520), (1024, 768, 2048)])
