@@ -36,6 +36,7 @@ SOURCES = [
     "gemm_f32.cu",
     "gemm_f32_tc.cu",
     "attention_plain.cu",
+    "attention_f32.cu",
     "sampling.cu",
     "gemm_tcgen05.cu",
     "gemm_chain.cu",

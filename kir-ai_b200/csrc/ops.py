@@ -1373,6 +1373,61 @@ def paged_attention_plain(q: torch.Tensor, cache: torch.Tensor, block_table: tor
     return out
 
 
+def attention_takes_f32_tiles(q: torch.Tensor, cache: torch.Tensor) -> bool:
+    """Whether float32 attention runs on the kernels that read a key row once for many query rows
+    (``csrc/attention_f32.cu``): heads of up to 128 columns in fours (16-byte loads), at most 64 query heads to a kv head
+    (the rows of a CTA), rows on 16-byte boundaries.  Every other form takes the plain kernel.  The 4B shape's layer: a prompt of
+    515 tokens 130 us here and 1,139 us plain, a decode step's 4 requests of about 106 tokens 6.4 and 23 us; the tiny model
+    (heads of 32, a window of 16) 5 and 8 us."""
+    return (q.dtype == torch.float32 and q.shape[2] % 4 == 0 and q.shape[2] <= 128 and q.shape[1] <= 64 * cache.shape[2]
+            and q.stride(0) % 4 == 0 and q.data_ptr() % 16 == 0 and cache.data_ptr() % 16 == 0)
+
+
+def attention_f32_prefill(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, query_start: torch.Tensor,
+                          context_len: torch.Tensor, max_query_len: int, window: Optional[int], scale: float,
+                          out: Optional[torch.Tensor] = None, chunk: Optional[int] = None, softcap: Optional[float] = None,
+                          keep_first: int = 0, sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """32-bit attention for runs of new tokens: what ``attention_prefill`` is in bfloat16, with the same arguments."""
+    _need_cuda(q, cache, block_table, query_start, context_len)
+    num_pages, kv_heads, page_size, head_dim = _cache_dims(cache)
+    rows, q_heads, qd, q_stride = _head_view(q)
+    assert qd == head_dim and q.dtype == torch.float32 and cache.dtype == torch.float32
+    requests = context_len.numel()
+    assert query_start.numel() == requests + 1 and query_start.dtype == torch.int32 and context_len.dtype == torch.int32
+    if out is None:
+        out = torch.empty((rows, q_heads * head_dim), dtype=q.dtype, device=q.device)
+    assert out.shape == (rows, q_heads * head_dim) and out.dtype == q.dtype and out.is_contiguous()
+    assert sinks is None or (sinks.is_cuda and sinks.dtype == torch.float32 and sinks.numel() == q_heads and sinks.is_contiguous())
+    _call("kirai_attention_f32_prefill", _ptr(q), _ptr(cache), _ptr(out), _ptr(block_table), _ptr(query_start), _ptr(context_len),
+          _i(requests), _i(max_query_len), _i(q_heads), _i(kv_heads), _i(head_dim), _l(q_stride), _i(page_size), _i(block_table.shape[1]),
+          _i(num_pages), _i(mask_code(window, chunk, keep_first)), _f(scale), _f(softcap or 0.0), _ptr(sinks), _ptr(error_flag(q.device)),
+          _stream(), detail=_attention_detail(q_heads, kv_heads, head_dim, window, chunk, keep_first))
+    return out
+
+
+def attention_f32_decode(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, context_len: torch.Tensor, longest: int,
+                         window: Optional[int], scale: float, out: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
+                         softcap: Optional[float] = None, keep_first: int = 0, sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """32-bit attention for a batch in which every request brings one token; ``longest``: the longest context, or a bound on it, by
+    which the launch is cut (any value is correct)."""
+    _need_cuda(q, cache, block_table, context_len)
+    num_pages, kv_heads, page_size, head_dim = _cache_dims(cache)
+    rows, q_heads, qd, q_stride = _head_view(q)
+    assert qd == head_dim and q.dtype == torch.float32 and cache.dtype == torch.float32
+    assert context_len.numel() == rows and context_len.dtype == torch.int32
+    if out is None:
+        out = torch.empty((rows, q_heads * head_dim), dtype=q.dtype, device=q.device)
+    assert out.shape == (rows, q_heads * head_dim) and out.dtype == q.dtype and out.is_contiguous()
+    assert sinks is None or (sinks.is_cuda and sinks.dtype == torch.float32 and sinks.numel() == q_heads and sinks.is_contiguous())
+    reach = (window + keep_first if window else None) or chunk or longest
+    _call("kirai_attention_f32_decode", _ptr(q), _ptr(cache), _ptr(out), _ptr(block_table), _ptr(context_len), _i(rows), _i(q_heads),
+          _i(kv_heads), _i(head_dim), _l(q_stride), _i(page_size), _i(block_table.shape[1]), _i(num_pages),
+          _i(mask_code(window, chunk, keep_first)), _f(scale), _f(softcap or 0.0), _ptr(sinks), _i(min(longest, reach)),
+          _i(sm_count(q.device)), _ptr(error_flag(q.device)), _stream(),
+          detail=_attention_detail(q_heads, kv_heads, head_dim, window, chunk, keep_first))
+    return out
+
+
 def attention_takes_tensor_cores(dtype: torch.dtype, head_dim: int) -> bool:
     """Whether attention over a cache of this dtype and head size runs on the tensor-core kernels (else the
     CUDA-core kernel, which takes any size)."""
@@ -1583,10 +1638,22 @@ def paged_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Ten
                     scale: float, chunk: Optional[int] = None, softcap: Optional[float] = None, keep_first: int = 0,
                     sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention of the product path over the paged cache for the tokens of ``batch``
-    (a kirai_b200.engine.batch.StepBatch).  float32 takes the plain kernel; bfloat16 takes the
+    (a kirai_b200.engine.batch.StepBatch).  float32 takes the 32-bit tile kernels, or the plain kernel for
+    forms they do not take (``attention_takes_f32_tiles``); bfloat16 takes the
     tensor-core kernels (the decode kernel when every request brings one token), or the plain
     kernel for head sizes they do not take (not a multiple of 8, or above 256)."""
     head_dim, q_heads, kv_heads = q.shape[2], q.shape[1], cache.shape[2]
+    if attention_takes_f32_tiles(q, cache):
+        rows = batch.num_requests if batch.decode_only else getattr(batch, "num_decode", 0)
+        form = dict(chunk=chunk, softcap=softcap, keep_first=keep_first, sinks=sinks)
+        out = torch.empty((q.shape[0], q_heads * head_dim), dtype=q.dtype, device=q.device)
+        if rows:
+            attention_f32_decode(q[:rows], cache, block_table[:rows], batch.context_len[:rows], batch.max_context_len, window, scale,
+                                 out=out[:rows], **form)
+        if rows < batch.num_requests:
+            attention_f32_prefill(q, cache, block_table[rows:], batch.query_start[rows:], batch.context_len[rows:], batch.max_query_len,
+                                  window, scale, out=out, **form)
+        return out
     fast = attention_takes_tensor_cores(q.dtype, head_dim) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0
     if not fast:
         return paged_attention_plain(q, cache, block_table, batch.request_of_token, batch.positions, window, scale,

@@ -820,3 +820,69 @@ def test_attention_with_block_tables_longer_than_the_shared_copy(ops):
         out = ops.attention_prefill(q, cache, table, qs, ctx, 1, None, scale, tcgen05=use_tcgen05).float().cpu().unflatten(1, (q_heads, head_dim))
         assert float((out[0, 0] - expected).abs().max()) <= 3e-2, use_tcgen05
     ops.check_device_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,page_size,form",
+                         [(32, 8, 128, 16, {}), (6, 2, 32, 16, {"window": 16}), (8, 1, 128, 5, {"window": 70, "keep_first": 3}),
+                          (5, 5, 4, 1, {"chunk": 48}), (12, 2, 80, 7, {"softcap": 3.0}), (16, 1, 64, 64, {"sinks": True}),
+                          (64, 1, 68, 16, {"window": 1}), (3, 1, 48, 8, {"chunk": 200, "sinks": True})])
+def test_32_bit_attention_tiles_against_64_bit_arithmetic(ops, q_heads, kv_heads, head_dim, page_size, form):
+    """Portions and single tokens through both 32-bit tile kernels.  Rows of the cache that no query may see hold NaN, and the
+    last token's value is infinite: neither may reach a row that does not see it."""
+    lengths, counts = [150, 5, 64, 1100], [71, 5, 1, 130]
+    cache, table, keys, values = paged_setup(torch.float32, lengths, kv_heads, head_dim, page_size, seed=3)
+    cache.fill_(float("nan"))
+    for r, n in enumerate(lengths):
+        values[r][n - 1, 0, head_dim - 1] = float("inf")
+        ops.kv_write(keys[r].to(DEV).contiguous(), values[r].to(DEV).contiguous(), cache, table,
+                     torch.full((n,), r, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV))
+    generator = torch.Generator().manual_seed(4)
+    q = torch.randn(sum(counts), q_heads + 2, head_dim, generator=generator).to(DEV)[:, :q_heads]  # rows with a stride of their own
+    scale = head_dim ** -0.5
+    sinks = torch.randn(q_heads, generator=generator).to(DEV) if form.get("sinks") else None
+    window, chunk, keep, cap = form.get("window"), form.get("chunk"), form.get("keep_first", 0), form.get("softcap")
+    options = dict(chunk=chunk, softcap=cap, keep_first=keep, sinks=sinks)
+
+    def expected(rows, r, positions):
+        k, v = (x[r].double().to(DEV).repeat_interleave(q_heads // kv_heads, dim=1) for x in (keys, values))
+        s = torch.einsum("thd,jhd->thj", rows.double(), k) * scale
+        s = cap * torch.tanh(s / cap) if cap else s
+        i, j = torch.tensor(positions, device=DEV)[:, None], torch.arange(len(k), device=DEV)[None, :]
+        seen = (j <= i) & ((i - j < window) | (j < keep) if window else j >= i - i % chunk if chunk else True)
+        s = s.masked_fill(~seen[:, None], -math.inf)
+        if sinks is not None:
+            s = torch.cat([s, sinks.double().view(1, -1, 1).expand(len(rows), -1, 1)], dim=-1)
+        p = torch.softmax(s, dim=-1)[..., : len(k)]
+        out = torch.einsum("thj,jhd->thd", p, v.nan_to_num(posinf=0.0))
+        out[(seen[:, -1])[:, None] & (torch.arange(q_heads, device=DEV) < q_heads // kv_heads), head_dim - 1] = math.inf
+        return out
+
+    assert ops.attention_takes_f32_tiles(q, cache)
+    # a score is a sum of up to 128 products, each rounded; weights and result follow it: (128 + 2) * 2^-24 * |q||k| scale
+    # bounds a score's error by 1e-4, its usual size is a tenth of that, and the values' mean moves by as much
+    bound = 3e-5
+    start = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    context = torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    fast = ops.attention_f32_prefill(q, cache, table, start, context, max(counts), window, scale, **options).unflatten(1, (q_heads, head_dim))
+    ends = torch.stack([q[int(e) - 1] for e in start[1:]])
+    alone = {longest: ops.attention_f32_decode(ends, cache, table, context, longest, window, scale, **options).unflatten(1, (q_heads, head_dim))
+             for longest in (1, 300, 1100)}  # one CTA, then clusters of CTAs (as many as the SMs hold)
+    ops.check_device_errors(torch.device(DEV))
+    for r, (n, count) in enumerate(zip(lengths, counts)):
+        want = expected(q[start[r] : start[r + 1]], r, list(range(n - count, n)))
+        for got, rows in [(fast[start[r] : start[r + 1]], want)] + [(a[r : r + 1], want[-1:]) for a in alone.values()]:
+            finite = torch.isfinite(rows)
+            assert torch.equal(torch.isfinite(got), finite)
+            assert float((got.double() - rows)[finite].abs().max()) <= bound, (r, float((got.double() - rows)[finite].abs().max()))
+
+
+def test_32_bit_attention_reports_a_missing_page(ops):
+    cache, table, keys, values = paged_setup(torch.float32, [40], 1, 32, 8)
+    q = rand(40, 2, 32)
+    table[0, 1] = -1
+    start, context = torch.tensor([0, 40], dtype=torch.int32, device=DEV), torch.tensor([40], dtype=torch.int32, device=DEV)
+    for call in (lambda: ops.attention_f32_prefill(q, cache, table, start, context, 40, None, 1.0),
+                 lambda: ops.attention_f32_decode(q[:1], cache, table, context, 40, None, 1.0)):
+        call()
+        with pytest.raises(ops.KernelError, match="no page"):
+            ops.check_device_errors(torch.device(DEV))
