@@ -74,6 +74,7 @@ struct GemmSmem {
                                           : (BN > 128 ? 4 : (BN > 64 ? (DEEP ? 6 : 3) : (DEEP ? (BN <= 16 ? 10 : (BN <= 32 ? 7 : 8)) : 4)));
     static constexpr int barrier_bytes = 2048;  // barriers [0, 256), row scales [256, 256 + 4 BN) (BN <= 256)
     static constexpr int stage_tokens = BN < 64 ? BN : 64;  // tokens that the staged stores take through shared memory at a time
+    // (from 1024 on, tiles of up to 64 tokens: the list of chosen experts)
     static_assert(!streaming || (2 * stages + 1) * 8 + 4 <= 256, "the streaming kernel's barriers must end before the row scales");
     static_assert(!DEEP || BN <= 32 || late_slots, "a long ring beside slots is for the smallest tiles");
     // LATE: what a CTA receives (from each other CTA the 16-token chunks that it owns, 8 KB each) and the staged tokens
@@ -115,7 +116,17 @@ struct Epilogue {
     // g = min(gate, gate_limit) and u = clamp(up, -gate_limit, gate_limit) the result is g sigmoid(gate_slope g) (u + 1).
     int gate_act = 0;
     float gate_limit = 0.0f, gate_slope = 1.0f;
+    // Products with the matrices of experts of which a step's few tokens use a part (weight-streaming kernel only): W's
+    // first chosen_experts * chosen_unit row tiles (chosen_columns: blocks of K) are the experts', chosen_unit to each,
+    // what stands behind them is always needed.  An expert whose gate is 0 for all chosen_tokens rows of `gates`
+    // [tokens, gates_stride] is not read: its row tiles are not computed and their part of C keeps what it held; its blocks
+    // of K, whose columns of A must be zero, are left out of the sum.  Null: every tile.
+    const float* gates = nullptr;
+    int gates_stride = 0, chosen_tokens = 0, chosen_experts = 0, chosen_unit = 1;
+    bool chosen_columns = false;
+    int chosen_tiles = 0;  // row tiles that the launch is expected to compute (host; picks the ring)
 };
+#define GEMM_MAX_CHOSEN 255  // experts whose numbers fit the list in the CTA's barrier page
 
 // Clock stamps of one CTA of the streaming kernel, written only when a buffer is given: 0 the CTA starts, 1 the kernel
 // before has finished (activations may be read), 2 the first stage is in shared memory, 3 the last product is done,
@@ -230,15 +241,52 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int x0 = blockIdx.x * GEMM_BM;  // first row of X in this tile
-    const int y0 = blockIdx.y * BN;       // first row of Y
-    const int total_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
-    const int kb_begin = blockIdx.z * k_blocks_per_split;
-    const int kb_end = min(total_k_blocks, kb_begin + k_blocks_per_split);
-    const int num_kb = max(0, kb_end - kb_begin);
+    const int y0 = blockIdx.y * BN;  // first row of Y
+    const int row_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;  // boxes of a row of tiles
+    int total_k_blocks = row_k_blocks, x_tile = blockIdx.x;
     const uint32_t rank = blockIdx.z;  // the cluster is (1, 1, splits) and the grid's z extent is splits
     pdl_launch_dependents();  // the next kernel may set itself up while this one streams
     if (threadIdx.x == 0) gemm_stamp(ep, 0);
+    const int* chosen_s = reinterpret_cast<const int*>(smem + STAGES * Smem::stage_bytes + 1024);  // how many, then which
+    if constexpr (SWAP && BN <= 64) {
+        if (ep.gates) {
+            // The list of the experts that some token uses, in ascending order; every CTA makes its own (a column of gates
+            // per lane).  It needs the kernel before this one, so such a launch cannot fetch weights ahead of it.
+            pdl_wait();
+            int* list = const_cast<int*>(chosen_s);
+            if (warp == 0) {
+                int count = 0;
+                for (int base = 0; base < ep.chosen_experts; base += 32) {
+                    const int e = base + lane;
+                    bool used = false;
+                    if (e < ep.chosen_experts) {
+#pragma unroll 4
+                        for (int t = 0; t < ep.chosen_tokens; ++t) used |= ep.gates[(size_t)t * ep.gates_stride + e] != 0.0f;
+                    }
+                    const uint32_t mask = __ballot_sync(0xffffffffu, used);
+                    if (used) list[1 + count + __popc(mask & ((1u << lane) - 1u))] = e;
+                    count += __popc(mask);
+                }
+                if (lane == 0) list[0] = count;
+            }
+            __syncthreads();
+            const int count = chosen_s[0], unit = ep.chosen_unit;
+            if (ep.chosen_columns) {
+                total_k_blocks -= (ep.chosen_experts - count) * unit;
+                k_blocks_per_split = (total_k_blocks + splits - 1) / splits;
+            } else {
+                // the tiles behind the experts' first, then the chosen experts': the CTAs with work are the first of the
+                // grid, which the device spreads evenly over its SMs
+                const int behind = (int)gridDim.x - ep.chosen_experts * unit, at = x_tile - behind;
+                if (at >= count * unit) return;  // (all CTAs of a cluster have the same tile)
+                x_tile = at < 0 ? ep.chosen_experts * unit + x_tile : chosen_s[1 + at / unit] * unit + at % unit;
+            }
+        }
+    }
+    const int x0 = x_tile * GEMM_BM;  // first row of X in this tile
+    const int kb_begin = blockIdx.z * k_blocks_per_split;
+    const int kb_end = min(total_k_blocks, kb_begin + k_blocks_per_split);
+    const int num_kb = max(0, kb_end - kb_begin);
 
     if (threadIdx.x == 0) {
         tma_prefetch_descriptor(&map_x);
@@ -279,7 +327,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // of the first ring of stages is fetched at once, and only the activations wait for it.
             const int x_first = SWAP ? 0 : 1, y_first = SWAP ? 1 : 0;  // which operand is the weights
             // tiled weights (SWAP only): this tile's boxes lie one after the other
-            const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)blockIdx.x * total_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
+            const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)x_tile * row_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
+            // this CTA's i-th block of K, counted from kb_begin: the i-th, but for the blocks of experts that are left out
+            auto block = [&](int i) {
+                if constexpr (SWAP && BN <= 64) {
+                    if (ep.gates && ep.chosen_columns) {
+                        const int at = kb_begin + i, unit = ep.chosen_unit, own = chosen_s[0] * unit;
+                        return (at < own ? chosen_s[1 + at / unit] * unit + at % unit : ep.chosen_experts * unit + at - own) - kb_begin;
+                    }
+                }
+                return i;
+            };
             auto load_x = [&](uint32_t dst, uint32_t full, int i) {
                 if (SWAP && boxes) bulk_load_1d(dst, boxes + (size_t)i * GEMM_BOX_BYTES, GEMM_BOX_BYTES, full);
                 else tma_load_2d(dst, &map_x, full, (kb_begin + i) * GEMM_BK, x0);
@@ -289,8 +347,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 const uint32_t full = smem_addr(&full_bar[i]);
                 mbar_expect_tx(full, Smem::stage_bytes);
                 const uint32_t dst = smem_addr(smem + i * Smem::stage_bytes);
-                const int k = (kb_begin + i) * GEMM_BK;
-                if (x_first == 0) load_x(dst, full, i);
+                const int at = block(i), k = (kb_begin + at) * GEMM_BK;
+                if (x_first == 0) load_x(dst, full, at);
                 if (y_first == 0) tma_load_2d(dst + Smem::x_bytes, &map_y, full, k, y0);
             }
             pdl_wait();  // what the kernel before wrote (the activations) is complete and visible
@@ -298,8 +356,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             for (int i = 0; i < head; ++i) {
                 const uint32_t full = smem_addr(&full_bar[i]);
                 const uint32_t dst = smem_addr(smem + i * Smem::stage_bytes);
-                const int k = (kb_begin + i) * GEMM_BK;
-                if (x_first == 1) load_x(dst, full, i);
+                const int at = block(i), k = (kb_begin + at) * GEMM_BK;
+                if (x_first == 1) load_x(dst, full, at);
                 if (y_first == 1) tma_load_2d(dst + Smem::x_bytes, &map_y, full, k, y0);
             }
             for (int i = head; i < num_kb; ++i) {
@@ -309,8 +367,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 const uint32_t full = smem_addr(&full_bar[s]);
                 mbar_expect_tx(full, Smem::stage_bytes);
                 const uint32_t dst = smem_addr(smem + s * Smem::stage_bytes);
-                const int k = (kb_begin + i) * GEMM_BK;
-                load_x(dst, full, i);
+                const int at = block(i), k = (kb_begin + at) * GEMM_BK;
+                load_x(dst, full, at);
                 tma_load_2d(dst + Smem::x_bytes, &map_y, full, k, y0);
             }
         }
@@ -1150,12 +1208,14 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
         const long clusters = (long)grid.x * grid.y;
         if constexpr (BN <= 128) {  // (tiles of 256 tokens have one configuration: four stages, one CTA per SM)
             // no more CTAs than SMs: one CTA per SM with the long ring (KIRAI_GEMM_DEEP=0 keeps the short one, to compare)
-            if (clusters * used <= sm_count() && deep_rings()) {
+            // (a product with the chosen experts alone: by the tiles that it is expected to compute)
+            const long busy = ep.chosen_tiles > 0 ? (long)ep.chosen_tiles * grid.y : clusters;
+            if (busy * used <= sm_count() && deep_rings()) {
                 using Deep = GemmSmem<BN, true, true>;
                 auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, true>;
                 cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Deep::total(Deep::max_splits));
                 if (err != cudaSuccess) return (int)err;
-                if (used > 1 && splits > 1 && clusters > max_resident_clusters(kernel, Deep::total(used), used)) continue;
+                if (used > 1 && splits > 1 && busy > max_resident_clusters(kernel, Deep::total(used), used)) continue;
                 return launch_pdl(kernel, grid, dim3(GEMM_THREADS), (size_t)Deep::total(used), stream, (unsigned)used, map_x,
                                   map_y, boxes, (OutT*)C, M, N, K, ldc, per_split, used, ep, error_flag);
             }
@@ -1278,6 +1338,33 @@ KIRAI_EXPORT int kirai_gemm_bf16_grouped(const void* A, const void* W, int tiled
     }
 #undef KIRAI_GROUPED
     return KIRAI_ERR_BAD_SIZE;
+}
+
+// A product of up to 64 tokens with the matrices of those experts alone that a token uses (see Epilogue::gates).
+//   gates [M, gates_stride] (float, on the device): nonzero where token m uses expert e < experts.
+//   columns 0: W [N, K] has `unit` tiles of 128 rows to each expert, then further rows that are always computed; the columns
+//   of C that belong to experts nobody uses are left as they were.  columns 1: every row of W has `unit` blocks of 64
+//   columns to each expert, then further columns that always count; columns of A that belong to experts nobody uses are not
+//   read.  expected_tiles (columns 0): row tiles that the launch will probably compute, by which it is cut.
+//   form 0: C bf16.  1: C float.
+KIRAI_EXPORT int kirai_gemm_bf16_chosen(const void* A, const void* W, int tiled, void* C, int M, int N, int K, long lda, long ldc,
+                                        int form, const float* gates, int gates_stride, int experts, int unit, int columns,
+                                        int expected_tiles, int* error_flag, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    const int pieces = columns ? (K + GEMM_BK - 1) / GEMM_BK : (N + GEMM_BM - 1) / GEMM_BM;
+    if (K <= 0 || M > 64 || !gates || gates_stride < experts || experts <= 0 || experts > GEMM_MAX_CHOSEN || unit <= 0 ||
+        (long)experts * unit > pieces || form < 0 || form > 1)
+        return KIRAI_ERR_BAD_SIZE;
+    Epilogue ep{nullptr, 0, 1.0f, 0.0f, nullptr, nullptr, nullptr, nullptr};
+    ep.gates = gates, ep.gates_stride = gates_stride, ep.chosen_tokens = M, ep.chosen_experts = experts, ep.chosen_unit = unit;
+    ep.chosen_columns = columns != 0;
+    int splits = 0;
+    if (!columns) {
+        ep.chosen_tiles = expected_tiles < 1 ? 1 : (expected_tiles < pieces ? expected_tiles : pieces);
+        splits = choose_splits(M, ep.chosen_tiles * GEMM_BM, K);
+    }
+    return form == 0 ? gemm_dispatch<bf16, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream)
+                     : gemm_dispatch<float, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream);
 }
 
 // The one entry point of the tensor-core product, A[M, K] (row stride lda) times W[N, K] transposed.

@@ -1268,6 +1268,41 @@ def linear_grouped(x: torch.Tensor, weight, groups: int, tile_group: torch.Tenso
     return out
 
 
+CHOSEN_MAX_ROWS = 64      # tokens of the weight-streaming kernel's tiles
+CHOSEN_MAX_EXPERTS = 255  # the list that every CTA makes
+
+
+def linear_chosen_takes(x: torch.Tensor, experts: int, expert_size: int, rows_of_expert: int) -> bool:
+    """Whether the products of a step of few tokens may read the matrices of the chosen experts alone: an expert's rows in the
+    first product are whole tiles of 128, its columns in the second whole blocks of 64, so that a tile or block belongs to
+    one expert."""
+    return (x.shape[0] <= CHOSEN_MAX_ROWS and experts <= CHOSEN_MAX_EXPERTS and rows_of_expert % 128 == 0 and expert_size % 64 == 0
+            and tcgen05_takes(x))
+
+
+def linear_chosen(x: torch.Tensor, weight, gates: torch.Tensor, experts: int, unit: int, columns: bool, expected_tiles: int = 1,
+                  out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
+    """``x`` [M, K] (bfloat16, at most 64 rows) times ``weight`` [N, K] transposed, reading only the matrices of experts that
+    some token uses: ``gates`` [M, >= experts] (float32) is nonzero there.
+
+    ``columns`` false: ``weight`` has ``unit`` tiles of 128 rows to each expert, then rows that are always computed; the
+    result's columns of an expert that nobody uses are NOT written (whatever memory held: multiply them by their zero gate
+    only where a zero gate gives zero whatever stands there, as ``gated_expert_gate`` and ``relu2_gate_`` do).
+    ``expected_tiles``: row tiles that will probably be computed, by which the launch is cut.
+    ``columns`` true: ``weight`` has ``unit`` blocks of 64 columns to each expert, then columns that always count; the columns of
+    ``x`` that belong to experts nobody uses are left out of the sums (they would add zeros)."""
+    m, k, n = _check_product(x, weight)
+    _need_cuda(gates)
+    assert m <= CHOSEN_MAX_ROWS and gates.dtype == torch.float32 and gates.dim() == 2 and gates.is_contiguous() and gates.shape[0] == m
+    tiled = isinstance(weight, TiledWeight)
+    out = torch.empty((m, n), dtype=out_dtype, device=x.device)
+    _call("kirai_gemm_bf16_chosen", _ptr(x), _ptr(weight.boxes if tiled else weight), _i(tiled), _ptr(out), _i(m), _i(n), _i(k),
+          _l(x.stride(0)), _l(n), _i(0 if out_dtype == torch.bfloat16 else 1), _ptr(gates), _i(gates.shape[1]), _i(experts), _i(unit),
+          _i(int(columns)), _i(expected_tiles), _ptr(error_flag(x.device)), _stream(),
+          detail=f" m={m} n={n} k={k}" if _timer is not None else "")
+    return out
+
+
 # ------------------------------------------------------------------- cache write
 def _cache_dims(cache: torch.Tensor):
     assert cache.dim() == 5 and cache.shape[1] == 2 and cache.is_contiguous(), "cache layer is [pages, 2, kv_heads, page, d]"

@@ -12,10 +12,14 @@ and multiplies by the token's routing weight of the column's expert (zero for
 an expert that was not chosen), and the down product then sums the chosen
 experts' outputs in its own accumulation.  Nothing depends on how many tokens
 an expert drew, so a step of single tokens can be captured in a graph; the
-price is that every expert's rows are computed for every token, experts / top
-times the arithmetic that the chosen experts alone would need.  For a step of
-few tokens that price is none: the products are bound by reading the weights,
-and a handful of tokens between them choose most experts anyway.
+price is that every chosen expert's rows are computed for every token.  For a
+step of few tokens that price is none: the products are bound by reading the
+weights.  In bfloat16 (up to 64 tokens, expert sizes in whole boxes of the
+weights) they read the chosen experts' matrices alone: each CTA looks the
+step's routing weights over on the device and takes a tile, or the blocks of
+K, of an expert that some token uses (``_reads_chosen``; 16 experts of which a
+token uses two, width 4096, expert size 1536, three tokens: the two products
+of a layer 94 us with all experts' matrices, 46 with the chosen ones).
 
 Steps of many tokens (``GROUPED_MIN_ROWS`` pairs of token and chosen expert, in
 bfloat16, expert and model width multiples of 128) sort their pairs by expert
@@ -141,7 +145,7 @@ class RoutedExperts(FeedForward):
         self.down_stacked = Linear([(prefix + n["down"].format(e=e), hidden_size) for e in range(experts)], expert_size)
         self.router: Optional[torch.Tensor] = None
         self.router_product: Optional[Linear] = None
-        self.grouped = False
+        self.grouped = self.leaves_out = False
 
     def weight_specs(self) -> Dict[str, WeightSpec]:
         shared = self.shared.weight_specs() if self.shared is not None else {}
@@ -171,6 +175,8 @@ class RoutedExperts(FeedForward):
             self.rule = {"correction": self.correction, "scale": self.weight_scale, "extra": 1 if self.shared_gate_name else 0}
         self.up.load(weights, rt)
         self.down.load(weights, rt)
+        # a token leaves some experts out, and the products of few tokens run on the weight-streaming kernel
+        self.leaves_out = rt.dtype == torch.bfloat16 and self.top < self.routes
         # sorting by expert pays only where a token uses a part of the experts, and needs whole 128-row boxes per expert
         self.grouped = (rt.dtype == torch.bfloat16 and self.top < self.routes and self.expert_size % 128 == 0
                         and self.hidden_size % 128 == 0 and hasattr(rt.ops, "linear_grouped"))
@@ -193,6 +199,30 @@ class RoutedExperts(FeedForward):
             return ops.router_choose_(self.router_product.forward(x, torch.float32), self.top, want_chosen, over_all=self.over_all,
                                       rule=self.rule)
         return ops.router_gates(x, self.router, self.top, want_chosen, over_all=self.over_all, rule=self.rule)
+
+    def _reads_chosen(self, x: torch.Tensor) -> bool:
+        """Whether a step of few tokens reads the chosen experts' matrices alone.  Every expert stays a candidate for the
+        products (which of them are read is known on the device only, so that such a step can be captured); what it saves
+        is the share of experts that nobody chose, (1 - top / routes)^tokens of them: at 16 experts of which a token uses two,
+        88 % of the bytes for one token, 66 % for three, 12 % for sixteen.  Against that stands the head start that the
+        products lose (they fetch no weights before the router has finished), about 1 us each."""
+        return (self.leaves_out and hasattr(self.rt.ops, "linear_chosen") and self.down.out_features % 8 == 0
+                and self.rt.ops.linear_chosen_takes(x, self.experts, self.expert_size, self.expert_size * (2 if self.gated else 1)))
+
+    def _up_few(self, x: torch.Tensor, gates: torch.Tensor) -> torch.Tensor:
+        """The stacked first product; columns of experts that nobody chose may be left unwritten (their gates are zero)."""
+        if not self._reads_chosen(x):
+            return self.up.forward(x)
+        unit = self.expert_size * (2 if self.gated else 1) // 128
+        read = self.experts * (1.0 - (1.0 - self.top / self.routes) ** x.shape[0])
+        behind = -(-self.up.out_features // 128) - self.experts * unit
+        return self.rt.ops.linear_chosen(x, self.up.weight, gates, self.experts, unit, False, int(read * unit) + behind)
+
+    def _down_few(self, hidden: torch.Tensor, gates: torch.Tensor, out_dtype: Optional[torch.dtype]) -> torch.Tensor:
+        if not self._reads_chosen(hidden):
+            return self.down.forward(hidden, out_dtype)
+        return self.rt.ops.linear_chosen(hidden, self.down.weight, gates, self.experts, self.expert_size // 64, True,
+                                         out_dtype=out_dtype or torch.bfloat16)
 
     def _sorts(self, rows: int) -> bool:
         return self.grouped and rows * self.top >= GROUPED_MIN_ROWS
@@ -221,11 +251,11 @@ class RoutedExperts(FeedForward):
             shared = self.shared.forward(x) if self.shared is not None else None
             return None, sorted_rows, shared, gates, share_col, same
         gates = self._route(x, False)
-        hidden = self.rt.ops.gated_expert_gate(self.up.forward(x), gates, self.expert_size, self.gate_act, self.limit, self.slope,
+        hidden = self.rt.ops.gated_expert_gate(self._up_few(x, gates), gates, self.expert_size, self.gate_act, self.limit, self.slope,
                                                interleaved=self.interleaved, experts=self.experts, shared_ff=self.shared_ff,
                                                shared_col=self.routes)
         shared = self.shared.forward(x) if self.shared is not None and not self.stacks_shared else None
-        return self.down.forward(hidden, torch.float32), None, shared, gates, share_col, same
+        return self._down_few(hidden, gates, torch.float32), None, shared, gates, share_col, same
 
     def adds_normed(self, rows: int) -> bool:
         """Optional, for a block that norms this part's OUTPUT: whether, for a batch of ``rows`` tokens, the part has
@@ -265,10 +295,10 @@ class RoutedExperts(FeedForward):
             out = ops.route_combine(y, slot_of, mix)
             return out if self.out_dtype == torch.float32 else ops.round_rows(out)
         gates = self._route(x, False)
-        hidden = self.up.forward(x)
+        hidden = self._up_few(x, gates)
         if self.gated:
             hidden = ops.gated_expert_gate(hidden, gates, self.expert_size, self.gate_act, self.limit, self.slope,
                                            interleaved=self.interleaved)
         else:
             ops.relu2_gate_(hidden, gates, self.expert_size)
-        return self.down.forward(hidden, self.out_dtype)
+        return self._down_few(hidden, gates, self.out_dtype)

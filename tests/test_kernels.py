@@ -886,3 +886,34 @@ def test_32_bit_attention_reports_a_missing_page(ops):
         call()
         with pytest.raises(ops.KernelError, match="no page"):
             ops.check_device_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("tokens", [1, 3, 16, 17, 64])
+@pytest.mark.parametrize("experts,unit,behind,width", [(16, 2, 296, 520), (3, 1, 0, 64), (40, 1, 64, 1000)])
+@pytest.mark.parametrize("tiled", [False, True])
+def test_products_with_the_chosen_experts_alone(ops, tokens, experts, unit, behind, width, tiled):
+    """Both forms against 64-bit arithmetic of the matrices that some token uses: no expert, one, a few, all of them."""
+    weight = rand(experts * unit * 128 + behind, width, dtype=torch.bfloat16)
+    wide = rand(width, experts * unit * 64 + behind, dtype=torch.bfloat16, seed=1)
+    x = rand(tokens, width, dtype=torch.bfloat16, seed=2)
+    as_given = ops.tile_weight if tiled else (lambda w: w)
+    for used in ([], [experts - 1], [0, experts // 2], list(range(experts))):
+        gates = torch.zeros(tokens, experts + 3, device=DEV)
+        gates[:, experts:] = 1.0  # columns beyond the experts' say nothing about them
+        for i, e in enumerate(used):
+            gates[i % tokens, e] = -0.25 if i else 1e-30
+        rows = torch.tensor([e in used for e in range(experts)], device=DEV).repeat_interleave(unit * 128)
+        rows = torch.cat([rows, torch.ones(behind, dtype=torch.bool, device=DEV)])
+        want = x.double() @ weight.double().T
+        for expected in (1, len(used) * unit + 3, 10 ** 6):
+            got = ops.linear_chosen(x, as_given(weight), gates, experts, unit, False, expected, torch.float32)
+            # 32-bit sums of `width` products of about 1 each: the usual bound, width * 2^-24 * sum |x w|, with its random walk
+            assert torch.allclose(got[:, rows].double(), want[:, rows], rtol=0, atol=width * 2.0 ** -20), (used, expected)
+        hidden = rand(tokens, wide.shape[1], dtype=torch.bfloat16, seed=3)
+        columns = torch.tensor([e in used for e in range(experts)], device=DEV).repeat_interleave(unit * 64)
+        columns = torch.cat([columns, torch.ones(behind, dtype=torch.bool, device=DEV)])
+        want = (hidden * columns).double() @ wide.double().T
+        hidden[:, ~columns] = float("nan")  # left out, not multiplied by zero
+        got = ops.linear_chosen(hidden, as_given(wide), gates, experts, unit, True, out_dtype=torch.float32)
+        assert torch.allclose(got.double(), want, rtol=0, atol=wide.shape[1] * 2.0 ** -20), used
+    ops.check_device_errors(torch.device(DEV))
