@@ -270,7 +270,7 @@ sample_rows_kernel(const float* __restrict__ logits, float* __restrict__ probs_s
 #define SC_TRIES 7  // values that a search step tries at once: the candidates shrink to an eighth a step
 
 struct SampleExchange {
-    float f[2][8];  // this CTA's contribution to the reduction in flight; two in turn, so that one cluster barrier a
+    float f[2][16];  // this CTA's contribution to the reduction in flight; two in turn, so that one cluster barrier a
     int i[2][2];    // reduction is enough (a slot is written again only after the barrier that follows its reading)
 };
 
@@ -298,24 +298,6 @@ __device__ __forceinline__ int sc_load_s32(const int* local, uint32_t rank) {
     return value;
 }
 
-// Block-wide sums of COUNT numbers at once (two block barriers for all of them); every thread gets the results, and
-// the order of the additions depends only on the block size.  scratch: 32 * COUNT floats of shared memory.
-template <int COUNT>
-__device__ __forceinline__ void sc_block_sums(float (&values)[COUNT], float* scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < COUNT; ++j) values[j] = warp_sum(values[j]);
-    __syncthreads();
-    if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < COUNT; ++j) scratch[warp * COUNT + j] = values[j];
-    }
-    __syncthreads();
-    const int warps = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int j = 0; j < COUNT; ++j) values[j] = warp_sum(lane < warps ? scratch[lane * COUNT + j] : 0.0f);
-}
-
 // Sums over the cluster of numbers that every thread of this CTA holds (its CTA's partial results), in rank order.
 // One thread per number reads the eight slots (every thread doing so was 57,000 remote loads a CTA and step) and
 // hands the totals on through `totals` (8 floats of shared memory).
@@ -337,20 +319,176 @@ __device__ __forceinline__ void sc_cluster_sum(float (&values)[COUNT], SampleExc
     turn ^= 1;  // (totals is written again only behind the next cluster barrier, which every thread reaches after this)
 }
 
-// G(v) = sum of the row's probabilities greater than v, for COUNT values at once.
-template <int COUNT>
-__device__ __forceinline__ void sc_sums_greater(const float* probs_s, int count, const float (&v)[COUNT], float (&g)[COUNT],
-                                                float* scratch, SampleExchange* ex, int& turn) {
+// A warp's sums of eight numbers a lane in one transposing butterfly (9 shuffles; eight sums of their own are 40), to
+// scratch[warp * 16 + j].
+__device__ __forceinline__ void sc_warp_sums(float (&g)[8], float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int j = 0; j < COUNT; ++j) g[j] = 0.0f;
+    for (int half = 4; half > 0; half >>= 1) {
+        const bool upper = lane & (half * 4);
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float mine = upper ? g[i + half] : g[i], other = upper ? g[i] : g[i + half];
+            g[i] = mine + __shfl_xor_sync(0xffffffffu, other, half * 4);
+        }
+    }
+    float sum = g[0];  // lane L: of number L / 4
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    if ((lane & 3) == 0) scratch[warp * 16 + (lane >> 2)] = sum;
+}
+
+// The warps' numbers scratch[warp * 16 + j], j < n <= 16, added up over the block (a warp to each number) and over the cluster
+// (in rank order): totals[j], and totals[16 + j] the share of the CTAs of lower rank.
+__device__ __forceinline__ void sc_totals(int n, const float* scratch, float* totals, SampleExchange* ex, int& turn) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    if (warp < n) {
+        const float of_block = warp_sum(lane < (int)(blockDim.x >> 5) ? scratch[lane * 16 + warp] : 0.0f);
+        if (lane == 0) ex->f[turn][warp] = of_block;
+    }
+    sc_sync();
+    if (warp < n) {
+        const float part = lane < SC_CTAS ? sc_load_f32(&ex->f[turn][warp], lane) : 0.0f;
+        float all = 0.0f, lower = 0.0f;
+#pragma unroll
+        for (int q = 0; q < SC_CTAS; ++q) {
+            const float of_rank = __shfl_sync(0xffffffffu, part, q);
+            if (q < (int)sc_rank()) lower += of_rank;
+            all += of_rank;
+        }
+        if (lane == 0) totals[warp] = all, totals[16 + warp] = lower;
+    }
+    __syncthreads();
+    turn ^= 1;
+}
+
+// ---- the usual row: few entries hold the nucleus
+// A model that is fairly sure of its next token has its nucleus in a handful of entries, and the two searches below, some
+// twenty passes over the slice with seven block-wide sums and a cluster barrier each, took 150 us a row for what a short sorted
+// list answers.  So the pass that normalises the probabilities also adds up and counts those above SC_CUTS fixed fractions
+// of the greatest one; the first cut above which the entries reach the target (top_p, or the draw's threshold where the
+// whole vocabulary is the nucleus) is taken, and if at most SC_LIST entries lie above it, the first CTA collects them,
+// orders them by counting how many stand before each, and walks their running sums.  Otherwise the searches run.
+// Temperature 0.7, top_p 0.9, 151,936 logits: 1 row 146 -> 21 us, 8 rows 174 -> 27, 64 rows 507 -> 73; where the searches run
+// (64 rows of nearly equal logits) 506 -> 371 us, by the sums' shorter reduction and the bracket that the cuts give.
+#define SC_CUTS 7
+#define SC_LIST 512
+__constant__ const float sc_cut[SC_CUTS] = {0.5f, 0.125f, 0.03125f, 0.0078125f, 0.001953125f, 0.00048828125f, 0.00006103515625f};
+
+struct ShortList {
+    unsigned long long key[SC_LIST];  // probability's bits, then the index's complement: greater keys come first
+    float value[SC_LIST];             // in order: probabilities, then their running sums
+    int index[SC_LIST];
+    int taken;  // entries that this CTA has written
+    int result;
+};
+
+// Normalises the slice in place and leaves in `row_s` what holds for the whole row: [j] the sum and [8 + j] the number of the
+// entries above cut j, [SC_CUTS] the sum of all; [24 + j] how many entries above cut j lie in CTAs of lower rank.
+__device__ __forceinline__ void sc_normalise_and_count(float* probs_s, int count, float total, float p_max, float* row_s, float* scratch,
+                                                       SampleExchange* ex, int& turn) {
+    static_assert(SC_CUTS == 7, "eight sums meet in one transposing butterfly, and a slot holds sixteen numbers");
+    float g[8] = {};
+    int n[SC_CUTS] = {};
+    float cut[SC_CUTS];
+#pragma unroll
+    for (int j = 0; j < SC_CUTS; ++j) cut[j] = p_max * sc_cut[j];
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        const float p = probs_s[i] / total;
+        probs_s[i] = p;
+        g[SC_CUTS] += p;
+        if (p > cut[SC_CUTS - 1]) {
+#pragma unroll
+            for (int j = 0; j < SC_CUTS; ++j)
+                if (p > cut[j]) g[j] += p, ++n[j];
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    sc_warp_sums(g, scratch);
+#pragma unroll
+    for (int j = 0; j < SC_CUTS; ++j) {
+        const int all = __reduce_add_sync(0xffffffffu, n[j]);
+        if (lane == 0) scratch[warp * 16 + 8 + j] = (float)all;  // (at most 2^17: exact)
+    }
+    sc_totals(8 + SC_CUTS, scratch, row_s, ex, turn);
+}
+
+// The entries of the row above `cut` (`n` of them, `before` in CTAs of lower rank) to the first CTA's list.
+__device__ __forceinline__ void sc_collect(const float* probs_s, int count, int first, float cut, int before, ShortList* list) {
+    if (threadIdx.x == 0) list->taken = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < count; i += blockDim.x) {
+        const float p = probs_s[i];
+        if (p > cut) {
+            const int at = before + atomicAdd(&list->taken, 1);
+            const unsigned long long key = ((unsigned long long)__float_as_uint(p) << 32) | (unsigned)~(first + i);
+            asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(sc_remote(&list->key[at], 0)), "l"(key) : "memory");
+        }
+    }
+    sc_sync();
+}
+
+// The first CTA: the entry at which the running sum of the ordered list reaches the threshold, which is `draw` times `whole`
+// or, where a nucleus is cut off, times the running sum that reaches `want`.
+__device__ __forceinline__ int sc_walk_list(ShortList* list, int n, bool cut_off, float want, float whole, float draw, int best_index) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < n) {
+        const unsigned long long mine = list->key[tid];
+        int place = 0;  // indices differ, so keys do
+        for (int k = 0; k < n; ++k) place += list->key[k] > mine;
+        list->value[place] = __uint_as_float((unsigned)(mine >> 32));
+        list->index[place] = (int)~(unsigned)mine;
+    }
+    if (tid == 0) list->result = -1;
+    __syncthreads();
+    if (tid < 32) {  // running sums: a lane adds up its run of the list, the lanes' totals meet in a scan
+        const int per = (n + 31) / 32, begin = min(lane * per, n), end = min(begin + per, n);
+        float sum = 0.0f;
+        for (int k = begin; k < end; ++k) list->value[k] = sum += list->value[k];
+        float ahead = sum;
+        for (int off = 1; off < 32; off <<= 1) {
+            const float other = __shfl_up_sync(0xffffffffu, ahead, off);
+            if (lane >= off) ahead += other;
+        }
+        const float offset = __shfl_up_sync(0xffffffffu, ahead, 1);
+        if (lane > 0)
+            for (int k = begin; k < end; ++k) list->value[k] += offset;
+    }
+    __syncthreads();
+    int last = n - 1;  // (rounding: the list reached the target when its sum was formed in another order)
+    if (cut_off) {
+        if (tid < n && list->value[tid] >= want && (tid == 0 || list->value[tid - 1] < want)) atomicMax(&list->result, tid);
+        __syncthreads();
+        if (list->result >= 0) last = list->result;
+        __syncthreads();
+        if (tid == 0) list->result = -1;
+        __syncthreads();
+        whole = list->value[last];
+    }
+    const float threshold = draw * whole;
+    if (!(threshold > 0.0f)) return best_index;
+    if (tid <= last && list->value[tid] >= threshold && (tid == 0 || list->value[tid - 1] < threshold)) atomicMax(&list->result, tid);
+    __syncthreads();
+    return list->index[list->result >= 0 ? list->result : last];
+}
+
+// G(v) = sum of the row's probabilities greater than v, for up to eight values at once.
+template <int COUNT>
+__device__ __forceinline__ void sc_sums_greater(const float* probs_s, int count, const float (&v)[COUNT], float (&out)[COUNT],
+                                                float* scratch, SampleExchange* ex, int& turn) {
+    static_assert(COUNT <= 8, "eight sums meet in one butterfly");
+    float g[8] = {};
     for (int i = threadIdx.x; i < count; i += blockDim.x) {
         const float p = probs_s[i];
 #pragma unroll
         for (int j = 0; j < COUNT; ++j)
             if (p > v[j]) g[j] += p;
     }
-    sc_block_sums<COUNT>(g, scratch);
-    sc_cluster_sum<COUNT>(g, ex, turn, scratch + 32 * COUNT);
+    sc_warp_sums(g, scratch);  // (every thread has left the reduction before: see the barrier at its end, and the reads below)
+    sc_totals(COUNT, scratch, scratch + 512, ex, turn);
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) out[j] = scratch[512 + j];
 }
 __device__ __forceinline__ float sc_sum_greater(const float* probs_s, int count, float value, float* scratch,
                                                 SampleExchange* ex, int& turn) {
@@ -360,12 +498,23 @@ __device__ __forceinline__ float sc_sum_greater(const float* probs_s, int count,
     return g[0];
 }
 
-// Smallest probability value v (a bit pattern in [0, hi_bits]) with G(v) < target; requires G(hi_bits) < target.
+// The cuts between which the boundary for `target` lies, as bit patterns: what the first pass has added up saves the searches
+// their first steps.
+__device__ __forceinline__ void sc_bracket(const float* above, float target, float p_max, unsigned& lo, unsigned& hi) {
+    lo = 0u, hi = __float_as_uint(p_max);
+#pragma unroll
+    for (int j = SC_CUTS - 1; j >= 0; --j)
+        if (above[j] >= target) lo = __float_as_uint(p_max * sc_cut[j]);  // the last that holds is the greatest
+#pragma unroll
+    for (int j = 0; j < SC_CUTS; ++j)
+        if (above[j] < target) hi = __float_as_uint(p_max * sc_cut[j]);  // the last that holds is the smallest
+}
+
+// Smallest probability value v (a bit pattern in [lo, hi]) with G(v) < target; requires G(hi) < target.
 // G does not grow with v, so SC_TRIES values cut the candidates [lo, hi] into SC_TRIES + 1 parts a step: everything
 // up to the last value that fails is out, the first value that passes is the new upper end.
-__device__ float sc_boundary_value(const float* probs_s, int count, float target, unsigned hi_bits, float* scratch,
+__device__ float sc_boundary_value(const float* probs_s, int count, float target, unsigned lo, unsigned hi, float* scratch,
                                    SampleExchange* ex, int& turn) {
-    unsigned lo = 0u, hi = hi_bits;
     while (lo < hi) {
         unsigned m[SC_TRIES];
         float v[SC_TRIES], g[SC_TRIES];
@@ -414,13 +563,15 @@ __device__ int sc_nth_equal(const float* probs_s, int count, int first, float va
     return result;
 }
 
-__global__ void __launch_bounds__(SC_THREADS)
+__global__ void __launch_bounds__(SC_THREADS, 2)
 sample_rows_cluster_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
                            const float* __restrict__ top_p, const float* __restrict__ draw, int* __restrict__ out,
                            int vocab, int per, int* __restrict__ error_flag) {
     pdl_launch_dependents();
     extern __shared__ float probs_s[];  // [per] this CTA's slice: logits first, then probabilities
-    __shared__ float scratch[32 * 8 + 8];  // block sums of up to 8 numbers, then the cluster's totals
+    __shared__ float scratch[32 * 16 + 32 + 8];  // the warps' sums of up to 16 numbers, the cluster's totals, and one total more
+    __shared__ float row_s[32];
+    __shared__ ShortList list;
     __shared__ int s_counts[SC_THREADS];
     __shared__ SampleExchange ex;
     const int r = blockIdx.y;
@@ -478,22 +629,37 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, const float* __rest
         acc += e;
     }
     float sums[1] = {block_sum(acc, scratch)};
-    sc_cluster_sum<1>(sums, &ex, turn, scratch + 32 * 8);
+    sc_cluster_sum<1>(sums, &ex, turn, scratch + 544);
     const float total = sums[0];
-    for (int i = threadIdx.x; i < count; i += blockDim.x) probs_s[i] = probs_s[i] / total;
-    __syncthreads();
     const float p_max = 1.0f / total;  // exp(0) / total: the probability of the greatest logit, nothing is greater
-    const unsigned hi_bits = __float_as_uint(p_max);
+    unsigned lo_bits, top_bits;
 
     const float want = top_p[r];
     float nucleus_total;
     float nucleus_value = 0.0f;
     int nucleus_ties = 0x7fffffff;
-    const float all = sc_sum_greater(probs_s, count, -1.0f, scratch, &ex, turn);
+    sc_normalise_and_count(probs_s, count, total, p_max, row_s, scratch, &ex, turn);
+    const float all = row_s[SC_CUTS];
+    const bool cut_off = !(want >= 1.0f || all < want);
+    const float target = cut_off ? want : draw[r] * all;
+    int above_cut = 0, before_me = 0;
+    float cut = -1.0f;
+#pragma unroll
+    for (int j = SC_CUTS - 1; j >= 0; --j)
+        if (row_s[j] >= target) above_cut = (int)row_s[8 + j], before_me = (int)row_s[24 + j], cut = p_max * sc_cut[j];
+    if (above_cut > 0 && above_cut <= SC_LIST) {
+        sc_collect(probs_s, count, first, cut, before_me, &list);
+        if (rank == 0) {
+            const int chosen = sc_walk_list(&list, above_cut, cut_off, want, all, draw[r], best_index);
+            if (threadIdx.x == 0) out[r] = chosen;
+        }
+        return;  // (the others wrote into the first CTA before the barrier in sc_collect, and nobody reads them any more)
+    }
     if (want >= 1.0f || all < want) {
         nucleus_total = all;
     } else {
-        nucleus_value = sc_boundary_value(probs_s, count, want, hi_bits, scratch, &ex, turn);
+        sc_bracket(row_s, want, p_max, lo_bits, top_bits);
+        nucleus_value = sc_boundary_value(probs_s, count, want, lo_bits, top_bits, scratch, &ex, turn);
         const float above = sc_sum_greater(probs_s, count, nucleus_value, scratch, &ex, turn);
         float running = above;
         int n = 0;
@@ -509,7 +675,8 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, const float* __rest
     if (!(threshold > 0.0f)) {
         chosen = best_index;
     } else {
-        float value = sc_boundary_value(probs_s, count, threshold, hi_bits, scratch, &ex, turn);
+        sc_bracket(row_s, threshold, p_max, lo_bits, top_bits);
+        float value = sc_boundary_value(probs_s, count, threshold, lo_bits, top_bits, scratch, &ex, turn);
         int n;
         if (value < nucleus_value) {
             value = nucleus_value;
@@ -529,7 +696,7 @@ sample_rows_cluster_kernel(const float* __restrict__ logits, const float* __rest
             int mine = 0;
             for (int i = threadIdx.x; i < count; i += blockDim.x) mine += (probs_s[i] == value);
             float ties[1] = {block_sum((float)mine, scratch)};
-            sc_cluster_sum<1>(ties, &ex, turn, scratch + 32 * 8);
+            sc_cluster_sum<1>(ties, &ex, turn, scratch + 544);
             const int total_ties = (int)(ties[0] + 0.5f);
             chosen = total_ties > 0 ? sc_nth_equal(probs_s, count, first, value, total_ties, s_counts, scratch, &ex, turn) : best_index;
         }

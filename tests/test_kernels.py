@@ -917,3 +917,30 @@ def test_products_with_the_chosen_experts_alone(ops, tokens, experts, unit, behi
         got = ops.linear_chosen(hidden, as_given(wide), gates, experts, unit, True, out_dtype=torch.float32)
         assert torch.allclose(got.double(), want, rtol=0, atol=wide.shape[1] * 2.0 ** -20), used
     ops.check_device_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("likely", [1, 2, 33, 511, 512, 513, 3000])
+@pytest.mark.parametrize("vocab", [32000, 151936])
+def test_sampling_where_few_entries_hold_the_nucleus(ops, likely, vocab):
+    """``likely`` entries far above the rest: up to 512 of them are collected and ordered, more are searched for.  Some tie."""
+    generator = torch.Generator().manual_seed(likely)
+    draws = torch.tensor([0.0, 0.2, 0.5, 0.77, 0.999])
+    logits = torch.randn(len(draws), vocab, generator=generator) - 30.0
+    for row in logits:
+        row[torch.randperm(vocab, generator=generator)[:likely]] = torch.randint(0, 8, (likely,), generator=generator) / 8.0 + 1.0
+    for top_p in (0.9, 1.0, 1e-6):
+        for temperature in (0.7, 1.0):
+            column = lambda v: torch.full((len(draws),), v, device=DEV)  # noqa: E731
+            got = ops.sample_rows(logits.to(DEV), column(temperature), column(top_p), draws.to(DEV)).tolist()
+            for row, draw in enumerate(draws.tolist()):
+                probs = torch.softmax(logits[row].double() / temperature, 0)
+                order = torch.argsort(-probs, stable=True)
+                running = torch.cumsum(probs[order], 0)
+                last = vocab - 1 if top_p >= 1.0 else int(torch.searchsorted(running, torch.tensor(top_p, dtype=torch.float64)))
+                place = int((order == got[row]).nonzero())
+                # 32-bit sums of up to 3,000 (and 152,000 tiny) terms, formed in another order: 2^-24 a rounding
+                slack, threshold = 3e-5, draw * float(running[last])
+                before = float(running[place - 1]) if place else 0.0
+                assert before - slack <= threshold <= float(running[place]) + slack, (row, top_p, place)
+                assert before <= float(running[last]) + slack
+    ops.check_device_errors(torch.device(DEV))
