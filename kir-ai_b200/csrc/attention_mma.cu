@@ -21,6 +21,8 @@
 // Key tiles start at absolute multiples of the tile size, so which keys share
 // a tile does not depend on how a prompt was cut.  head_dim: any multiple of 8
 // up to 256 (the tile is padded with zeros to 64, 128 or 256 columns).
+#include <climits>
+
 #include "sm100.cuh"
 #include "tensor_map.cuh"
 
@@ -574,17 +576,18 @@ struct DecodeTile {
 
 // Shared memory of the decode kernel: the query tile, per warp a ring of DC_STAGES (K tile, V tile)
 // filled by TMA, one mbarrier per ring slot; after the key loop the ring is reused to merge the warps.
-template <int D>
+template <int D, int W = DecodeTile<D>::WARPS>
 struct DecodeSmem {
     static constexpr int BN = DecodeTile<D>::BN;
-    static constexpr int DC_WARPS = DecodeTile<D>::WARPS;
+    static constexpr int DC_WARPS = W;
     static constexpr int q_bytes = 16 * D * 2;
     static constexpr int tile_bytes = BN * D * 2;
     static constexpr int ring_bytes = DC_WARPS * DC_STAGES * 2 * tile_bytes;
     static constexpr int merge_bytes = DC_WARPS * 16 * (D + 2) * 4;
     static constexpr int body = q_bytes + (ring_bytes > merge_bytes ? ring_bytes : merge_bytes);
     static constexpr int table_entries = 1024;  // block-table entries kept in shared memory (longer ranges read global memory)
-    static constexpr int prefix_entries = 1025;  // balanced kernel: where each request's tiles start (up to 1,024 requests)
+    static constexpr bool all_forms = W == DecodeTile<D>::WARPS;  // CTAs of fewer warps are for the split kernel without merging
+    static constexpr int prefix_entries = all_forms ? 1025 : 1;  // balanced kernel: where each request's tiles start (up to 1,024 requests)
     static constexpr int rope_offset = body + DC_WARPS * DC_STAGES * 8 + table_entries * 4 + prefix_entries * 4 + 12;  // 16-byte aligned
     // fused q/k preparation: cos [D / 2], sin [D / 2] of the request's position, then the q and the k norm's weights [D] each
     static constexpr int rope_bytes = 3 * D * 4;
@@ -593,7 +596,7 @@ struct DecodeSmem {
     // shared memory; outside the ring, which the first CTA may still be streaming through (heads up to 128 only:
     // wider heads leave no room)
     static constexpr int pair_offset = rope_offset + rope_bytes;
-    static constexpr int pair_bytes = D <= 128 ? 16 * (D + 2) * 4 : 0;
+    static constexpr int pair_bytes = all_forms && D <= 128 ? 16 * (D + 2) * 4 : 0;
     static constexpr int total = pair_offset + pair_bytes + 1024;  // + slack to align to 1024
 };
 
@@ -618,7 +621,12 @@ struct DecodeArgs {
     float eps;
     bf16* cache;
     unsigned long long* stamps;  // null, or [CTAs][8] clock stamps (ns) of the decode kernel, for measurements
+    // A launch of several waves hands out the requests with the longest contexts first (a block takes the request of its
+    // place in that order), so that the last wave is made of the shortest: 64 requests of 131 to 1,500 tokens, 8 kv heads, in CTAs
+    // of 4 warps 53 -> 41 us a layer.
+    int longest_first;
 };
+#define DECODE_MAX_SORTED 512  // requests of such a launch: every block orders them
 
 // Clock stamps of one CTA of the decode kernel (split form), written only when a buffer is given: 0 the CTA starts,
 // 1 the kernel before has finished, 2 the queries are in shared memory, 3 the warps have attended their tiles,
@@ -742,12 +750,12 @@ __device__ __forceinline__ void append_new_token(const DecodeArgs& args, const f
 // CTA's first work: the tiles that earlier steps filled are requested before griddepcontrol.wait, the rest after.
 // t_begin and t_end count the tiles that the query walks (`runs`: a window that keeps the sequence's first `keep` keys
 // walks those keys' tiles and then the window's; without kept keys walked tile v is key tile runs.first + v).
-template <int D, bool HEADS>
+template <int D, bool HEADS, int W = DecodeTile<D>::WARPS>
 __device__ __forceinline__ int decode_attend_range(const CUtensorMap& kv_map, const DecodeArgs& args, uint8_t* smem, int req,
                                                    int kv_head, int pos, int key_lo, int last_tile, int t_begin, int t_end,
                                                    int k_base, bool first, bf16* __restrict__ out,
                                                    float* __restrict__ dst_partial, long partial_stride, TileRuns runs, int keep) {
-    using Smem = DecodeSmem<D>;
+    using Smem = DecodeSmem<D, W>;
     constexpr int BN = Smem::BN;
     constexpr int DC_WARPS = Smem::DC_WARPS;
     constexpr int PANELS = D / 64;
@@ -1005,9 +1013,9 @@ __device__ __forceinline__ int decode_attend_range(const CUtensorMap& kv_map, co
 }
 
 // One barrier per ring slot and warp; called by every thread before the first range.
-template <int D>
+template <int D, int W = DecodeTile<D>::WARPS>
 __device__ __forceinline__ void decode_init_barriers(uint8_t* smem) {
-    using Smem = DecodeSmem<D>;
+    using Smem = DecodeSmem<D, W>;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint64_t* bars = (uint64_t*)(smem + Smem::body) + warp * DC_STAGES;
     if (lane == 0) {
@@ -1015,6 +1023,28 @@ __device__ __forceinline__ void decode_init_barriers(uint8_t* smem) {
         sm100::mbar_fence_init();
     }
     __syncthreads();
+}
+
+// The request with the n-th longest context (the lower index first among equal ones), found by the whole block; `lens`:
+// `requests` ints (rounded up to four) of shared memory on a 16-byte boundary that nobody uses yet.
+__device__ __forceinline__ int nth_longest(const int* __restrict__ context_len, int requests, int n, int* lens) {
+    __shared__ int found;
+    const int padded = (requests + 3) & ~3;
+    for (int r = threadIdx.x; r < padded; r += blockDim.x) lens[r] = r < requests ? context_len[r] : INT_MIN;
+    __syncthreads();
+    for (int r = threadIdx.x; r < requests; r += blockDim.x) {
+        const int mine = lens[r];
+        int before = 0;
+#pragma unroll 4
+        for (int k = 0; k < padded; k += 4) {
+            const int4 other = *reinterpret_cast<const int4*>(lens + k);
+            before += (other.x > mine || (other.x == mine && k < r)) + (other.y > mine || (other.y == mine && k + 1 < r)) +
+                      (other.z > mine || (other.z == mine && k + 2 < r)) + (other.w > mine || (other.w == mine && k + 3 < r));
+        }
+        if (before == n) found = r;
+    }
+    __syncthreads();
+    return found;
 }
 
 // partial: [requests, q_heads, splits, head_dim + 2] floats: unnormalised output, then max (log2 domain), then sum.
@@ -1034,17 +1064,19 @@ __device__ __forceinline__ void decode_init_barriers(uint8_t* smem) {
 // arithmetic of attention_merge_splits_kernel, and stores the result: no buffer in global memory and no second kernel,
 // whose way through a kernel boundary cost 4.5 us a layer at 8 requests.  The slots (group rows each) share
 // DecodeSmem::pair_bytes, which the launch checks.
-template <int D, bool HEADS, bool PAIR>
-__global__ void __launch_bounds__(DecodeTile<D>::WARPS * 32)
+template <int D, bool HEADS, bool PAIR, int W = DecodeTile<D>::WARPS>
+__global__ void __launch_bounds__(W * 32)
 attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, DecodeArgs args, bf16* __restrict__ out,
                         float* __restrict__ partial, const int* __restrict__ context_len, int num_splits) {
     pdl_launch_dependents();
     decode_stamp(args, 0);
-    using Smem = DecodeSmem<D>;
+    using Smem = DecodeSmem<D, W>;
     constexpr int BN = Smem::BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int split = blockIdx.x, kv_head = blockIdx.y, req = blockIdx.z;
+    const int split = blockIdx.x, kv_head = blockIdx.y;
+    const int req = !PAIR && args.longest_first ? nth_longest(context_len, gridDim.z, blockIdx.z, reinterpret_cast<int*>(smem + Smem::q_bytes))
+                                                : (int)blockIdx.z;
     const int group = args.q_heads / args.kv_heads;
     const int pos = context_len[req] - 1;
     const int keep = mask_keep(args.window);
@@ -1056,7 +1088,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, DecodeArgs a
     const int t_begin = split * per_split;
     const int t_end = min(tiles, t_begin + per_split);
     if (threadIdx.x == 0) sm100::tma_prefetch_descriptor(&kv_map);
-    decode_init_barriers<D>(smem);
+    decode_init_barriers<D, W>(smem);
     if (PAIR) {
         const int stride = args.head_dim + 2;
         float* own = reinterpret_cast<float*>(smem + Smem::q_bytes + Smem::merge_bytes);  // this CTA's rows, behind its warps' merge buffer
@@ -1094,7 +1126,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, DecodeArgs a
     }
     float* dst_partial = num_splits == 1 ? nullptr
         : partial + (((size_t)req * args.q_heads + kv_head * group) * num_splits + split) * (args.head_dim + 2);
-    decode_attend_range<D, HEADS>(kv_map, args, smem, req, kv_head, pos, key_lo, last_tile, t_begin, t_end, 0, true, out,
+    decode_attend_range<D, HEADS, W>(kv_map, args, smem, req, kv_head, pos, key_lo, last_tile, t_begin, t_end, 0, true, out,
                                   dst_partial, (long)num_splits * (args.head_dim + 2), runs, keep);
     decode_stamp(args, 4);
 }
@@ -1197,51 +1229,64 @@ attention_decode_balanced_kernel(const __grid_constant__ CUtensorMap kv_map, Dec
     if (first) pdl_wait();  // a CTA without work still orders itself after the kernel before it
 }
 
-// One block per (request, query head): adds up the pieces of a pair that more than one CTA of the balanced kernel
-// attended, in CTA order; a pair finished inside one CTA is left as that CTA wrote it.
-__global__ void __launch_bounds__(128)
+// A warp per (request, query head): adds up the pieces of a pair that more than one CTA of the balanced kernel
+// attended, in CTA order; a pair finished inside one CTA is left as that CTA wrote it.  (A block per (request, query
+// head), each with a scan of its own over the requests, took 4.3 us at 64 requests of 32 heads.)
+#define MERGE_WARPS 8
+__global__ void __launch_bounds__(MERGE_WARPS * 32)
 attention_merge_balanced_kernel(const float* __restrict__ partial, bf16* __restrict__ out,
                                 const int* __restrict__ context_len, int requests, int q_heads, int kv_heads,
                                 int head_dim, int window, int tile_keys, int ctas, const float* __restrict__ sinks) {
     pdl_launch_dependents();
     __shared__ int prefix[DECODE_MAX_REQUESTS + 1];
-    __shared__ float warp_max[4];
-    const int req = blockIdx.x / q_heads, head = blockIdx.x % q_heads;
-    const int group = q_heads / kv_heads, kv_head = head / group, row = head % group;
     decode_tile_prefix(context_len, requests, window, tile_keys, prefix);
+    const int lane = threadIdx.x & 31;
+    const long at = (long)blockIdx.x * MERGE_WARPS + (threadIdx.x >> 5);
+    pdl_wait();
+    if (at >= (long)requests * q_heads) return;
+    const int req = (int)(at / q_heads), head = (int)(at - (long)req * q_heads);
+    const int group = q_heads / kv_heads, kv_head = head / group, row = head % group;
     const int my_tiles = prefix[req + 1] - prefix[req];
     const long total = (long)kv_heads * prefix[requests];
     const long start = (long)kv_heads * prefix[req] + (long)kv_head * my_tiles;
-    pdl_wait();
-    bf16* dst = out + ((size_t)req * q_heads + head) * head_dim;
+    bf16* dst = out + at * head_dim;
     if (my_tiles == 0) {
-        for (int col = threadIdx.x; col < head_dim; col += blockDim.x) dst[col] = from_f32<bf16>(0.0f);
+        for (int col = lane; col < head_dim; col += 32) dst[col] = from_f32<bf16>(0.0f);
         return;
     }
     const long per_cta = (total + ctas - 1) / ctas;
     const int c_first = (int)(start / per_cta), c_last = (int)((start + my_tiles - 1) / per_cta);
     if (c_first == c_last) return;  // finished by its CTA
-    const int stride = head_dim + 2;
+    const int stride = head_dim + 2;  // (even, as head_dim is: a lane takes two columns at a time)
     // piece of CTA c: slot 0 unless the pair starts inside that CTA's range (only c_first can)
     const int first_slot = start == (long)c_first * per_cta ? 0 : 1;
     auto piece = [&](int c) { return partial + (((size_t)c * 2 + (c == c_first ? first_slot : 0)) * 16 + row) * stride; };
     float m_all = -INFINITY;
-    for (int c = c_first + (int)threadIdx.x; c <= c_last; c += blockDim.x) m_all = fmaxf(m_all, piece(c)[head_dim]);
+    for (int c = c_first + lane; c <= c_last; c += 32) m_all = fmaxf(m_all, piece(c)[head_dim]);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m_all = fmaxf(m_all, __shfl_xor_sync(0xffffffffu, m_all, d));
-    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m_all;
-    __syncthreads();
-    m_all = fmaxf(fmaxf(warp_max[0], warp_max[1]), fmaxf(warp_max[2], warp_max[3]));
-    for (int col = threadIdx.x; col < head_dim; col += blockDim.x) {
-        float acc = 0.0f, l_all = 0.0f;
+    for (int col0 = 0; col0 < head_dim; col0 += 128) {
+        float2 acc[2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+        float l_all = 0.0f;
+        const int a = col0 + 2 * lane, b = a + 64;
 #pragma unroll 4
         for (int c = c_first; c <= c_last; ++c) {
             const float* src = piece(c);
-            const float weight = src[head_dim] == -INFINITY ? 0.0f : exp2f(src[head_dim] - m_all);
-            acc += src[col] * weight;
-            l_all += src[head_dim + 1] * weight;
+            const float2 tail = *reinterpret_cast<const float2*>(src + head_dim);  // maximum, sum
+            const float2 x = a < head_dim ? *reinterpret_cast<const float2*>(src + a) : make_float2(0.0f, 0.0f);
+            const float2 y = b < head_dim ? *reinterpret_cast<const float2*>(src + b) : make_float2(0.0f, 0.0f);
+            const float weight = tail.x == -INFINITY ? 0.0f : exp2f(tail.x - m_all);
+            acc[0].x += x.x * weight, acc[0].y += x.y * weight, acc[1].x += y.x * weight, acc[1].y += y.y * weight;
+            l_all += tail.y * weight;
         }
-        dst[col] = from_f32<bf16>(softmax_value(acc, m_all, l_all, sinks, head));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int col = h ? b : a;
+            if (col < head_dim) {
+                dst[col] = from_f32<bf16>(softmax_value(acc[h].x, m_all, l_all, sinks, head));
+                dst[col + 1] = from_f32<bf16>(softmax_value(acc[h].y, m_all, l_all, sinks, head));
+            }
+        }
     }
 }
 
@@ -1323,7 +1368,7 @@ int decode_launch(const void* q, const void* cache, void* out, float* partial, c
                   const int* context_len, int requests, int q_heads, int kv_heads, int head_dim, long q_row_stride,
                   int page_size, int table_width, int num_pages, int window, float scale, int num_splits,
                   int* error_flag, cudaStream_t stream, const FuseQK* fuse = nullptr, float softcap = 0.0f,
-                  const float* sinks = nullptr) {
+                  const float* sinks = nullptr, int crowd_warps = 0) {
     using Smem = DecodeSmem<D>;
     const int box_rows = page_size < Smem::BN ? page_size : Smem::BN;
     if (Smem::BN % box_rows != 0 || page_size % box_rows != 0) return KIRAI_ERR_UNSUPPORTED;  // page sizes: powers of two
@@ -1348,6 +1393,25 @@ int decode_launch(const void* q, const void* cache, void* out, float* partial, c
     args.stamps = g_decode_stamps;
     if (g_decode_stamps) g_decode_stamps += 8 * 1024;  // the next launch's stamps follow
     dim3 grid(num_splits, kv_heads, requests);
+    if (crowd_warps > 0) {
+        if (pair || fuse || !heads || requests > DECODE_MAX_SORTED) return KIRAI_ERR_UNSUPPORTED;
+        args.longest_first = 1;
+    }
+    if (crowd_warps == 4) {
+        if constexpr (D <= 128) {
+            using Small = DecodeSmem<D, 4>;
+            static_assert(2 * (Small::total + 1024) <= 228 * 1024, "two of these CTAs to an SM");
+            auto half = attention_decode_kernel<D, true, false, 4>;
+            err = cudaFuncSetAttribute(half, cudaFuncAttributeMaxDynamicSharedMemorySize, Small::total);
+            if (err != cudaSuccess) return (int)err;
+            const int status = launch_pdl(half, grid, dim3(Small::DC_WARPS * 32), (size_t)Small::total, stream, 1u, kv_map, args,
+                                          (bf16*)out, partial, context_len, num_splits);
+            if (status || num_splits == 1) return status;
+            return launch_pdl(attention_merge_splits_kernel, dim3(requests * q_heads), dim3(128), 0, stream, 1u, (const float*)partial,
+                              (bf16*)out, head_dim, num_splits, q_heads, sinks);
+        }
+        return KIRAI_ERR_UNSUPPORTED;
+    }
     if (pair)
         return launch_pdl_clusters(kernel, grid, dim3(Smem::DC_WARPS * 32), (size_t)Smem::total, stream, dim3(num_splits, 1, 1),
                                    kv_map, args, (bf16*)out, partial, context_len, num_splits);
@@ -1383,7 +1447,8 @@ int decode_balanced_launch(const void* q, const void* cache, void* out, float* p
     int status = launch_pdl(kernel, dim3(ctas), dim3(Smem::DC_WARPS * 32), (size_t)Smem::total, stream, 1u, kv_map, args,
                             (bf16*)out, partial, context_len, requests);
     if (status) return status;
-    return launch_pdl(attention_merge_balanced_kernel, dim3(requests * q_heads), dim3(128), 0, stream, 1u,
+    return launch_pdl(attention_merge_balanced_kernel, dim3((unsigned)(((long)requests * q_heads + MERGE_WARPS - 1) / MERGE_WARPS)),
+                      dim3(MERGE_WARPS * 32), 0, stream, 1u,
                       (const float*)partial, (bf16*)out, context_len, requests, q_heads, kv_heads, head_dim, window,
                       (int)Smem::BN, ctas, sinks);
 }
@@ -1509,6 +1574,27 @@ KIRAI_EXPORT int kirai_attention_decode_bf16(const void* q, const void* cache, v
     return attention_decode_entry(q, cache, out, partial, block_table, context_len, requests, q_heads, kv_heads, head_dim,
                                   q_row_stride, page_size, table_width, num_pages, window, scale, 0.0f, num_splits, error_flag,
                                   stream);
+}
+
+// For more (request, kv head) pairs than SMs, so that CTAs run one behind another: requests with the longest contexts come
+// first, and a CTA has 8 warps (one CTA to an SM) or 4 (two to an SM: one streams while the other sets up or merges).  Groups of
+// up to eight heads of up to 128 columns, up to 512 requests.  softcap 0, sinks null: none.  partial: as above (splits > 1).
+KIRAI_EXPORT int kirai_attention_decode_crowd_bf16(const void* q, const void* cache, void* out, float* partial, const int* block_table,
+                                                   const int* context_len, int requests, int q_heads, int kv_heads, int head_dim,
+                                                   long q_row_stride, int page_size, int table_width, int num_pages, int window,
+                                                   float scale, float softcap, const float* sinks, int num_splits, int warps,
+                                                   int* error_flag, cudaStream_t stream) {
+    if (requests <= 0) return 0;
+    const int bad = check_common(q_heads, kv_heads, head_dim, q_row_stride, q);
+    if (bad) return bad;
+    if (q_heads / kv_heads > 8 || head_dim > 128 || requests > DECODE_MAX_SORTED) return KIRAI_ERR_UNSUPPORTED;
+    if (num_splits < 1 || num_splits > 65535 || (num_splits > 1 && !partial) || (warps != 4 && warps != 8)) return KIRAI_ERR_BAD_SIZE;
+    return head_dim <= 64 ? decode_launch<64>(q, cache, out, partial, block_table, context_len, requests, q_heads, kv_heads, head_dim,
+                                              q_row_stride, page_size, table_width, num_pages, window, scale, num_splits, error_flag, stream,
+                                              nullptr, softcap, sinks, warps)
+                          : decode_launch<128>(q, cache, out, partial, block_table, context_len, requests, q_heads, kv_heads, head_dim,
+                                               q_row_stride, page_size, table_width, num_pages, window, scale, num_splits, error_flag, stream,
+                                               nullptr, softcap, sinks, warps);
 }
 
 // The same with a soft cap on the scores (0: none) and `window` < 0 for a chunked mask.

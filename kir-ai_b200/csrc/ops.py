@@ -1669,6 +1669,66 @@ def attention_decode_balanced(q: torch.Tensor, cache: torch.Tensor, block_table:
     return out
 
 
+def attention_decode_crowd(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, context_len: torch.Tensor,
+                           window: Optional[int], scale: float, num_splits: int = 1, warps: int = 8, out: Optional[torch.Tensor] = None,
+                           chunk: Optional[int] = None, softcap: Optional[float] = None, keep_first: int = 0,
+                           sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``attention_decode`` for more (request, kv head) pairs than SMs: requests with the longest contexts first, CTAs of 8 warps
+    (one to an SM) or of 4 (two to an SM); see ``decode_crowd_plan``."""
+    _need_cuda(q, cache, block_table, context_len)
+    num_pages, kv_heads, page_size, head_dim = _cache_dims(cache)
+    rows, q_heads, qd, q_stride = _head_view(q)
+    assert qd == head_dim and q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16
+    assert context_len.numel() == rows and context_len.dtype == torch.int32
+    assert sinks is None or (sinks.is_cuda and sinks.dtype == torch.float32 and sinks.numel() == q_heads and sinks.is_contiguous())
+    if out is None:
+        out = torch.empty((rows, q_heads * head_dim), dtype=q.dtype, device=q.device)
+    assert out.shape == (rows, q_heads * head_dim) and out.dtype == q.dtype and out.is_contiguous()
+    partial = None
+    if num_splits > 1:
+        partial = torch.empty((rows, q_heads, num_splits, head_dim + 2), dtype=torch.float32, device=q.device)
+    _call("kirai_attention_decode_crowd_bf16", _ptr(q), _ptr(cache), _ptr(out), _ptr(partial), _ptr(block_table), _ptr(context_len),
+          _i(rows), _i(q_heads), _i(kv_heads), _i(head_dim), _l(q_stride), _i(page_size), _i(block_table.shape[1]), _i(num_pages),
+          _i(mask_code(window, chunk, keep_first)), _f(scale), _f(softcap or 0.0), _ptr(sinks), _i(num_splits), _i(warps),
+          _ptr(error_flag(q.device)), _stream(), detail=_attention_detail(q_heads, kv_heads, head_dim, window, chunk, keep_first))
+    return out
+
+
+DECODE_MAX_SORTED = 512  # requests whose order every CTA of ``attention_decode_crowd`` works out
+
+
+def decode_crowd_plan(context_lens, kv_heads: int, reach: Optional[int] = None, sms: int = DEFAULT_SMS, head_dim: int = 128,
+                      group: int = 4) -> Optional[tuple]:
+    """How a batch of more (request, kv head) pairs than SMs is attended: (warps of a CTA, ranges of a request's keys), or
+    None where another kernel should (few pairs, wide heads, a few contexts so long that only equal ranges for all SMs help).
+
+    A CTA of w warps that has t key tiles takes about ceil(t / w) rounds plus a set-up and a merge, 1.27 us a round and 4.4 us
+    with 8 warps and an SM to itself, 1.07 and 7.1 with 4 warps and half an SM; more than one range costs 4 us for
+    the second kernel.  CTAs come longest first, so the launch ends close to the greatest of these lower bounds: the longest
+    CTA; the sum over the slots; for every k the k + 1 shortest of the k * slots + 1 longest (some slot has k + 1 of them);
+    and the bytes.  Against measurements of 29 batches of 18 to 64 requests (8 kv heads of 128, contexts of 20 to 20,000
+    tokens) the times come out within a tenth.  In us, 1,000 tokens each: 32 requests 37 with 8 warps and 31 with 4 (floor 20),
+    48 of 1,300 tokens 64 and 66 (39); 20 of 500 to 3,000 tokens 41 and 61, two ranges 51 and 44 (25).  The
+    balanced kernel: 42, 63, 47, and 97 at 64 requests of 131 to 1,500 tokens, where 4 warps take 47."""
+    requests = len(context_lens)
+    if requests * kv_heads <= sms or requests > DECODE_MAX_SORTED or head_dim > 128 or group > 8 or kv_heads > sms:
+        return None
+    tiles = sorted((-(-(min(int(n), reach) if reach else int(n)) // 16) for n in context_lens), reverse=True)
+    bytes_us = kv_heads * sum(tiles) * head_dim * 64 / 5.9e6
+    best, best_us = None, 1.35 * (-(-(-(-kv_heads * sum(tiles) // sms)) // 8) + 9.5) + 6.0 * requests * kv_heads / sms  # the balanced kernel
+    for warps, splits in ((8, 1), (4, 1), (4, 2), (4, 3)):
+        slots = (sms if warps == 8 else 2 * sms) // kv_heads  # a request's heads are alike: in units of requests
+        per_round, fixed = (1.27, 4.4) if warps == 8 else (1.07, 7.1)
+        costs = [-(-t // (splits * warps)) * per_round + fixed for t in tiles]  # of each of a request's ranges, longest first
+        us = max(costs[0], splits * sum(costs) / slots, bytes_us)
+        for k in range(1, (splits * requests - 1) // slots + 1):
+            us = max(us, sum(costs[i // splits] for i in range(k * slots - k, k * slots + 1)))
+        us += 0.0 if splits == 1 else 4.0
+        if us < best_us:
+            best, best_us = (warps, splits), us
+    return best
+
+
 def paged_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, batch, window: Optional[int],
                     scale: float, chunk: Optional[int] = None, softcap: Optional[float] = None, keep_first: int = 0,
                     sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -1724,15 +1784,20 @@ def _decode_rows(q, cache, block_table, batch, rows: int, window: Optional[int],
     # the batch may say which kernel (a captured step does: its lengths change between replays); otherwise
     # the host's copy of the lengths decides; KIRAI_DECODE_BALANCED=0 or 1 overrides both
     balanced = getattr(batch, "decode_balanced", None)
+    crowd = getattr(batch, "decode_crowd", None)
     longest = batch.max_context_len
     if balanced is None:
         lens = [start + count for start, count in zip(batch.start_positions[:rows], batch.query_lens[:rows])]
-        balanced, _ = decode_plan(lens, kv_heads, reach, sms=sm_count(q.device), room=room, head_dim=q.shape[2],
-                                  group=q.shape[1] // kv_heads)
+        crowd = decode_crowd_plan(lens, kv_heads, reach, sms=sm_count(q.device), head_dim=q.shape[2], group=q.shape[1] // kv_heads)
+        balanced = False if crowd else decode_plan(lens, kv_heads, reach, sms=sm_count(q.device), room=room, head_dim=q.shape[2],
+                                                   group=q.shape[1] // kv_heads)[0]
         longest = max(lens)
     forced = os.environ.get("KIRAI_DECODE_BALANCED")
     if forced in ("0", "1"):
-        balanced = forced == "1"
+        balanced, crowd = forced == "1", None
+    if crowd and q.shape[2] <= 128 and q.shape[1] // kv_heads <= 8:  # (a captured step's layers may differ in their heads)
+        attention_decode_crowd(q, cache, block_table, context_len, window, scale, crowd[1], crowd[0], out=out, **mask)
+        return
     if balanced and rows <= 1024:
         attention_decode_balanced(q, cache, block_table, context_len, window, scale, out=out, **mask)
         return

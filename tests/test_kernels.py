@@ -944,3 +944,29 @@ def test_sampling_where_few_entries_hold_the_nucleus(ops, likely, vocab):
                 assert before - slack <= threshold <= float(running[place]) + slack, (row, top_p, place)
                 assert before <= float(running[last]) + slack
     ops.check_device_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim,page_size,form",
+                         [(32, 8, 128, 16, {}), (4, 4, 64, 8, {"window": 20}), (8, 1, 96, 64, {"softcap": 5.0}), (6, 2, 48, 1, {"sinks": True}),
+                          (4, 2, 128, 16, {"chunk": 48}), (7, 1, 128, 32, {"window": 37, "keep_first": 5})])
+def test_decode_attention_of_crowds(ops, q_heads, kv_heads, head_dim, page_size, form):
+    """The decode attention for many requests (the longest first) against the plain kernel, with both sizes of CTAs, whole and in
+    ranges (more ranges than a request has tiles, too); requests of one token, of whole tiles, of a tile and one, and of equal length."""
+    lengths = [1, 150, 16, 17, 300, 5, 64, 33, 64, 150, 1]
+    cache, table, keys, values = paged_setup(torch.bfloat16, lengths, kv_heads, head_dim, page_size, seed=5)
+    for r, n in enumerate(lengths):
+        ops.kv_write(keys[r].to(DEV).contiguous(), values[r].to(DEV).contiguous(), cache, table,
+                     torch.full((n,), r, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV))
+    q = rand(len(lengths), q_heads, head_dim, dtype=torch.bfloat16, scale=2.0)
+    scale, context = head_dim ** -0.5, torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    sinks = rand(q_heads) if form.get("sinks") else None
+    options = dict(chunk=form.get("chunk"), softcap=form.get("softcap"), keep_first=form.get("keep_first", 0), sinks=sinks)
+    window = form.get("window")
+    plain = ops.paged_attention_plain(q.float(), cache.float(), table, torch.arange(len(lengths), dtype=torch.int32, device=DEV), context - 1,
+                                      window, scale, **options)
+    for warps in (4, 8):
+        for splits in (1, 2, 3, 21):
+            got = ops.attention_decode_crowd(q, cache, table, context, window, scale, splits, warps, **options)
+            # weights and result are rounded to bfloat16 (2^-9 each) on values of up to about 4
+            assert float((got.float() - plain).abs().max()) <= 2.5e-2, (warps, splits)
+    ops.check_device_errors(torch.device(DEV))

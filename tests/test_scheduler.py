@@ -183,6 +183,22 @@ def test_decode_plan_prefers_the_balanced_kernel_only_for_uneven_or_badly_filled
     assert decode_plan([], 8) == (False, 1)
 
 
+def test_decode_crowd_plan_follows_the_measured_batches():
+    """More (request, kv head) pairs than SMs: CTAs of 8 warps where a long request would set the time of smaller ones or one wave
+    holds the batch, of 4 warps for many alike, ranges for a few very long ones; nothing else is taken."""
+    from kirai_b200.csrc.ops import decode_crowd_plan
+
+    assert decode_crowd_plan([1000] * 18, 8) is None                        # 144 CTAs fit the SMs
+    assert decode_crowd_plan([1000] * 64, 8, head_dim=256) is None and decode_crowd_plan([1000] * 64, 8, group=16) is None
+    assert decode_crowd_plan([1000] * 513, 8) is None and decode_crowd_plan([], 8) is None
+    assert decode_crowd_plan([1000] * 32, 8) == (4, 1) and decode_crowd_plan([1000] * 64, 8) == (4, 1)
+    uneven = [3000 - 2500 * i // 19 for i in range(20)]
+    assert decode_crowd_plan(uneven, 8) == (8, 1)
+    assert decode_crowd_plan(uneven, 8, reach=256) == (4, 1)                # a window makes them equal
+    assert decode_crowd_plan([6000 - 5950 * i // 23 for i in range(24)], 8) == (4, 3)
+    assert decode_crowd_plan([200_000] + [100] * 30, 8) is None             # equal ranges for all SMs
+
+
 def test_decode_plan_over_random_batches_respects_the_kernels_limits():
     """Whatever the batch, the planner names a split count that the decode kernel takes (1 to 64 ranges, never more
     ranges than key tiles), and ranges are merged inside the kernel only where the device said the clusters fit and
