@@ -164,6 +164,22 @@ __device__ __forceinline__ float softmax_inverse(float m, float sum, const float
     return keep / (sum * keep + exp2f(s - top));
 }
 
+// ---- two 32-bit multiply-adds an instruction, each rounded as a single one is
+typedef unsigned long long f32x2;
+
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ void unpair(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+
 static inline int launch_status() { return (int)cudaGetLastError(); }
 
 // ---- programmatic dependent launch -----------------------------------------

@@ -889,18 +889,23 @@ def _state_chunked(batch, state_rows: int, walk_limit: Optional[int]) -> bool:
     return bool(fn(ctypes.c_int(state_rows)))
 
 
-def _state_side(batch, tokens: int, heads: int, rows: int, cols: int, normaliser: bool, device, chain_limit: Optional[int]):
-    """(units, state, normaliser, marks): the buffers of a step whose chunks run side by side, or (0, None, None, None)."""
+def _state_side(batch, tokens: int, heads: int, groups: int, rows: int, cols: int, normaliser: bool, device, chain_limit: Optional[int]):
+    """(units, state, normaliser, marks, scores): the buffers of a step whose chunks run side by side, or (0, None, None, None,
+    None); ``scores`` (queries times keys of a chunk, ``groups`` sets of them) only for sizes that can be read in 16 bytes."""
     fn = library().kirai_state_chunk_tokens
     fn.restype = ctypes.c_int
-    units = tokens // int(fn()) + batch.num_requests
+    chunk = int(fn())
+    units = tokens // chunk + batch.num_requests
     limit = STATE_CHAIN_LIMIT if chain_limit is None else chain_limit
     if batch.max_query_len <= limit or units * heads * rows * cols * 4 > STATE_SIDE_BYTES:
-        return 0, None, None, None
+        return 0, None, None, None, None
     state = torch.empty((units, heads, rows, cols), dtype=torch.float32, device=device)
     norm = torch.empty((units, heads, rows), dtype=torch.float32, device=device) if normaliser else None
     marks = torch.empty((units, heads, 3), dtype=torch.float32, device=device)
-    return units, state, norm, marks
+    scores = None
+    if rows % 4 == 0 and cols % 4 == 0:
+        scores = torch.empty((units, groups, chunk, chunk), dtype=torch.float32, device=device)
+    return units, state, norm, marks, scores
 
 
 def ssm_walk(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, skip: torch.Tensor,
@@ -920,10 +925,11 @@ def ssm_walk(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     assert state.dtype == torch.float32 and state.dim() == 2 and state.is_contiguous()
     y = torch.empty((xbc.shape[0], inner), dtype=torch.float32, device=xbc.device)
     if _state_chunked(batch, state_size, walk_limit):
-        units, side, _, marks = _state_side(batch, xbc.shape[0], heads, state_size, head_dim, False, xbc.device, chain_limit)
+        units, side, _, marks, scores = _state_side(batch, xbc.shape[0], heads, groups, state_size, head_dim, False, xbc.device, chain_limit)
         _call("kirai_ssm_chunks", _ptr(xbc), _ptr(dt), _l(dt.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state),
               _l(state.shape[1]), _l(ssm_offset), _ptr(batch.query_start), _ptr(batch.slots), _ptr(y), _i(batch.num_requests),
-              _i(heads), _i(groups), _i(state_size), _i(head_dim), _i(state.shape[0]), _i(units), _ptr(side), _ptr(marks), _stream())
+              _i(heads), _i(groups), _i(state_size), _i(head_dim), _i(state.shape[0]), _i(units), _ptr(side), _ptr(marks), _ptr(scores),
+              _stream())
         return y
     _call("kirai_ssm_walk", _ptr(xbc), _ptr(dt), _l(dt.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state),
           _l(state.shape[1]), _l(ssm_offset), _ptr(batch.query_start), _ptr(batch.slots), _ptr(y), _i(batch.num_requests),
@@ -949,12 +955,12 @@ def matrix_memory_walk(rows: torch.Tensor, in_bias: Optional[torch.Tensor], keep
     assert state.dtype == torch.float32 and state.dim() == 2 and state.is_contiguous()
     o = torch.empty((rows.shape[0], heads * value_dim), dtype=torch.float32, device=rows.device)
     if _state_chunked(batch, key_dim, walk_limit):
-        units, side, norm, marks = _state_side(batch, rows.shape[0], heads, key_dim, value_dim, True, rows.device, chain_limit)
+        units, side, norm, marks, scores = _state_side(batch, rows.shape[0], heads, heads, key_dim, value_dim, True, rows.device, chain_limit)
         tail = None if units else torch.empty((batch.num_requests, heads, key_dim + 1), dtype=torch.float32, device=rows.device)
         _call("kirai_matrix_memory_chunks", _ptr(rows), _l(rows.stride(0)), _ptr(in_bias), _ptr(keep_bias), _f(cap), _f(q_scale),
               _ptr(state), _l(state.shape[1]), _ptr(batch.query_start), _ptr(batch.slots), _ptr(o), _ptr(tail),
               _i(batch.num_requests), _i(heads), _i(key_dim), _i(value_dim), _i(state.shape[0]), _i(units), _ptr(side), _ptr(norm),
-              _ptr(marks), _stream())
+              _ptr(marks), _ptr(scores), _stream())
         return o
     _call("kirai_matrix_memory_walk", _ptr(rows), _l(rows.stride(0)), _ptr(in_bias), _ptr(keep_bias), _f(cap), _f(q_scale),
           _ptr(state), _l(state.shape[1]), _ptr(batch.query_start), _ptr(batch.slots), _ptr(o), _i(batch.num_requests), _i(heads),
@@ -993,7 +999,7 @@ def channel_scan(rows: torch.Tensor, up: torch.Tensor, bias: torch.Tensor, tau: 
     units = tokens // chunk + batch.num_requests
     tiles = torch.empty((units, heads, 2 * key_dim + chunk, chunk), dtype=torch.float32, device=rows.device)
     kept = torch.empty((units, heads, key_dim), dtype=torch.float32, device=rows.device)
-    side = _state_side(batch, tokens, heads, key_dim, value_dim, False, rows.device, chain_limit)[1]
+    side = _state_side(batch, tokens, heads, 0, key_dim, value_dim, False, rows.device, chain_limit)[1]
     _call("kirai_channel_chunks", *common, _ptr(o), _ptr(tiles), _ptr(kept), _ptr(side), *sizes, _i(units), _stream())
     gate = rows[:, 2 * width + heads * value_dim : 2 * width + 2 * heads * value_dim]
     return gated_group_norm(o, gate, norm, eps, heads, False, out_dtype, silu_after=True)

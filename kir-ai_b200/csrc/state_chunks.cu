@@ -344,6 +344,7 @@ struct ChunkSide {
     float* U;      // [chunks of the step, heads, d, dv]: a chunk's own share, then the state at its start
     float* u;      // [chunks, heads, d]: likewise for the normaliser (matrix memory)
     float* marks;  // [chunks, heads, 3]: X'_last, G_last, then the maximum at the chunk's start
+    float* scores;  // [chunks, groups, CHUNK, CHUNK]: q_t . k_s, or null
 };
 
 template <int J>
@@ -455,6 +456,259 @@ __global__ void __launch_bounds__(THREADS) chunk_out_kernel(const ChunkScan a, c
         a.state[slot * a.state_len + a.m_off + head] = w.scal[2];
 }
 
+// ---- the same for rows that can be read 16 bytes at a time ------------------------------------------------------------
+// The kernels above take q . k anew in every block of a chunk's heads and columns, copy q and k four bytes at a time into
+// tiles turned by bank-conflicting stores, and feed 16 FMAs from five shared-memory reads.  Where d, dv, the strides and the
+// addresses allow 16-byte copies these take their place: q . k is made once per (chunk, group) by blocks of
+// the first launch that have no other work; tiles keep the rows as they lie; a block has 64 value columns; a thread multiplies 4 x 4
+// (read-out) or 8 x 4 (state) values from 16-byte reads with two FMAs an instruction.  Bound by the FMA pipe and the traffic of the states (d dv
+// floats per chunk and head, written, carried and read).  Three requests, 2,030 tokens, one launch each, us before and now: 128 heads of a
+// state of 128 x 64 with one group, own shares 433 and 142, read-outs 691 and 228; 16 heads of 128 x 256, 233 and 91, 363 and 130.
+constexpr int COLS = 64;           // value columns a block
+constexpr int SPITCH = CHUNK + 4;  // floats a row of the scores' tile
+
+__device__ __forceinline__ void copy_async_16(float* to, const float* from, bool present) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from), "r"(present ? 16 : 0)
+                 : "memory");
+}
+// `rows` rows of `width` floats (a multiple of 4) from `from` into a tile of row pitch `pitch`; rows from `len` on are zero.
+__device__ __forceinline__ void fetch_rows(float* tile, int pitch, const float* from, long stride, int rows, int len, int width) {
+    const int quads = width >> 2;
+    for (int i = threadIdx.x; i < rows * quads; i += THREADS) {
+        const int t = i / quads, c = i - t * quads;
+        copy_async_16(tile + t * pitch + 4 * c, from + (t < len ? t * stride + 4 * c : 0), t < len);
+    }
+}
+
+__host__ __device__ inline long local_rows_floats(int d) { return (long)CHUNK * (d + 4) + CHUNK * COLS + 5 * CHUNK + 8; }
+__host__ __device__ inline long scores_floats(int d) { return 2L * CHUNK * (d + 4); }
+__host__ __device__ inline long out_rows_floats(int d) {
+    return (long)CHUNK * (d + 4) + CHUNK * SPITCH + CHUNK * COLS + (long)d * COLS + d + 6 * CHUNK + 8;
+}
+
+// q_t . k_s of a chunk's tokens, t >= s, [t][s]; a thread has t = 4 ty + i, s = tx + 16 j.
+__device__ __forceinline__ void chunk_raw_scores(const ChunkScan& a, const ChunkSide& side, const ChunkPlace& at, int group, float* smem) {
+    const int d = a.d, pitch = d + 4, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    float* Q = smem;
+    float* K = smem + CHUNK * pitch;
+    fetch_rows(Q, pitch, a.q + (long)group * d + at.row0 * a.q_stride, a.q_stride, CHUNK, at.len, d);
+    fetch_rows(K, pitch, a.k + (long)group * d + at.row0 * a.k_stride, a.k_stride, CHUNK, at.len, d);
+    copies_wait();
+    __syncthreads();
+    f32x2 acc[4][4] = {};
+    for (int kd = 0; kd < d; kd += 4) {
+        ulonglong2 qv[4], kv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(Q + (4 * ty + i) * pitch + kd);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const ulonglong2*>(K + (tx + 16 * j) * pitch + kd);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fma2(acc[i][j], qv[i].x, kv[j].x), fma2(acc[i][j], qv[i].y, kv[j].y);
+    }
+    float* to = side.scores + ((long)blockIdx.x * a.groups + group) * CHUNK * CHUNK;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float even, odd;
+            unpair(acc[i][j], even, odd);
+            to[(4 * ty + i) * CHUNK + tx + 16 * j] = even + odd;
+        }
+}
+
+// As chunk_local_kernel; blocks with blockIdx.z == pieces make the scores.
+__global__ void __launch_bounds__(THREADS, 3) chunk_local_rows_kernel(const ChunkScan a, const ChunkSide side, int requests, int pieces) {
+    extern __shared__ __align__(16) float smem[];
+    pdl_launch_dependents();
+    const int head = blockIdx.y, d = a.d, tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int group = head / (a.heads / a.groups);
+    ChunkPlace at;
+    const bool found = find_chunk(a.query_start, requests, blockIdx.x, at);
+    pdl_wait();
+    if (!found) return;
+    if ((int)blockIdx.z == pieces) {
+        if (head % (a.heads / a.groups) == 0) chunk_raw_scores(a, side, at, group, smem);
+        return;
+    }
+    const int col0 = blockIdx.z * COLS, cols = min(COLS, a.dv - col0), pitch = d + 4;
+    float* K = smem;
+    float* V = K + CHUNK * pitch;
+    float* B = V + CHUNK * COLS;
+    float *X = B + CHUNK, *C = X + CHUNK, *Last = C + CHUNK, *Floor = Last + CHUNK, *scal = Floor + CHUNK;
+    fetch_rows(K, pitch, a.k + (long)group * d + at.row0 * a.k_stride, a.k_stride, CHUNK, at.len, d);
+    fetch_rows(V, COLS, a.v + (long)head * a.dv + col0 + at.row0 * a.v_stride, a.v_stride, CHUNK, at.len, cols);
+    if (tid < 32) chunk_gates(a, head, at.row0, at.len, a.memory ? -INFINITY : 0.0f, B, X, C, Last, Floor, scal);
+    copies_wait();
+    __syncthreads();
+    const long unit = (long)blockIdx.x * a.heads + head;
+    if (blockIdx.z == 0) {
+        if (a.memory)
+            for (int kd = tid; kd < d; kd += THREADS) {
+                float acc = 0.0f;
+                for (int s = 0; s < at.len; ++s) acc = fmaf(Last[s], K[s * pitch + kd], acc);
+                side.u[unit * d + kd] = acc;
+            }
+        if (tid == 0) side.marks[unit * 3] = scal[3], side.marks[unit * 3 + 1] = scal[4];
+    }
+    for (int i = tid; i < at.len * (COLS / 4); i += THREADS) {
+        float4* v = reinterpret_cast<float4*>(V) + i;
+        const float weight = Last[i / (COLS / 4)];
+        *v = make_float4(v->x * weight, v->y * weight, v->z * weight, v->w * weight);
+    }
+    __syncthreads();
+    float* U = side.U + unit * d * a.dv + col0 + 4 * tx;
+    for (int r0 = 0; r0 < d; r0 += 128) {
+        const int first = r0 + 4 * ty, second = r0 + 64 + 4 * ty;  // this thread's rows, four each
+        const float* k0 = K + (first < d ? first : 0);
+        const float* k1 = K + (second < d ? second : 0);
+        f32x2 acc[8][2] = {};
+#pragma unroll 4
+        for (int s = 0; s < at.len; ++s) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(V + s * COLS + 4 * tx);
+            const float4 x = *reinterpret_cast<const float4*>(k0 + s * pitch), y = *reinterpret_cast<const float4*>(k1 + s * pitch);
+            const float ks[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const f32x2 kk = pair(ks[i], ks[i]);
+                fma2(acc[i][0], kk, v.x), fma2(acc[i][1], kk, v.y);
+            }
+        }
+        if (4 * tx >= cols) continue;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int kd = (i < 4 ? first : second) + (i & 3);
+            if (kd >= d) continue;
+            float4 out;
+            unpair(acc[i][0], out.x, out.y), unpair(acc[i][1], out.z, out.w);
+            *reinterpret_cast<float4*>(U + (long)kd * a.dv) = out;
+        }
+    }
+}
+
+// As chunk_out_kernel, from the scores that the launch above left.
+__global__ void __launch_bounds__(THREADS, 2) chunk_out_rows_kernel(const ChunkScan a, const ChunkSide side, int requests) {
+    extern __shared__ __align__(16) float smem[];
+    pdl_launch_dependents();
+    const int head = blockIdx.y, col0 = blockIdx.z * COLS, cols = min(COLS, a.dv - col0);
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, d = a.d, pitch = d + 4;
+    float* Q = smem;
+    float* P = Q + CHUNK * pitch;     // [t][s]
+    float* V = P + CHUNK * SPITCH;    // [s][COLS]
+    float* S = V + CHUNK * COLS;      // [d][COLS]: the state at the chunk's start
+    float* N = S + (long)d * COLS;
+    float* B = N + d;
+    float *X = B + CHUNK, *C = X + CHUNK, *Last = C + CHUNK, *Floor = Last + CHUNK, *under = Floor + CHUNK, *scal = under + CHUNK;
+    ChunkPlace at;
+    const bool found = find_chunk(a.query_start, requests, blockIdx.x, at);
+    const int slot = found ? a.slots[at.request] : -1;
+    pdl_wait();
+    if (!found || slot < 0 || slot >= a.num_slots) return;
+    const int group = head / (a.heads / a.groups);
+    const long unit = (long)blockIdx.x * a.heads + head;
+    fetch_rows(Q, pitch, a.q + (long)group * d + at.row0 * a.q_stride, a.q_stride, CHUNK, at.len, d);
+    fetch_rows(P, SPITCH, side.scores + ((long)blockIdx.x * a.groups + group) * CHUNK * CHUNK, CHUNK, CHUNK, CHUNK, CHUNK);
+    fetch_rows(V, COLS, a.v + (long)head * a.dv + col0 + at.row0 * a.v_stride, a.v_stride, CHUNK, at.len, cols);
+    fetch_rows(S, COLS, side.U + unit * d * a.dv + col0, a.dv, d, d, cols);
+    if (a.memory) fetch_rows(N, d, side.u + unit * d, d, 1, 1, d);
+    const float m0 = a.memory ? side.marks[unit * 3 + 2] : 0.0f;
+    if (tid < 32) chunk_gates(a, head, at.row0, at.len, m0, B, X, C, Last, Floor, scal);
+    copies_wait();
+    __syncthreads();
+    for (int i = tid; i < CHUNK * CHUNK; i += THREADS) {
+        const int t = i / CHUNK, s = i % CHUNK;
+        float* p = P + t * SPITCH + s;
+        *p = s <= t && t < at.len ? *p * a.q_scale * expf(B[s] - X[t]) * C[s] : 0.0f;
+    }
+    __syncthreads();
+    if (a.memory) {  // what a token's read-out is divided by; four threads to a token
+        const int t = tid >> 2, part = tid & 3;
+        float carried = 0.0f, fresh = 0.0f;
+        for (int kd = 4 * part; kd < d; kd += 16) {
+            const float4 q = *reinterpret_cast<const float4*>(Q + t * pitch + kd), n = *reinterpret_cast<const float4*>(N + kd);
+            carried = fmaf(q.x, n.x, fmaf(q.y, n.y, fmaf(q.z, n.z, fmaf(q.w, n.w, carried))));
+        }
+        for (int s = part; s <= t; s += 4) fresh += P[t * SPITCH + s];
+        float den = fmaf(carried, expf(m0 - X[t]) * a.q_scale, fresh);
+        den += __shfl_xor_sync(0xffffffffu, den, 1);
+        den += __shfl_xor_sync(0xffffffffu, den, 2);
+        if (part == 0) under[t] = 1.0f / (fmaxf(fabsf(den), Floor[t]) + 1e-6f);
+    }
+    // tokens 4 ty + i at columns 4 tx .. + 3: q from the state, then the scores from the values
+    f32x2 o[4][2] = {};
+#pragma unroll 2
+    for (int kd = 0; kd < d; kd += 4) {
+        float4 q[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4*>(Q + (4 * ty + i) * pitch + kd);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(S + (kd + e) * COLS + 4 * tx);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float w = e == 0 ? q[i].x : e == 1 ? q[i].y : e == 2 ? q[i].z : q[i].w;
+                const f32x2 ww = pair(w, w);
+                fma2(o[i][0], ww, v.x), fma2(o[i][1], ww, v.y);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float carried = expf(m0 - X[4 * ty + i]) * a.q_scale;
+        const f32x2 cc = pair(carried, carried);
+        o[i][0] = mul2(o[i][0], cc), o[i][1] = mul2(o[i][1], cc);
+    }
+    for (int s = 0; s < 4 * ty + 4; s += 4) {
+        float4 p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(P + (4 * ty + i) * SPITCH + s);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(V + (s + e) * COLS + 4 * tx);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float w = e == 0 ? p[i].x : e == 1 ? p[i].y : e == 2 ? p[i].z : p[i].w;
+                const f32x2 ww = pair(w, w);
+                fma2(o[i][0], ww, v.x), fma2(o[i][1], ww, v.y);
+            }
+        }
+    }
+    if (a.memory) __syncthreads();
+    if (4 * tx < cols) {
+        const float skip = a.memory ? 0.0f : a.skip[head];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int t = 4 * ty + i;
+            if (t >= at.len) continue;
+            float4 out;
+            unpair(o[i][0], out.x, out.y), unpair(o[i][1], out.z, out.w);
+            if (a.memory) {
+                const float factor = under[t];
+                out.x *= factor, out.y *= factor, out.z *= factor, out.w *= factor;
+            } else {
+                const float4 v = *reinterpret_cast<const float4*>(V + t * COLS + 4 * tx);
+                out.x = fmaf(skip, v.x, out.x), out.y = fmaf(skip, v.y, out.y), out.z = fmaf(skip, v.z, out.z), out.w = fmaf(skip, v.w, out.w);
+            }
+            *reinterpret_cast<float4*>(a.out + (at.row0 + t) * ((long)a.heads * a.dv) + (long)head * a.dv + col0 + 4 * tx) = out;
+        }
+    }
+    if (a.memory && tid == 0 && blockIdx.z == 0 && at.chunk == at.chunks - 1)
+        a.state[slot * a.state_len + a.m_off + head] = scal[2];
+}
+
+// Whether these rows can be read 16 bytes at a time and the tiles fit (the scores' buffer says that the caller made one).
+bool rows_in_quads(const ChunkScan& a, const ChunkSide& side) {
+    const uintptr_t bases = (uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.out | (uintptr_t)side.U | (uintptr_t)side.u | (uintptr_t)side.scores;
+    if (!side.scores || bases % 16 != 0 || a.d % 4 != 0 || a.dv % 4 != 0 || (a.q_stride | a.k_stride | a.v_stride) % 4 != 0) return false;
+    int device = 0, limit = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+        return false;
+    const long most = out_rows_floats(a.d) > scores_floats(a.d) ? out_rows_floats(a.d) : scores_floats(a.d);
+    return most * 4 <= limit;
+}
+
 // A thread per (request, head, entry): the new normaliser and maximum go to the request's slot.
 __global__ void chunk_tail_kernel(const float* __restrict__ tail, float* __restrict__ state, long state_len, long n_off, long m_off,
                                   const int* __restrict__ query_start, const int* __restrict__ slots, int requests, int heads, int d,
@@ -499,6 +753,24 @@ int chunk_scan_launch(ChunkScan a, int requests, int units, ChunkSide side, cuda
     const int runs = cols_pitch(a.cols) / 16;
     const int pieces = (a.dv + a.cols - 1) / a.cols;
     static long granted[3][5] = {};  // (one device a process)
+    if (units > 0 && rows_in_quads(a, side)) {
+        const int wide = (a.dv + COLS - 1) / COLS;
+        const long local_bytes = 4 * (local_rows_floats(a.d) > scores_floats(a.d) ? local_rows_floats(a.d) : scores_floats(a.d));
+        const long out_bytes = 4 * out_rows_floats(a.d);
+        static long granted_rows[2] = {};
+        int status = grant_shared(chunk_local_rows_kernel, local_bytes, &granted_rows[0]);
+        if (status == 0) status = grant_shared(chunk_out_rows_kernel, out_bytes, &granted_rows[1]);
+        if (status == 0)
+            status = launch_pdl(chunk_local_rows_kernel, dim3(units, a.heads, wide + 1), dim3(THREADS), (size_t)local_bytes, stream, 1u, a, side,
+                                requests, wide);
+        const long entries = (long)a.d * a.dv + (a.memory ? a.d : 0);
+        if (status == 0)
+            status = launch_pdl(chunk_carry_kernel, dim3(requests, a.heads, (unsigned)((entries + 255) / 256)), dim3(256), 0, stream, 1u,
+                                a, side, requests);
+        if (status == 0)
+            status = launch_pdl(chunk_out_rows_kernel, dim3(units, a.heads, wide), dim3(THREADS), (size_t)out_bytes, stream, 1u, a, side, requests);
+        return status;
+    }
     if (units > 0) {
         auto local = KIRAI_BY_RUNS(runs, chunk_local_kernel);
         auto out = KIRAI_BY_RUNS(runs, chunk_out_kernel);
@@ -542,7 +814,7 @@ KIRAI_EXPORT int kirai_state_chunk_tokens() { return CHUNK; }
 KIRAI_EXPORT int kirai_ssm_chunks(const float* xbc, const float* dt_raw, long dt_stride, const float* dt_bias, const float* a_log,
                                   const float* d_skip, float* state, long state_len, long ssm_off, const int* query_start,
                                   const int* slots, float* y, int requests, int heads, int groups, int N, int P, int num_slots,
-                                  int units, float* side_state, float* side_marks, cudaStream_t stream) {
+                                  int units, float* side_state, float* side_marks, float* side_scores, cudaStream_t stream) {
     if (requests <= 0) return 0;
     if (heads <= 0 || groups <= 0 || heads % groups || N <= 0 || P <= 0 || ssm_off < 0 || ssm_off + (long)heads * N * P > state_len)
         return KIRAI_ERR_BAD_SIZE;
@@ -556,17 +828,17 @@ KIRAI_EXPORT int kirai_ssm_chunks(const float* xbc, const float* dt_raw, long dt
     a.query_start = query_start, a.slots = slots, a.out = y;
     a.heads = heads, a.groups = groups, a.d = N, a.dv = P, a.num_slots = num_slots, a.memory = 0;
     if (units > 0 && (!side_state || !side_marks)) return KIRAI_ERR_BAD_SIZE;
-    return chunk_scan_launch(a, requests, units, ChunkSide{side_state, nullptr, side_marks}, stream);
+    return chunk_scan_launch(a, requests, units, ChunkSide{side_state, nullptr, side_marks, side_scores}, stream);
 }
 
 // The matrix memory in chunks; the arguments of kirai_matrix_memory_walk and `tail` [requests, heads, d + 1] (float32), or
 // for the chunks side by side (units > 0) side_state [units, heads, d, dv], side_norm [units, heads, d], side_marks
-// [units, heads, 3].
+// [units, heads, 3] and side_scores [units, heads, 64, 64] or null.
 KIRAI_EXPORT int kirai_matrix_memory_chunks(const float* rows, long row_stride, const float* in_bias, const float* keep_bias,
                                             float cap, float q_scale, float* state, long state_len, const int* query_start,
                                             const int* slots, float* o, float* tail, int requests, int heads, int d, int dv,
                                             int num_slots, int units, float* side_state, float* side_norm, float* side_marks,
-                                            cudaStream_t stream) {
+                                            float* side_scores, cudaStream_t stream) {
     if (requests <= 0) return 0;
     if (heads <= 0 || d <= 0 || dv <= 0 || !(cap > 0.0f) || (!tail && units <= 0) || (long)heads * d * dv + (long)heads * d + heads > state_len)
         return KIRAI_ERR_BAD_SIZE;
@@ -582,5 +854,5 @@ KIRAI_EXPORT int kirai_matrix_memory_chunks(const float* rows, long row_stride, 
     a.query_start = query_start, a.slots = slots, a.out = o;
     a.heads = heads, a.groups = heads, a.d = d, a.dv = dv, a.num_slots = num_slots, a.memory = 1;
     if (units > 0 && (!side_state || !side_norm || !side_marks)) return KIRAI_ERR_BAD_SIZE;
-    return chunk_scan_launch(a, requests, units, ChunkSide{side_state, side_norm, side_marks}, stream);
+    return chunk_scan_launch(a, requests, units, ChunkSide{side_state, side_norm, side_marks, side_scores}, stream);
 }

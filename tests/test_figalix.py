@@ -988,3 +988,42 @@ def test_command_line_generates(tiny):
     assert result.returncode == 0, result.stderr
     expected = _plain_greedy(tiny["config"], tiny["weights"], prompt, 6)
     assert json.loads(result.stdout.strip().splitlines()[-1])["token_ids"] == expected
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,groups,d,dv", [(6, 2, 128, 64), (2, 1, 256, 72), (1, 1, 4, 4), (3, 3, 132, 132)])
+@pytest.mark.parametrize("memory", [False, True])
+def test_chunks_side_by_side_from_aligned_rows_equal_those_from_any_rows(heads, groups, d, dv, memory):
+    """The kernels that read rows 16 bytes at a time against the ones for any address (the same rows one float further on):
+    portions of one token up to several chunks, states that are not zero, sizes around a tile of 64 columns and 128 rows."""
+    from part_helpers import Session
+    from kirai_b200.parts.base import StateNeed
+    from kirai_b200.csrc import ops
+
+    gen = torch.Generator().manual_seed(d + dv)
+    lens = [9, 64, 65, 300, 1, 127]
+    L = heads * d * dv + heads * d + heads
+    session = Session([StateNeed((L,), torch.float32)], torch.float32, page_size=4, num_pages=4, num_slots=8)
+    batch = session.batch([(f"r{i}", n) for i, n in enumerate(lens)])
+    T = sum(lens)
+    width = heads * (2 * d + dv + 2) if memory else heads * dv + 2 * groups * d
+    values = torch.randn((T, width), generator=gen).cuda()
+    state = torch.randn((8, L), generator=gen).cuda()
+    gate = [torch.randn(heads, generator=gen).cuda() for _ in range(3)]
+    dt = torch.randn((T, heads), generator=gen).cuda()
+    outs = []
+    for shift in (0, 1):
+        st = state.clone()
+        if memory:
+            wide = -(-width // 4) * 4 + 4
+            rows = torch.zeros(T * wide + 8, device="cuda")[shift : shift + T * wide].view(T, wide)
+            rows[:, :width] = values
+            out = ops.matrix_memory_walk(rows, gate[0], gate[1] + 3.0, 15.0, d ** -0.5, st, batch, heads, d, dv, 0, 0)
+        else:
+            rows = torch.zeros(T * width + 8, device="cuda")[shift : shift + T * width].view(T, width)
+            rows.copy_(values)
+            out = ops.ssm_walk(rows, dt, gate[0] - 3.0, gate[1], gate[2], st, 0, batch, heads, groups, d, dv, 0, 0)
+        outs.append((out, st))
+    for fast, general in zip(*outs):
+        # 32-bit sums of up to 300 terms in another order: a few 2^-24 of the terms' size, which is that of the greatest results
+        assert torch.isfinite(general).all() and float((fast - general).abs().max()) <= 3e-5 * float(general.abs().max())
