@@ -1027,3 +1027,41 @@ def test_chunks_side_by_side_from_aligned_rows_equal_those_from_any_rows(heads, 
     for fast, general in zip(*outs):
         # 32-bit sums of up to 300 terms in another order: a few 2^-24 of the terms' size, which is that of the greatest results
         assert torch.isfinite(general).all() and float((fast - general).abs().max()) <= 3e-5 * float(general.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [4, 96, 1024, 1028, 4096, 4100, 16384, 16388])
+@pytest.mark.parametrize("rows", [1, 3, 70])
+def test_sums_under_a_tanh_and_pairs_of_normed_rows_from_aligned_rows(rows, width):
+    """The kernels with 16-byte accesses against 64-bit arithmetic and against the ones for any address (the same rows one
+    float further on), with and without terms to add, rows picked out, both result types."""
+    from kirai_b200.csrc import ops
+
+    gen = torch.Generator().manual_seed(width + rows)
+    resid, d1, d2 = (torch.randn((rows, width), generator=gen) for _ in range(3))
+    w, b = torch.randn(width, generator=gen), torch.randn(width, generator=gen)
+    alpha = torch.tensor([0.7])
+    picked = torch.randint(0, rows, (5,), generator=gen, dtype=torch.int32)
+
+    def placed(t, shift):
+        out = torch.zeros(t.numel() + 8, dtype=t.dtype, device="cuda")[shift : shift + t.numel()].view(t.shape)
+        return out.copy_(t)
+
+    for shift in (0, 1):
+        for first, second in ((d1, d2), (d1, None), (None, None)):
+            for index in (None, picked):
+                for dtype in (torch.float32, torch.bfloat16):
+                    stream = placed(resid, shift)
+                    got = ops.add_dyt(stream, [placed(d, shift) if d is not None else None for d in (first, second)], 0.5,
+                                      alpha.cuda(), placed(w, shift), placed(b, shift), dtype, index.cuda() if index is not None else None)
+                    total = resid.double() + 0.5 * ((first.double() if first is not None else 0.0) + (second.double() if second is not None else 0.0))
+                    chosen = total if index is None else total[index.long()]
+                    want = torch.tanh(0.7 * chosen) * w.double() + b.double()
+                    # a few roundings of values of up to about 8 in 32 bits; one more of the result in bfloat16
+                    bound = 8.0 * 2.0 ** -20 if dtype == torch.float32 else 8.0 * 2.0 ** -8
+                    assert float((got.double().cpu() - want).abs().max()) <= bound
+                    left = total if index is None else resid.double()
+                    assert float((stream.double().cpu() - left).abs().max()) <= 8.0 * 2.0 ** -22
+        got = ops.rms_pair_mean(placed(d1, shift), placed(d2, shift), placed(w, shift), placed(b, shift), 1e-6).double().cpu()
+        unit = lambda x: x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-6)  # noqa: E731
+        assert float((got - 0.5 * (unit(d1) * w.double() + unit(d2) * b.double())).abs().max()) <= 16.0 * 2.0 ** -19
