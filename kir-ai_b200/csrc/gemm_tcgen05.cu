@@ -1126,8 +1126,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
 // reads 48 for the same products.  The kernel above is bound by its load thread, at 0.40 us a block of K whatever the tile's
 // width (the MMAs of 256 columns need 0.28 at full clocks); here the weights and the rows of A have a load thread each, a block
 // takes 0.32 us at 256 columns and less for narrower tiles, which fill the last round of a launch better (see pair_width).  Bound by
-// the tensor cores and the power cap.  2,048 tokens, us before and now: 8B q/k/v 90 and 81, o 63 and 60, gate/up 317 and 272, down 176
-// and 154; 4B o 47 and 34, down 115 and 77; 32B o 185 and 125, down 528 and 346.
+// the tensor cores and the power cap.  2,048 tokens, us before and now: 8B q/k/v 90 and 77, o 63 and 57, gate/up 317 and 272, down 176
+// and 141; 4B o 47 and 34, down 115 and 77; 32B o 185 and 125, down 528 and 346.
 //
 // Each CTA's load threads fill its own ring and count on its own barriers.  In the second CTA a thread of the otherwise idle
 // MMA warp passes "this stage is full" on to the first CTA (peer_full), whose MMA thread waits for both; its commits free
@@ -1156,7 +1156,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
     const int half = tile_n >> 1;  // weight rows of a stage
-    const int stage_bytes = X_BYTES + half * GEMM_BK * 2;  // (tile_n is a multiple of 32)
+    const int stage_bytes = X_BYTES + half * GEMM_BK * 2;
     const int stages = min(PAIR_MAX_RING, PAIR_RING_BYTES / stage_bytes);
     const int m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), total_tiles = m_tiles * ((N + tile_n - 1) / tile_n);
     const int num_kb = (K + GEMM_BK - 1) / GEMM_BK;
@@ -1320,19 +1320,18 @@ static int sm_count() {
     }();
     return count;
 }
-// The width of the pairs' tiles: the one whose rounds of tiles are shortest together.  An MMA of a pair (256 rows) takes whole
-// multiples of 32 columns, nothing between.  A round takes as long as its tiles are wide, down to about 168 columns (a block of K then
-// takes 0.26 us, what loading and announcing it takes); narrower than 256 only for a thirty-second less at least.  Measured at
-// 2,048 tokens, us at 256 columns and at the chosen width: N 2560, K 9728 98 and 77 (160: 128 tiles in two rounds, 80 at 256
-// take two as well); N 5120, K 25600 468 and 346 (192: three rounds either way); N 24576, K 4096 290 and 272 (224); and where
-// 256 stays: N 4096, K 12288 154 and 158 (160), N 19456, K 2560 137 and 142 (224).
+// The width of the pairs' tiles: the one whose rounds of tiles are shortest together.  A round takes as long as its tiles are
+// wide, down to about 168 columns (a block of K then takes 0.26 us, what loading and announcing it takes).  Measured at 2,048
+// tokens, us at 256 columns and at the chosen width: N 2560, K 9728 98 and 77 (160: 128 tiles in two rounds, 80 at 256
+// take two as well); N 5120, K 25600 468 and 346 (192: three rounds either way); N 6144, K 4096 81 and 77 (240); N 24576,
+// K 4096 290 and 272 (224).
 static int pair_width(int M, int N, int pairs) {
     const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
     int best = PAIR_BN;
     long best_cost = 0;
-    for (int width = PAIR_BN; width >= 160; width -= 32) {
+    for (int width = PAIR_BN; width >= 160; width -= 16) {
         const long tiles = m_tiles * ((N + width - 1) / width), cost = (tiles + pairs - 1) / pairs * (width < 168 ? 168 : width);
-        if (width == PAIR_BN || cost * 32 < best_cost * 31) best = width, best_cost = cost;
+        if (width == PAIR_BN || cost < best_cost) best = width, best_cost = cost;
     }
     return best;
 }

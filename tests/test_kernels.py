@@ -972,8 +972,7 @@ def test_decode_attention_of_crowds(ops, q_heads, kv_heads, head_dim, page_size,
     ops.check_device_errors(torch.device(DEV))
 
 
-@pytest.mark.parametrize("m,n,k", [(257, 136, 64), (300, 4096, 72), (515, 1000, 520), (700, 5128, 1024), (1605, 2560, 136), (2100, 6144, 64), (4000, 336, 128),
-                                   (131, 19456, 64), (900, 2560, 256), (2048, 5120, 128), (2048, 24576, 64)])
+@pytest.mark.parametrize("m,n,k", [(257, 136, 64), (300, 4096, 72), (515, 1000, 520), (700, 5128, 1024), (1605, 2560, 136), (2100, 6144, 64), (4000, 336, 128)])
 def test_products_of_many_tokens_by_pairs_of_ctas(ops, m, n, k):
     """The product kernel of many tokens against 64-bit sums: a second CTA without rows or without weights, tiles of every width
     that begin and end inside a box, K that ends inside a block; both weight layouts, both result types, both activations and
