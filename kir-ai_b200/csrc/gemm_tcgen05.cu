@@ -824,55 +824,6 @@ __device__ __forceinline__ void epilogue_residual_norm_coalesced(const Epilogue&
     }
 }
 
-// Sixteen adjacent columns of one row of the product, from column `column` (a multiple of 16) on, through the epilogue to `row`
-// (EPI 0, 1 and 3).
-template <typename OutT, int EPI>
-__device__ __forceinline__ void store_columns(const Epilogue& ep, OutT* __restrict__ row, float (&v)[16], int column, int N) {
-    if (EPI == 3) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = v[j] > 0.0f ? v[j] * v[j] : 0.0f;
-    }
-    if (EPI == 1) {
-        // 8 gate columns, then their 8 up columns: 8 outputs at column / 2
-        OutT* dst = row + (column >> 1);
-        if (column + 16 <= N && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
-            uint32_t packed[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                __nv_bfloat162 pair = __floats2bfloat162_rn(gate_mul(ep, v[2 * j], v[2 * j + 8]), gate_mul(ep, v[2 * j + 1], v[2 * j + 9]));
-                packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-            }
-            *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (column + j + 8 < N) dst[j] = from_f32<OutT>(gate_mul(ep, v[j], v[j + 8]));
-        }
-        return;
-    }
-    OutT* dst = row + column;
-    const bool full = (column + 16 <= N) && (((uintptr_t)dst & 15) == 0);
-    if (full && sizeof(OutT) == 2) {
-        uint32_t packed[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-            packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-        }
-        uint4* out = reinterpret_cast<uint4*>(dst);
-        out[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        out[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-    } else if (full && sizeof(OutT) == 4) {
-        float4* out = reinterpret_cast<float4*>(dst);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) out[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (column + j < N) dst[j] = from_f32<OutT>(v[j]);
-    }
-}
-
 template <int BN, typename OutT, int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
@@ -1070,6 +1021,10 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) * my_scale;
+                if (EPI == 3) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = v[j] > 0.0f ? v[j] * v[j] : 0.0f;
+                }
                 if (EPI == 2) {
                     float* res = ep.residual + (size_t)x_row * N + y0 + c0;
                     OutT* dst = C + (size_t)x_row * ldc + y0 + c0;
@@ -1100,8 +1055,44 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
                             }
                         }
                     }
+                } else if (EPI == 1) {
+                    // columns y0 + c0 .. + 15 are 8 gate rows then their 8 up rows: 8 outputs at (y0 + c0) / 2
+                    OutT* dst = C + (size_t)x_row * ldc + ((y0 + c0) >> 1);
+                    if (y0 + c0 + 16 <= N && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
+                        uint32_t packed[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            __nv_bfloat162 pair = __floats2bfloat162_rn(gate_mul(ep, v[2 * j], v[2 * j + 8]), gate_mul(ep, v[2 * j + 1], v[2 * j + 9]));
+                            packed[j] = *reinterpret_cast<uint32_t*>(&pair);
+                        }
+                        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (y0 + c0 + j + 8 < N) dst[j] = from_f32<OutT>(gate_mul(ep, v[j], v[j + 8]));
+                    }
                 } else {
-                    store_columns<OutT, EPI>(ep, C + (size_t)x_row * ldc, v, y0 + c0, N);
+                    OutT* dst = C + (size_t)x_row * ldc + y0 + c0;
+                    const bool full = (y0 + c0 + 16 <= N) && (((uintptr_t)dst & 15) == 0);
+                    if (full && sizeof(OutT) == 2) {
+                        uint32_t packed[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                            packed[j] = *reinterpret_cast<uint32_t*>(&pair);
+                        }
+                        uint4* out = reinterpret_cast<uint4*>(dst);
+                        out[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                        out[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                    } else if (full && sizeof(OutT) == 4) {
+                        float4* out = reinterpret_cast<float4*>(dst);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) out[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (y0 + c0 + j < N) dst[j] = from_f32<OutT>(v[j]);
+                    }
                 }
             }
             if (EPI == 2 && x_row < M) ep.sumsq_out[(size_t)n_tile * M + x_row] = row_sq;  // this column tile's share
@@ -1120,197 +1111,6 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
     }
 }
 
-// The same product by pairs of CTAs (a cluster of two on neighbouring SMs, cta_group::2): a pair makes a tile of 256 rows of A and
-// tile_n weight rows with one MMA stream.  Each CTA holds its own 128 rows of A and half of the weight rows in shared memory
-// and the result of its rows in its tensor memory, so that a block of K costs an SM 32 KB from L2 (tile_n 256) where the kernel above
-// reads 48 for the same products.  The kernel above is bound by its load thread, at 0.40 us a block of K whatever the tile's
-// width (the MMAs of 256 columns need 0.28 at full clocks); here the weights and the rows of A have a load thread each, a block
-// takes 0.32 us at 256 columns and less for narrower tiles, which fill the last round of a launch better (see pair_width).  Bound by
-// the tensor cores and the power cap.  2,048 tokens, us before and now: 8B q/k/v 90 and 77, o 63 and 57, gate/up 317 and 272, down 176
-// and 141; 4B o 47 and 34, down 115 and 77; 32B o 185 and 125, down 528 and 346.
-//
-// Each CTA's load threads fill its own ring and count on its own barriers.  In the second CTA a thread of the otherwise idle
-// MMA warp passes "this stage is full" on to the first CTA (peer_full), whose MMA thread waits for both; its commits free
-// the stage, and announce the accumulator, in both CTAs; the epilogue warps of both give the accumulator back to the first.
-// Not for grouped products (the two halves of a tile could belong to different matrices).
-#define PAIR_BN 256
-#define PAIR_RING_BYTES (192 * 1024)
-#define PAIR_MAX_RING 10
-#define PAIR_THREADS 224
-template <typename OutT, int EPI>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
-gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
-                         const uint8_t* __restrict__ w_tiled, OutT* __restrict__ C, int M, int N, int K, long ldc, Epilogue ep,
-                         int tile_n, int* __restrict__ error_flag) {
-    constexpr int X_BYTES = GEMM_BM * GEMM_BK * 2;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = (uint64_t*)(smem + PAIR_RING_BYTES);
-    uint64_t* full_bar = bars;                        // [ring] TMA -> this CTA's MMA warp
-    uint64_t* empty_bar = bars + PAIR_MAX_RING;       // [ring] MMA -> TMA
-    uint64_t* peer_full = bars + 2 * PAIR_MAX_RING;   // [ring] in the first CTA: the second one's stage is full
-    uint64_t* acc_full = bars + 3 * PAIR_MAX_RING;    // [2] MMA -> epilogue
-    uint64_t* acc_empty = acc_full + 2;               // [2] in the first CTA: both epilogues -> MMA
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int half = tile_n >> 1;  // weight rows of a stage
-    const int stage_bytes = X_BYTES + half * GEMM_BK * 2;
-    const int stages = min(PAIR_MAX_RING, PAIR_RING_BYTES / stage_bytes);
-    const int m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM), total_tiles = m_tiles * ((N + tile_n - 1) / tile_n);
-    const int num_kb = (K + GEMM_BK - 1) / GEMM_BK;
-    pdl_launch_dependents();
-
-    if (threadIdx.x == 0) {
-        tma_prefetch_descriptor(&map_x);
-        tma_prefetch_descriptor(&map_y);
-        for (int s = 0; s < stages; ++s) {
-            mbar_init(smem_addr(&full_bar[s]), 2);  // the two load threads
-            mbar_init(smem_addr(&empty_bar[s]), 1);
-            mbar_init(smem_addr(&peer_full[s]), 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(smem_addr(&acc_full[b]), 1);
-            mbar_init(smem_addr(&acc_empty[b]), 8);  // one arrival per epilogue warp of both CTAs
-        }
-        mbar_fence_init();
-    }
-    if (warp == 1) {
-        tmem_alloc_pair(smem_addr(tmem_slot), 2 * PAIR_BN);
-        tmem_relinquish_pair();
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();  // both CTAs' barriers and tensor memory are there
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    bool ok = true;
-
-    if (warp == 0) {
-        if (elect_one()) {
-            // the weights: this CTA's half of the tile's rows, from the boxes of 128 rows that hold them (a tile's half begins and
-            // ends at a multiple of 8 rows, so that every piece keeps its place in the swizzle's groups of 8; rows past the last
-            // box are left out, their columns of the accumulator are never stored).  They do not depend on the kernel before
-            const int box_rows = (N + GEMM_BM - 1) / GEMM_BM * GEMM_BM;
-            int stage = 0;
-            uint32_t round = 0;  // how often the ring has wrapped
-            for (int t = pair; t < total_tiles && ok; t += pairs) {
-                const int first = (t / m_tiles) * tile_n + rank * half;
-                const int rows = max(0, min(half, box_rows - first));
-                const int inside = first & (GEMM_BM - 1), head = min(GEMM_BM - inside, rows);
-                const uint8_t* src = w_tiled + (size_t)(first / GEMM_BM) * num_kb * GEMM_BOX_BYTES;
-                const uint8_t* next = src + (size_t)num_kb * GEMM_BOX_BYTES;  // the box of the rows behind
-                src += inside * (GEMM_BK * 2);
-                const uint32_t head_bytes = head * (GEMM_BK * 2), tail_bytes = (rows - head) * (GEMM_BK * 2);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (round > 0 && !mbar_wait(smem_addr(&empty_bar[stage]), (round - 1u) & 1u)) { ok = false; break; }
-                    const uint32_t full = smem_addr(&full_bar[stage]), dst = smem_addr(smem + stage * stage_bytes) + X_BYTES;
-                    if (w_tiled) {
-                        mbar_expect_tx(full, head_bytes + tail_bytes);
-                        if (head_bytes) bulk_load_1d(dst, src, head_bytes, full);
-                        if (tail_bytes) bulk_load_1d(dst + head_bytes, next, tail_bytes, full);
-                        src += GEMM_BOX_BYTES, next += GEMM_BOX_BYTES;
-                    } else {
-                        mbar_expect_tx(full, half * (GEMM_BK * 2));
-                        tma_load_2d(dst, &map_y, full, kb * GEMM_BK, first);
-                    }
-                    if (++stage == stages) stage = 0, ++round;
-                }
-            }
-        }
-    } else if (warp == 6) {
-        if (elect_one()) {
-            // this CTA's rows of A, by a thread of their own: one thread that asked for both set the pace
-            pdl_wait();
-            int stage = 0;
-            uint32_t round = 0;
-            for (int t = pair; t < total_tiles && ok; t += pairs) {
-                const int row = (2 * (t % m_tiles) + rank) * GEMM_BM;
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (round > 0 && !mbar_wait(smem_addr(&empty_bar[stage]), (round - 1u) & 1u)) { ok = false; break; }
-                    const uint32_t full = smem_addr(&full_bar[stage]);
-                    mbar_expect_tx(full, X_BYTES);
-                    tma_load_2d(smem_addr(smem + stage * stage_bytes), &map_x, full, kb * GEMM_BK, row);
-                    if (++stage == stages) stage = 0, ++round;
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (elect_one()) {
-            const uint32_t idesc = instr_desc_bf16(2 * GEMM_BM, tile_n);
-            int s = 0, local = 0;
-            uint32_t round = 0;
-            for (int t = pair; t < total_tiles && ok; t += pairs, ++local) {
-                const int buf = local & 1;
-                // both epilogues must have drained this accumulator (two tiles ago)
-                if (rank == 0 && local >= 2 && !mbar_wait(smem_addr(&acc_empty[buf]), (uint32_t)((local >> 1) - 1) & 1u)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * PAIR_BN);
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(smem_addr(&full_bar[s]), round & 1u)) { ok = false; break; }
-                    if (rank == 1) {
-                        mbar_arrive_remote(smem_addr(&peer_full[s]), 0);
-                    } else {
-                        if (!mbar_wait(smem_addr(&peer_full[s]), round & 1u)) { ok = false; break; }
-                        tc_fence_after();
-                        const uint32_t x_addr = smem_addr(smem + s * stage_bytes);
-                        const uint64_t desc_x = smem_desc_k_major_sw128(x_addr);
-                        const uint64_t desc_y = smem_desc_k_major_sw128(x_addr + X_BYTES);
-#pragma unroll
-                        for (int k = 0; k < GEMM_BK / 16; ++k)
-                            mma_bf16_ss_pair(tmem_acc, desc_x + (uint64_t)(2 * k), desc_y + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        mma_commit_pair(smem_addr(&empty_bar[s]));
-                    }
-                    if (++s == stages) s = 0, ++round;
-                }
-                if (ok && rank == 0) mma_commit_pair(smem_addr(&acc_full[buf]));
-            }
-        }
-    } else {
-        const int lane_group = warp & 3;
-        const int tile_row = lane_group * 32 + lane;
-        pdl_wait();  // the output buffer may still be read by the kernel before this one
-        int local = 0;
-        for (int t = pair; t < total_tiles; t += pairs, ++local) {
-            const int buf = local & 1;
-            const int y0 = (t / m_tiles) * tile_n;
-            const int x_row = (2 * (t % m_tiles) + rank) * GEMM_BM + tile_row;
-            if (!mbar_wait(smem_addr(&acc_full[buf]), (uint32_t)(local >> 1) & 1u)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * PAIR_BN) + ((uint32_t)(lane_group * 32) << 16);
-            const float my_scale = (ep.row_sumsq && x_row < M) ? row_scale_of(ep, x_row, M) : 1.0f;
-#pragma unroll 1
-            for (int c0 = 0; c0 < tile_n; c0 += 16) {
-                if (y0 + c0 >= N) break;  // uniform across the warp
-                uint32_t r[16];
-                tmem_load_32x16(tmem_acc + (uint32_t)c0, r);
-                tmem_load_wait();
-                __syncwarp();
-                if (x_row < M) {
-                    float v[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) * my_scale;
-                    store_columns<OutT, EPI>(ep, C + (size_t)x_row * ldc, v, y0 + c0, N);
-                }
-                __syncwarp();
-            }
-            // this warp has read its lanes of the accumulator: hand it back to the MMA thread
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(smem_addr(&acc_empty[buf]), 0);
-        }
-    }
-    if (!ok) atomicExch(error_flag, KIRAI_FLAG_WAIT_RAN_OUT);
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();  // nobody's shared or tensor memory is used any more, and no arrival is on its way
-    if (warp == 1) {
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, 2 * PAIR_BN);
-    }
-}
-
 static int sm_count() {
     static const int count = [] {
         int device = 0, value = 0;
@@ -1320,43 +1120,6 @@ static int sm_count() {
     }();
     return count;
 }
-// The width of the pairs' tiles: the one whose rounds of tiles are shortest together.  A round takes as long as its tiles are
-// wide, down to about 168 columns (a block of K then takes 0.26 us, what loading and announcing it takes).  Measured at 2,048
-// tokens, us at 256 columns and at the chosen width: N 2560, K 9728 98 and 77 (160: 128 tiles in two rounds, 80 at 256
-// take two as well); N 5120, K 25600 468 and 346 (192: three rounds either way); N 6144, K 4096 81 and 77 (240); N 24576,
-// K 4096 290 and 272 (224).
-static int pair_width(int M, int N, int pairs) {
-    const long m_tiles = (M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
-    int best = PAIR_BN;
-    long best_cost = 0;
-    for (int width = PAIR_BN; width >= 160; width -= 16) {
-        const long tiles = m_tiles * ((N + width - 1) / width), cost = (tiles + pairs - 1) / pairs * (width < 168 ? 168 : width);
-        if (width == PAIR_BN || cost < best_cost) best = width, best_cost = cost;
-    }
-    return best;
-}
-
-template <typename OutT, int EPI>
-static int launch_pairs(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
-                        const Epilogue& ep, int* error_flag, cudaStream_t stream) {
-    const int most = sm_count() / 2;
-    if (most <= 0) return KIRAI_ERR_UNSUPPORTED;  // the device did not say how many SMs it has
-    const int tile_n = pair_width(M, N, most);
-    CUtensorMap map_a, map_w;
-    if (!tmap::bf16_2d_sw128(&map_a, A, M, K, lda, GEMM_BM, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
-    if (tiled) map_w = map_a;  // not read: the boxes are fetched by address
-    else if (!tmap::bf16_2d_sw128(&map_w, W, (uint64_t)N, K, K, tile_n / 2, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
-    if (tiled && ((uintptr_t)W & 15)) return KIRAI_ERR_BAD_ALIGN;
-    const long tiles = (long)((M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((N + tile_n - 1) / tile_n);
-    auto kernel = gemm_tcgen05_pair_kernel<OutT, EPI>;
-    constexpr int smem_bytes = PAIR_RING_BYTES + 1024 + 1024;  // the ring, barriers, slack to align to 1024
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (err != cudaSuccess) return (int)err;
-    return launch_pdl_clusters(kernel, dim3((unsigned)(2 * (tiles < most ? tiles : most))), dim3(PAIR_THREADS), (size_t)smem_bytes, stream,
-                               dim3(2, 1, 1), map_a, map_w, tiled ? (const uint8_t*)W : (const uint8_t*)nullptr, (OutT*)C, M, N, K, ldc, ep,
-                               tile_n, error_flag);
-}
-
 template <int BN, typename OutT, int EPI>
 static int launch_persistent(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
                              const Epilogue& ep, int* error_flag, cudaStream_t stream, int groups = 1) {
@@ -1521,8 +1284,7 @@ static int gemm_dispatch(const void* A, const void* W, bool tiled, void* C, int 
     if (M <= 256 && EPI == 2 && N % 8 == 0 && (M <= 128 || one_wave)) return KIRAI_ERR_BAD_ALIGN;  // see kirai_gemm_bf16_residual_parts
 #undef KIRAI_GEMM_CASE
     if (N <= 128) return launch_persistent<128, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
-    if constexpr (EPI == 2) return launch_persistent<256, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
-    else return launch_pairs<OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
+    return launch_persistent<256, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
 }
 
 // Split count that the entry points pick for splits <= 0.

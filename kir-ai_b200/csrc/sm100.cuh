@@ -54,15 +54,6 @@ __device__ __forceinline__ bool mbar_wait_limited(uint32_t bar, uint32_t parity,
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return mbar_wait_limited(bar, parity, KIRAI_WAIT_LIMIT); }
 
-// Arrives on the barrier that lies at `bar` in CTA `rank` of the cluster.  For handing on what the tensor cores and TMA have
-// done (their own completion, seen by this thread, comes before): no ordinary store is published by it, and a release at
-// cluster scope, a fence of about 0.9 us, would stand in every stage of a ring.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar, uint32_t rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(bar), "r"(rank));
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
-
 // The same for waits on the critical path of a pipeline (between an MMA and the warps that consume
 // its result): polls without sleeping for a long while, so that the wake-up adds no latency.
 __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity) {
@@ -156,27 +147,6 @@ __device__ __forceinline__ void mma_bf16_ss(uint32_t tmem_d, uint64_t desc_a, ui
 // Arrives on the barrier when every MMA issued so far by this thread is done.
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// The forms for a pair of CTAs (cta_group::2): both allocate, the first one's thread issues, a commit arrives on the barrier at
-// the same place in both.
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t columns) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t columns) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
-}
-__device__ __forceinline__ void mma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
-                 : "memory");
 }
 
 // 32 consecutive 32-bit columns of this thread's lane (warp w of a warpgroup reads lanes 32 (w % 4) ..).

@@ -970,28 +970,3 @@ def test_decode_attention_of_crowds(ops, q_heads, kv_heads, head_dim, page_size,
             # weights and result are rounded to bfloat16 (2^-9 each) on values of up to about 4
             assert float((got.float() - plain).abs().max()) <= 2.5e-2, (warps, splits)
     ops.check_device_errors(torch.device(DEV))
-
-
-@pytest.mark.parametrize("m,n,k", [(257, 136, 64), (300, 4096, 72), (515, 1000, 520), (700, 5128, 1024), (1605, 2560, 136), (2100, 6144, 64), (4000, 336, 128)])
-def test_products_of_many_tokens_by_pairs_of_ctas(ops, m, n, k):
-    """The product kernel of many tokens against 64-bit sums: a second CTA without rows or without weights, tiles of every width
-    that begin and end inside a box, K that ends inside a block; both weight layouts, both result types, both activations and
-    the row scale."""
-    x, w = rand(m, k, dtype=torch.bfloat16), rand(n, k, dtype=torch.bfloat16, seed=1)
-    want = x.double() @ w.double().T
-    # 32-bit sums of k products of about 1: a random walk of roundings, far below k * 2^-20
-    for weight in (w, ops.tile_weight(w)):
-        assert float((ops.linear_tcgen05(x, weight, torch.float32).double() - want).abs().max()) <= k * 2.0 ** -20
-        assert torch.allclose(ops.linear_tcgen05(x, weight).double(), want, rtol=2.0 ** -8, atol=k * 2.0 ** -20)
-        if n % 16 == 0:
-            gate, up = want.unflatten(1, (n // 16, 2, 8)).unbind(2)
-            gated = (torch.nn.functional.silu(gate) * up).flatten(1)
-            got = ops.linear_tcgen05(x, weight, swiglu=True).double()
-            # the result's rounding, and silu's fast exponential and division (2^-21 each) on sums off by k * 2^-20
-            assert float(((got - gated).abs() / (gated.abs() + 1.0)).max()) <= 2.0 ** -8 + k * 2.0 ** -17
-        assert torch.allclose(ops.linear_tcgen05(x, weight, relu2=True).double(), want.clamp(min=0.0) ** 2, rtol=2.0 ** -7, atol=k * 2.0 ** -14)
-        sumsq = torch.rand(2, m, device=DEV) + 0.5
-        scale = 1.0 / (sumsq.double().sum(0) / 7.0 + 1e-3).sqrt()
-        got = ops.linear_tcgen05(x, weight, torch.float32, row_scale=(sumsq, 7.0, 1e-3)).double()
-        assert float((got - want * scale[:, None]).abs().max()) <= 3.0 * k * 2.0 ** -20 + float(want.abs().max()) * 2.0 ** -20
-    ops.check_device_errors(torch.device(DEV))
