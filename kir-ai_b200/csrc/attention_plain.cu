@@ -1,7 +1,9 @@
 // Plain causal grouped-query attention over the paged cache: one block per
 // (token, query head), keys walked in position order, scores, softmax and the
-// weighted sum in 32-bit.  It serves the true 32-bit path and is the reference
-// beside the tensor-core attention kernels.
+// weighted sum in 32-bit.  It serves the forms of the true 32-bit path that
+// attention_f32.cu does not take, and is the reference beside the other attention
+// kernels.  A token's result does not depend on the rest of the step here; there the
+// cut of a request's keys follows the number of requests.
 //
 // Token t of request r at absolute position pos reads the keys at positions
 // [lo, pos] of r, lo = max(0, pos - window + 1) with a window, else 0

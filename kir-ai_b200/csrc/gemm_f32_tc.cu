@@ -1,12 +1,15 @@
 // 32-bit matrix product C[M, N] = A[M, K] * W[N, K]^T for many rows of A on the fifth-generation tensor cores.
 //
-// A float has 24 significant bits and a bf16 eight: every float is the sum of three bf16 values exactly, its top eight
-// bits, the next eight of what is left, and the rest.  With both operands cut that way the product of two floats is the
-// sum of nine products of bf16 values, which the tensor cores form exactly; the three smallest (2^-24 of the whole and
-// below, less than a 32-bit rounding) are left out and six are summed: lo hi, mid mid, hi lo, mid hi, hi mid, hi hi, in
+// A float has 24 significant bits and a bf16 eight: every float (from 2^-110 on) is the sum of three bf16 values exactly, the
+// nearest one, the nearest to what is left, and the rest.  With both operands cut that way the product of two floats is the
+// sum of nine products of bf16 values, which the tensor cores form exactly.  To nearest, a second cut is at most 2^-8 and a
+// third 2^-17 of the value, of either sign: the three smallest products are at most 2^-24 of the whole together (0.87 x 2^-24 of
+// 4 million pairs, 0 on average; cuts that drop bits leave out up to 7.8 x 2^-24, always of the product's sign).  They are
+// left out and six are summed: lo hi, mid mid, hi lo, mid hi, hi mid, hi hi, in
 // this order.  The tensor cores' own additions drop low bits instead of rounding, so they only sum over 32 values of K;
-// every such block of partial sums is then added to the tile's sums in registers by ordinary 32-bit additions.  The
-// result is nearer to the exact one than a chain of 32-bit FMAs (measured: see the launcher).
+// every such block of partial sums is then added to the tile's sums in registers by ordinary 32-bit additions.  From 32 values
+// of K on the result is nearer to the exact one than a chain of 32-bit FMAs, where no single product outweighs the others
+// (measured: see the launcher).  A row of C depends on how the product was cut, and that on the number of rows.
 //
 // A CTA computes 128 columns of C (128 rows of W fill the MMA) for BN rows of A.  Three planes of A are made by a kernel
 // of their own, once per product (A is small beside W), and come in by TMA as the K-major B operand.  W comes in as it
@@ -73,16 +76,18 @@ __device__ __forceinline__ uint64_t smem_desc_k_major_sw64(uint32_t addr) {
     return desc;
 }
 
-// Two floats cut into three pairs of bf16 (the first in the lower half): each cut takes the top half of the bits, which
-// is the top eight significant ones, and the subtractions are exact.
+// Two floats cut into three pairs of bf16 (the first in the lower half), each cut the nearest bf16 to what is left: the
+// subtractions are exact, and what the second leaves has at most eight bits, so that the third takes all of it (above 2^-110:
+// bits of a value below 2^-133 have no place in a bf16).
 __device__ __forceinline__ void cut_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    const uint32_t xb = __float_as_uint(x), yb = __float_as_uint(y);
-    hi = __byte_perm(xb, yb, 0x7632);
-    const float xr = x - __uint_as_float(xb & 0xffff0000u), yr = y - __uint_as_float(yb & 0xffff0000u);
-    const uint32_t xc = __float_as_uint(xr), yc = __float_as_uint(yr);
-    mid = __byte_perm(xc, yc, 0x7632);
-    const float xl = xr - __uint_as_float(xc & 0xffff0000u), yl = yr - __uint_as_float(yc & 0xffff0000u);
-    lo = __byte_perm(__float_as_uint(xl), __float_as_uint(yl), 0x7632);
+    auto nearest = [](float a, float b) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+        return *reinterpret_cast<const uint32_t*>(&v);
+    };
+    hi = nearest(x, y);
+    const float xr = x - __uint_as_float(hi << 16), yr = y - __uint_as_float(hi & 0xffff0000u);
+    mid = nearest(xr, yr);
+    lo = nearest(xr - __uint_as_float(mid << 16), yr - __uint_as_float(mid & 0xffff0000u));
 }
 
 // planes[3][M][pitch] of A[M, K]; K a multiple of 4, a thread four columns of a row.
@@ -385,8 +390,9 @@ static Cut choose_cut(int M, int N, int K) {
 // `splits` CTAs (1 to 8).
 // Measured at 515 rows of the 4B shape's products (6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728): 80, 72,
 // 296 and 143 us (204, 150, 173 and 179 TFLOP/s of 32-bit arithmetic, six times that in the tensor cores), where the plain
-// kernel took 5.3 ms together (20 TFLOP/s).  2-norm of the error over that of the result 1.3e-7 to 3.3e-7, the plain
-// kernel's 9e-7 to 1.8e-6.
+// kernel took 5.3 ms together (20 TFLOP/s).  2-norm of the error over that of the result, in 2^-24, here and in the plain kernel:
+// normal values 0.79 and 0.68 at K = 4, 0.80 and 1.24 at 16, 0.96 and 1.7 at 32, 1.7 and 15 at 2,560, 2.4 and 29 at 9,728; values of one
+// sign 0.90 and 0.60, 1.0 and 1.06, 1.0 and 1.4, 1.3 and 13, 1.3 and 26.
 KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_, void* C_, int M, int N, int K, long lda, long ldc,
                                    int bn, int splits, int* error_flag, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;

@@ -1,9 +1,10 @@
 // Plain matrix product on the CUDA cores: C[M, N] = A[M, K] * W[N, K]^T with
 // 32-bit fused multiply-adds, k walked in order for every output element (no
 // split along K), so an output row does not depend on which other rows are in
-// the batch.  With float operands this is the true 32-bit path of every linear
-// layer; with bf16 operands it is the plain reference beside the tensor-core
-// kernel.  Any M, N, K >= 1; A and C may have row strides.
+// the batch.  With float operands it takes the products of the true 32-bit path
+// that gemm_f32.cu (up to 8 rows) and gemm_f32_tc.cu (more) do not (rows off 16-byte
+// boundaries, sums of fewer than 32 values); with bf16 operands it is the plain
+// reference beside the tensor-core kernel.  Any M, N, K >= 1; A and C may have row strides.
 #include "common.cuh"
 
 #define BM 64

@@ -1903,6 +1903,9 @@ def linear_f32_rows(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     return out
 
 
+F32_TC_MIN_K = 32  # shorter sums have fewer roundings than the three cuts and the tensor cores' additions (K of 4: 0.68 against 0.79 x 2^-24)
+
+
 def linear_f32_tc_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether ``linear_f32_tc`` runs for these operands: rows of float32 on 16-byte boundaries."""
     return (x.dtype == torch.float32 and x.shape[0] > 0 and x.shape[1] > 0 and x.shape[1] % 4 == 0 and x.stride(0) % 4 == 0
@@ -1910,8 +1913,8 @@ def linear_f32_tc_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
 
 def linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, tile_rows: int = 0, splits: int = 0) -> torch.Tensor:
-    """float32 ``x`` [M, K] times ``weight`` [N, K] transposed on the tensor cores, every float as three bf16 values: at
-    least as exact as 32-bit FMAs.  ``tile_rows`` (32, 64, 128 or 192) and ``splits`` (1 to 8) force how the product is
+    """float32 ``x`` [M, K] times ``weight`` [N, K] transposed on the tensor cores, every float as three bf16 values: from 32
+    values of K on nearer to the exact product than 32-bit FMAs (``F32_TC_MIN_K``).  ``tile_rows`` (32, 64, 128 or 192) and ``splits`` (1 to 8) force how the product is
     cut into CTAs; 0 leaves it to the kernel's rule."""
     _need_cuda(x, weight)
     assert x.dim() == 2 and weight.dim() == 2 and weight.is_contiguous() and weight.dtype == torch.float32
@@ -2190,7 +2193,8 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """The linear layer of the product path: for float32, where rows can be read 16 bytes at a time, a kernel that streams
-    the weights (up to 8 rows) or products of values cut in three on the tensor cores, else the plain kernel; for bfloat16 the tcgen05 kernel, or the
+    the weights (up to 8 rows) or products of values cut in three on the tensor cores (sums of 32 values and more), else the
+    plain kernel: a row's last bits depend on how many rows stand beside it; for bfloat16 the tcgen05 kernel, or the
     CUDA-core kernel when K is not a multiple of 8 (TMA cannot read such rows)."""
     if isinstance(weight, TiledWeight):
         return linear_tcgen05(x if tcgen05_takes(x) else x.contiguous(), weight, out_dtype)
@@ -2199,7 +2203,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if weight.dtype == torch.float32 and out_dtype in (None, torch.float32):
         if linear_f32_rows_takes(x, weight):
             return linear_f32_rows(x, weight)
-        if linear_f32_tc_takes(x, weight):
+        if x.shape[1] >= F32_TC_MIN_K and linear_f32_tc_takes(x, weight):
             return linear_f32_tc(x, weight)
     return linear_plain(x, weight, out_dtype)
 

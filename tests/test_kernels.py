@@ -163,6 +163,35 @@ def test_linear_float32_on_tensor_cores(ops, m, n, k):
         ops.linear_f32_tc(rand(m, k + 9)[:, 1 : 1 + k], w)
 
 
+@pytest.mark.parametrize("k", [4, 8, 16, 32])
+def test_linear_float32_on_tensor_cores_leaves_out_less_than_a_rounding(ops, k):
+    """Products of one sign, where what is left out cannot cancel: mantissas whose second and third cuts would be the greatest
+    if a cut dropped bits, ones just under a power of two, and values spread evenly over a binade."""
+    worst, full = 1.0 + 2.0 ** -7 - 2.0 ** -23, 2.0 - 2.0 ** -23
+    for x, w in ((torch.full((33, k), worst), torch.full((130, k), worst)), (torch.full((33, k), full), torch.full((130, k), worst)),
+                 (torch.full((33, k), full), torch.full((130, k), full)), (rand(33, k, seed=5).abs().cpu() % 1 + 1, rand(130, k, seed=6).abs().cpu() % 1 + 1)):
+        x, w = x.to(DEV), w.to(DEV)
+        expected = x.double() @ w.double().T
+        # to nearest, the second cut is at most 2^-8 and the third 2^-17 of a value's leading bit: the products left out are within
+        # 2^-24 (1 + 2^-8) of the whole; the tensor cores drop at most 2^-23 at each of the two additions of the greatest products
+        # (sixteen values of K each) and 2^-8 of that at the smaller ones'
+        bound = (1.01 + 2 * 2.0 * (1 + 5 * 2.0 ** -8)) * 2.0 ** -24 * expected
+        assert bool(((ops.linear_f32_tc(x, w).double() - expected).abs() <= bound).all())
+        # short sums, which 32-bit FMAs round less often, take those
+        assert torch.equal(ops.linear(x, w), ops.linear_f32_tc(x, w) if k >= 32 else ops.linear_plain(x, w))
+
+
+@pytest.mark.parametrize("k", [32, 64, 100, 2560])
+def test_linear_float32_on_tensor_cores_is_nearer_than_a_chain_of_roundings(ops, k):
+    """The 2-norm of the error against that of the plain kernel, over 20,000 sums: values of both signs and of one."""
+    for one_sign in (False, True):
+        x, w = rand(64, k, seed=7), rand(320, k, seed=8)
+        x, w = (x.abs() + 1.0, w.abs() + 1.0) if one_sign else (x, w)
+        expected = x.double() @ w.double().T
+        error = [float((f(x, w).double() - expected).norm()) for f in (ops.linear_f32_tc, ops.linear_plain)]
+        assert error[0] < error[1], (one_sign, error)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 128, 64), (3, 200, 136), (16, 1000, 512), (48, 520, 1032), (64, 4096, 264),
                                    (65, 264, 192), (100, 1000, 2080), (128, 4096, 4096), (129, 520, 1032),
                                    (200, 96, 64), (256, 4096, 2112), (257, 264, 192), (300, 1000, 520), (1024, 768, 2048)])
