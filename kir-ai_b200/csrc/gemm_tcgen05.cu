@@ -116,17 +116,23 @@ struct Epilogue {
     // g = min(gate, gate_limit) and u = clamp(up, -gate_limit, gate_limit) the result is g sigmoid(gate_slope g) (u + 1).
     int gate_act = 0;
     float gate_limit = 0.0f, gate_slope = 1.0f;
-    // Products with the matrices of experts of which a step's few tokens use a part (weight-streaming kernel only): W's
-    // first chosen_experts * chosen_unit row tiles (chosen_columns: blocks of K) are the experts', chosen_unit to each,
-    // what stands behind them is always needed.  An expert whose gate is 0 for all chosen_tokens rows of `gates`
-    // [tokens, gates_stride] is not read: its row tiles are not computed and their part of C keeps what it held; its blocks
-    // of K, whose columns of A must be zero, are left out of the sum.  Null: every tile.
-    const float* gates = nullptr;
-    int gates_stride = 0, chosen_tokens = 0, chosen_experts = 0, chosen_unit = 1;
-    bool chosen_columns = false;
-    int chosen_tiles = 0;  // row tiles that the launch is expected to compute (host; picks the ring)
+};
+
+// A product with the matrices of experts of which a step's few tokens use a part (weight-streaming kernel, up to 64 tokens,
+// plain stores): W's first `experts` * `unit` row tiles (columns: blocks of K) are the experts', `unit` to each, what stands
+// behind them is always needed.  An expert whose gate is 0 for all `tokens` rows of `gates` [tokens, stride] is not read: its
+// row tiles are not computed and their part of C keeps what it held; its blocks of K, whose columns of A must be zero, are
+// left out of the sum.  (How the blocks of K fall to the CTAs of a split, and so the order of a row's sum, follows the
+// experts that the step's tokens chose together.)  Instances of the kernel of their own take this as one more argument: as fields that
+// every instance looked at, a one-request step of the 8B shape took 24.6 ms in place of 24.2.
+struct ChosenExperts {
+    const float* gates;
+    int stride, tokens, experts, unit;
+    bool columns;
+    int expected_tiles;  // row tiles that the launch is expected to compute (host; picks the ring); 0 for columns
 };
 #define GEMM_MAX_CHOSEN 255  // experts whose numbers fit the list in the CTA's barrier page
+__device__ __forceinline__ const ChosenExperts& chosen_of(const ChosenExperts& chosen) { return chosen; }
 
 // Clock stamps of one CTA of the streaming kernel, written only when a buffer is given: 0 the CTA starts, 1 the kernel
 // before has finished (activations may be read), 2 the first stage is in shared memory, 3 the last product is done,
@@ -209,12 +215,15 @@ __device__ __forceinline__ float gate_mul(const Epilogue& ep, float gate, float 
 // which adds the slots in rank order and stores the result: no partial sum goes to global memory.
 // EPI 0 stores C.  EPI 1 expects W's rows interleaved in eights (8 gate rows, the 8 matching up
 // rows, ...) and stores silu(gate) * up, [M, N / 2].
-template <int BN, bool SWAP, typename OutT, int EPI, bool DEEP>
+// Chosen: nothing, or ChosenExperts.
+template <int BN, bool SWAP, typename OutT, int EPI, bool DEEP, typename... Chosen>
 __global__ void __launch_bounds__(GEMM_THREADS, GemmSmem<BN, DEEP, true>::ctas_per_sm)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const uint8_t* __restrict__ w_tiled, OutT* __restrict__ C, int M, int N, int K, long ldc,
-                    int k_blocks_per_split, int splits, Epilogue ep, int* __restrict__ error_flag) {
+                    int k_blocks_per_split, int splits, Epilogue ep, int* __restrict__ error_flag, Chosen... chosen) {
     using Smem = GemmSmem<BN, DEEP, true>;
+    constexpr bool CHOSEN = sizeof...(Chosen) > 0;
+    static_assert(!CHOSEN || (SWAP && BN <= 64 && EPI == 0), "the list lies behind the row scales of up to 64 tokens");
     constexpr int STAGES = Smem::stages;
     constexpr bool LATE = Smem::late_slots;  // what other CTAs send lies in the receiver's ring (see GemmSmem)
     // Tiles of 32 tokens and more, split along K: every CTA of the cluster sums and stores a share of the tile's
@@ -241,52 +250,54 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int x_tile = blockIdx.x;
+    int x0 = blockIdx.x * GEMM_BM;   // first row of X in this tile
     const int y0 = blockIdx.y * BN;  // first row of Y
-    const int row_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;  // boxes of a row of tiles
-    int total_k_blocks = row_k_blocks, x_tile = blockIdx.x;
+    const int total_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
+    int kb_begin = blockIdx.z * k_blocks_per_split;
+    int kb_end = min(total_k_blocks, kb_begin + k_blocks_per_split);
+    int num_kb = max(0, kb_end - kb_begin);
     const uint32_t rank = blockIdx.z;  // the cluster is (1, 1, splits) and the grid's z extent is splits
-    pdl_launch_dependents();  // the next kernel may set itself up while this one streams
+    if constexpr (!CHOSEN) pdl_launch_dependents();  // the next kernel may set itself up while this one streams
     if (threadIdx.x == 0) gemm_stamp(ep, 0);
     const int* chosen_s = reinterpret_cast<const int*>(smem + STAGES * Smem::stage_bytes + 1024);  // how many, then which
-    if constexpr (SWAP && BN <= 64) {
-        if (ep.gates) {
-            // The list of the experts that some token uses, in ascending order; every CTA makes its own (a column of gates
-            // per lane).  It needs the kernel before this one, so such a launch cannot fetch weights ahead of it.
-            pdl_wait();
-            int* list = const_cast<int*>(chosen_s);
-            if (warp == 0) {
-                int count = 0;
-                for (int base = 0; base < ep.chosen_experts; base += 32) {
-                    const int e = base + lane;
-                    bool used = false;
-                    if (e < ep.chosen_experts) {
+    if constexpr (CHOSEN) {
+        // The list of the experts that some token uses, in ascending order; every CTA makes its own (a column of gates
+        // per lane).  It needs the kernel before this one, so such a launch cannot fetch weights ahead of it; and a CTA that has
+        // waited without tensor memory of its own lets later kernels start only once it has that (below), so that none of
+        // them can take the columns and then wait for this one.
+        const ChosenExperts& ce = chosen_of(chosen...);
+        pdl_wait();
+        int* list = const_cast<int*>(chosen_s);
+        if (warp == 0) {
+            int count = 0;
+            for (int base = 0; base < ce.experts; base += 32) {
+                const int e = base + lane;
+                bool used = false;
+                if (e < ce.experts) {
 #pragma unroll 4
-                        for (int t = 0; t < ep.chosen_tokens; ++t) used |= ep.gates[(size_t)t * ep.gates_stride + e] != 0.0f;
-                    }
-                    const uint32_t mask = __ballot_sync(0xffffffffu, used);
-                    if (used) list[1 + count + __popc(mask & ((1u << lane) - 1u))] = e;
-                    count += __popc(mask);
+                    for (int t = 0; t < ce.tokens; ++t) used |= ce.gates[(size_t)t * ce.stride + e] != 0.0f;
                 }
-                if (lane == 0) list[0] = count;
+                const uint32_t mask = __ballot_sync(0xffffffffu, used);
+                if (used) list[1 + count + __popc(mask & ((1u << lane) - 1u))] = e;
+                count += __popc(mask);
             }
-            __syncthreads();
-            const int count = chosen_s[0], unit = ep.chosen_unit;
-            if (ep.chosen_columns) {
-                total_k_blocks -= (ep.chosen_experts - count) * unit;
-                k_blocks_per_split = (total_k_blocks + splits - 1) / splits;
-            } else {
-                // the tiles behind the experts' first, then the chosen experts': the CTAs with work are the first of the
-                // grid, which the device spreads evenly over its SMs
-                const int behind = (int)gridDim.x - ep.chosen_experts * unit, at = x_tile - behind;
-                if (at >= count * unit) return;  // (all CTAs of a cluster have the same tile)
-                x_tile = at < 0 ? ep.chosen_experts * unit + x_tile : chosen_s[1 + at / unit] * unit + at % unit;
-            }
+            if (lane == 0) list[0] = count;
+        }
+        __syncthreads();
+        const int count = chosen_s[0];
+        if (ce.columns) {
+            const int read = total_k_blocks - (ce.experts - count) * ce.unit, share = (read + splits - 1) / splits;
+            kb_begin = blockIdx.z * share, kb_end = min(read, kb_begin + share), num_kb = max(0, kb_end - kb_begin);
+        } else {
+            // the tiles behind the experts' first, then the chosen experts': the CTAs with work are the first of the
+            // grid, which the device spreads evenly over its SMs
+            const int behind = (int)gridDim.x - ce.experts * ce.unit, at = x_tile - behind;
+            if (at >= count * ce.unit) return;  // (all CTAs of a cluster have the same tile)
+            x_tile = at < 0 ? ce.experts * ce.unit + x_tile : chosen_s[1 + at / ce.unit] * ce.unit + at % ce.unit;
+            x0 = x_tile * GEMM_BM;
         }
     }
-    const int x0 = x_tile * GEMM_BM;  // first row of X in this tile
-    const int kb_begin = blockIdx.z * k_blocks_per_split;
-    const int kb_end = min(total_k_blocks, kb_begin + k_blocks_per_split);
-    const int num_kb = max(0, kb_end - kb_begin);
 
     if (threadIdx.x == 0) {
         tma_prefetch_descriptor(&map_x);
@@ -305,6 +316,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if constexpr (CHOSEN) pdl_launch_dependents();
     const uint32_t tmem_base = *tmem_slot;
     float res[16];  // EPI 2: the stream's values under this thread's 16 outputs
     float norm_w = 0.0f;
@@ -327,13 +339,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // of the first ring of stages is fetched at once, and only the activations wait for it.
             const int x_first = SWAP ? 0 : 1, y_first = SWAP ? 1 : 0;  // which operand is the weights
             // tiled weights (SWAP only): this tile's boxes lie one after the other
-            const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)x_tile * row_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
+            const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)x_tile * total_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
             // this CTA's i-th block of K, counted from kb_begin: the i-th, but for the blocks of experts that are left out
             auto block = [&](int i) {
-                if constexpr (SWAP && BN <= 64) {
-                    if (ep.gates && ep.chosen_columns) {
-                        const int at = kb_begin + i, unit = ep.chosen_unit, own = chosen_s[0] * unit;
-                        return (at < own ? chosen_s[1 + at / unit] * unit + at % unit : ep.chosen_experts * unit + at - own) - kb_begin;
+                if constexpr (CHOSEN) {
+                    const ChosenExperts& ce = chosen_of(chosen...);
+                    if (ce.columns) {
+                        const int at = kb_begin + i, unit = ce.unit, own = chosen_s[0] * unit;
+                        return (at < own ? chosen_s[1 + at / unit] * unit + at % unit : ce.experts * unit + at - own) - kb_begin;
                     }
                 }
                 return i;
@@ -392,7 +405,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 }
                 mma_commit(smem_addr(&empty_bar[s]));  // frees the stage once these MMAs have read it
             }
-            mma_commit(smem_addr(done_bar));
+            if (!CHOSEN || num_kb > 0) mma_commit(smem_addr(done_bar));  // (nobody waits for it without products)
         }
     } else {
         pdl_wait();  // the output buffer may still be read by the kernel before this one
@@ -1176,9 +1189,9 @@ static long max_resident_clusters(Kernel kernel, int smem_bytes, int cluster_z) 
     return answer;
 }
 
-template <int BN, bool SWAP, typename OutT, int EPI>
+template <int BN, bool SWAP, typename OutT, int EPI, typename... Chosen>
 static int launch_config(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
-                         int splits, const Epilogue& ep, int* error_flag, cudaStream_t stream) {
+                         int splits, const Epilogue& ep, int* error_flag, cudaStream_t stream, const Chosen&... chosen) {
     using Smem = GemmSmem<BN, false, true>;
     CUtensorMap map_x, map_y;
     const void* x_ptr = SWAP ? W : A;
@@ -1209,19 +1222,23 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
         if constexpr (BN <= 128) {  // (tiles of 256 tokens have one configuration: four stages, one CTA per SM)
             // no more CTAs than SMs: one CTA per SM with the long ring (KIRAI_GEMM_DEEP=0 keeps the short one, to compare)
             // (a product with the chosen experts alone: by the tiles that it is expected to compute)
-            const long busy = ep.chosen_tiles > 0 ? (long)ep.chosen_tiles * grid.y : clusters;
+            long busy = clusters;
+            if constexpr (sizeof...(Chosen) > 0) {
+                const long expected = (chosen.expected_tiles + ... + 0);
+                if (expected > 0) busy = expected * grid.y;
+            }
             if (busy * used <= sm_count() && deep_rings()) {
                 using Deep = GemmSmem<BN, true, true>;
-                auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, true>;
+                auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, true, Chosen...>;
                 cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Deep::total(Deep::max_splits));
                 if (err != cudaSuccess) return (int)err;
                 if (used > 1 && splits > 1 && busy > max_resident_clusters(kernel, Deep::total(used), used)) continue;
                 return launch_pdl(kernel, grid, dim3(GEMM_THREADS), (size_t)Deep::total(used), stream, (unsigned)used, map_x,
-                                  map_y, boxes, (OutT*)C, M, N, K, ldc, per_split, used, ep, error_flag);
+                                  map_y, boxes, (OutT*)C, M, N, K, ldc, per_split, used, ep, error_flag, chosen...);
             }
         }
         if (used > Smem::max_splits) continue;  // (tiles of 128 tokens split only with the long ring)
-        auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, false>;
+        auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, false, Chosen...>;
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::total(Smem::max_splits));
         if (err != cudaSuccess) return (int)err;
         // launches of more CTAs than SMs run in waves anyway; only a launch meant to be one wave is fitted
@@ -1229,7 +1246,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
             clusters > max_resident_clusters(kernel, Smem::total(used), used))
             continue;
         return launch_pdl(kernel, grid, dim3(GEMM_THREADS), (size_t)Smem::total(used), stream, (unsigned)used, map_x, map_y,
-                          boxes, (OutT*)C, M, N, K, ldc, per_split, used, ep, error_flag);
+                          boxes, (OutT*)C, M, N, K, ldc, per_split, used, ep, error_flag, chosen...);
     }
 }
 
@@ -1340,7 +1357,7 @@ KIRAI_EXPORT int kirai_gemm_bf16_grouped(const void* A, const void* W, int tiled
     return KIRAI_ERR_BAD_SIZE;
 }
 
-// A product of up to 64 tokens with the matrices of those experts alone that a token uses (see Epilogue::gates).
+// A product of up to 64 tokens with the matrices of those experts alone that a token uses (see ChosenExperts).
 //   gates [M, gates_stride] (float, on the device): nonzero where token m uses expert e < experts.
 //   columns 0: W [N, K] has `unit` tiles of 128 rows to each expert, then further rows that are always computed; the columns
 //   of C that belong to experts nobody uses are left as they were.  columns 1: every row of W has `unit` blocks of 64
@@ -1355,16 +1372,18 @@ KIRAI_EXPORT int kirai_gemm_bf16_chosen(const void* A, const void* W, int tiled,
     if (K <= 0 || M > 64 || !gates || gates_stride < experts || experts <= 0 || experts > GEMM_MAX_CHOSEN || unit <= 0 ||
         (long)experts * unit > pieces || form < 0 || form > 1)
         return KIRAI_ERR_BAD_SIZE;
-    Epilogue ep{nullptr, 0, 1.0f, 0.0f, nullptr, nullptr, nullptr, nullptr};
-    ep.gates = gates, ep.gates_stride = gates_stride, ep.chosen_tokens = M, ep.chosen_experts = experts, ep.chosen_unit = unit;
-    ep.chosen_columns = columns != 0;
-    int splits = 0;
-    if (!columns) {
-        ep.chosen_tiles = expected_tiles < 1 ? 1 : (expected_tiles < pieces ? expected_tiles : pieces);
-        splits = choose_splits(M, ep.chosen_tiles * GEMM_BM, K);
-    }
-    return form == 0 ? gemm_dispatch<bf16, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream)
-                     : gemm_dispatch<float, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream);
+    if (K % 8 != 0 || lda % 8 != 0) return KIRAI_ERR_BAD_ALIGN;
+    const Epilogue ep{nullptr, 0, 1.0f, 0.0f, nullptr, nullptr, nullptr, nullptr};
+    ChosenExperts chosen{gates, gates_stride, M, experts, unit, columns != 0, 0};
+    if (!columns) chosen.expected_tiles = expected_tiles < 1 ? 1 : (expected_tiles < pieces ? expected_tiles : pieces);
+    const int splits = choose_splits(M, columns ? N : chosen.expected_tiles * GEMM_BM, K);
+#define KIRAI_CHOSEN(BN)                                                                                                                      \
+    return form == 0 ? launch_config<BN, true, bf16, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream, chosen) \
+                     : launch_config<BN, true, float, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream, chosen)
+    if (M <= 16) KIRAI_CHOSEN(16);
+    if (M <= 32) KIRAI_CHOSEN(32);
+    KIRAI_CHOSEN(64);
+#undef KIRAI_CHOSEN
 }
 
 // The one entry point of the tensor-core product, A[M, K] (row stride lda) times W[N, K] transposed.
