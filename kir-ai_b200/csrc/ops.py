@@ -1286,6 +1286,27 @@ def linear_chosen_takes(x: torch.Tensor, experts: int, expert_size: int, rows_of
             and tcgen05_takes(x))
 
 
+def linear_chosen_pays(tokens: int, experts: int, share: float, n: int, k: int, expert_bytes: int, columns: bool,
+                       sms: Optional[int] = None) -> bool:
+    """Whether a product [tokens, k] x [n, k] is expected to be faster by ``linear_chosen`` than whole: ``share`` of the experts
+    is used by some token, ``expert_bytes`` of the matrix belong to experts.  What it saves is the reading of the others, at
+    about 6 TB/s.  Against that stand 4 us (no weights are fetched before the kernel ahead has finished) and the list that every
+    CTA makes, 0.15 us for four tokens and 32 experts in each wave of CTAs; with chosen columns also the load thread, which
+    needs 0.33 us to find and fetch a block of K (in a launch of 128 CTAs a block takes 0.35 us of the memory's time anyway,
+    in one of 64 half of that).  Measured with these weights alone in a graph, us a layer whole, first product chosen, both: 16
+    experts of which a token uses two, width 4096, expert size 1536: 3 tokens 100, 68, 52; 12 tokens 103, 93, 92; 20 tokens 110, 113,
+    116; 64 tokens 121, 129, 135.  64 experts of which it uses four, width 2048, expert size 768: 8 tokens 104, 77, 73; 16 tokens 107,
+    97, 108; 32 tokens 123, 125, 147.  128 of which it uses eight: 8 tokens 195, 135, 125; 16 tokens 201, 170, 189; 64 tokens 273, 358, 416."""
+    sms, tiles = sms or DEFAULT_SMS, -(-n // 128)
+    splits = min(4, max(1, (2 * sms + tiles) // (2 * tiles)))
+    whole_us = expert_bytes / 6.0e6
+    listing_us = 0.15 * -(-tokens // 4) * -(-experts // 32) * -(-tiles * splits // (2 * sms))
+    read_us = share * whole_us
+    if columns:
+        read_us = max(read_us, share * expert_bytes / (n * 128) / splits * 0.33)
+    return read_us + listing_us + 4.0 < whole_us
+
+
 def linear_chosen(x: torch.Tensor, weight, gates: torch.Tensor, experts: int, unit: int, columns: bool, expected_tiles: int = 1,
                   out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     """``x`` [M, K] (bfloat16, at most 64 rows) times ``weight`` [N, K] transposed, reading only the matrices of experts that

@@ -14,12 +14,14 @@ experts' outputs in its own accumulation.  Nothing depends on how many tokens
 an expert drew, so a step of single tokens can be captured in a graph; the
 price is that every chosen expert's rows are computed for every token.  For a
 step of few tokens that price is none: the products are bound by reading the
-weights.  In bfloat16 (up to 64 tokens, expert sizes in whole boxes of the
-weights) they read the chosen experts' matrices alone: each CTA looks the
-step's routing weights over on the device and takes a tile, or the blocks of
-K, of an expert that some token uses (``_reads_chosen``; 16 experts of which a
-token uses two, width 4096, expert size 1536, three tokens: the two products
-of a layer 94 us with all experts' matrices, 46 with the chosen ones).
+weights.  In bfloat16 (expert sizes in whole boxes of the weights) the few
+tokens of a step that leave enough experts out (``_reads_chosen``) read the
+chosen experts' matrices alone: each CTA looks the step's routing weights over
+on the device and takes a tile, or the blocks of K, of an expert that some
+token uses (16 experts of which a token uses two, width 4096, expert size
+1536, three tokens: router and products of a layer 100 us with all experts'
+matrices, 52 with the chosen ones).  A token's sum over K is then cut among CTAs by
+what the step's tokens chose together, so its last bits depend on them.
 
 Steps of many tokens (``GROUPED_MIN_ROWS`` pairs of token and chosen expert, in
 bfloat16, expert and model width multiples of 128) sort their pairs by expert
@@ -200,26 +202,35 @@ class RoutedExperts(FeedForward):
                                       rule=self.rule)
         return ops.router_gates(x, self.router, self.top, want_chosen, over_all=self.over_all, rule=self.rule)
 
-    def _reads_chosen(self, x: torch.Tensor) -> bool:
-        """Whether a step of few tokens reads the chosen experts' matrices alone.  Every expert stays a candidate for the
-        products (which of them are read is known on the device only, so that such a step can be captured); what it saves
-        is the share of experts that nobody chose, (1 - top / routes)^tokens of them: at 16 experts of which a token uses two,
-        88 % of the bytes for one token, 66 % for three, 12 % for sixteen.  Against that stands the head start that the
-        products lose (they fetch no weights before the router has finished), about 1 us each."""
-        return (self.leaves_out and hasattr(self.rt.ops, "linear_chosen") and self.down.out_features % 8 == 0
-                and self.rt.ops.linear_chosen_takes(x, self.experts, self.expert_size, self.expert_size * (2 if self.gated else 1)))
+    def _share_read(self, tokens: int) -> float:
+        """The share of the experts that some of ``tokens`` tokens use, if every choice is as likely."""
+        return 1.0 - (1.0 - self.top / self.routes) ** tokens
+
+    def _reads_chosen(self, x: torch.Tensor, columns: bool) -> bool:
+        """Whether the first (``columns``: the second) product of a step of few tokens reads the chosen experts' matrices alone.
+        Every expert stays a candidate for the products (which of them are read is known on the device only, so that such a
+        step can be captured); what it saves is the experts that nobody chose, (1 - top / routes)^tokens of them: at 16
+        experts of which a token uses two, 88 % of the bytes for one token, 66 % for three, 12 % for sixteen, nothing for sixty.
+        ``ops.linear_chosen_pays`` has what stands against that."""
+        rows = self.expert_size * (2 if self.gated else 1)
+        if not (self.leaves_out and hasattr(self.rt.ops, "linear_chosen") and self.down.out_features % 8 == 0
+                and self.rt.ops.linear_chosen_takes(x, self.experts, self.expert_size, rows)):
+            return False
+        n, k = (self.hidden_size, x.shape[1]) if columns else (self.up.out_features, self.hidden_size)
+        return self.rt.ops.linear_chosen_pays(x.shape[0], self.experts, self._share_read(x.shape[0]), n, k,
+                                              2 * self.experts * self.hidden_size * (self.expert_size if columns else rows), columns)
 
     def _up_few(self, x: torch.Tensor, gates: torch.Tensor) -> torch.Tensor:
         """The stacked first product; columns of experts that nobody chose may be left unwritten (their gates are zero)."""
-        if not self._reads_chosen(x):
+        if not self._reads_chosen(x, False):
             return self.up.forward(x)
         unit = self.expert_size * (2 if self.gated else 1) // 128
-        read = self.experts * (1.0 - (1.0 - self.top / self.routes) ** x.shape[0])
+        read = self.experts * self._share_read(x.shape[0])
         behind = -(-self.up.out_features // 128) - self.experts * unit
         return self.rt.ops.linear_chosen(x, self.up.weight, gates, self.experts, unit, False, int(read * unit) + behind)
 
     def _down_few(self, hidden: torch.Tensor, gates: torch.Tensor, out_dtype: Optional[torch.dtype]) -> torch.Tensor:
-        if not self._reads_chosen(hidden):
+        if not self._reads_chosen(hidden, True):
             return self.down.forward(hidden, out_dtype)
         return self.rt.ops.linear_chosen(hidden, self.down.weight, gates, self.experts, self.expert_size // 64, True,
                                          out_dtype=out_dtype or torch.bfloat16)

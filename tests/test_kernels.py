@@ -948,6 +948,31 @@ def test_products_with_the_chosen_experts_alone(ops, tokens, experts, unit, behi
     ops.check_device_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("heads_on", [False, True])
+@pytest.mark.parametrize("tokens", [1, 5, 16, 33, 64])
+def test_experts_are_the_same_whole_and_chosen(ops, monkeypatch, tokens, heads_on):
+    """The part with each product whole and each reading the chosen experts alone, with a shared branch stacked behind the
+    experts and without: the gates' zeros stand for what is not read, whatever memory held there."""
+    from part_helpers import load_part
+    from kirai_b200.parts.experts import RoutedExperts
+    from kirai_b200.parts.swiglu import SwiGLU
+
+    shared = SwiGLU("shared.", 256, 192) if heads_on else None
+    more = dict(scoring="softmax_corrected", weight_scale=1.0, shared=shared, shared_gate="sg") if heads_on else {}
+    part = RoutedExperts("m.", 256, 128, 12, 2, activation="silu_gated", **more)
+    load_part(part, torch.bfloat16, seed=3)
+    x = rand(tokens, 256, dtype=torch.bfloat16, seed=4)
+    results = []
+    for up, down in ((False, False), (True, False), (False, True), (True, True)):
+        monkeypatch.setattr(ops, "linear_chosen_pays", lambda *a, **k: down if a[6] else up)
+        torch.full((tokens, part.up.out_features), float("nan"), dtype=torch.bfloat16, device=DEV)  # what an unwritten column may hold
+        results.append(part.forward(x).float())
+    ops.check_device_errors(torch.device(DEV))
+    for result in results[1:]:
+        # the same products in 32-bit sums of another order, then one rounding to bfloat16
+        assert float((result - results[0]).abs().max()) <= 2.0 ** -7 * float(results[0].abs().max())
+
+
 @pytest.mark.parametrize("likely", [1, 2, 33, 511, 512, 513, 3000])
 @pytest.mark.parametrize("vocab", [32000, 151936])
 def test_sampling_where_few_entries_hold_the_nucleus(ops, likely, vocab):

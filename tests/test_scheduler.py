@@ -199,6 +199,34 @@ def test_decode_crowd_plan_follows_the_measured_batches():
     assert decode_crowd_plan([200_000] + [100] * 30, 8) is None             # equal ranges for all SMs
 
 
+def test_products_with_chosen_experts_are_taken_where_they_were_measured_faster():
+    """Every measured step whose two ways differ by more than a twentieth: (experts, top, width, expert size, rows behind the
+    experts, tokens, us whole, first product chosen, both)."""
+    import kirai_b200  # noqa: F401
+    from kirai_b200.csrc.ops import linear_chosen_pays
+
+    measured = [
+        (16, 2, 4096, 1536, 0, 1, 102, 56, 32), (16, 2, 4096, 1536, 0, 3, 100, 68, 52), (16, 2, 4096, 1536, 0, 8, 101, 79, 71),
+        (16, 2, 4096, 1536, 0, 12, 103, 93, 92), (16, 2, 4096, 1536, 0, 20, 110, 113, 116), (16, 2, 4096, 1536, 0, 32, 112, 117, 122),
+        (16, 2, 4096, 1536, 0, 64, 121, 129, 135), (16, 2, 4096, 1536, 1536, 3, 111, 75, 60), (16, 2, 4096, 1536, 1536, 12, 114, 100, 96),
+        (16, 2, 4096, 1536, 1536, 64, 129, 136, 142), (8, 2, 4096, 2048, 0, 1, 73, 47, 33), (8, 2, 4096, 2048, 0, 3, 73, 60, 55),
+        (8, 2, 4096, 2048, 0, 12, 73, 75, 80), (8, 2, 4096, 2048, 0, 64, 85, 89, 94), (64, 4, 2048, 768, 0, 1, 102, 64, 35),
+        (64, 4, 2048, 768, 0, 3, 103, 67, 48), (64, 4, 2048, 768, 0, 8, 104, 77, 73), (64, 4, 2048, 768, 0, 12, 105, 85, 90),
+        (64, 4, 2048, 768, 0, 16, 107, 97, 108), (64, 4, 2048, 768, 0, 32, 123, 125, 147), (64, 4, 2048, 768, 0, 64, 139, 168, 197),
+        (128, 8, 2048, 768, 0, 1, 191, 113, 57), (128, 8, 2048, 768, 0, 8, 195, 135, 125), (128, 8, 2048, 768, 0, 12, 197, 153, 158),
+        (128, 8, 2048, 768, 0, 16, 201, 170, 189), (128, 8, 2048, 768, 0, 32, 229, 230, 274), (128, 8, 2048, 768, 0, 64, 273, 358, 416),
+    ]
+    for experts, top, width, ff, behind, tokens, whole, first, both in measured:
+        share = 1.0 - (1.0 - top / experts) ** tokens
+        up = linear_chosen_pays(tokens, experts, share, experts * 2 * ff + 2 * behind, width, 4 * experts * ff * width, False)
+        down = linear_chosen_pays(tokens, experts, share, width, experts * ff + behind, 2 * experts * ff * width, True)
+        if abs(first - whole) > 0.05 * whole:
+            assert up == (first < whole), (experts, tokens)
+        if abs(both - first) > 0.05 * whole:
+            assert down == (both < first), (experts, tokens)
+    assert not linear_chosen_pays(1, 8, 0.125, 2048, 64, 8 * 2 * 128 * 64 * 2, False)  # a small layer has nothing to save
+
+
 def test_decode_plan_over_random_batches_respects_the_kernels_limits():
     """Whatever the batch, the planner names a split count that the decode kernel takes (1 to 64 ranges, never more
     ranges than key tiles), and ranges are merged inside the kernel only where the device said the clusters fit and
