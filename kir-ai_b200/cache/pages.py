@@ -112,6 +112,7 @@ class GroupSpec:
     key_dim: Optional[int] = None    # columns of a row that keys use (None: all)
     value_dim: Optional[int] = None  # columns of a row that values use (None: all)
     keep_first: int = 0  # a window never gives back the pages of a request's first so many tokens
+    group: Optional[int] = None  # the most query heads to a kv head among the layers (None: some layer does not say)
 
 
 @dataclass(eq=False)

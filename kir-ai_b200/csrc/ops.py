@@ -1724,8 +1724,14 @@ def attention_decode_crowd(q: torch.Tensor, cache: torch.Tensor, block_table: to
 DECODE_MAX_SORTED = 512  # requests whose order every CTA of ``attention_decode_crowd`` works out
 
 
+def decode_crowd_serves(requests: int, kv_heads: int, head_dim: int, group: Optional[int], sms: int) -> bool:
+    """Whether ``attention_decode_crowd`` is for such a layer: more (request, kv head) pairs than SMs, and sizes that it takes."""
+    return (sms < requests * kv_heads and requests <= DECODE_MAX_SORTED and head_dim <= 128 and group is not None and group <= 8
+            and kv_heads <= sms)
+
+
 def decode_crowd_plan(context_lens, kv_heads: int, reach: Optional[int] = None, sms: int = DEFAULT_SMS, head_dim: int = 128,
-                      group: int = 4) -> Optional[tuple]:
+                      group: Optional[int] = 4) -> Optional[tuple]:
     """How a batch of more (request, kv head) pairs than SMs is attended: (warps of a CTA, ranges of a request's keys), or
     None where another kernel should (few pairs, wide heads, a few contexts so long that only equal ranges for all SMs help).
 
@@ -1738,7 +1744,7 @@ def decode_crowd_plan(context_lens, kv_heads: int, reach: Optional[int] = None, 
     48 of 1,300 tokens 64 and 66 (39); 20 of 500 to 3,000 tokens 41 and 61, two ranges 51 and 44 (25).  The
     balanced kernel: 42, 63, 47, and 97 at 64 requests of 131 to 1,500 tokens, where 4 warps take 47."""
     requests = len(context_lens)
-    if requests * kv_heads <= sms or requests > DECODE_MAX_SORTED or head_dim > 128 or group > 8 or kv_heads > sms:
+    if not decode_crowd_serves(requests, kv_heads, head_dim, group, sms):
         return None
     tiles = sorted((-(-(min(int(n), reach) if reach else int(n)) // 16) for n in context_lens), reverse=True)
     bytes_us = kv_heads * sum(tiles) * head_dim * 64 / 5.9e6
@@ -1822,7 +1828,8 @@ def _decode_rows(q, cache, block_table, batch, rows: int, window: Optional[int],
     forced = os.environ.get("KIRAI_DECODE_BALANCED")
     if forced in ("0", "1"):
         balanced, crowd = forced == "1", None
-    if crowd and q.shape[2] <= 128 and q.shape[1] // kv_heads <= 8:  # (a captured step's layers may differ in their heads)
+    # (a captured step's layers may differ in their heads: those that the crowd's kernel is not for take the step's other plan)
+    if crowd and decode_crowd_serves(rows, kv_heads, q.shape[2], q.shape[1] // kv_heads, sm_count(q.device)):
         attention_decode_crowd(q, cache, block_table, context_len, window, scale, crowd[1], crowd[0], out=out, **mask)
         return
     if balanced and rows <= 1024:

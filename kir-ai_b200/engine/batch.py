@@ -52,7 +52,8 @@ class StepBatch:
     decode_balanced: Optional[bool] = None
     # into how many ranges that kernel cuts a request's keys (None or 0: decided from the longest context above)
     decode_splits: Optional[int] = None
-    # for more (request, kv head) pairs than SMs: (warps of a CTA, ranges), see ops.decode_crowd_plan (None: not such a batch)
+    # for layers of more (request, kv head) pairs than SMs: (warps of a CTA, ranges), see ops.decode_crowd_plan (None: not such a
+    # batch); layers that ops.decode_crowd_serves does not name take the two above
     decode_crowd: Optional[tuple] = None
 
     @property

@@ -211,19 +211,21 @@ class DecodeGraphs:
         captured step: the widest need decides).  The ranges are planned for the lengths that the requests have, not
         for the longest that the block tables' bucket could hold: at 7 requests of 4,100 tokens that is 2 ranges, not
         the 5 that 8,192 tokens would want (3.55 against 3.67 ms a step).  Third: how more (request, kv head) pairs than SMs
-        are attended (ops.decode_crowd_plan), which then decides."""
+        are attended (ops.decode_crowd_plan) by the layers that ops.decode_crowd_serves; where that is every layer the
+        other two are left at nothing, so that they do not make more captures."""
         ops = self.runner.rt.ops
         groups = list(self.runner.cache.groups)
         if not groups:
             return False, 0, None
         need = max(groups, key=lambda g: g.window or (1 << 60))
         device = self.runner.rt.device
-        crowd = ops.decode_crowd_plan(context_lens, need.kv_heads, need.window, sms=ops.sm_count(device), head_dim=need.head_dim)
-        if crowd:
+        sms = ops.sm_count(device)
+        crowd = ops.decode_crowd_plan(context_lens, need.kv_heads, need.window, sms=sms, head_dim=need.head_dim, group=need.group)
+        if crowd and all(ops.decode_crowd_serves(len(context_lens), g.kv_heads, g.head_dim, g.group, sms) for g in groups):
             return False, 0, crowd
-        balanced, splits = ops.decode_plan(context_lens, need.kv_heads, need.window, sms=ops.sm_count(device),
+        balanced, splits = ops.decode_plan(context_lens, need.kv_heads, need.window, sms=sms,
                                            room=ops.decode_cluster_room(device, need.head_dim), head_dim=need.head_dim)
-        return balanced, (0 if balanced else splits), None
+        return balanced, (0 if balanced else splits), crowd
 
     @staticmethod
     def batch_bucket(requests: int) -> int:

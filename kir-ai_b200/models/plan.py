@@ -16,7 +16,7 @@ from typing import Dict, List, Optional
 
 import torch
 
-from ..parts.base import Norm, NormedSum, Runtime, ScaledSum, StreamCopy, StreamUpdate, WeightSpec
+from ..parts.base import KVCacheNeed, Norm, NormedSum, Runtime, ScaledSum, StreamCopy, StreamUpdate, WeightSpec
 from ..parts.block import Block
 from ..parts.embedding import Embedding, OutputHead
 
@@ -97,6 +97,8 @@ class ModelPlan:
                     raise PlanError(f"order[{step}]: cache layer {call.cache} is read before any call wrote it")
                 if needs[call.cache] != need:
                     raise PlanError(f"order[{step}]: reader needs {need}, cache layer {call.cache} holds {needs[call.cache]}")
+                if isinstance(need, KVCacheNeed):
+                    needs[call.cache] = needs[call.cache].also_read_by(need)
         if sorted(needs) != list(range(len(needs))):
             raise PlanError(f"cache layers must be numbered 0..n-1 without gaps, got {sorted(needs)}")
         self.cache_needs = [needs[i] for i in range(len(needs))]

@@ -160,8 +160,8 @@ class GQAttention(Mixer):
     def cache_need(self):
         if self.wide:
             return KVCacheNeed(self.kv_heads, self.pad_dim, self.window, key_dim=self.head_dim, value_dim=self.value_dim,
-                               keep_first=self.keep_first)
-        return KVCacheNeed(self.kv_heads, self.head_dim, self.window)
+                               keep_first=self.keep_first, group=self.q_heads // self.kv_heads)
+        return KVCacheNeed(self.kv_heads, self.head_dim, self.window, group=self.q_heads // self.kv_heads)
 
     @property
     def capture_safe(self) -> bool:

@@ -15,7 +15,7 @@ per-variant flags).
 """
 from __future__ import annotations
 
-from dataclasses import dataclass
+from dataclasses import dataclass, field, replace
 from typing import Dict, Optional, Tuple
 
 import torch
@@ -54,7 +54,8 @@ class KVCacheNeed:
     tokens for good: a window under which every position still sees the sequence's first tokens).  ``head_dim`` is the width of a
     cache row.  Keys and values may be narrower than the row and differ from each other
     (``key_dim``, ``value_dim``; None: the whole row): the columns beyond them are never written
-    and stay zero, so kernels that read whole rows compute the same scores and sums."""
+    and stay zero, so kernels that read whole rows compute the same scores and sums.  ``group``: query heads to a kv
+    head, for choosing kernels (None: not said, and kernels that take only some groups are not chosen ahead)."""
 
     kv_heads: int
     head_dim: int
@@ -62,6 +63,11 @@ class KVCacheNeed:
     key_dim: Optional[int] = None
     value_dim: Optional[int] = None
     keep_first: int = 0
+    group: Optional[int] = field(default=None, compare=False)  # (layers of other groups may share a cache layer)
+
+    def also_read_by(self, other: "KVCacheNeed") -> "KVCacheNeed":
+        """This need with the larger group of the two (None where one does not say)."""
+        return replace(self, group=max(self.group, other.group) if self.group and other.group else None)
 
 
 @dataclass(frozen=True)

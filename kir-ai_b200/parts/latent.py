@@ -92,7 +92,7 @@ class LatentAttention(Mixer):
         self.q_norm = self.kv_norm = None
 
     def cache_need(self) -> KVCacheNeed:
-        return KVCacheNeed(1, self.pad_dim, None, key_dim=self.row, value_dim=self.kv_rank)
+        return KVCacheNeed(1, self.pad_dim, None, key_dim=self.row, value_dim=self.kv_rank, group=self.heads)
 
     @property
     def capture_safe(self) -> bool:

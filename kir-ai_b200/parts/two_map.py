@@ -49,7 +49,8 @@ class TwoMapAttention(Mixer):
         self.factor = None  # lambda
 
     def cache_need(self) -> KVCacheNeed:
-        return KVCacheNeed(self.kv_heads, self.pad_dim, None, key_dim=2 * self.head_dim, value_dim=self.value_dim)
+        return KVCacheNeed(self.kv_heads, self.pad_dim, None, key_dim=2 * self.head_dim, value_dim=self.value_dim,
+                           group=2 * self.heads // self.kv_heads)
 
     def weight_specs(self) -> Dict[str, WeightSpec]:
         return {**self.qkv.weight_specs(), **self.out.weight_specs(),

@@ -227,6 +227,46 @@ def test_products_with_chosen_experts_are_taken_where_they_were_measured_faster(
     assert not linear_chosen_pays(1, 8, 0.125, 2048, 64, 8 * 2 * 128 * 64 * 2, False)  # a small layer has nothing to save
 
 
+def test_captured_steps_plan_for_the_heads_that_the_layers_have():
+    """A captured step of more pairs than SMs takes the plan that an eager one takes: the crowd's kernel only where it serves the
+    layers' groups and heads, and beside layers that it does not serve the plan that those would have without it."""
+    from types import SimpleNamespace
+
+    import kirai_b200  # noqa: F401
+    from kirai_b200.csrc import ops
+    from kirai_b200.engine.graphs import DecodeGraphs
+    from kirai_b200.parts.attention import GQAttention
+    from kirai_b200.parts.base import KVCacheNeed
+
+    fake_ops = SimpleNamespace(decode_plan=ops.decode_plan, decode_crowd_plan=ops.decode_crowd_plan,
+                               decode_crowd_serves=getattr(ops, "decode_crowd_serves", None), sm_count=lambda device: 148,
+                               decode_cluster_room=lambda device, head_dim, group=4: (lambda cluster: 148 // cluster))
+
+    def plan(needs, lens):
+        cache = CacheManager(needs, page_size=16, num_pages=4, num_slots=1, device=None)
+        graphs = DecodeGraphs(SimpleNamespace(rt=SimpleNamespace(ops=fake_ops, device="cuda:0"), cache=cache))
+        return graphs._plan(lens)
+
+    def attention(q_heads, kv_heads, head_dim, **more):
+        return GQAttention("", 64, q_heads, kv_heads, head_dim, None, **more).cache_need()
+
+    lens = [100 + 3000 * i // 63 for i in range(64)]
+    crowd = ops.decode_crowd_plan(lens, 8)
+    assert crowd is not None and ops.decode_plan(lens, 4)[0] is True
+    assert plan([attention(32, 8, 128)] * 3, lens) == (False, 0, crowd)
+    assert plan([attention(64, 4, 128)], lens) == (True, 0, None)            # 16 query heads to a kv head
+    assert plan([attention(32, 8, 128), attention(32, 8, 256)], lens)[2] == crowd
+    for other in (attention(128, 8, 128, window=4096), attention(16, 8, 256, window=4096), attention(8, 1, 128, window=4096)):
+        both = plan([attention(32, 8, 128), other], lens)
+        assert both == ((True, 0, crowd) if ops.decode_plan(lens, 8)[0] else (False, ops.decode_plan(lens, 8)[1], crowd))
+    assert plan([attention(32, 8, 128), attention(128, 8, 128)], lens)[2] is None  # one pool, the larger group counts
+    shared = attention(32, 8, 128).also_read_by(attention(128, 8, 128))                # a layer that reads another's pages
+    assert shared == attention(32, 8, 128) and shared.group == 16 and plan([shared], lens)[2] is None
+    assert attention(32, 8, 128).also_read_by(KVCacheNeed(8, 128, None)).group is None
+    assert plan([KVCacheNeed(8, 128, None)], lens)[2] is None                # a mixer that does not say its group
+    assert plan([attention(32, 8, 128)], [1000] * 18) == (False, ops.decode_plan([1000] * 18, 8)[1], None)
+
+
 def test_decode_plan_over_random_batches_respects_the_kernels_limits():
     """Whatever the batch, the planner names a split count that the decode kernel takes (1 to 64 ranges, never more
     ranges than key tiles), and ranges are merged inside the kernel only where the device said the clusters fit and
