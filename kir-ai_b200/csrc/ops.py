@@ -891,19 +891,21 @@ def _state_chunked(batch, state_rows: int, walk_limit: Optional[int]) -> bool:
 
 def _state_side(batch, tokens: int, heads: int, groups: int, rows: int, cols: int, normaliser: bool, device, chain_limit: Optional[int]):
     """(units, state, normaliser, marks, scores): the buffers of a step whose chunks run side by side, or (0, None, None, None,
-    None); ``scores`` (queries times keys of a chunk, ``groups`` sets of them) only for sizes that can be read in 16 bytes."""
+    None); ``scores`` (queries times keys of a chunk, ``groups`` sets of them) only for sizes that can be read in 16 bytes, and where
+    the limit takes them beside the states (with narrow heads they are the greater part: 16 times the states at 16 x 16)."""
     fn = library().kirai_state_chunk_tokens
     fn.restype = ctypes.c_int
     chunk = int(fn())
     units = tokens // chunk + batch.num_requests
     limit = STATE_CHAIN_LIMIT if chain_limit is None else chain_limit
-    if batch.max_query_len <= limit or units * heads * rows * cols * 4 > STATE_SIDE_BYTES:
+    state_bytes = units * heads * rows * cols * 4
+    if batch.max_query_len <= limit or state_bytes > STATE_SIDE_BYTES:
         return 0, None, None, None, None
     state = torch.empty((units, heads, rows, cols), dtype=torch.float32, device=device)
     norm = torch.empty((units, heads, rows), dtype=torch.float32, device=device) if normaliser else None
     marks = torch.empty((units, heads, 3), dtype=torch.float32, device=device)
     scores = None
-    if rows % 4 == 0 and cols % 4 == 0:
+    if rows % 4 == 0 and cols % 4 == 0 and state_bytes + units * groups * chunk * chunk * 4 <= STATE_SIDE_BYTES:
         scores = torch.empty((units, groups, chunk, chunk), dtype=torch.float32, device=device)
     return units, state, norm, marks, scores
 

@@ -990,6 +990,27 @@ def test_command_line_generates(tiny):
     assert json.loads(result.stdout.strip().splitlines()[-1])["token_ids"] == expected
 
 
+@pytest.mark.parametrize("heads,groups,d,dv", [(128, 1, 128, 64), (16, 16, 128, 256), (64, 64, 32, 32), (64, 64, 16, 16), (8, 8, 4, 4), (8, 8, 6, 5)])
+def test_buffers_of_chunks_side_by_side_stay_within_their_limit(heads, groups, d, dv):
+    """States and scores together, at step sizes around the limit of each: the scores are left out first (the kernels for any
+    address, which need none, then run), and where the states alone are too many there are no buffers at all."""
+    from types import SimpleNamespace
+    from kirai_b200.csrc import ops
+
+    chunk, limit, seen = 64, ops.STATE_SIDE_BYTES, set()
+    state, scores = heads * d * dv * 4, groups * chunk * chunk * 4  # bytes of a unit
+    for units in (3, limit // (state + scores), limit // (state + scores) + 1, limit // state, limit // state + 1):
+        batch = SimpleNamespace(num_requests=1, max_query_len=1 << 30)
+        got = ops._state_side(batch, (units - 1) * chunk, heads, groups, d, dv, False, "meta", 0)
+        assert got[0] in (0, units)
+        held = sum(t.numel() * 4 for t in (got[1], got[4]) if t is not None)
+        assert held <= limit
+        assert (got[0] > 0) == (units * state <= limit)
+        assert (got[4] is not None) == (d % 4 == 0 and dv % 4 == 0 and units * (state + scores) <= limit)
+        seen.add((got[0] > 0, got[4] is not None))
+    assert seen == ({(True, True), (True, False), (False, False)} if d % 4 == 0 and dv % 4 == 0 else {(True, False), (False, False)})
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("heads,groups,d,dv", [(6, 2, 128, 64), (2, 1, 256, 72), (1, 1, 4, 4), (3, 3, 132, 132)])
 @pytest.mark.parametrize("memory", [False, True])
