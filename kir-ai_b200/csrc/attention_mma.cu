@@ -1026,7 +1026,8 @@ __device__ __forceinline__ void decode_init_barriers(uint8_t* smem) {
 }
 
 // The request with the n-th longest context (the lower index first among equal ones), found by the whole block; `lens`:
-// `requests` ints (rounded up to four) of shared memory on a 16-byte boundary that nobody uses yet.
+// `requests` ints (rounded up to four) of shared memory on a 16-byte boundary that nobody uses yet and that TMA never
+// writes (ordinary stores and reads there would need a proxy fence before TMA's).
 __device__ __forceinline__ int nth_longest(const int* __restrict__ context_len, int requests, int n, int* lens) {
     __shared__ int found;
     const int padded = (requests + 3) & ~3;
@@ -1075,8 +1076,11 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, DecodeArgs a
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const int split = blockIdx.x, kv_head = blockIdx.y;
-    const int req = !PAIR && args.longest_first ? nth_longest(context_len, gridDim.z, blockIdx.z, reinterpret_cast<int*>(smem + Smem::q_bytes))
-                                                : (int)blockIdx.z;
+    // (the lengths lie where the block table will)
+    static_assert(DECODE_MAX_SORTED <= Smem::table_entries && (Smem::body + Smem::DC_WARPS * DC_STAGES * 8) % 16 == 0, "room for the lengths");
+    const int req = !PAIR && args.longest_first
+                        ? nth_longest(context_len, gridDim.z, blockIdx.z, reinterpret_cast<int*>(smem + Smem::body + Smem::DC_WARPS * DC_STAGES * 8))
+                        : (int)blockIdx.z;
     const int group = args.q_heads / args.kv_heads;
     const int pos = context_len[req] - 1;
     const int keep = mask_keep(args.window);

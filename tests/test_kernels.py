@@ -1024,3 +1024,25 @@ def test_decode_attention_of_crowds(ops, q_heads, kv_heads, head_dim, page_size,
             # weights and result are rounded to bfloat16 (2^-9 each) on values of up to about 4
             assert float((got.float() - plain).abs().max()) <= 2.5e-2, (warps, splits)
     ops.check_device_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("requests,kv_heads,head_dim", [(511, 1, 64), (512, 2, 128), (203, 4, 128)])
+def test_decode_attention_of_the_largest_crowds(ops, requests, kv_heads, head_dim):
+    """As many requests as a launch orders by length, and numbers that are no multiple of four; many of equal length.  Every request
+    has to be attended once, whatever the place of its length in shared memory."""
+    generator = torch.Generator().manual_seed(requests)
+    lengths = torch.randint(1, 80, (requests,), generator=generator).tolist()
+    cache, table, keys, values = paged_setup(torch.bfloat16, lengths, kv_heads, head_dim, 16, seed=6)
+    for r, n in enumerate(lengths):
+        ops.kv_write(keys[r].to(DEV).contiguous(), values[r].to(DEV).contiguous(), cache, table,
+                     torch.full((n,), r, dtype=torch.int32, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV))
+    q = rand(requests, 2 * kv_heads, head_dim, dtype=torch.bfloat16, scale=2.0)
+    scale, context = head_dim ** -0.5, torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    plain = ops.paged_attention_plain(q.float(), cache.float(), table, torch.arange(requests, dtype=torch.int32, device=DEV), context - 1,
+                                      None, scale)
+    for warps, splits in ((4, 1), (8, 1), (4, 2)):
+        for _ in range(3):
+            got = ops.attention_decode_crowd(q, cache, table, context, None, scale, splits, warps)
+            # weights and result are rounded to bfloat16 (2^-9 each) on values of up to about 4
+            assert float((got.float() - plain).abs().max()) <= 2.5e-2, (warps, splits)
+    ops.check_device_errors(torch.device(DEV))
