@@ -1754,6 +1754,8 @@ def decode_crowd_plan(context_lens, kv_heads: int, reach: Optional[int] = None, 
     for warps, splits in ((8, 1), (4, 1), (4, 2), (4, 3)):
         slots = (sms if warps == 8 else 2 * sms) // kv_heads  # a request's heads are alike: in units of requests
         per_round, fixed = (1.27, 4.4) if warps == 8 else (1.07, 7.1)
+        if max(-(-tiles[0] // (splits * warps)) * per_round + fixed, bytes_us) + (0.0 if splits == 1 else 4.0) >= best_us:
+            continue  # (the longest request alone rules the form out)
         costs = [-(-t // (splits * warps)) * per_round + fixed for t in tiles]  # of each of a request's ranges, longest first
         us = max(costs[0], splits * sum(costs) / slots, bytes_us)
         for k in range(1, (splits * requests - 1) // slots + 1):
@@ -1805,6 +1807,24 @@ def paged_attention(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Ten
                              chunk=chunk, softcap=softcap, keep_first=keep_first, sinks=sinks)
 
 
+def _decode_choice(batch, rows: int, kv_heads: int, reach: Optional[int], sms: int, room, head_dim: int, group: int) -> tuple:
+    """(crowd, balanced, longest context) of the first ``rows`` requests of a step that runs eagerly.  Layers alike get the same
+    answer, which the step's batch keeps: the plans walk all requests in Python, 40 us at 64 of them, and a model has dozens
+    of layers (a batch that keeps nothing is planned anew each time)."""
+    lens = [start + count for start, count in zip(batch.start_positions[:rows], batch.query_lens[:rows])]
+    plans = getattr(batch, "decode_plans", None)
+    key = (rows, kv_heads, reach, sms, head_dim, group)
+    known = plans.get(key) if plans is not None else None
+    if known is not None and known[0] == lens:
+        return known[1]
+    crowd = decode_crowd_plan(lens, kv_heads, reach, sms=sms, head_dim=head_dim, group=group)
+    balanced = False if crowd else decode_plan(lens, kv_heads, reach, sms=sms, room=room, head_dim=head_dim, group=group)[0]
+    choice = (crowd, balanced, max(lens))
+    if plans is not None:
+        plans[key] = (lens, choice)
+    return choice
+
+
 def _decode_rows(q, cache, block_table, batch, rows: int, window: Optional[int], scale: float, out: torch.Tensor,
                  chunk: Optional[int] = None, softcap: Optional[float] = None, keep_first: int = 0,
                  sinks: Optional[torch.Tensor] = None) -> None:
@@ -1822,11 +1842,7 @@ def _decode_rows(q, cache, block_table, batch, rows: int, window: Optional[int],
     crowd = getattr(batch, "decode_crowd", None)
     longest = batch.max_context_len
     if balanced is None:
-        lens = [start + count for start, count in zip(batch.start_positions[:rows], batch.query_lens[:rows])]
-        crowd = decode_crowd_plan(lens, kv_heads, reach, sms=sm_count(q.device), head_dim=q.shape[2], group=q.shape[1] // kv_heads)
-        balanced = False if crowd else decode_plan(lens, kv_heads, reach, sms=sm_count(q.device), room=room, head_dim=q.shape[2],
-                                                   group=q.shape[1] // kv_heads)[0]
-        longest = max(lens)
+        crowd, balanced, longest = _decode_choice(batch, rows, kv_heads, reach, sm_count(q.device), room, q.shape[2], q.shape[1] // kv_heads)
     forced = os.environ.get("KIRAI_DECODE_BALANCED")
     if forced in ("0", "1"):
         balanced, crowd = forced == "1", None

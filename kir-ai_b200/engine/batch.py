@@ -55,6 +55,8 @@ class StepBatch:
     # for layers of more (request, kv head) pairs than SMs: (warps of a CTA, ranges), see ops.decode_crowd_plan (None: not such a
     # batch); layers that ops.decode_crowd_serves does not name take the two above
     decode_crowd: Optional[tuple] = None
+    # how the step's single tokens are attended, worked out once for all layers alike: (rows, heads and reach) -> (lengths, plan)
+    decode_plans: dict = field(default_factory=dict)
 
     @property
     def decode_only(self) -> bool:

@@ -267,6 +267,34 @@ def test_captured_steps_plan_for_the_heads_that_the_layers_have():
     assert plan([attention(32, 8, 128)], [1000] * 18) == (False, ops.decode_plan([1000] * 18, 8)[1], None)
 
 
+def test_a_step_plans_its_decode_attention_once_for_layers_alike(monkeypatch):
+    """Layers of the same heads and reach share one plan of the step; other heads, another reach and changed lengths are
+    planned for themselves, and the answers are those of the plans."""
+    from types import SimpleNamespace
+
+    from kirai_b200.csrc import ops
+
+    calls = []
+    crowd_plan, plan = ops.decode_crowd_plan, ops.decode_plan
+    monkeypatch.setattr(ops, "decode_crowd_plan", lambda *a, **k: calls.append("crowd") or crowd_plan(*a, **k))
+    monkeypatch.setattr(ops, "decode_plan", lambda *a, **k: calls.append("plan") or plan(*a, **k))
+    room = lambda cluster: 148 // cluster  # noqa: E731
+    for lens in ([1000] * 32, [200_000] + [100] * 30, [700, 900]):
+        batch = SimpleNamespace(start_positions=[n - 1 for n in lens] + [5], query_lens=[1] * len(lens) + [9], decode_plans={})
+        crowd = crowd_plan(lens, 8)
+        expected = (crowd, False if crowd else plan(lens, 8, room=room)[0], max(lens))
+        calls.clear()
+        for _ in range(36):
+            assert ops._decode_choice(batch, len(lens), 8, None, 148, room, 128, 4) == expected
+        assert len(calls) <= 2
+        assert ops._decode_choice(batch, len(lens), 8, 64, 148, room, 128, 4)[0] == crowd_plan(lens, 8, 64)
+        assert ops._decode_choice(batch, len(lens), 2, None, 148, room, 256, 16) == (None, plan(lens, 2, room=room, head_dim=256, group=16)[0], max(lens))
+        batch.start_positions[0] += 100_000
+        assert ops._decode_choice(batch, len(lens), 8, None, 148, room, 128, 4)[2] == lens[0] + 100_000
+        del batch.decode_plans
+        assert ops._decode_choice(batch, len(lens), 8, None, 148, room, 128, 4)[2] == lens[0] + 100_000
+
+
 def test_decode_plan_over_random_batches_respects_the_kernels_limits():
     """Whatever the batch, the planner names a split count that the decode kernel takes (1 to 64 ranges, never more
     ranges than key tiles), and ranges are merged inside the kernel only where the device said the clusters fit and
