@@ -120,7 +120,7 @@ template <int BN>
 __global__ void __launch_bounds__(THREADS, Shape<BN>::ctas)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const float* __restrict__ A,
                    const float* __restrict__ W, float* __restrict__ C, int M, int N, int K, long lda, long ldc, int blocks_per_split,
-                   int* __restrict__ error_flag) {
+                   int constant, int* __restrict__ error_flag) {
     using S = Shape<BN>;
     constexpr int WS = S::w_stages, AS = S::a_stages, HALF = BN / 2;
     extern __shared__ uint8_t smem_raw[];
@@ -247,7 +247,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
     } else if (warp == WORKERS) {
         if (elect_one()) {
-            // W does not depend on the kernel before this one
+            if (!constant) pdl_wait();  // constant weights do not depend on the kernel before this one, nor on the one before that
             int i = 0;
             for (; i < blocks; ++i) {
                 const int s = i % WS;
@@ -335,7 +335,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
 template <int BN>
 int launch_tc(const float* A, const float* W, const bf16* planes, float* C, int M, int N, int K, long lda, long ldc, int pitch, int splits,
-              int* error_flag, cudaStream_t stream) {
+              int constant, int* error_flag, cudaStream_t stream) {
     using S = Shape<BN>;
     CUtensorMap map_w, map_a;
     if (!tmap::matrix_boxes<0>(&map_w, W, (uint64_t)N, (uint64_t)K, (uint64_t)K, TILE_N)) return KIRAI_ERR_BAD_ALIGN;
@@ -346,7 +346,7 @@ int launch_tc(const float* A, const float* W, const bf16* planes, float* C, int 
     const int blocks = (K + BLOCK_K - 1) / BLOCK_K;
     const dim3 grid((unsigned)((N + TILE_N - 1) / TILE_N), (unsigned)((M + BN - 1) / BN), (unsigned)splits);
     return launch_pdl(kernel, grid, dim3(THREADS), (size_t)S::total, stream, (unsigned)splits, map_w, map_a, A, W, C, M, N, K, lda, ldc,
-                      (blocks + splits - 1) / splits, error_flag);
+                      (blocks + splits - 1) / splits, constant, error_flag);
 }
 
 }  // namespace
@@ -387,14 +387,15 @@ static Cut choose_cut(int M, int N, int K) {
 
 // planes: 3 M pitch bf16 of scratch, pitch = K rounded up to a multiple of 8.  K and the row stride of A multiples of 4, A, W
 // and planes on 16-byte boundaries.  bn 0: the cut is chosen here; else 32, 64, 128 or 192 rows of A to a tile and K over
-// `splits` CTAs (1 to 8).
+// `splits` CTAs (1 to 8).  constant: W is not written by the kernel ahead in the stream (weights of a loaded model), and is fetched
+// before that has finished.
 // Measured at 515 rows of the 4B shape's products (6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728): 80, 72,
 // 296 and 143 us (204, 150, 173 and 179 TFLOP/s of 32-bit arithmetic, six times that in the tensor cores), where the plain
 // kernel took 5.3 ms together (20 TFLOP/s).  2-norm of the error over that of the result, in 2^-24, here and in the plain kernel:
 // normal values 0.79 and 0.68 at K = 4, 0.80 and 1.24 at 16, 0.96 and 1.7 at 32, 1.7 and 15 at 2,560, 2.4 and 29 at 9,728; values of one
 // sign 0.90 and 0.60, 1.0 and 1.06, 1.0 and 1.4, 1.3 and 13, 1.3 and 26.
 KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_, void* C_, int M, int N, int K, long lda, long ldc,
-                                   int bn, int splits, int* error_flag, cudaStream_t stream) {
+                                   int bn, int splits, int constant, int* error_flag, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || (long)3 * M > 0x7fffffffL || splits < 0 || splits > 8) return KIRAI_ERR_BAD_SIZE;
     if (K % 4 != 0 || lda % 4 != 0 || (((uintptr_t)A_ | (uintptr_t)W_ | (uintptr_t)planes_) & 15) != 0) return KIRAI_ERR_BAD_ALIGN;
@@ -409,10 +410,10 @@ KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_
     if (status != 0) return status;
     float* C = (float*)C_;
     switch (cut.bn) {
-        case 32: return launch_tc<32>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, error_flag, stream);
-        case 64: return launch_tc<64>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, error_flag, stream);
-        case 128: return launch_tc<128>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, error_flag, stream);
-        case 192: return launch_tc<192>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, error_flag, stream);
+        case 32: return launch_tc<32>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+        case 64: return launch_tc<64>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+        case 128: return launch_tc<128>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+        case 192: return launch_tc<192>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
     }
     return KIRAI_ERR_BAD_SIZE;
 }

@@ -1938,14 +1938,16 @@ def linear_f32_rows_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
-def linear_f32_rows(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """float32 ``x`` [M, K] times ``weight`` [N, K] transposed for up to 8 rows, with 32-bit FMAs: the weights are streamed."""
+def linear_f32_rows(x: torch.Tensor, weight: torch.Tensor, constant: bool = False) -> torch.Tensor:
+    """float32 ``x`` [M, K] times ``weight`` [N, K] transposed for up to 8 rows, with 32-bit FMAs: the weights are streamed.
+    ``constant`` as in ``linear``."""
     _need_cuda(x, weight)
     assert x.dim() == 2 and weight.dim() == 2 and weight.is_contiguous() and weight.dtype == torch.float32
     assert x.shape[1] == weight.shape[1] and linear_f32_rows_takes(x, weight)
     m, k, n = x.shape[0], x.shape[1], weight.shape[0]
     out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-    _call("kirai_gemm_f32_rows", _ptr(x), _ptr(weight), _ptr(out), _i(m), _i(n), _i(k), _l(x.stride(0)), _l(n), _stream())
+    _call("kirai_gemm_f32_rows", _ptr(x), _ptr(weight), _ptr(out), _i(m), _i(n), _i(k), _l(x.stride(0)), _l(n), _i(int(constant)),
+          _stream())
     return out
 
 
@@ -1958,10 +1960,10 @@ def linear_f32_tc_takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
             and x.stride(1) == 1 and x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0)
 
 
-def linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, tile_rows: int = 0, splits: int = 0) -> torch.Tensor:
+def linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, tile_rows: int = 0, splits: int = 0, constant: bool = False) -> torch.Tensor:
     """float32 ``x`` [M, K] times ``weight`` [N, K] transposed on the tensor cores, every float as three bf16 values: from 32
     values of K on nearer to the exact product than 32-bit FMAs (``F32_TC_MIN_K``).  ``tile_rows`` (32, 64, 128 or 192) and ``splits`` (1 to 8) force how the product is
-    cut into CTAs; 0 leaves it to the kernel's rule."""
+    cut into CTAs; 0 leaves it to the kernel's rule.  ``constant`` as in ``linear``."""
     _need_cuda(x, weight)
     assert x.dim() == 2 and weight.dim() == 2 and weight.is_contiguous() and weight.dtype == torch.float32
     assert x.shape[1] == weight.shape[1] and linear_f32_tc_takes(x, weight)
@@ -1969,7 +1971,7 @@ def linear_f32_tc(x: torch.Tensor, weight: torch.Tensor, tile_rows: int = 0, spl
     out = torch.empty((m, n), dtype=torch.float32, device=x.device)
     planes = torch.empty((3, m, (k + 7) // 8 * 8), dtype=torch.bfloat16, device=x.device)
     _call("kirai_gemm_f32_tc", _ptr(x), _ptr(weight), _ptr(planes), _ptr(out), _i(m), _i(n), _i(k), _l(x.stride(0)), _l(n),
-          _i(tile_rows), _i(splits), _ptr(error_flag(x.device)), _stream())
+          _i(tile_rows), _i(splits), _i(int(constant)), _ptr(error_flag(x.device)), _stream())
     return out
 
 
@@ -2237,20 +2239,22 @@ def interleave_gate_up(gate: torch.Tensor, up: torch.Tensor) -> torch.Tensor:
     return torch.stack([gate.view(inter // 8, 8, k), up.view(inter // 8, 8, k)], dim=1).reshape(2 * inter, k).contiguous()
 
 
-def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None, constant: bool = False) -> torch.Tensor:
     """The linear layer of the product path: for float32, where rows can be read 16 bytes at a time, a kernel that streams
     the weights (up to 8 rows) or products of values cut in three on the tensor cores (sums of 32 values and more), else the
     plain kernel: a row's last bits depend on how many rows stand beside it; for bfloat16 the tcgen05 kernel, or the
-    CUDA-core kernel when K is not a multiple of 8 (TMA cannot read such rows)."""
+    CUDA-core kernel when K is not a multiple of 8 (TMA cannot read such rows).  ``constant``: no kernel still under way
+    writes the weight (it belongs to a loaded model), so that float32 products may fetch it before the kernel ahead in
+    the stream has finished, as the tcgen05 kernel does with any weight."""
     if isinstance(weight, TiledWeight):
         return linear_tcgen05(x if tcgen05_takes(x) else x.contiguous(), weight, out_dtype)
     if tcgen05_takes(x):
         return linear_tcgen05(x, weight, out_dtype)
     if weight.dtype == torch.float32 and out_dtype in (None, torch.float32):
         if linear_f32_rows_takes(x, weight):
-            return linear_f32_rows(x, weight)
+            return linear_f32_rows(x, weight, constant)
         if x.shape[1] >= F32_TC_MIN_K and linear_f32_tc_takes(x, weight):
-            return linear_f32_tc(x, weight)
+            return linear_f32_tc(x, weight, constant=constant)
     return linear_plain(x, weight, out_dtype)
 
 

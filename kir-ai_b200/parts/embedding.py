@@ -122,5 +122,5 @@ class OutputHead(Part):
         self.weight = _table(weights, rt, self.weight_name, self.hidden_size)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        logits = self.rt.ops.linear(x, self.weight, torch.float32)
+        logits = self.rt.ops.linear(x, self.weight, torch.float32, constant=True)
         return self.rt.ops.softcap_(logits, self.softcap) if self.softcap else logits

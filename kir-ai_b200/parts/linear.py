@@ -79,7 +79,7 @@ class Linear(Part):
     def forward(self, x, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
         if isinstance(x, UnscaledNorm):
             return self.rt.ops.linear_tcgen05(x.rows, self.weight, out_dtype, row_scale=x.row_scale())
-        return self.rt.ops.linear(x, self.weight, out_dtype)
+        return self.rt.ops.linear(x, self.weight, out_dtype, constant=True)
 
     # Largest batch for which a norm is folded into the products around it: every batch that the weight-streaming
     # products take.  Measured on the 8B layer sizes (ms a decode step, folded against separate): one request 4 %

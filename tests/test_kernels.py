@@ -163,6 +163,25 @@ def test_linear_float32_on_tensor_cores(ops, m, n, k):
         ops.linear_f32_tc(rand(m, k + 9)[:, 1 : 1 + k], w)
 
 
+@pytest.mark.parametrize("m", [1, 8, 40, 200])
+def test_linear_float32_reads_weights_that_the_kernel_before_it_wrote(ops, m):
+    """A weight made by the launch just ahead in the stream, one after the other in the same memory; and the same bits from
+    weights that are said to be constant, once they are."""
+    x, base = rand(m, 1024), rand(4096, 1024, seed=2)
+    w = torch.empty_like(base)
+    factors = [2.0 ** (i % 7 - 3) for i in range(40)]
+    results = []
+    for factor in factors:
+        torch.mul(base, factor, out=w)
+        results.append(ops.linear(x, w))
+    torch.cuda.synchronize()
+    want = ops.linear(x, base, constant=True)
+    assert torch.equal(want, ops.linear(x, base))
+    for factor, got in zip(factors, results):
+        assert torch.equal(got, want * factor)  # (powers of two: every rounding is the same)
+    ops.check_device_errors(torch.device(DEV))
+
+
 @pytest.mark.parametrize("k", [4, 8, 16, 32])
 def test_linear_float32_on_tensor_cores_leaves_out_less_than_a_rounding(ops, k):
     """Products of one sign, where what is left out cannot cancel: mantissas whose second and third cuts would be the greatest
