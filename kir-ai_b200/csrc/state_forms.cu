@@ -44,7 +44,7 @@ __global__ void add_dyt_kernel(float* __restrict__ resid, const float* __restric
 
 // The same with 16-byte accesses, four adjacent columns a thread: nothing is summed over a row, so a row goes over as many
 // blocks as it has 1,024 columns (one block per row, 16 dependent rounds of 4 bytes a thread, took 10.6 us a launch at three rows of
-// 4,096; 2.1 us now).  The weights are asked for before the kernel before this one has finished.
+// 4,096; 2.1 us now).
 template <typename O>
 __device__ __forceinline__ void store_four(O* to, const float (&v)[4]);
 template <>
@@ -61,10 +61,10 @@ __global__ void __launch_bounds__(256) add_dyt_vec_kernel(float* __restrict__ re
                                                           const int* __restrict__ row_index, int width) {
     pdl_launch_dependents();
     const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
-    if (c >= width) return pdl_wait();
+    pdl_wait();
+    if (c >= width) return;
     const float a = alpha[0];
     const float4 wv = *reinterpret_cast<const float4*>(w + c), bv = *reinterpret_cast<const float4*>(b + c);
-    pdl_wait();
     const long row = blockIdx.x;
     const long src = row_index ? row_index[row] : row;
     float4 v = *reinterpret_cast<const float4*>(resid + src * width + c);

@@ -1083,6 +1083,13 @@ def test_sums_under_a_tanh_and_pairs_of_normed_rows_from_aligned_rows(rows, widt
                     assert float((got.double().cpu() - want).abs().max()) <= bound
                     left = total if index is None else resid.double()
                     assert float((stream.double().cpu() - left).abs().max()) <= 8.0 * 2.0 ** -22
+        # weights that the launch just ahead in the stream wrote
+        scaled, gain, offset = placed(resid, shift), placed(w, shift), placed(b, shift)
+        for factor in (2.0, 0.25, 2.0):
+            gain.mul_(factor), offset.mul_(factor)
+            got = ops.add_dyt(scaled, [None, None], 0.5, alpha.cuda(), gain, offset, torch.float32, None)
+        want = torch.tanh(0.7 * resid.double()) * w.double() + b.double()
+        assert float((got.double().cpu() - want).abs().max()) <= 8.0 * 2.0 ** -20
         got = ops.rms_pair_mean(placed(d1, shift), placed(d2, shift), placed(w, shift), placed(b, shift), 1e-6).double().cpu()
         unit = lambda x: x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-6)  # noqa: E731
         assert float((got - 0.5 * (unit(d1) * w.double() + unit(d2) * b.double())).abs().max()) <= 16.0 * 2.0 ** -19
