@@ -17,7 +17,8 @@
 // columns.  The warp's sums for all (head, key) pairs are made by one transposing butterfly, 31 shuffles for 32 sums, after
 // which a lane owns one score; weights go back by shuffles.  Bound by the latency of the loads (4 requests of about 106 tokens:
 // 6.4 us a layer, plain kernel 23); long contexts are cut over
-// a cluster of CTAs that merge through distributed shared memory, one CTA per 128 keys and at most eight.
+// a cluster of CTAs that merge through distributed shared memory, one CTA per 128 keys and at most eight, and as many as run
+// at once: the order of a request's sums, and so its last bits, follow the number of requests and the longest of them.
 #include "common.cuh"
 
 #define AF_ROWS 64

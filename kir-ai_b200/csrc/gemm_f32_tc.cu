@@ -389,8 +389,8 @@ static Cut choose_cut(int M, int N, int K) {
 // and planes on 16-byte boundaries.  bn 0: the cut is chosen here; else 32, 64, 128 or 192 rows of A to a tile and K over
 // `splits` CTAs (1 to 8).  constant: W is not written by the kernel ahead in the stream (weights of a loaded model), and is fetched
 // before that has finished.
-// Measured at 515 rows of the 4B shape's products (6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728): 80, 72,
-// 296 and 143 us (204, 150, 173 and 179 TFLOP/s of 32-bit arithmetic, six times that in the tensor cores), where the plain
+// Measured at 515 rows of the 4B shape's products (6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728): 81, 71,
+// 298 and 147 us (201, 152, 172 and 174 TFLOP/s of 32-bit arithmetic, six times that in the tensor cores), where the plain
 // kernel took 5.3 ms together (20 TFLOP/s).  2-norm of the error over that of the result, in 2^-24, here and in the plain kernel:
 // normal values 0.79 and 0.68 at K = 4, 0.80 and 1.24 at 16, 0.96 and 1.7 at 32, 1.7 and 15 at 2,560, 2.4 and 29 at 9,728; values of one
 // sign 0.90 and 0.60, 1.0 and 1.06, 1.0 and 1.4, 1.3 and 13, 1.3 and 26.

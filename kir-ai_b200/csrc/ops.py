@@ -1742,9 +1742,10 @@ def decode_crowd_plan(context_lens, kv_heads: int, reach: Optional[int] = None, 
     the second kernel.  CTAs come longest first, so the launch ends close to the greatest of these lower bounds: the longest
     CTA; the sum over the slots; for every k the k + 1 shortest of the k * slots + 1 longest (some slot has k + 1 of them);
     and the bytes.  Against measurements of 29 batches of 18 to 64 requests (8 kv heads of 128, contexts of 20 to 20,000
-    tokens) the times come out within a tenth.  In us, 1,000 tokens each: 32 requests 37 with 8 warps and 31 with 4 (floor 20),
-    48 of 1,300 tokens 64 and 66 (39); 20 of 500 to 3,000 tokens 41 and 61, two ranges 51 and 44 (25).  The
-    balanced kernel: 42, 63, 47, and 97 at 64 requests of 131 to 1,500 tokens, where 4 warps take 47."""
+    tokens), each launch timed alone, the times come out within a tenth.  Launches back to back in a graph, as a step has them,
+    take some 7 us less, and the order among the forms is the same: 32 requests of 1,000 tokens 30 us with 8 warps, 24 with 4, 33 with 4
+    in two ranges (bytes: 20), 48 of 1,300 tokens 54, 58, 58 (39), 20 of 500 to 3,000 tokens 31, 52, 34 (22), 64 of 131 to 1,500
+    tokens 51, 40, 57 (33); the balanced kernel 34, 55, 39 and 70 to 101 (as the requests lie)."""
     requests = len(context_lens)
     if not decode_crowd_serves(requests, kv_heads, head_dim, group, sms):
         return None
