@@ -43,6 +43,8 @@ using namespace sm100;
 #define GEMM_BK 64
 #define GEMM_THREADS 192
 #define GEMM_BOX_BYTES (GEMM_BM * GEMM_BK * 2)  // one box of tiled weights
+#define GEMM_BARRIER_BYTES 2048                 // persistent kernel: barriers behind the ring
+#define GEMM_MAX_STAGES 12                      // persistent kernel: the longest ring
 
 // Shared memory of one CTA: the ring of stages, the barriers, then (only with split-K) one slot
 // per CTA of the cluster for the partial tiles.  The swapped, weight-streaming case (BN <= 64)
@@ -756,9 +758,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
 // ---------------------------------------------------------------- many tokens: persistent kernel
 // One CTA per SM walks tiles t = blockIdx.x, + gridDim.x, ... (token tile fastest, so CTAs that
-// run side by side share a weight tile in L2).  Tensor memory holds two accumulators of BN
-// columns: while the epilogue warps read one back, convert and store it, the MMA thread already
-// fills the other with the next tile, and the TMA warp runs ahead across tile borders.
+// run side by side share a weight tile in L2).  A tile is 128 or 256 rows by `width` columns, whatever the
+// launch found best (`persistent_tile`).  Tensor memory holds two accumulators.  Tiles of 128 rows take turns with
+// them: while the epilogue warps read one back, convert and store it, the MMA thread already
+// fills the other with the next tile, and the TMA warp runs ahead across tile borders.  A tile of 256 rows uses
+// both, one for each half of its rows, which share the weights in shared memory (a third less from L2 a product); four epilogue warps a
+// half take it to registers at once, and the next tile's products follow half by half.
+// What bounds it: on many full rounds the power cap (8B gate/up at 2,048 tokens, 1.39 PFLOP/s sustained where cuBLAS ran
+// at 1.30; products without loads 246 us, loads without products 169, both 297), on few the last round.  A second load
+// thread made no difference (300 us).
 // Tried and taken out: the last wave shared out evenly (its tiles' k-blocks cut into one range per SM, partial tiles
 // through a workspace, summed in the order of the ranges by the CTA that counts last).  Even with the sums left out
 // the 8B shapes at 2,048 tokens gained 0 to 4 % (q, k, v 99 to 95 us, o 72 to 71, gate/up 283 to 282, down 166 to
@@ -837,24 +845,25 @@ __device__ __forceinline__ void epilogue_residual_norm_coalesced(const Epilogue&
     }
 }
 
-template <int BN, typename OutT, int EPI>
-__global__ void __launch_bounds__(GEMM_THREADS, 1)
+template <int MT, typename OutT, int EPI>
+__global__ void __launch_bounds__(64 + 128 * MT, 1)
 gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                                const uint8_t* __restrict__ w_tiled, OutT* __restrict__ C, int M, int N, int K, long ldc,
-                               Epilogue ep, int* __restrict__ error_flag) {
-    using Smem = GemmSmem<BN>;
-    constexpr int STAGES = Smem::stages;
+                               int width, int stages, Epilogue ep, int* __restrict__ error_flag) {
+    static_assert(MT == 1 || EPI != 2, "the residual-and-norm epilogue is built for tiles of 128 rows");
+    constexpr int ROWS = MT * GEMM_BM, X_BYTES = MT * GEMM_BOX_BYTES;
+    const int stage_bytes = X_BYTES + width * (GEMM_BK * 2);
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = (uint64_t*)(smem + STAGES * Smem::stage_bytes);
-    uint64_t* full_bar = bars;                    // [STAGES] TMA -> MMA
-    uint64_t* empty_bar = bars + STAGES;          // [STAGES] MMA -> TMA
-    uint64_t* acc_full = bars + 2 * STAGES;       // [2] MMA -> epilogue
-    uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA
-    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
+    uint64_t* bars = (uint64_t*)(smem + stages * stage_bytes);
+    uint64_t* full_bar = bars;                         // [stages] TMA -> MMA
+    uint64_t* empty_bar = bars + GEMM_MAX_STAGES;      // [stages] MMA -> TMA
+    uint64_t* acc_full = bars + 2 * GEMM_MAX_STAGES;   // [2] MMA -> epilogue, one per accumulator
+    uint64_t* acc_empty = acc_full + 2;                // [2] epilogue -> MMA
+    uint32_t* tmem_slot = (uint32_t*)(acc_full + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m_tiles = (M + GEMM_BM - 1) / GEMM_BM, n_tiles = (N + BN - 1) / BN;
+    const int m_tiles = (M + ROWS - 1) / ROWS, n_tiles = (N + width - 1) / width;
     const int total_tiles = m_tiles * n_tiles;
     const int num_kb = (K + GEMM_BK - 1) / GEMM_BK;
     pdl_launch_dependents();
@@ -862,18 +871,18 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
     if (threadIdx.x == 0) {
         tma_prefetch_descriptor(&map_x);
         tma_prefetch_descriptor(&map_y);
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(smem_addr(&full_bar[s]), 1);
             mbar_init(smem_addr(&empty_bar[s]), 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_addr(&acc_full[b]), 1);
-            mbar_init(smem_addr(&acc_empty[b]), 4);  // one arrival per epilogue warp
+            mbar_init(smem_addr(&acc_empty[b]), 4);  // one arrival per epilogue warp of the accumulator
         }
         mbar_fence_init();
     }
     if (warp == 1) {
-        tmem_alloc(smem_addr(tmem_slot), 2 * tmem_columns<BN>());
+        tmem_alloc(smem_addr(tmem_slot), 512);  // two accumulators, 256 columns apart
         tmem_relinquish();
     }
     tc_fence_before();
@@ -884,8 +893,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
 
     if (warp == 0) {
         if (elect_one()) {
-            // Walks this CTA's (tile, k-block) sequence and the ring of stages with counters only: this thread's
-            // issue rate bounds the kernel, and a division per k-block showed in the product's time.
+            // Walks this CTA's (tile, k-block) sequence and the ring of stages with counters only.
             struct Cursor {
                 int t, kb, stage, m_tile, n_tile;
                 uint32_t round;  // how often the ring has wrapped
@@ -902,27 +910,36 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
             };
             auto advance = [&](Cursor& c) {
                 if (++c.kb == num_kb) { c.kb = 0, c.t += (int)gridDim.x; place(c); }
-                if (++c.stage == STAGES) { c.stage = 0, ++c.round; }
+                if (++c.stage == stages) { c.stage = 0, ++c.round; }
             };
             const int row_tiles = (N + GEMM_BM - 1) / GEMM_BM;
             auto issue = [&](const Cursor& c, bool weights, bool activations) {
                 const uint32_t full = smem_addr(&full_bar[c.stage]);
-                const uint32_t dst = smem_addr(smem + c.stage * Smem::stage_bytes);
+                const uint32_t dst = smem_addr(smem + c.stage * stage_bytes);
+                // (rows of A past the last one: a whole half of the tile is left out, a part of one reads zeros)
+                const bool second = MT == 2 && c.m_tile * ROWS + GEMM_BM < M;
+                const uint32_t x_bytes = second ? 2 * GEMM_BOX_BYTES : GEMM_BOX_BYTES;
                 if (weights && w_tiled) {
-                    // BN / 128 boxes of 128 weight rows, stacked as the MMA reads them; a box past the last row
-                    // tile is left out (its columns of the accumulator are never stored)
-                    const int first = c.n_tile * (BN / GEMM_BM);
-                    const int boxes = min(BN / GEMM_BM, row_tiles - first);
-                    mbar_expect_tx(full, Smem::x_bytes + boxes * GEMM_BOX_BYTES);
-                    const uint8_t* src = w_tiled + ((size_t)(first + c.group * row_tiles) * num_kb + c.kb) * GEMM_BOX_BYTES;
-                    for (int b = 0; b < boxes; ++b)
-                        bulk_load_1d(dst + Smem::x_bytes + b * GEMM_BOX_BYTES, src + (size_t)b * num_kb * GEMM_BOX_BYTES,
-                                     GEMM_BOX_BYTES, full);
+                    // `width` rows from the tile's first on, in pieces that stay inside a box of 128 rows (whole groups of 8
+                    // rows, over which the swizzle repeats); rows past the last box are left out (their columns of the
+                    // accumulator are never stored)
+                    int row = c.n_tile * width, left = min(width, row_tiles * GEMM_BM - row);
+                    mbar_expect_tx(full, x_bytes + (uint32_t)left * (GEMM_BK * 2));
+                    uint32_t to = dst + X_BYTES;
+                    while (left > 0) {
+                        const int in = row & (GEMM_BM - 1), take = min(GEMM_BM - in, left);
+                        bulk_load_1d(to, w_tiled + ((size_t)((row >> 7) + c.group * row_tiles) * num_kb + c.kb) * GEMM_BOX_BYTES + in * (GEMM_BK * 2),
+                                     (uint32_t)take * (GEMM_BK * 2), full);
+                        row += take, left -= take, to += (uint32_t)take * (GEMM_BK * 2);
+                    }
                 } else if (weights) {
-                    mbar_expect_tx(full, Smem::stage_bytes);
-                    tma_load_2d(dst + Smem::x_bytes, &map_y, full, c.kb * GEMM_BK, c.group * N + c.n_tile * BN);
+                    mbar_expect_tx(full, x_bytes + (uint32_t)width * (GEMM_BK * 2));
+                    tma_load_2d(dst + X_BYTES, &map_y, full, c.kb * GEMM_BK, c.group * N + c.n_tile * width);
                 }
-                if (activations) tma_load_2d(dst, &map_x, full, c.kb * GEMM_BK, c.m_tile * GEMM_BM);
+                if (activations) {
+                    tma_load_2d(dst, &map_x, full, c.kb * GEMM_BK, c.m_tile * ROWS);
+                    if (second) tma_load_2d(dst + GEMM_BOX_BYTES, &map_x, full, c.kb * GEMM_BK, c.m_tile * ROWS + GEMM_BM);
+                }
             };
             // The weights do not depend on the kernel before this one: the first ring of weight tiles is
             // fetched at once, and only the activation tiles wait for that kernel to finish.
@@ -930,7 +947,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
             place(ahead);
             Cursor behind = ahead;
             int head = 0;
-            for (; head < STAGES && ahead.t < total_tiles; ++head) { issue(ahead, true, false); advance(ahead); }
+            for (; head < stages && ahead.t < total_tiles; ++head) { issue(ahead, true, false); advance(ahead); }
             pdl_wait();
             for (int i = 0; i < head; ++i) { issue(behind, false, true); advance(behind); }
             while (ahead.t < total_tiles) {
@@ -941,35 +958,47 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
         }
     } else if (warp == 1) {
         if (elect_one()) {
-            constexpr uint32_t idesc = instr_desc_bf16(GEMM_BM, BN);
-            int it = 0, handled = 0;
+            const uint32_t idesc = instr_desc_bf16(GEMM_BM, width);
+            int stage = 0, handled = 0;
+            uint32_t parity = 0;   // of the ring's current round
+            int used[2] = {0, 0};  // tiles that each accumulator has held
             if (ep.tile_group) pdl_wait();
             for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
                 if (ep.tile_group && ep.tile_group[t % m_tiles] < 0) continue;
-                const int local = handled++;
-                const int buf = local & 1;
-                // the epilogue must have drained this accumulator (two tiles ago)
-                if (local >= 2 && !mbar_wait(smem_addr(&acc_empty[buf]), (uint32_t)((local >> 1) - 1) & 1u)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * tmem_columns<BN>());
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(smem_addr(&full_bar[s]), (uint32_t)(it / STAGES) & 1u)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t x_addr = smem_addr(smem + s * Smem::stage_bytes);
-                    const uint64_t desc_x = smem_desc_k_major_sw128(x_addr);
-                    const uint64_t desc_y = smem_desc_k_major_sw128(x_addr + Smem::x_bytes);
+                // one row tile: the tiles take turns with the accumulators; two: each half of the rows has one
+                const int first = MT == 1 ? (handled++ & 1) : 0;
+                const int halves = MT == 2 && (t % m_tiles) * ROWS + GEMM_BM < M ? 2 : 1;
+                const int seen = MT == 1 ? (first ? used[1] : used[0]) : 0;
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    if (!mbar_wait(smem_addr(&full_bar[stage]), parity)) { ok = false; break; }
+                    const uint32_t x_addr = smem_addr(smem + stage * stage_bytes);
+                    const uint64_t desc_y = smem_desc_k_major_sw128(x_addr + X_BYTES);
 #pragma unroll
-                    for (int k = 0; k < GEMM_BK / 16; ++k)
-                        mma_bf16_ss(tmem_acc, desc_x + (uint64_t)(2 * k), desc_y + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    mma_commit(smem_addr(&empty_bar[s]));
+                    for (int h = 0; h < MT; ++h) {
+                        if (h >= halves) break;
+                        const int acc = MT == 1 ? first : h, before = MT == 1 ? seen : used[h];
+                        // the epilogue must have drained this accumulator
+                        if (kb == 0 && before > 0 && !mbar_wait(smem_addr(&acc_empty[acc]), (uint32_t)(before - 1) & 1u)) { ok = false; break; }
+                        tc_fence_after();
+                        const uint64_t desc_x = smem_desc_k_major_sw128(x_addr + h * GEMM_BOX_BYTES);
+#pragma unroll
+                        for (int k = 0; k < GEMM_BK / 16; ++k)
+                            mma_bf16_ss(tmem_base + (uint32_t)acc * 256u, desc_x + (uint64_t)(2 * k), desc_y + (uint64_t)(2 * k), idesc,
+                                        (kb > 0 || k > 0) ? 1u : 0u);
+                        if (kb == num_kb - 1) mma_commit(smem_addr(&acc_full[acc]));
+                    }
+                    if (!ok) break;
+                    mma_commit(smem_addr(&empty_bar[stage]));
+                    if (++stage == stages) stage = 0, parity ^= 1u;
                 }
-                if (!ok) break;
-                mma_commit(smem_addr(&acc_full[buf]));
+                if (MT == 2) ++used[0], used[1] += halves - 1;
+                else if (first) ++used[1];
+                else ++used[0];
             }
         }
     } else {
         const int lane_group = warp & 3;
+        const int half = (warp - 2) >> 2;  // two row tiles: which 128 rows this warp stores
         const int tile_row = lane_group * 32 + lane;
         pdl_wait();  // the output buffer may still be read by the kernel before this one
         // whether the residual-and-norm epilogue can take its coalesced form (whole 16-byte pieces everywhere)
@@ -978,10 +1007,12 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
         int handled = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
             if (ep.tile_group && ep.tile_group[t % m_tiles] < 0) continue;
-            const int local = handled++;
-            const int buf = local & 1;
             const int n_tile = t / m_tiles;
-            const int x0 = (t % m_tiles) * GEMM_BM, y0 = n_tile * BN;
+            const int x0 = (t % m_tiles) * ROWS + half * GEMM_BM, y0 = n_tile * width;
+            if (MT == 2 && x0 >= M) continue;  // a half without rows
+            const int local = handled++;
+            const int buf = MT == 1 ? local & 1 : half;
+            const uint32_t parity = (uint32_t)(MT == 1 ? local >> 1 : local) & 1u;
             const int x_row = x0 + tile_row;
             // EPI 2: the stream's values are fetched two chunks of 16 columns ahead of their use, the first two
             // before this tile's products are done
@@ -996,52 +1027,48 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
                 const int gr = x0 + lane_group * 32 + lane;
                 if (gr < M) {
                     const char* line = reinterpret_cast<const char*>(ep.residual + (size_t)gr * N + y0);
-                    const int bytes = min(BN, N - y0) * 4;
+                    const int bytes = min(width, N - y0) * 4;
                     for (int off = 0; off < bytes; off += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(line + off));
                 }
             }
-            if (!mbar_wait(smem_addr(&acc_full[buf]), (uint32_t)(local >> 1) & 1u)) { ok = false; break; }
+            const float my_scale = (EPI != 2 && ep.row_sumsq && x_row < M) ? row_scale_of(ep, x_row, M) : 1.0f;
+            if (!mbar_wait(smem_addr(&acc_full[buf]), parity)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * tmem_columns<BN>()) + ((uint32_t)(lane_group * 32) << 16);
-            if (EPI == 2 && sizeof(OutT) == 2 && coalesced) {
-                float4* stage = reinterpret_cast<float4*>(smem + STAGES * Smem::stage_bytes + Smem::barrier_bytes) + lane_group * 256;
-                epilogue_residual_norm_coalesced(ep, reinterpret_cast<__nv_bfloat16*>(C), ldc, tmem_acc, stage, x0 + lane_group * 32,
-                                                 y0, BN, M, N, n_tile, lane);
+            const uint32_t tmem_acc = tmem_base + (uint32_t)buf * 256u + ((uint32_t)(lane_group * 32) << 16);
+            auto release = [&] {  // this warp has read its lanes of the accumulator: hand it back to the MMA thread
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_addr(&acc_empty[buf]));
-                continue;
-            }
-            const float my_scale = (ep.row_sumsq && x_row < M) ? row_scale_of(ep, x_row, M) : 1.0f;
-            float row_sq = 0.0f;
+            };
+            if constexpr (EPI == 2) {
+                if (sizeof(OutT) == 2 && coalesced) {
+                    float4* stage = reinterpret_cast<float4*>(smem + stages * stage_bytes + GEMM_BARRIER_BYTES) + lane_group * 256;
+                    epilogue_residual_norm_coalesced(ep, reinterpret_cast<__nv_bfloat16*>(C), ldc, tmem_acc, stage, x0 + lane_group * 32,
+                                                     y0, width, M, N, n_tile, lane);
+                    release();
+                    continue;
+                }
+                float row_sq = 0.0f;
 #pragma unroll 1
-            for (int c0 = 0; c0 < BN; c0 += 16) {
-                if (y0 + c0 >= N) break;  // uniform across the warp
-                float4 w4[4];
-                if (EPI == 2) {
+                for (int c0 = 0; c0 < width; c0 += 16) {
+                    if (y0 + c0 >= N) break;  // uniform across the warp
+                    float4 w4[4];
                     if (c0 > 0) { cur = next; next = after; }
-                    load_residual_chunk(ep, x_row, c0 + 32 < BN ? y0 + c0 + 32 : N, M, N, after);
+                    load_residual_chunk(ep, x_row, c0 + 32 < width ? y0 + c0 + 32 : N, M, N, after);
                     if (cur.vector) {
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) w4[q4] = reinterpret_cast<const float4*>(ep.norm_weight + y0 + c0)[q4];
                     }
-                }
-                const bool vector = EPI == 2 && cur.vector;
-                uint32_t r[16];
-                tmem_load_32x16(tmem_acc + (uint32_t)c0, r);
-                tmem_load_wait();
-                if (x_row >= M) continue;
-                float v[16];
+                    uint32_t r[16];
+                    tmem_load_32x16(tmem_acc + (uint32_t)c0, r);
+                    tmem_load_wait();
+                    if (x_row >= M) continue;
+                    float v[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) * my_scale;
-                if (EPI == 3) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = v[j] > 0.0f ? v[j] * v[j] : 0.0f;
-                }
-                if (EPI == 2) {
+                    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
                     float* res = ep.residual + (size_t)x_row * N + y0 + c0;
                     OutT* dst = C + (size_t)x_row * ldc + y0 + c0;
-                    if (vector && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
+                    if (cur.vector && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
                         uint32_t packed[8];
 #pragma unroll
                         for (int q4 = 0; q4 < 4; ++q4) {
@@ -1068,51 +1095,97 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
                             }
                         }
                     }
-                } else if (EPI == 1) {
-                    // columns y0 + c0 .. + 15 are 8 gate rows then their 8 up rows: 8 outputs at (y0 + c0) / 2
-                    OutT* dst = C + (size_t)x_row * ldc + ((y0 + c0) >> 1);
-                    if (y0 + c0 + 16 <= N && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
-                        uint32_t packed[4];
+                }
+                if (x_row < M) ep.sumsq_out[(size_t)n_tile * M + x_row] = row_sq;  // this column tile's share
+                release();
+            } else {
+                // EPI 1: 16 columns are 8 gate rows then their 8 up rows, and make 8 outputs
+                constexpr int PER = EPI == 1 ? 8 : 16;  // outputs of a chunk of 16 columns
+                OutT* const row_out = C + (size_t)x_row * ldc + (EPI == 1 ? y0 >> 1 : y0);
+                const bool aligned = ((uintptr_t)C & 15) == 0 && (ldc * (long)sizeof(OutT)) % 16 == 0;
+                auto values = [&](int c0, float (&v)[PER]) {
+                    uint32_t r[16];
+                    tmem_load_32x16(tmem_acc + (uint32_t)c0, r);
+                    tmem_load_wait();
+                    if (EPI == 1) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            __nv_bfloat162 pair = __floats2bfloat162_rn(gate_mul(ep, v[2 * j], v[2 * j + 8]), gate_mul(ep, v[2 * j + 1], v[2 * j + 9]));
-                            packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-                        }
-                        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                        for (int j = 0; j < 8; ++j) v[j] = gate_mul(ep, __uint_as_float(r[j]) * my_scale, __uint_as_float(r[j + 8]) * my_scale);
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (y0 + c0 + j + 8 < N) dst[j] = from_f32<OutT>(gate_mul(ep, v[j], v[j + 8]));
+                        for (int j = 0; j < PER; ++j) {
+                            v[j] = __uint_as_float(r[j]) * my_scale;
+                            if (EPI == 3) v[j] = v[j] > 0.0f ? v[j] * v[j] : 0.0f;
+                        }
+                    }
+                };
+                if constexpr (MT == 2 && sizeof(OutT) == 2) {
+                    // The next tile's products wait for this accumulator: the row is taken into registers as it will be
+                    // stored, and the accumulator handed back before anything is written.
+                    uint32_t packed[16][PER / 2];
+#pragma unroll
+                    for (int c = 0; c < 16; ++c) {
+                        if (16 * c < width) {
+                            float v[PER];
+                            values(16 * c, v);
+#pragma unroll
+                            for (int j = 0; j < PER / 2; ++j) {
+                                __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                                packed[c][j] = *reinterpret_cast<uint32_t*>(&pair);
+                            }
+                        }
+                    }
+                    release();
+                    if (x_row < M) {
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) {
+                            if (16 * c >= width || y0 + 16 * c >= N) break;
+                            OutT* dst = row_out + c * PER;
+                            if (aligned && y0 + 16 * c + 16 <= N) {
+#pragma unroll
+                                for (int q = 0; q < PER / 8; ++q)
+                                    reinterpret_cast<uint4*>(dst)[q] = make_uint4(packed[c][4 * q], packed[c][4 * q + 1], packed[c][4 * q + 2], packed[c][4 * q + 3]);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < PER; ++j) {
+                                    const __nv_bfloat162 pair = *reinterpret_cast<const __nv_bfloat162*>(&packed[c][j / 2]);
+                                    if (y0 + 16 * c + (EPI == 1 ? 8 + j : j) < N) dst[j] = j & 1 ? pair.y : pair.x;
+                                }
+                            }
+                        }
                     }
                 } else {
-                    OutT* dst = C + (size_t)x_row * ldc + y0 + c0;
-                    const bool full = (y0 + c0 + 16 <= N) && (((uintptr_t)dst & 15) == 0);
-                    if (full && sizeof(OutT) == 2) {
-                        uint32_t packed[8];
+#pragma unroll 1
+                    for (int c0 = 0; c0 < width; c0 += 16) {
+                        if (y0 + c0 >= N) break;  // uniform across the warp
+                        float v[PER];
+                        values(c0, v);
+                        if (x_row >= M) continue;
+                        OutT* dst = row_out + (EPI == 1 ? c0 >> 1 : c0);
+                        if (aligned && y0 + c0 + 16 <= N) {
+                            if (sizeof(OutT) == 2) {
+                                uint32_t packed[PER / 2];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                            packed[j] = *reinterpret_cast<uint32_t*>(&pair);
+                                for (int j = 0; j < PER / 2; ++j) {
+                                    __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                                    packed[j] = *reinterpret_cast<uint32_t*>(&pair);
+                                }
+#pragma unroll
+                                for (int q = 0; q < PER / 8; ++q)
+                                    reinterpret_cast<uint4*>(dst)[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < PER / 4; ++j)
+                                    reinterpret_cast<float4*>(dst)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < PER; ++j)
+                                if (y0 + c0 + (EPI == 1 ? 8 + j : j) < N) dst[j] = from_f32<OutT>(v[j]);
                         }
-                        uint4* out = reinterpret_cast<uint4*>(dst);
-                        out[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        out[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                    } else if (full && sizeof(OutT) == 4) {
-                        float4* out = reinterpret_cast<float4*>(dst);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) out[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (y0 + c0 + j < N) dst[j] = from_f32<OutT>(v[j]);
                     }
+                    release();
                 }
             }
-            if (EPI == 2 && x_row < M) ep.sumsq_out[(size_t)n_tile * M + x_row] = row_sq;  // this column tile's share
-            // this warp has read its lanes of the accumulator: hand it back to the MMA thread
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_addr(&acc_empty[buf]));
         }
     }
     if (!ok) atomicExch(error_flag, 4);
@@ -1120,7 +1193,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 2 * tmem_columns<BN>());
+        tmem_dealloc(tmem_base, 512);
     }
 }
 
@@ -1133,25 +1206,88 @@ static int sm_count() {
     }();
     return count;
 }
-template <int BN, typename OutT, int EPI>
-static int launch_persistent(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
-                             const Epilogue& ep, int* error_flag, cudaStream_t stream, int groups = 1) {
-    using Smem = GemmSmem<BN>;
+
+// The tile (128 * row_tiles rows, `width` columns) of a product of many tokens, and the stages of its ring.
+//
+// A launch runs in rounds of one tile an SM, and what few rounds cost is decided by how full the last one is: tiles of 128 x 256
+// made 160 tiles of the 4B shape's down product at 2,048 tokens, two rounds on 148 SMs, 121 us; 144 tiles of 256 x 144 make one,
+// 78 us (o 50 to 35 us; the 32B shape's o 164 to 129, down 515 to 384, q/k/v 169 to 154; the 8B shape's down 163 to 139; at 300
+// tokens the 4B shape's o 26 to 18 us with tiles of 128 x 64, whose 120 tiles keep more SMs busy than 30).  So the tile is the
+// one with the least cost by the rule below, in which a block of K costs a tile of 128 rows as much as width + 80 columns
+// (1.17 ns each) and one of 256 rows 1.95 * (width + 32) (its two halves share the weights' way through L2), a round that is
+// partly empty a quarter less for what is empty (the others get its share of L2 and power), and a tile of 256 rows its epilogue
+// on top, during which its accumulators are not free: 1,000 columns where a row goes to registers before it is stored, 3,000 where the
+// activation is worked out or 32-bit values are stored first.  128 x 256, which many full rounds run best, is left for
+// 6 % or more, and widths that cut the weights' boxes in pieces count 1.5 % more.  Fitted to 44 shapes (4B, 8B and 32B layers, 300 to
+// 2,048 tokens), each timed at 24 tiles: what it picks is 0.5 % slower than the best on average, 9 % at most.
+// Grouped products, whose tiles without rows are known on the device alone, and the residual-and-norm epilogue, whose
+// callers count its column tiles, keep 128 x 256.
+struct PersistentTile {
+    int row_tiles, width;
+};
+static int persistent_stages(int row_tiles, int width) {
+    const int stages = 200 * 1024 / (row_tiles * GEMM_BOX_BYTES + width * GEMM_BK * 2);
+    return stages < GEMM_MAX_STAGES ? stages : GEMM_MAX_STAGES;
+}
+static PersistentTile persistent_tile(int M, int N, int K, int epi, bool grouped, size_t out_bytes) {
+    if (epi == 2 || grouped) return PersistentTile{1, N <= 128 ? 128 : 256};
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    const double k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
+    PersistentTile best{1, 256};
+    double least = 0.0;
+    for (int row_tiles = 1; row_tiles <= 2; ++row_tiles) {
+        const long m_tiles = (M + row_tiles * GEMM_BM - 1) / (row_tiles * GEMM_BM);
+        for (int width = 256; width >= (row_tiles == 1 ? 48 : 96); width -= 16) {
+            const long tiles = m_tiles * ((N + width - 1) / width), whole = (tiles + sms - 1) / sms;
+            const double rounds = whole == 1 ? 1.0 : 0.25 * tiles / sms + 0.75 * whole;
+            const double block = row_tiles == 1 ? width + 80.0 : 1.95 * (width + 32.0);
+            const double exposed = row_tiles == 1 ? 0.0 : (epi == 1 || out_bytes == 4 ? 3000.0 : 1000.0);
+            double cost = rounds * (k_blocks * block + exposed);
+            if (row_tiles == 1 && width == 256) cost *= 0.94;
+            if (width % 64 != 0) cost *= 1.015;
+            if (least == 0.0 || cost < least) least = cost, best = PersistentTile{row_tiles, width};
+        }
+    }
+    return best;
+}
+// What the rule picks: 1,000 * row tiles + columns (form as in kirai_gemm_bf16_general).
+KIRAI_EXPORT int kirai_gemm_bf16_many_tile(int M, int N, int K, int form) {
+    const int epi = form == 3 ? 2 : (form == 2 || form == 5 || form == 7 ? 1 : (form == 4 ? 3 : 0));
+    const PersistentTile tile = persistent_tile(M, N, K, epi, false, form == 1 ? 4 : 2);
+    return 1000 * tile.row_tiles + tile.width;
+}
+
+template <int MT, typename OutT, int EPI>
+static int launch_persistent_tile(int width, const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
+                                  const Epilogue& ep, int* error_flag, cudaStream_t stream, int groups) {
     CUtensorMap map_a, map_w;
     if (!tmap::bf16_2d_sw128(&map_a, A, M, K, lda, GEMM_BM, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
     if (tiled) map_w = map_a;  // not read: the boxes are fetched by address
-    else if (!tmap::bf16_2d_sw128(&map_w, W, (uint64_t)N * groups, K, K, BN, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
+    else if (!tmap::bf16_2d_sw128(&map_w, W, (uint64_t)N * groups, K, K, width, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
     if (tiled && ((uintptr_t)W & 15)) return KIRAI_ERR_BAD_ALIGN;
-    const long tiles = (long)((M + GEMM_BM - 1) / GEMM_BM) * ((N + BN - 1) / BN);
+    const long tiles = (long)((M + MT * GEMM_BM - 1) / (MT * GEMM_BM)) * ((N + width - 1) / width);
     const int sms = sm_count();
     if (sms <= 0) return KIRAI_ERR_UNSUPPORTED;  // the device did not say how many SMs it has
     const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-    auto kernel = gemm_tcgen05_persistent_kernel<BN, OutT, EPI>;
-    const int smem_bytes = Smem::total(1) + (EPI == 2 ? 4 * 32 * 32 * 4 : 0);  // + the epilogue's staging buffers
+    const int stages = persistent_stages(MT, width);
+    auto kernel = gemm_tcgen05_persistent_kernel<MT, OutT, EPI>;
+    const int smem_bytes = stages * (MT * GEMM_BOX_BYTES + width * GEMM_BK * 2) + GEMM_BARRIER_BYTES + 1024 +  // + slack to align the ring
+                           (EPI == 2 ? 4 * 32 * 32 * 4 : 0);                                                   // + the epilogue's staging buffers
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (err != cudaSuccess) return (int)err;
-    return launch_pdl(kernel, dim3(grid), dim3(GEMM_THREADS), (size_t)smem_bytes, stream, 1u, map_a, map_w,
-                      tiled ? (const uint8_t*)W : (const uint8_t*)nullptr, (OutT*)C, M, N, K, ldc, ep, error_flag);
+    return launch_pdl(kernel, dim3(grid), dim3(64 + 128 * MT), (size_t)smem_bytes, stream, 1u, map_a, map_w,
+                      tiled ? (const uint8_t*)W : (const uint8_t*)nullptr, (OutT*)C, M, N, K, ldc, width, stages, ep, error_flag);
+}
+
+template <typename OutT, int EPI>
+static int launch_persistent(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
+                             const Epilogue& ep, int* error_flag, cudaStream_t stream, int groups = 1) {
+    const PersistentTile tile = persistent_tile(M, N, K, EPI, ep.tile_group != nullptr, sizeof(OutT));
+    if constexpr (EPI != 2) {
+        if (tile.row_tiles == 2)
+            return launch_persistent_tile<2, OutT, EPI>(tile.width, A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream, groups);
+    }
+    return launch_persistent_tile<1, OutT, EPI>(tile.width, A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream, groups);
 }
 
 static bool deep_rings() {
@@ -1300,8 +1436,7 @@ static int gemm_dispatch(const void* A, const void* W, bool tiled, void* C, int 
     if (M <= 256 && one_wave && streams_wide_tiles(C, ldc, sizeof(OutT), N, EPI, ep)) KIRAI_GEMM_CASE(256, true);
     if (M <= 256 && EPI == 2 && N % 8 == 0 && (M <= 128 || one_wave)) return KIRAI_ERR_BAD_ALIGN;  // see kirai_gemm_bf16_residual_parts
 #undef KIRAI_GEMM_CASE
-    if (N <= 128) return launch_persistent<128, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
-    return launch_persistent<256, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
+    return launch_persistent<OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
 }
 
 // Split count that the entry points pick for splits <= 0.
@@ -1341,9 +1476,7 @@ KIRAI_EXPORT int kirai_gemm_bf16_grouped(const void* A, const void* W, int tiled
     if (tiled && N % GEMM_BM != 0) return KIRAI_ERR_BAD_SIZE;
     Epilogue ep{nullptr, 0, 1.0f, 0.0f, nullptr, nullptr, nullptr, nullptr};
     ep.tile_group = tile_group;
-#define KIRAI_GROUPED(OutT, EPI)                                                                                                  \
-    return N <= 128 ? launch_persistent<128, OutT, EPI>(A, W, tiled != 0, C, M, N, K, lda, ldc, ep, error_flag, stream, groups) \
-                    : launch_persistent<256, OutT, EPI>(A, W, tiled != 0, C, M, N, K, lda, ldc, ep, error_flag, stream, groups)
+#define KIRAI_GROUPED(OutT, EPI) return launch_persistent<OutT, EPI>(A, W, tiled != 0, C, M, N, K, lda, ldc, ep, error_flag, stream, groups)
     switch (form) {
         case 0: KIRAI_GROUPED(bf16, 0);
         case 1: KIRAI_GROUPED(float, 0);

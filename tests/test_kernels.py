@@ -247,6 +247,37 @@ def test_linear_tcgen05_against_plain(ops, m, n, k, out_dtype):
     ops.check_device_errors(torch.device(DEV))
 
 
+# tiles of the many-token kernel that the rule picks on 148 SMs: 128 and 256 rows (with a last tile of one half, or of a part of
+# one), widths that cut weight boxes, columns beyond the last whole tile or box, a K that ends inside a block
+@pytest.mark.parametrize("m,n,k", [(300, 2560, 64), (300, 6144, 72), (640, 2568, 136), (1100, 2560, 264), (1408, 4104, 1096),
+                                   (1600, 4096, 2056), (1920, 2560, 2056), (2049, 2600, 2056), (1200, 6160, 2056)])
+def test_many_token_products_of_every_tile(ops, m, n, k):
+    x, w = rand(m, k, dtype=torch.bfloat16, scale=0.5), rand(n, k, dtype=torch.bfloat16, scale=0.1, seed=3)
+    tiled = ops.tile_weight(w)
+    # 32-bit sums of k products in another order: k roundings of 2^-24, at most, on sums of |products| (and torch's own)
+    expected, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    out = ops.linear_tcgen05(x, tiled, torch.float32)
+    assert bool(((out.double() - expected).abs() <= 2 * k * 2.0 ** -24 * size).all())
+    assert torch.equal(out, ops.linear_tcgen05(x, w, torch.float32))
+    # 16-bit results are those sums rounded once; the same bits whatever tile makes them
+    assert torch.equal(ops.linear_tcgen05(x, tiled), out.bfloat16())
+    assert torch.equal(ops.linear_tcgen05(x, w), out.bfloat16())
+    assert torch.equal(ops.linear_relu2(x, tiled), (out.clamp(min=0.0) ** 2).bfloat16())
+    if n % 16 == 0:
+        gate, up = out.view(m, n // 16, 2, 8)[:, :, 0].reshape(m, -1), out.view(m, n // 16, 2, 8)[:, :, 1].reshape(m, -1)
+        act = ops.linear_tcgen05(x, tiled, swiglu=True).double()
+        exact = gate.double() / (1.0 + torch.exp(-gate.double())) * up.double()
+        assert bool(((act - exact).abs() <= (2.0 ** -8 + 2.0 ** -18) * exact.abs() + 1e-30).all())  # one rounding to 16 bits, fast exp and division
+    ops.check_device_errors(torch.device(DEV))
+
+
+def test_many_token_products_take_the_tiles_tested_above(ops):
+    pick = ops.library().kirai_gemm_bf16_many_tile
+    shapes = test_many_token_products_of_every_tile.pytestmark[0].args[1]
+    tiles = {divmod(pick(m, n, k, form), 1000) for m, n, k in shapes for form in (0, 1, 2)}
+    assert {rows for rows, _ in tiles} == {1, 2} and len({width for _, width in tiles}) >= 6 and any(width % 128 for _, width in tiles)
+
+
 def test_linear_refuses_rows_that_tma_cannot_read(ops):
     x, w = rand(4, 70, dtype=torch.bfloat16), rand(32, 70, dtype=torch.bfloat16)
     with pytest.raises(ops.KernelError):
