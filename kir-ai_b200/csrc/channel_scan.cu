@@ -530,9 +530,16 @@ __global__ void __launch_bounds__(WALK_THREADS, 512 / WALK_THREADS) channel_walk
     const long first = a.query_start[request];
     const int count = (int)(a.query_start[request + 1] - first);
     const int slot = a.slots[request];
+    float* S = a.state + slot * a.state_len + (long)head * d * dv;
+    if (slot >= 0 && slot < a.num_slots && count > 0) {
+        // the state that the last step left lies in memory, as does the decays' matrix
+        for (long i = tid * 32L; i < (long)d * dv; i += WALK_THREADS * 32L) prefetch_l2(S + i);
+        const int lines = (d + 31) / 32;
+        for (int i = tid; i < a.rank * lines; i += WALK_THREADS)
+            prefetch_l2(a.up + (long)(i / lines) * a.heads * d + (long)head * d + (i % lines) * 32);
+    }
     pdl_wait();
     if (slot < 0 || slot >= a.num_slots || count <= 0) return;
-    float* S = a.state + slot * a.state_len + (long)head * d * dv;
     Cols<V> held[HOLD ? HELD : 1];
     if (HOLD && phase < phases && group < groups_all) {
 #pragma unroll

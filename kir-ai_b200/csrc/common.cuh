@@ -41,6 +41,13 @@ __device__ __forceinline__ float from_f32<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat16_rn(v); }
 
+// Asks for the line that holds `p` to be brought into L2.  Unlike a load this may be done ahead of pdl_wait(), whoever writes
+// the line: L2 is where every SM's loads and stores meet, so a later load finds what was written last.  Kernels of few rows ask
+// for weights and states this way while the kernel before them still runs: between two uses in a decode step gigabytes of
+// other weights have gone through L2, and a first load from memory costs about a microsecond.
+#define PREFETCH_ROWS 148  // a kernel with a block per row asks ahead up to so many rows; with more, blocks that start later find the lines
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int offset = 16; offset > 0; offset >>= 1) v += __shfl_xor_sync(0xffffffffu, v, offset);

@@ -151,6 +151,9 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __res
                                        const int* __restrict__ row_index, float* __restrict__ resid_out, int hidden,
                                        float eps) {
     pdl_launch_dependents();
+    if (gridDim.x <= PREFETCH_ROWS) {
+        for (int i = threadIdx.x * 32; i < hidden; i += blockDim.x * 32) prefetch_l2(weight + i);
+    }
     pdl_wait();
     __shared__ float scratch[32];
     const int row = blockIdx.x;
@@ -158,18 +161,20 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ resid, const T* __res
     const float* x = resid + (size_t)src * hidden;
     const T* d = delta ? delta + (size_t)src * hidden : nullptr;
     float* sum_dst = row_index ? resid_out + (size_t)row * hidden : resid + (size_t)src * hidden;
-    float4 v[VEC];
+    float4 v[VEC], dv[VEC];
     float acc = 0.0f;
+    // (all loads before the first store, which might be to what a later one reads for all that the compiler knows)
 #pragma unroll
     for (int n = 0; n < VEC; ++n) {
         const int i = (n * blockDim.x + threadIdx.x) * 4;
-        v[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[n] = i < hidden ? Vec4<float>::load(x + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (d && i < hidden) dv[n] = Vec4<T>::load(d + i);
+    }
+#pragma unroll
+    for (int n = 0; n < VEC; ++n) {
+        const int i = (n * blockDim.x + threadIdx.x) * 4;
         if (i < hidden) {
-            v[n] = Vec4<float>::load(x + i);
-            if (d) {
-                const float4 dv = Vec4<T>::load(d + i);
-                v[n].x += dv.x; v[n].y += dv.y; v[n].z += dv.z; v[n].w += dv.w;
-            }
+            if (d) v[n].x += dv[n].x, v[n].y += dv[n].y, v[n].z += dv[n].z, v[n].w += dv[n].w;
             if (d || row_index) Vec4<float>::store(sum_dst + i, v[n]);
             acc = fmaf(v[n].x, v[n].x, acc);
             acc = fmaf(v[n].y, v[n].y, acc);

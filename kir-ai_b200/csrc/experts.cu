@@ -176,7 +176,6 @@ router_gates_few_kernel(const T* __restrict__ x, long x_stride, const float* __r
                         int* __restrict__ chosen_ids, float* __restrict__ chosen_weights, int* __restrict__ arrivals, int hidden,
                         int experts, int top, RouterRule rule) {
     pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ float logits_s[];  // [experts]
     __shared__ float part_s[ROUTER_WARPS];
     __shared__ int is_last;
@@ -184,6 +183,8 @@ router_gates_few_kernel(const T* __restrict__ x, long x_stride, const float* __r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* row = x + (size_t)token * x_stride;
     const float* w = router + (size_t)e * hidden;
+    for (int i = threadIdx.x * 32; i < hidden; i += ROUTER_WARPS * 32 * 32) prefetch_l2(w + i);
+    pdl_wait();
     float* out = gates + (size_t)token * (experts + rule.extra);
     float dot = 0.0f;
     if (hidden % 4 == 0 && x_stride % 4 == 0 && (((uintptr_t)x | (uintptr_t)router) & 15) == 0) {
@@ -601,6 +602,9 @@ template <int VEC>
 __global__ void terms_norm_add_kernel(float* __restrict__ resid, const FeedForwardTerms f, const float* __restrict__ norm_weight,
                                       bf16* __restrict__ copy, int hidden, float eps) {
     pdl_launch_dependents();
+    if (gridDim.x <= PREFETCH_ROWS) {
+        for (int i = threadIdx.x * 32; i < hidden; i += blockDim.x * 32) prefetch_l2(norm_weight + i);
+    }
     pdl_wait();
     __shared__ float scratch[32];
     const int token = blockIdx.x;
@@ -609,14 +613,15 @@ __global__ void terms_norm_add_kernel(float* __restrict__ resid, const FeedForwa
     const float share = f.shared && f.share_col >= 0 ? f.gates[(size_t)token * f.gates_stride + f.share_col] : 1.0f;
     const float same = same_weight(f, token);
     float4* dst = reinterpret_cast<float4*>(resid + base);
-    float4 kept[VEC], stream[VEC];
+    const float4* w4 = reinterpret_cast<const float4*>(norm_weight);
+    float4 kept[VEC], stream[VEC], w[VEC];
     float acc = 0.0f;
 #pragma unroll
     for (int n = 0; n < VEC; ++n) {
         const int i = threadIdx.x + n * blockDim.x;
         kept[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < quads) {
-            stream[n] = dst[i];
+            stream[n] = dst[i], w[n] = w4[i];
             if (f.routed) kept[n] = load4(f.routed + base + 4 * (size_t)i);
             if (f.sorted) {
                 for (int j = 0; j < f.top; ++j) {
@@ -631,14 +636,12 @@ __global__ void terms_norm_add_kernel(float* __restrict__ resid, const FeedForwa
     }
     const float variance = block_sum(acc, scratch) / (float)hidden + eps;
     const float scale = variance == 0.0f ? 0.0f : 1.0f / sqrtf(variance);
-    const float4* w4 = reinterpret_cast<const float4*>(norm_weight);
 #pragma unroll
     for (int n = 0; n < VEC; ++n) {
         const int i = threadIdx.x + n * blockDim.x;
         if (i < quads) {
             float4 r = stream[n];
-            const float4 w = w4[i];
-            r.x += kept[n].x * scale * w.x, r.y += kept[n].y * scale * w.y, r.z += kept[n].z * scale * w.z, r.w += kept[n].w * scale * w.w;
+            r.x += kept[n].x * scale * w[n].x, r.y += kept[n].y * scale * w[n].y, r.z += kept[n].z * scale * w[n].z, r.w += kept[n].w * scale * w[n].w;
             dst[i] = r;
             if (copy) {
                 const __nv_bfloat162 lo = __floats2bfloat162_rn(r.x, r.y), hi = __floats2bfloat162_rn(r.z, r.w);

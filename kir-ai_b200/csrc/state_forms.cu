@@ -61,6 +61,7 @@ __global__ void __launch_bounds__(256) add_dyt_vec_kernel(float* __restrict__ re
                                                           const int* __restrict__ row_index, int width) {
     pdl_launch_dependents();
     const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (gridDim.x <= PREFETCH_ROWS && (threadIdx.x & 7) == 0 && c < width) prefetch_l2(w + c), prefetch_l2(b + c);
     pdl_wait();
     if (c >= width) return;
     const float a = alpha[0];
@@ -149,10 +150,13 @@ __global__ void rms_pair_mean_vec_kernel(const float* __restrict__ a, const floa
                                          const float* __restrict__ wb, float eps, float* __restrict__ out, int width) {
     __shared__ float2 scratch[32];
     pdl_launch_dependents();
+    if (gridDim.x <= PREFETCH_ROWS) {
+        for (int i = threadIdx.x * 32; i < width; i += blockDim.x * 32) prefetch_l2(wa + i), prefetch_l2(wb + i);
+    }
     pdl_wait();
     const float* pa = a + (long)blockIdx.x * width;
     const float* pb = b + (long)blockIdx.x * width;
-    float4 x[4], y[4];
+    float4 x[4], y[4], u[4], v[4];
     float sa = 0.0f, sb = 0.0f;
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -160,6 +164,7 @@ __global__ void rms_pair_mean_vec_kernel(const float* __restrict__ a, const floa
         const bool inside = c < width;
         x[n] = inside ? *reinterpret_cast<const float4*>(pa + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         y[n] = inside ? *reinterpret_cast<const float4*>(pb + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (inside) u[n] = *reinterpret_cast<const float4*>(wa + c), v[n] = *reinterpret_cast<const float4*>(wb + c);
     }
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -176,10 +181,9 @@ __global__ void rms_pair_mean_vec_kernel(const float* __restrict__ a, const floa
     for (int n = 0; n < 4; ++n) {
         const int c = (n * blockDim.x + threadIdx.x) * 4;
         if (c >= width) break;
-        const float4 u = *reinterpret_cast<const float4*>(wa + c), v = *reinterpret_cast<const float4*>(wb + c);
         *reinterpret_cast<float4*>(out + (long)blockIdx.x * width + c) =
-            make_float4(0.5f * (x[n].x * ra * u.x + y[n].x * rb * v.x), 0.5f * (x[n].y * ra * u.y + y[n].y * rb * v.y),
-                        0.5f * (x[n].z * ra * u.z + y[n].z * rb * v.z), 0.5f * (x[n].w * ra * u.w + y[n].w * rb * v.w));
+            make_float4(0.5f * (x[n].x * ra * u[n].x + y[n].x * rb * v[n].x), 0.5f * (x[n].y * ra * u[n].y + y[n].y * rb * v[n].y),
+                        0.5f * (x[n].z * ra * u[n].z + y[n].z * rb * v[n].z), 0.5f * (x[n].w * ra * u[n].w + y[n].w * rb * v[n].w));
     }
 }
 
@@ -293,9 +297,12 @@ __global__ void __launch_bounds__(1024) gated_group_norm_vec_kernel(const float*
                                                                     O* __restrict__ out, int groups, int group_width, int mode) {
     __shared__ float scratch[32];
     pdl_launch_dependents();
-    pdl_wait();
     const long row = blockIdx.x / groups;
     const int c0 = (int)(blockIdx.x - row * groups) * group_width;
+    if (gridDim.x <= PREFETCH_ROWS) {
+        for (int i = threadIdx.x * 32; i < group_width; i += blockDim.x * 32) prefetch_l2(weight + c0 + i);
+    }
+    pdl_wait();
     const float* py = y + row * y_stride + c0;
     const float* pg = gate + row * g_stride + c0;
     float4 v[VEC], g[VEC];
@@ -382,6 +389,18 @@ KIRAI_EXPORT int kirai_gated_group_norm_bf16(const float* y, long y_stride, cons
     return gated_group_norm_launch<bf16>(y, y_stride, gate, g_stride, weight, eps, out, rows, groups, group_width, mode, stream);
 }
 
+// (WIDE walks) A state that the last step left lies in memory: its lines are asked for ahead of the wait, a lane for each of the
+// rows that its warp will read (`mine` is the thread's own column p of row 0, lane 0's the first of the warp's 32).
+template <int REGS>
+__device__ __forceinline__ void prefetch_state_rows(const float* mine, int lane, int p, int s, int split, int rows, int cols) {
+    if (p - lane >= cols) return;
+#pragma unroll
+    for (int i = 0; i < (REGS + 31) / 32; ++i) {
+        const int row = s + (lane + 32 * i) * split;
+        if (lane + 32 * i < REGS && row < rows) prefetch_l2(mine - lane + (long)row * cols);
+    }
+}
+
 // ------------------------------------------------------------------ state-space walk
 // Block (request, head); thread (p, s): column p of the head's state [N, P], rows s, s + SPLIT, ...
 // WIDE (a block has whole runs of 32 columns): the threads of a warp have adjacent columns of the same rows, so that the state is
@@ -407,10 +426,11 @@ __global__ void __launch_bounds__(256) ssm_walk_kernel(const float* __restrict__
     const int group = head / (heads / groups);
     const int inner = heads * P, channels = inner + 2 * groups * N;
     const float decay_rate = -expf(a_log[head]), skip = d_skip[head], bias = dt_bias[head];
-    pdl_wait();
-    if (slot < 0 || slot >= num_slots) return;
     const bool live = p < P;
     float* mine = state + slot * state_len + ssm_off + ((long)head * N) * P + p;
+    if (WIDE && slot >= 0 && slot < num_slots) prefetch_state_rows<REGS>(mine, threadIdx.x & 31, p, s, split, N, P);
+    pdl_wait();
+    if (slot < 0 || slot >= num_slots) return;
     float S[REGS];
 #pragma unroll
     for (int i = 0; i < REGS; ++i) {
@@ -513,11 +533,12 @@ __global__ void __launch_bounds__(256) matrix_memory_walk_kernel(const float* __
     const int count = (int)(query_start[request + 1] - first);
     const int slot = slots[request];
     const float ib = in_bias ? in_bias[head] : 0.0f, fb = keep_bias ? keep_bias[head] : 0.0f;
-    pdl_wait();
-    if (slot < 0 || slot >= num_slots) return;
     const bool live = p < dv;
     float* base = state + slot * state_len;
     float* mine = base + ((long)head * d) * dv + p;
+    if (WIDE && slot >= 0 && slot < num_slots) prefetch_state_rows<REGS>(mine, threadIdx.x & 31, p, s, split, d, dv);
+    pdl_wait();
+    if (slot < 0 || slot >= num_slots) return;
     const float* norm = base + (long)heads * d * dv + (long)head * d;
     const float* peak_at = base + (long)heads * d * dv + (long)heads * d + head;
     float S[REGS], nn[REGS];
