@@ -125,6 +125,11 @@ __device__ __forceinline__ float ex2_approx(float x) {
 __device__ __forceinline__ uint32_t pack2_weights(float lo, float hi) {
     return __byte_perm(__float_as_uint(lo) + 0x8000u, __float_as_uint(hi) + 0x8000u, 0x7632);
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
@@ -413,10 +418,10 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
                     if (!((j >= lo || j < keep) && j <= pos)) s[i] = __float_as_uint(-INFINITY);
                 }
             }
-            // the row's maximum (four running maxima, so that the chain of dependent compares is short)
+            // the row's maximum (four running maxima, so that the chain of dependent compares is short; two scores an instruction)
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int i = 0; i < TA_BN; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(s[i]));
+            for (int i = 0; i < TA_BN; i += 2) mx[(i >> 1) & 3] = max3(mx[(i >> 1) & 3], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
             const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;  // the factor is positive
             const float m_new = fmaxf(m_used, m_tile);
             const bool grow = m_new > m_used + 8.0f || (m_used == -INFINITY && m_new != -INFINITY);
@@ -447,22 +452,28 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
                 }
             }
             const float m_sub = m_used == -INFINITY ? 0.0f : m_used;
-            // the weights: exp2(s * scale - m), one fused multiply-add and one ex2.approx per key (-inf gives 0);
+            // the weights: exp2(s * scale - m), half a packed multiply-add and one ex2.approx per key (-inf gives 0);
             // their 32 columns of bf16 pairs go over the first half of this tile's S buffer
-            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const f32x2 scale2 = pair(scale_log2, scale_log2), minus_m = pair(-m_sub, -m_sub);
+            f32x2 sum[2] = {pair(0.0f, 0.0f), pair(0.0f, 0.0f)};
 #pragma unroll
             for (int c = 0; c < TA_BN / 32; ++c) {
                 uint32_t p[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float a = ex2_approx(fmaf(__uint_as_float(s[c * 32 + 2 * i]), scale_log2, -m_sub));
-                    const float b = ex2_approx(fmaf(__uint_as_float(s[c * 32 + 2 * i + 1]), scale_log2, -m_sub));
-                    sum[i & 3] += a + b;
+                    f32x2 e = minus_m;
+                    fma2(e, pair(__uint_as_float(s[c * 32 + 2 * i]), __uint_as_float(s[c * 32 + 2 * i + 1])), scale2);
+                    float a, b;
+                    unpair(e, a, b);
+                    a = ex2_approx(a), b = ex2_approx(b);
+                    sum[i & 1] = add2(sum[i & 1], pair(a, b));
                     p[i] = pack2_weights(a, b);
                 }
                 tmem_store_32x16(s_buf + (uint32_t)(c * 16), p);
             }
-            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+            float even, odd;
+            unpair(add2(sum[0], sum[1]), even, odd);
+            l += even + odd;
             tmem_store_wait();
             if (!seen_before && !mbar_wait_hot(smem_addr(o_ready), (uint32_t)(it - 1) & 1u)) { ok = false; break; }
             tc_fence_before();
