@@ -12,6 +12,7 @@ flag that ``check_device_errors`` reads.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -93,18 +94,31 @@ launch_count = 0  # entry points called so far (each launches one to three kerne
 launch_counts: dict = {}  # the same by entry point: which kernels a step used, and how often (Engine.stats reports it)
 
 
-def _call(name: str, *args, detail: str = "") -> None:
+def _call(name: str, *args, detail: str = "", argtypes: Optional[tuple] = None) -> None:
     """Launches one entry point on the current stream.  Products that were held back to be launched together
     (see ``chained_products``) go first: launches keep the order in which they were asked for."""
     if _pending:
         flush_products()
-    _launch(name, *args, detail=detail)
+    _launch(name, *args, detail=detail, argtypes=argtypes)
 
 
-def _launch(name: str, *args, detail: str = "") -> None:
-    global launch_count
+_entry_points: dict = {}  # by name: the library's functions that return a status
+
+
+def _entry(name: str, argtypes: Optional[tuple]):
+    """The entry point ``name``, looked up once.  With ``argtypes`` it takes plain numbers (addresses among them): a product
+    has 22 arguments, and a ctypes object for each of them took the host about as long as the launch itself."""
     fn = getattr(library(), name)
     fn.restype = ctypes.c_int
+    if argtypes is not None:
+        fn.argtypes = argtypes
+    _entry_points[name] = fn
+    return fn
+
+
+def _launch(name: str, *args, detail: str = "", argtypes: Optional[tuple] = None) -> None:
+    global launch_count
+    fn = _entry_points.get(name) or _entry(name, argtypes)
     if _timer is not None:
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
@@ -153,8 +167,26 @@ _l = ctypes.c_long
 _f = ctypes.c_float
 
 
+def _types(letters: str) -> tuple:
+    """The argument types of an entry point that takes plain numbers: p an address, i an int, l a long, f a float."""
+    return tuple({"p": ctypes.c_void_p, "i": _i, "l": _l, "f": _f}[letter] for letter in letters)
+
+
+def _address(tensor: Optional[torch.Tensor]) -> Optional[int]:
+    return None if tensor is None else tensor.data_ptr()
+
+
+def _stream_address() -> int:
+    if _raw_stream is not None and _raw_device is not None:
+        return _raw_stream(_raw_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
 def error_flag(device: torch.device) -> torch.Tensor:
     """The int32 device word that kernels set instead of faulting."""
+    flag = _error_flags.get(device)
+    if flag is not None:
+        return flag
     key = torch.device(device)
     if key.index is None:
         key = torch.device("cuda", torch.cuda.current_device())
@@ -215,6 +247,9 @@ def embedding(table, ids: torch.Tensor, out: Optional[torch.Tensor] = None) -> t
 
 
 # --------------------------------------------------------------------- RMSNorm
+_ADD_RMSNORM_TYPES = _types("pppppp" "ii" "f" "p")
+
+
 def add_rmsnorm(resid: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor, eps: float,
                 out_dtype: torch.dtype, row_index: Optional[torch.Tensor] = None):
     """``resid += delta`` (32-bit, in place), then RMSNorm of the sum in ``out_dtype``.
@@ -234,8 +269,8 @@ def add_rmsnorm(resid: torch.Tensor, delta: Optional[torch.Tensor], weight: torc
     if row_index is not None:
         assert row_index.dtype == torch.int32 and row_index.is_contiguous()
         summed = torch.empty((rows, hidden), dtype=torch.float32, device=resid.device)
-    _call(f"kirai_add_rmsnorm_{_suffix(out_dtype)}", _ptr(resid), _ptr(delta), _ptr(weight), _ptr(out),
-          _ptr(row_index), _ptr(summed), _i(rows), _i(hidden), _f(eps), _stream())
+    _call("kirai_add_rmsnorm_" + _suffix(out_dtype), resid.data_ptr(), _address(delta), weight.data_ptr(), out.data_ptr(),
+          _address(row_index), _address(summed), rows, hidden, eps, _stream_address(), argtypes=_ADD_RMSNORM_TYPES)
     return (out, summed) if row_index is not None else out
 
 
@@ -1353,6 +1388,9 @@ def kv_write(k: torch.Tensor, v: torch.Tensor, cache: torch.Tensor, block_table:
           _i(page_size), _i(block_table.shape[1]), _i(num_pages), _ptr(error_flag(k.device)), _stream())
 
 
+_QK_TYPES = _types("pppppppp" "iiiii" "f" "iiii" "pp")
+
+
 def qk_norm_rope_kv_write_(qkv: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int,
                            q_weight: Optional[torch.Tensor], k_weight: Optional[torch.Tensor],
                            inv_freq: Optional[torch.Tensor], eps: float, cache: Optional[torch.Tensor],
@@ -1370,11 +1408,10 @@ def qk_norm_rope_kv_write_(qkv: torch.Tensor, q_heads: int, kv_heads: int, head_
     for w in (q_weight, k_weight):
         assert w is None or (w.dtype == torch.float32 and w.numel() == head_dim and w.is_contiguous())
     assert inv_freq is None or (inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2)
-    _call(f"kirai_qk_norm_rope_kv_write_{_suffix(qkv.dtype)}", _ptr(qkv), _ptr(q_weight), _ptr(k_weight),
-          _ptr(inv_freq), _ptr(cache if write_cache else None), _ptr(block_table), _ptr(request_of_token),
-          _ptr(positions), _i(qkv.shape[0]), _i(q_heads), _i(kv_heads), _i(head_dim), _i(head_dim), _f(eps),
-          _i(page_size), _i(block_table.shape[1]), _i(num_pages), _i(1 if write_cache else 0),
-          _ptr(error_flag(qkv.device)), _stream())
+    _call("kirai_qk_norm_rope_kv_write_" + _suffix(qkv.dtype), qkv.data_ptr(), _address(q_weight), _address(k_weight),
+          _address(inv_freq), cache.data_ptr() if write_cache else None, block_table.data_ptr(), request_of_token.data_ptr(),
+          positions.data_ptr(), qkv.shape[0], q_heads, kv_heads, head_dim, head_dim, eps, page_size, block_table.shape[1], num_pages,
+          1 if write_cache else 0, error_flag(qkv.device).data_ptr(), _stream_address(), argtypes=_QK_TYPES)
 
 
 # --------------------------------------------------------------------- attention
@@ -1522,6 +1559,9 @@ def attention_prefill_takes_tcgen05(q_heads: int, kv_heads: int, head_dim: int, 
     return head_dim <= 256 and head_dim % 8 == 0 and 128 % group == 0 and page_size & (page_size - 1) == 0
 
 
+_PREFILL_TYPES = [_types("pppppp" "iiiii" "l" "iiii" "f" + cap + "pp") for cap in ("", "f", "fp")]  # by what ``_capped`` adds
+
+
 def attention_prefill(q: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, query_start: torch.Tensor,
                       context_len: torch.Tensor, max_query_len: int, window: Optional[int], scale: float,
                       tcgen05: Optional[bool] = None, out: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
@@ -1542,10 +1582,10 @@ def attention_prefill(q: torch.Tensor, cache: torch.Tensor, block_table: torch.T
         out = torch.empty((rows, q_heads * head_dim), dtype=q.dtype, device=q.device)
     assert out.shape == (rows, q_heads * head_dim) and out.dtype == q.dtype and out.is_contiguous()
     name, cap = _capped("kirai_attention_prefill_tc_bf16" if tcgen05 else "kirai_attention_prefill_bf16", softcap, sinks, q_heads)
-    _call(name, _ptr(q), _ptr(cache), _ptr(out),
-          _ptr(block_table), _ptr(query_start), _ptr(context_len), _i(requests), _i(max_query_len), _i(q_heads), _i(kv_heads),
-          _i(head_dim), _l(q_stride), _i(page_size), _i(block_table.shape[1]), _i(num_pages), _i(mask_code(window, chunk, keep_first)), _f(scale),
-          *cap, _ptr(error_flag(q.device)), _stream(), detail=_attention_detail(q_heads, kv_heads, head_dim, window, chunk, keep_first))
+    _call(name, q.data_ptr(), cache.data_ptr(), out.data_ptr(), block_table.data_ptr(), query_start.data_ptr(), context_len.data_ptr(),
+          requests, max_query_len, q_heads, kv_heads, head_dim, q_stride, page_size, block_table.shape[1], num_pages,
+          mask_code(window, chunk, keep_first), scale, *cap, error_flag(q.device).data_ptr(), _stream_address(),
+          detail=_attention_detail(q_heads, kv_heads, head_dim, window, chunk, keep_first), argtypes=_PREFILL_TYPES[len(cap)])
     return out
 
 
@@ -2090,18 +2130,18 @@ def _chain_workspace(device: torch.device) -> torch.Tensor:
     return _chain_workspaces[key]
 
 
+_GEMM_TYPES = _types("pp" "i" "p" "iii" "ll" "ii" "piff" "ppp" "ff" "pp")
+
+
 def _launch_product(item) -> None:
     x, weight, out, n, k, width, splits, form, row_scale, resid, norm_weight, sumsq_out, gate = item
     tiled = isinstance(weight, TiledWeight)
-    if row_scale is not None:
-        sumsq, count, eps = row_scale
-        scale_args = (_ptr(sumsq), _i(sumsq.shape[0]), _f(float(count)), _f(float(eps)))
-    else:
-        scale_args = (_ptr(None), _i(0), _f(1.0), _f(0.0))
-    _launch("kirai_gemm_bf16_general", _ptr(x), _ptr(weight.boxes if tiled else weight), _i(tiled), _ptr(out), _i(x.shape[0]),
-            _i(n), _i(k), _l(x.stride(0)), _l(width), _i(splits), _i(form), *scale_args,
-            _ptr(resid), _ptr(norm_weight), _ptr(sumsq_out), _f(gate[0]), _f(gate[1]), _ptr(error_flag(x.device)), _stream(),
-            detail=f" m={x.shape[0]} n={n} k={k} form={form}" if _timer is not None else "")
+    sumsq, count, eps = row_scale if row_scale is not None else (None, 1.0, 0.0)
+    rows = x.shape[0]
+    _launch("kirai_gemm_bf16_general", x.data_ptr(), weight.boxes.data_ptr() if tiled else weight.data_ptr(), tiled, out.data_ptr(), rows,
+            n, k, x.stride(0), width, splits, form, _address(sumsq), 0 if sumsq is None else sumsq.shape[0], count, eps,
+            _address(resid), _address(norm_weight), _address(sumsq_out), gate[0], gate[1], error_flag(x.device).data_ptr(), _stream_address(),
+            detail=f" m={rows} n={n} k={k} form={form}" if _timer is not None else "", argtypes=_GEMM_TYPES)
 
 
 def flush_products() -> None:
@@ -2199,6 +2239,11 @@ def linear_tcgen05(x: torch.Tensor, weight, out_dtype: Optional[torch.dtype] = N
     return out
 
 
+@functools.lru_cache(maxsize=4096)
+def _residual_parts(m: int, n: int) -> int:
+    return int(library().kirai_gemm_bf16_residual_parts(_i(m), _i(n)))
+
+
 def linear_residual_norm(x: torch.Tensor, weight, resid: torch.Tensor, norm_weight: torch.Tensor,
                          splits: int = 0) -> tuple:
     """``resid`` [M, N] (float32, in place) += ``x`` [M, K] times ``weight`` [N, K] transposed, on the tensor cores;
@@ -2208,7 +2253,7 @@ def linear_residual_norm(x: torch.Tensor, weight, resid: torch.Tensor, norm_weig
     _need_cuda(resid, norm_weight)
     assert resid.dtype == torch.float32 and resid.shape == (m, n) and resid.is_contiguous()
     assert norm_weight.dtype == torch.float32 and norm_weight.shape == (n,) and norm_weight.is_contiguous()
-    parts = int(library().kirai_gemm_bf16_residual_parts(_i(m), _i(n)))
+    parts = _residual_parts(m, n)
     rows = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
     sumsq = torch.empty((parts, m), dtype=torch.float32, device=x.device)
     _gemm(x, weight, rows, n, k, n, splits, 3, None, resid, norm_weight, sumsq)
