@@ -113,9 +113,10 @@ class CacheManager:
     def open(self, request_id) -> Optional[RequestPages]:
         request = self.tables.open(request_id)
         if request is not None:
-            for tensor in self.state.values():
-                if tensor is not None:
-                    tensor[request.slot].zero_()
+            # (all layers' slots in one launch: one at a time took the host 10 us each before a request's first step)
+            slots = [tensor[request.slot] for tensor in self.state.values() if tensor is not None]
+            if slots:
+                torch._foreach_zero_(slots)
         return request
 
     def can_reserve(self, request: RequestPages, new_tokens: int) -> bool:

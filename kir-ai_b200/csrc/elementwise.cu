@@ -867,20 +867,24 @@ KIRAI_EXPORT int kirai_add_residual_bf16(float* resid, const void* delta, long c
 // ------------------------------------------------------------- decode advance
 // After a captured decode step: the sampled tokens become the next step's input
 // and every request moves one position on, so the same graph can be replayed
-// without the host in between.
+// without the host in between.  `report` (may be null) receives the device error word, so that a step's tokens and its
+// error word can lie side by side and reach the host in one copy.
 __global__ void decode_advance_kernel(int* __restrict__ token_ids, const int* __restrict__ sampled,
-                                      int* __restrict__ positions, int* __restrict__ context_len, int count) {
+                                      int* __restrict__ positions, int* __restrict__ context_len, int count,
+                                      const int* __restrict__ error_flag, int* __restrict__ report) {
     pdl_launch_dependents();
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0 && report) *report = *error_flag;
     if (i >= count) return;
     token_ids[i] = sampled[i];
     positions[i] += 1;
     context_len[i] += 1;
 }
 KIRAI_EXPORT int kirai_decode_advance(int* token_ids, const int* sampled, int* positions, int* context_len, int count,
-                                      cudaStream_t stream) {
+                                      const int* error_flag, int* report, cudaStream_t stream) {
     if (count <= 0) return 0;
-    const int pdl_status = launch_pdl(decode_advance_kernel, dim3((count + 127) / 128), dim3(128), 0, stream, 1u, token_ids, sampled, positions, context_len, count);
+    if (report && !error_flag) return KIRAI_ERR_BAD_SIZE;
+    const int pdl_status = launch_pdl(decode_advance_kernel, dim3((count + 127) / 128), dim3(128), 0, stream, 1u, token_ids, sampled, positions, context_len, count, error_flag, report);
     return pdl_status;
 }

@@ -2315,13 +2315,16 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def decode_advance(token_ids: torch.Tensor, sampled: torch.Tensor, positions: torch.Tensor, context_len: torch.Tensor) -> None:
-    """token_ids <- sampled; positions += 1; context_len += 1 (all int32 [R], on the device)."""
+def decode_advance(token_ids: torch.Tensor, sampled: torch.Tensor, positions: torch.Tensor, context_len: torch.Tensor,
+                   report: Optional[torch.Tensor] = None) -> None:
+    """token_ids <- sampled; positions += 1; context_len += 1 (all int32 [R], on the device); ``report`` [1] (int32) receives
+    the device error word as the kernels before left it."""
     _need_cuda(token_ids, sampled, positions, context_len)
     for t in (token_ids, sampled, positions, context_len):
         assert t.dtype == torch.int32 and t.is_contiguous() and t.numel() == token_ids.numel()
+    assert report is None or (report.dtype == torch.int32 and report.numel() == 1 and report.device == token_ids.device)
     _call("kirai_decode_advance", _ptr(token_ids), _ptr(sampled), _ptr(positions), _ptr(context_len),
-          _i(token_ids.numel()), _stream())
+          _i(token_ids.numel()), _ptr(error_flag(token_ids.device)), _ptr(report), _stream())
 
 
 # ---------------------------------------------------------------------- sampling

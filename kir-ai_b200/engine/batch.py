@@ -63,8 +63,9 @@ class StepBatch:
         return self.max_query_len == 1
 
 
-def build_batch(entries: Sequence[StepEntry], cache, device) -> StepBatch:
-    """Packs the entries (whose pages are already reserved) into a StepBatch on ``device``.
+def build_batch(entries: Sequence[StepEntry], cache, device, token_arrays: Optional[Sequence[Optional[np.ndarray]]] = None) -> StepBatch:
+    """Packs the entries (whose pages are already reserved) into a StepBatch on ``device``.  ``token_arrays``: their
+    tokens as arrays, where the caller has them already.
 
     Inside the batch the requests that bring one token come first (in their order), then the others (in theirs);
     ``want_rows`` still lists the wanted places in the order of ``entries`` and of each ``want``, so the caller's
@@ -85,7 +86,8 @@ def build_batch(entries: Sequence[StepEntry], cache, device) -> StepBatch:
     row = 0
     for index, entry in enumerate(entries):
         n = query_lens[index]
-        token_ids[row : row + n] = np.asarray(entry.tokens, dtype=np.int64)
+        tokens = token_arrays[order[index]] if token_arrays is not None else None
+        token_ids[row : row + n] = np.asarray(entry.tokens, dtype=np.int64) if tokens is None else tokens
         positions[row : row + n] = np.arange(starts[index], starts[index] + n, dtype=np.int32)
         request_of_token[row : row + n] = index
         first_row[order[index]] = row

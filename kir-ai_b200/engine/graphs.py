@@ -43,8 +43,10 @@ class DecodeGraph:
         self.table_width = table_width
         device = runner.rt.device
         groups = len(runner.cache.groups)
-        # packed int32 inputs: token_ids, positions, context_len, slots, then one table per group
-        self.sections = [B, B, B, B] + [B * table_width] * groups
+        # packed int32 inputs: token_ids (and behind them the error word, which goes back to the host with the tokens),
+        # positions, context_len, slots, one table per group, and the bits of the sampling's temperatures, top-ps and draws:
+        # one copy each way a step (each cost the host about 8 us and the device 5 us between two steps)
+        self.sections = [B + 1, B, B, B] + [B * table_width] * groups + [3 * B]
         offsets, cursor = [], 0
         for size in self.sections:
             offsets.append(cursor)
@@ -54,18 +56,18 @@ class DecodeGraph:
         # other for the step after it
         self.host_ints = [torch.zeros(cursor, dtype=torch.int32).pin_memory() for _ in range(2)]
         self.dev_ints = torch.zeros(cursor, dtype=torch.int32, device=device)
-        self.host_floats = [torch.zeros(3 * B, dtype=torch.float32).pin_memory() for _ in range(2)]
         self.loads = 0
-        self.dev_floats = torch.zeros(3 * B, dtype=torch.float32, device=device)
         self.fixed = torch.arange(B + 1, dtype=torch.int32, device=device)
 
         def section(i, source):
             return source[offsets[i] : offsets[i] + self.sections[i]]
 
-        self.token_ids, self.positions = section(0, self.dev_ints), section(1, self.dev_ints)
+        self.results = section(0, self.dev_ints)  # after a step: the tokens it sampled, then the error word
+        self.token_ids, self.positions = self.results[:B], section(1, self.dev_ints)
+        self.dev_floats = section(4 + groups, self.dev_ints).view(torch.float32)
         self.context_len, self.slots = section(2, self.dev_ints), section(3, self.dev_ints)
         self.tables = [section(4 + g, self.dev_ints).view(B, table_width) for g in range(groups)]
-        self._host = [[section(i, ints) for i in range(len(self.sections))] for ints in self.host_ints]
+        self._host = [[section(i, ints.numpy()) for i in range(len(self.sections))] for ints in self.host_ints]
         self.batch = StepBatch(
             num_tokens=B, num_requests=B, token_ids=self.token_ids, positions=self.positions,
             request_of_token=self.fixed[:B], query_start=self.fixed, context_len=self.context_len, slots=self.slots,
@@ -80,8 +82,7 @@ class DecodeGraph:
         self.kernels_per_replay = 0
         # results of launched steps come back through pinned buffers, two of them in turn: a step's result is
         # read by the host while the step after it is already queued
-        self.host_tokens = [torch.zeros(B, dtype=torch.int32).pin_memory() for _ in range(2)]
-        self.host_flag = [torch.zeros(1, dtype=torch.int32).pin_memory() for _ in range(2)]
+        self.host_results = [torch.zeros(B + 1, dtype=torch.int32).pin_memory() for _ in range(2)]
         self.launches = 0
 
     def _body(self) -> None:
@@ -92,42 +93,39 @@ class DecodeGraph:
         B = self.num_requests
         floats = self.dev_floats
         self.tokens_out = ops.sample_rows(logits, floats[:B], floats[B : 2 * B], floats[2 * B :])
-        ops.decode_advance(self.token_ids, self.tokens_out, self.positions, self.context_len)
+        ops.decode_advance(self.token_ids, self.tokens_out, self.positions, self.context_len, self.results[B:])
 
     def load_inputs(self, token_ids: Optional[Sequence[int]], positions: Sequence[int], slots: Sequence[int],
                     tables: Sequence[np.ndarray], temperatures: Sequence[float], top_ps: Sequence[float],
                     draws: Sequence[float]) -> None:
-        """Copies a step's inputs from pinned host memory to the fixed device buffers (two copies).
+        """Copies a step's inputs from pinned host memory to the fixed device buffers (one copy).
         ``token_ids`` None leaves the token buffer as the step before left it: the tokens it sampled."""
         B = self.num_requests
         turn = self.loads & 1
         self.loads += 1
-        host, host_ints, host_floats = self._host[turn], self.host_ints[turn], self.host_floats[turn]
+        host, host_ints = self._host[turn], self.host_ints[turn]
         if token_ids is not None:
-            host[0].copy_(torch.as_tensor(token_ids, dtype=torch.int32))
-        position_tensor = torch.as_tensor(positions, dtype=torch.int32)
-        host[1].copy_(position_tensor)
-        host[2].copy_(position_tensor + 1)
-        host[3].copy_(torch.as_tensor(slots, dtype=torch.int32))
+            host[0][:B] = token_ids
+        host[1][:] = positions
+        np.add(host[1], 1, out=host[2])
+        host[3][:] = slots
         for g, table in enumerate(tables):
-            padded = np.full((B, self.table_width), -1, dtype=np.int32)
-            padded[:, : table.shape[1]] = table
-            host[4 + g].copy_(torch.from_numpy(padded.reshape(-1)))
-        host_floats[:B] = torch.as_tensor(temperatures, dtype=torch.float32)
-        host_floats[B : 2 * B] = torch.as_tensor(top_ps, dtype=torch.float32)
-        host_floats[2 * B :] = torch.as_tensor(draws, dtype=torch.float32)
+            rows = host[4 + g].reshape(B, self.table_width)
+            rows[:, : table.shape[1]] = table
+            rows[:, table.shape[1] :] = -1
+        floats = host[-1].view(np.float32)
+        floats[:B], floats[B : 2 * B], floats[2 * B :] = temperatures, top_ps, draws
         first = 0 if token_ids is not None else self.offsets[1]
         self.dev_ints[first:].copy_(host_ints[first:], non_blocking=True)
-        self.dev_floats.copy_(host_floats, non_blocking=True)
 
     @property
     def input_bytes(self) -> int:
-        return self.host_ints[0].numel() * 4 + self.host_floats[0].numel() * 4
+        return self.host_ints[0].numel() * 4
 
     @property
     def ahead_input_bytes(self) -> int:
         """What a step copies that takes its tokens from the step before it on the device."""
-        return (self.host_ints[0].numel() - self.offsets[1]) * 4 + self.host_floats[0].numel() * 4
+        return (self.host_ints[0].numel() - self.offsets[1]) * 4
 
     def capture(self) -> None:
         """Runs the step once eagerly (so that everything lazy has happened), then captures it.
@@ -174,8 +172,7 @@ class DecodeGraph:
         index = self.launches & 1
         self.launches += 1
         self.graph.replay()
-        self.host_tokens[index].copy_(self.tokens_out, non_blocking=True)
-        self.host_flag[index].copy_(self.runner.rt.ops.error_flag(self.runner.rt.device), non_blocking=True)
+        self.host_results[index].copy_(self.results, non_blocking=True)
         event = torch.cuda.Event()
         event.record()
         return LaunchedStep(self, index, event)
@@ -190,11 +187,10 @@ class LaunchedStep:
     def wait(self) -> List[int]:
         """Waits for the step; raises if a kernel set the device error word; returns the sampled tokens."""
         self.event.synchronize()
-        ops = self.graph.runner.rt.ops
-        value = int(self.graph.host_flag[self.index][0])
-        if value != 0:
-            ops.check_device_errors(self.graph.runner.rt.device)  # reads, clears and raises
-        return self.graph.host_tokens[self.index].tolist()
+        *tokens, error = self.graph.host_results[self.index].tolist()
+        if error != 0:
+            self.graph.runner.rt.ops.check_device_errors(self.graph.runner.rt.device)  # reads, clears and raises
+        return tokens
 
 
 class DecodeGraphs:

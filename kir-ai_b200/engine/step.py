@@ -12,8 +12,9 @@ concurrent requests as independent threads.
 """
 from __future__ import annotations
 
-from typing import Optional, Sequence
+from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .batch import StepEntry, build_batch
@@ -27,8 +28,19 @@ class StepError(ValueError):
     """A malformed step (bad token id, empty run, wanted place out of range...)."""
 
 
-def check_entries(entries: Sequence[StepEntry], vocab_size: int, max_positions: Optional[int]) -> None:
+def _token_array(tokens) -> Optional[np.ndarray]:
+    """The token ids as one array (None where numpy cannot make one of them)."""
+    try:
+        array = np.asarray(tokens, dtype=np.int64)
+    except (OverflowError, TypeError, ValueError):
+        return None
+    return array if array.ndim == 1 else None
+
+
+def check_entries(entries: Sequence[StepEntry], vocab_size: int, max_positions: Optional[int]) -> List[Optional[np.ndarray]]:
+    """Raises for a malformed step; returns every entry's tokens as an array."""
     seen = set()
+    arrays: List[Optional[np.ndarray]] = []
     for entry in entries:
         request = entry.request
         if id(request) in seen:
@@ -39,9 +51,13 @@ def check_entries(entries: Sequence[StepEntry], vocab_size: int, max_positions: 
         n = len(entry.tokens)
         if n == 0:
             raise StepError(f"request {request.request_id!r} brings no tokens")
-        for token in entry.tokens:
-            if not 0 <= int(token) < vocab_size:
-                raise StepError(f"token id {token} outside vocab size {vocab_size}")
+        # (a loop over a portion of 2,048 tokens took 0.2 ms, with the device waiting; it is left to name the bad one)
+        array = _token_array(entry.tokens)
+        if array is None or array.min() < 0 or array.max() >= vocab_size:
+            for token in entry.tokens:
+                if not 0 <= int(token) < vocab_size:
+                    raise StepError(f"token id {token} outside vocab size {vocab_size}")
+        arrays.append(array)
         for place in entry.want:
             if not 0 <= int(place) < n:
                 raise StepError(f"request {request.request_id!r}: wanted place {place} is outside its {n} tokens")
@@ -49,6 +65,7 @@ def check_entries(entries: Sequence[StepEntry], vocab_size: int, max_positions: 
             raise StepError(
                 f"request {request.request_id!r}: {request.length + n} tokens exceed the model's {max_positions} positions"
             )
+    return arrays
 
 
 def reserve_all(entries: Sequence[StepEntry], cache) -> None:
@@ -70,9 +87,9 @@ def run_step(model, cache, entries: Sequence[StepEntry], *, check_errors: bool =
     """Runs one step; returns logits [wanted, vocab] (float32, on the device) or None if nothing is wanted."""
     if not entries:
         return None
-    check_entries(entries, model.plan.vocab_size, model.plan.max_positions)
+    arrays = check_entries(entries, model.plan.vocab_size, model.plan.max_positions)
     reserve_all(entries, cache)
-    batch = build_batch(entries, cache, model.rt.device)
+    batch = build_batch(entries, cache, model.rt.device, arrays)
     resid, delta = model.forward(batch, cache)
     logits = model.logits(resid, delta, batch.want_rows) if batch.num_want else None
     for entry in entries:
