@@ -1096,3 +1096,49 @@ def test_decode_attention_of_the_largest_crowds(ops, requests, kv_heads, head_di
             # weights and result are rounded to bfloat16 (2^-9 each) on values of up to about 4
             assert float((got.float() - plain).abs().max()) <= 2.5e-2, (warps, splits)
     ops.check_device_errors(torch.device(DEV))
+
+
+@pytest.mark.parametrize("tokens,rot_dims,norm", [(1, 64, False), (3, 128, True), (255, 64, True), (256, 64, True), (300, 32, False)])
+def test_rotated_heads_spread_over_blocks(ops, tokens, rot_dims, norm):
+    """Below 256 tokens a token's heads go over several blocks (29 here: a last block with part of its warps idle); every row is
+    what the token makes alone, and the rotation's formula."""
+    nq, nkv, dim, page = 17, 6, 128, 16
+    rows = rand(tokens, (nq + 2 * nkv) * dim, seed=tokens)
+    freq = (10000.0 ** (-torch.arange(rot_dims // 2, dtype=torch.float64) * 2 / rot_dims)).float().to(DEV)
+    weights = dict(q_norm=(1.0 + 0.1 * rand(dim, seed=1)).contiguous(), k_norm=(1.0 + 0.1 * rand(dim, seed=2)).contiguous(), norm_eps=1e-6) if norm else {}
+    pages = -(-tokens // page)
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(3)).int().view(1, -1).to(DEV)
+    positions, request = torch.arange(tokens, dtype=torch.int32, device=DEV), torch.zeros(tokens, dtype=torch.int32, device=DEV)
+
+    def prepare(cache, first, last):
+        return ops.qkv_rope_write(rows[first:last], nq, nkv, dim, dim, dim, None, None, None, None, freq, 0, rot_dims, cache, table,
+                                  request[first:last], positions[first:last], torch.float32, **weights)
+
+    whole, one = (torch.zeros(pages, 2, nkv, page, dim, device=DEV) for _ in range(2))
+    q = prepare(whole, 0, tokens)
+    alone = torch.cat([prepare(one, t, t + 1) for t in range(tokens)])
+    ops.check_device_errors(torch.device(DEV))
+    assert torch.equal(q, alone) and torch.equal(whole, one)
+    x = rows[:, : nq * dim].double().view(tokens, nq, dim)
+    if norm:
+        x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6) * weights["q_norm"].double()
+    angle = (positions.float()[:, None] * freq[None]).double()
+    half = rot_dims // 2
+    c, s, a, b = angle.cos()[:, None], angle.sin()[:, None], x[..., :half], x[..., half:rot_dims]
+    expected = torch.cat([a * c - b * s, b * c + a * s, x[..., rot_dims:]], dim=-1)
+    # a handful of 32-bit operations on values of a few units (the sum of squares has 128 terms in a tree of depth 9)
+    assert float((q.double() - expected).abs().max()) <= 16 * 2.0 ** -24 * float(expected.abs().max())
+
+
+def test_the_error_word_leaves_a_step_beside_its_tokens(ops):
+    sampled = torch.tensor([5, 9, 2], dtype=torch.int32, device=DEV)
+    results = torch.full((4,), 77, dtype=torch.int32, device=DEV)
+    positions, lengths = torch.tensor([3, 4, 5], dtype=torch.int32, device=DEV), torch.tensor([4, 5, 6], dtype=torch.int32, device=DEV)
+    flag = ops.error_flag(torch.device(DEV))
+    for word in (0, 3):
+        flag.fill_(word)
+        ops.decode_advance(results[:3], sampled, positions, lengths, results[3:])
+        assert results.tolist() == [5, 9, 2, word]
+    flag.zero_()
+    ops.decode_advance(results[:3], sampled, positions, lengths)
+    assert results.tolist() == [5, 9, 2, 3] and positions.tolist() == [6, 7, 8] and lengths.tolist() == [7, 8, 9]

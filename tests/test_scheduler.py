@@ -377,3 +377,17 @@ def test_native_scheduler_decides_as_the_python_model_does():
         assert got == expected, f"seed {seed}"
         evictions += preempted
     assert evictions > 20  # the workloads do run out of pages
+
+
+@pytest.mark.parametrize("tokens,good", [([0, 5, 99], True), ([3, -1], False), ([100], False), ([5] * 40 + [1 << 70], False), ((7, 8), True)])
+def test_a_steps_tokens_are_checked_as_an_array(tokens, good):
+    from kirai_b200.engine.batch import StepEntry
+    from kirai_b200.engine.step import StepError, check_entries
+
+    cache = CacheManager([KVCacheNeed(1, 8, None)], page_size=4, num_pages=64, num_slots=2, device=None)
+    entries = [StepEntry(cache.open("a"), tokens, [])]
+    if good:
+        assert check_entries(entries, 100, None)[0].tolist() == list(tokens)
+    else:
+        with pytest.raises(StepError, match="outside vocab size 100"):
+            check_entries(entries, 100, None)
