@@ -143,7 +143,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
                             long q_row_stride, int page_size, int box_rows, int piece_rows, int table_width, int num_pages,
                             int window, ScoreForm form, int* __restrict__ error_flag) {
     pdl_launch_dependents();
-    pdl_wait();
     using Smem = TcAttnSmem<D>;
     constexpr int PANELS = Smem::panels;
     const float scale_log2 = form.cap_log2 != 0.0f ? 1.0f : form.scale_log2;  // capped scores are in the exponent's units already
@@ -203,30 +202,42 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
         mbar_init(smem_addr(o_ready), 1);
         mbar_fence_init();
     }
-    if (warp == 1) {
-        tmem_alloc(smem_addr(tmem_slot), TaTmem<D>::cols);
-        tmem_relinquish();
-    }
-    // Q tile: row r is token (row0 + r) / group, head kv_head * group + (row0 + r) % group
     {
-        constexpr int CH = D / 8;
-        const int chunks_used = head_dim / 8;
-        for (int id = tid; id < TA_ROWS * CH; id += TA_THREADS) {
-            const int r = id / CH, chunk = id % CH;
-            const int row = row0 + r;
-            uint4 value = make_uint4(0u, 0u, 0u, 0u);
-            if (row < rows_total && chunk < chunks_used) {
-                const int token = row / group, head = kv_head * group + row % group;
-                value = *reinterpret_cast<const uint4*>(q + (size_t)(q_begin + token) * q_row_stride + (size_t)head * head_dim + chunk * 8);
-            }
-            *reinterpret_cast<uint4*>(smem + panel_offset<TA_ROWS>(r, chunk)) = value;
-        }
-        // the block table of the keys this CTA reads
+        // the block table of the keys this CTA reads (like the lengths above it came with the step's inputs, which no kernel
+        // ahead writes; what kernels make, the queries and this step's keys and values, is read after the wait)
         const int* table_g = block_table + (long)req * table_width;
         const int first_page = runs.kept ? 0 : (first_tile * TA_BN) / page_size;
         const int last_page = min(table_width - 1, pos_last / page_size);
         if (last_page - first_page < Smem::table_entries)
             for (int i = first_page + tid; i <= last_page; i += TA_THREADS) table_s[i - first_page] = table_g[i];
+    }
+    pdl_wait();
+    if (warp == 1) {
+        tmem_alloc(smem_addr(tmem_slot), TaTmem<D>::cols);
+        tmem_relinquish();
+    }
+    // Q tile: row r is token (row0 + r) / group, head kv_head * group + (row0 + r) % group; ten pieces of 16 bytes of a thread
+    // are asked for before the first is stored (one at a time, with a division each, they were a third of a short prompt's launch)
+    {
+        constexpr int CH = D / 8, PIECES = 10;
+        const int chunks_used = head_dim / 8, group_shift = __ffs(group) - 1;  // (the group divides 128)
+        for (int first = tid; first < TA_ROWS * CH; first += TA_THREADS * PIECES) {
+            uint4 value[PIECES];
+#pragma unroll
+            for (int n = 0; n < PIECES; ++n) {
+                const int id = first + n * TA_THREADS, chunk = id % CH, row = row0 + id / CH;
+                value[n] = make_uint4(0u, 0u, 0u, 0u);
+                if (id < TA_ROWS * CH && row < rows_total && chunk < chunks_used) {
+                    const int token = row >> group_shift, head = (kv_head << group_shift) + (row & (group - 1));
+                    value[n] = *reinterpret_cast<const uint4*>(q + (size_t)(q_begin + token) * q_row_stride + (size_t)head * head_dim + chunk * 8);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < PIECES; ++n) {
+                const int id = first + n * TA_THREADS;
+                if (id < TA_ROWS * CH) *reinterpret_cast<uint4*>(smem + panel_offset<TA_ROWS>(id / CH, id % CH)) = value[n];
+            }
+        }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the MMAs read the Q tile through the async proxy
     tc_fence_before();
