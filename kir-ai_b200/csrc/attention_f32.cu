@@ -5,8 +5,9 @@
 // many query rows.
 //
 // Prompt kernel: a CTA takes 64 query rows of one kv head's group (64 / group tokens, all heads of the group) over tiles of 64
-// keys.  128 threads hold 8 x 4 scores and 8 x (head columns / 16) results each; the operands of four columns come from
-// shared memory as 16-byte loads (16 wavefronts for 128 FMAs a lane, so that the FMA pipe and not shared memory sets the
+// keys.  256 threads hold 4 x 4 scores and 4 x (head columns / 16) results each (with 128 threads and 8 x 4 an SM had eight
+// warps, too few to hide the barriers of a tile); the operands of four columns come from
+// shared memory as 16-byte loads (12 wavefronts for 64 FMAs a lane, so that the FMA pipe and not shared memory sets the
 // pace), and `fma.rn.f32x2` halves the instructions.  Bound by the FMA pipe: the 4B shape's layer (32 heads of 128, 8 kv
 // heads) at 515 tokens is 2.2 GFLOP, 30 us at 72 TFLOP/s; measured 130 us (plain kernel: 1,139), the heaviest row tile's nine key tiles one after
 // another setting the end.  Weights overlay the key tile, so that a CTA takes 101 KB and
@@ -23,7 +24,9 @@
 
 #define AF_ROWS 64
 #define AF_KEYS 64
-#define AF_THREADS 128
+#define AF_THREADS 256
+#define AF_TY (AF_THREADS / 16)   // threads along the query rows (sixteen stand along the keys and the columns)
+#define AF_R (AF_ROWS / AF_TY)    // query rows of a thread
 #define AF_PSTRIDE (AF_KEYS + 4)
 
 __device__ __forceinline__ void copy_16(float* dst, const float* src, bool present) {
@@ -51,14 +54,14 @@ __device__ __forceinline__ long key_row(const int* table, int j, int page_size, 
 // The weighted sum of one tile.  EDGE: some row of the CTA does not see some key of the tile; such a key's value is then
 // not multiplied at all (a weight of 0 would still make NaN of an infinite value that the row may not see).
 template <int DP, bool EDGE>
-__device__ __forceinline__ void weighted_sum(f32x2 (&o)[8][DP / 32], const float* __restrict__ p_s, const float* __restrict__ v_s,
-                                             const long* __restrict__ base_s, int key0, const int (&pos)[8], int window, int keep,
+__device__ __forceinline__ void weighted_sum(f32x2 (&o)[AF_R][DP / 32], const float* __restrict__ p_s, const float* __restrict__ v_s,
+                                             const long* __restrict__ base_s, int key0, const int (&pos)[AF_R], int window, int keep,
                                              int ty, int tx) {
 #pragma unroll 2
     for (int k = 0; k < AF_KEYS; k += 4) {
-        float4 p[8];
+        float4 p[AF_R];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) p[i] = *reinterpret_cast<const float4*>(p_s + (ty + 8 * i) * AF_PSTRIDE + k);
+        for (int i = 0; i < AF_R; ++i) p[i] = *reinterpret_cast<const float4*>(p_s + (ty + AF_TY * i) * AF_PSTRIDE + k);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             f32x2 v[DP / 32];
@@ -70,7 +73,7 @@ __device__ __forceinline__ void weighted_sum(f32x2 (&o)[8][DP / 32], const float
             const int j = key0 + k + u;
             const bool present = EDGE ? base_s[k + u] >= 0 : true;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < AF_R; ++i) {
                 if (EDGE && !(present && j <= pos[i] && (j >= first_visible_key(pos[i], window) || j < keep))) continue;
                 const float w = u == 0 ? p[i].x : u == 1 ? p[i].y : u == 2 ? p[i].z : p[i].w;
                 const f32x2 ww = pair(w, w);
@@ -87,7 +90,7 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
                              const int* __restrict__ block_table, const int* __restrict__ query_start,
                              const int* __restrict__ context_len, int q_heads, int kv_heads, int head_dim, long q_row_stride,
                              int page_size, int table_width, int num_pages, int mask, float scale, float softcap,
-                             const float* __restrict__ sinks, int* __restrict__ error_flag) {
+                             const float* __restrict__ sinks, int first_tiles, int* __restrict__ error_flag) {
     extern __shared__ float4 smem4[];
     float* q_s = reinterpret_cast<float*>(smem4);        // [AF_ROWS][DP + 4]
     float* k_s = q_s + AF_ROWS * (DP + 4);               // [AF_KEYS][DP + 4], then the weights [AF_ROWS][AF_PSTRIDE]
@@ -102,7 +105,10 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
     const int tokens_per_tile = AF_ROWS / group;
     const int row0 = query_start[request], run = query_start[request + 1] - row0;
     const int row_tiles = (run + tokens_per_tile - 1) / tokens_per_tile;
-    const int row_tile = row_tiles - 1 - (int)blockIdx.y;  // the longest rows of keys are handed out first
+    // the longest rows of keys are handed out first; where all CTAs start at once, two to an SM (`first_tiles` > 0), the second
+    // ones, from row tile `first_tiles` of the order on, come shortest first, so that an SM's two add up alike
+    const int place = blockIdx.y;
+    const int row_tile = first_tiles > 0 && row_tiles == (int)gridDim.y && place >= first_tiles ? place - first_tiles : row_tiles - 1 - place;
     if (row_tile < 0) return;
     const int token0 = row_tile * tokens_per_tile;
     const int first_pos = context_len[request] - run;
@@ -112,9 +118,9 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
     const int* table = block_table + (long)request * table_width;
     const int columns4 = head_dim >> 2;
 
-    int pos[8];
+    int pos[AF_R];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) pos[i] = min(first_pos + token0 + (ty + 8 * i) / group, last_pos);
+    for (int i = 0; i < AF_R; ++i) pos[i] = min(first_pos + token0 + (ty + AF_TY * i) / group, last_pos);
     const int tile_first_pos = first_pos + token0;
     const int lo_first = first_visible_key(tile_first_pos, window);
     const int lo_last = first_visible_key(last_pos, window);
@@ -153,10 +159,10 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
     fetch(k_s, DP + 4, 0, 0);
     copy_commit();
 
-    f32x2 o[8][DP / 32];
-    float m[8], l[8];
+    f32x2 o[AF_R][DP / 32];
+    float m[AF_R], l[AF_R];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < AF_R; ++i) {
         m[i] = -INFINITY, l[i] = 0.0f;
 #pragma unroll
         for (int c = 0; c < DP / 32; ++c) o[i][c] = 0ull;
@@ -173,20 +179,20 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
         copy_commit();
         if (it + 1 < tiles) find_rows(it + 1);
 
-        f32x2 s2[8][4];
+        f32x2 s2[AF_R][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < AF_R; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s2[i][j] = 0ull;
 #pragma unroll 2
         for (int c = 0; c < head_dim; c += 4) {
-            ulonglong2 a[8], b[4];
+            ulonglong2 a[AF_R], b[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const ulonglong2*>(k_s + (tx + 16 * j) * (DP + 4) + c);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 8 * i) * (DP + 4) + c);
+            for (int i = 0; i < AF_R; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + AF_TY * i) * (DP + 4) + c);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < AF_R; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     fma2(s2[i][j], a[i].x, b[j].x);
@@ -195,7 +201,7 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
         }
         __syncthreads();  // the keys have been read: the weights take their place
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < AF_R; ++i) {
             float s[4];
             bool seen[4];
             float top = m[i];
@@ -218,7 +224,7 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
             for (int j = 0; j < 4; ++j) {
                 const float w = seen[j] ? expf(s[j] - top) : 0.0f;
                 sum += w;
-                p_s[(ty + 8 * i) * AF_PSTRIDE + tx + 16 * j] = w;
+                p_s[(ty + AF_TY * i) * AF_PSTRIDE + tx + 16 * j] = w;
             }
             l[i] = l[i] * corr + sum;  // this thread's keys only; the sixteen threads of a row meet at the end
             m[i] = top;
@@ -237,11 +243,11 @@ attention_f32_prefill_kernel(const float* __restrict__ q, const float* __restric
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < AF_R; ++i) {
         float sum = l[i];
 #pragma unroll
         for (int offset = 8; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
-        const int r = ty + 8 * i, token = token0 + r / group;
+        const int r = ty + AF_TY * i, token = token0 + r / group;
         if (r >= tokens_per_tile * group || token >= run) continue;
         const int head = kv_head * group + r % group;
         float* row = out + ((size_t)(row0 + token) * q_heads + head) * head_dim;
@@ -441,9 +447,16 @@ static int attention_f32_prefill_launch(dim3 grid, cudaStream_t stream, const fl
     const size_t smem = (size_t)(AF_ROWS * (DP + 4) + AF_KEYS * (DP + 4) + AF_KEYS * DP) * sizeof(float);
     const cudaError_t err = cudaFuncSetAttribute(attention_f32_prefill_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
+    static const int sms = [] {
+        int device = 0, value = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
+        return value;
+    }();
+    const long ctas = (long)grid.x * grid.y;
+    const int first_tiles = grid.z == 1 && ctas > sms && ctas <= 2L * sms ? sms / (int)grid.x : 0;
     return launch_pdl(attention_f32_prefill_kernel<DP>, grid, dim3(AF_THREADS), smem, stream, 1u, q, cache, out, block_table,
                       query_start, context_len, q_heads, kv_heads, head_dim, q_row_stride, page_size, table_width, num_pages,
-                      mask, scale, softcap, sinks, error_flag);
+                      mask, scale, softcap, sinks, first_tiles, error_flag);
 }
 
 // Runs of new tokens: query_start [requests + 1] rows of q and out, context_len [requests] tokens in the cache after the step.
