@@ -357,13 +357,17 @@ int launch_tc(const float* A, const float* W, const bf16* planes, float* C, int 
 // A split has to save a twentieth.  (Of all cuts, swept over 4 weight sizes and 9 to 800 rows, this takes the fastest.)
 struct Cut {
     int bn, splits;
+    float us;  // by the times above
 };
+static constexpr int cut_rows[4] = {32, 64, 128, 192};
+static constexpr float cut_block_us[4] = {0.66f, 0.58f, 0.70f, 0.88f};
 static Cut choose_cut(int M, int N, int K) {
-    constexpr int bns[4] = {32, 64, 128, 192}, cuts[5] = {1, 2, 3, 4, 8}, at_once[5] = {148, 148, 120, 132, 112};
-    constexpr float block_us[4] = {0.66f, 0.58f, 0.70f, 0.88f};
+    constexpr int cuts[5] = {1, 2, 3, 4, 8}, at_once[5] = {148, 148, 120, 132, 112};
+    constexpr const int* bns = cut_rows;
+    constexpr const float* block_us = cut_block_us;
     const int blocks = (K + BLOCK_K - 1) / BLOCK_K;
     const long columns = (N + TILE_N - 1) / TILE_N;
-    Cut best{192, 1};
+    Cut best{192, 1, 0.0f};
     float least = 0.0f;
     for (int b = 0; b < 4; ++b) {
         if (b > 0 && bns[b - 1] >= M) break;  // one tile already takes every row
@@ -378,11 +382,43 @@ static Cut choose_cut(int M, int N, int K) {
             const float total = (float)rounds * (8.0f + us * (float)((blocks + s - 1) / s)) * (s > 1 ? 1.05f : 1.0f);
             if (least == 0.0f || total < least) {
                 least = total;
-                best = Cut{bns[b], s};
+                best = Cut{bns[b], s, total};
             }
         }
     }
     return best;
+}
+
+// Where a product's tiles fill a few rounds and a little of one more (456 CTAs of 192 rows on 148 SMs: four rounds, the last with
+// 12), the columns of the whole rounds are one launch and the rest a second one with a cut of its own, finer along K, which
+// starts as the first one's CTAs end.  How many columns (a multiple of TILE_N) the first launch takes and its rows a tile;
+// 0 where one launch is as good to a twentieth.
+static int whole_rounds(int M, int N, int K, float single_us, int* bn) {
+    const int blocks = (K + BLOCK_K - 1) / BLOCK_K;
+    const long columns = (N + TILE_N - 1) / TILE_N;
+    float least = 0.95f * single_us;
+    int taken = 0;
+    for (int b = 0; b < 4; ++b) {
+        if (b > 0 && cut_rows[b - 1] >= M) break;
+        const long row_tiles = (M + cut_rows[b] - 1) / cut_rows[b], room = cut_rows[b] <= 64 ? 296 : 148;
+        const long rounds = columns * row_tiles / room, first = rounds * room / row_tiles;
+        if (rounds < 1 || first < 1 || first >= columns) continue;
+        const float us = (cut_rows[b] == 64 ? 0.90f : cut_block_us[b]) * (float)blocks;
+        const float total = (float)rounds * (8.0f + us) + choose_cut(M, (int)(N - first * TILE_N), K).us;
+        if (total < least) least = total, taken = (int)first * TILE_N, *bn = cut_rows[b];
+    }
+    return taken;
+}
+
+static int launch_cut(const Cut& cut, const float* A, const float* W, bf16* planes, float* C, int M, int N, int K, long lda, long ldc, int pitch,
+                      int constant, int* error_flag, cudaStream_t stream) {
+    switch (cut.bn) {
+        case 32: return launch_tc<32>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+        case 64: return launch_tc<64>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+        case 128: return launch_tc<128>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+        case 192: return launch_tc<192>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+    }
+    return KIRAI_ERR_BAD_SIZE;
 }
 
 // planes: 3 M pitch bf16 of scratch, pitch = K rounded up to a multiple of 8.  K and the row stride of A multiples of 4, A, W
@@ -399,7 +435,9 @@ KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || (long)3 * M > 0x7fffffffL || splits < 0 || splits > 8) return KIRAI_ERR_BAD_SIZE;
     if (K % 4 != 0 || lda % 4 != 0 || (((uintptr_t)A_ | (uintptr_t)W_ | (uintptr_t)planes_) & 15) != 0) return KIRAI_ERR_BAD_ALIGN;
-    const Cut cut = bn == 0 ? choose_cut(M, N, K) : Cut{bn, splits > 0 ? splits : 1};
+    const Cut cut = bn == 0 ? choose_cut(M, N, K) : Cut{bn, splits > 0 ? splits : 1, 0.0f};
+    int first_bn = 0;
+    const int first = bn == 0 && splits == 0 ? whole_rounds(M, N, K, cut.us, &first_bn) : 0;
     const int pitch = (K + 7) / 8 * 8;
     const long quads = (long)M * (K / 4);
     const long cut_blocks = (quads + 255) / 256;
@@ -409,11 +447,11 @@ KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_
     const int status = launch_pdl(f32_planes_kernel, dim3((unsigned)cut_blocks), dim3(256), 0, stream, 1u, A, planes, M, K, lda, pitch);
     if (status != 0) return status;
     float* C = (float*)C_;
-    switch (cut.bn) {
-        case 32: return launch_tc<32>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
-        case 64: return launch_tc<64>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
-        case 128: return launch_tc<128>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
-        case 192: return launch_tc<192>(A, W, planes, C, M, N, K, lda, ldc, pitch, cut.splits, constant, error_flag, stream);
+    if (first > 0) {
+        const int done = launch_cut(Cut{first_bn, 1, 0.0f}, A, W, planes, C, M, first, K, lda, ldc, pitch, constant, error_flag, stream);
+        if (done != 0) return done;
+        return launch_cut(choose_cut(M, N - first, K), A, W + (size_t)first * K, planes, C + first, M, N - first, K, lda, ldc, pitch, constant,
+                          error_flag, stream);
     }
-    return KIRAI_ERR_BAD_SIZE;
+    return launch_cut(cut, A, W, planes, C, M, N, K, lda, ldc, pitch, constant, error_flag, stream);
 }

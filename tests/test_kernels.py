@@ -163,6 +163,19 @@ def test_linear_float32_on_tensor_cores(ops, m, n, k):
         ops.linear_f32_tc(rand(m, k + 9)[:, 1 : 1 + k], w)
 
 
+# products whose tiles fill whole rounds of 148 SMs and a little of another: two launches (192, 128 and 32 rows a tile), the second
+# with a part of a tile of columns, K split, a part of a block of K
+@pytest.mark.parametrize("m,n,k", [(515, 19456, 516), (576, 6400 + 60, 1028), (128, 19200, 700), (30, 38400 + 4, 260)])
+def test_linear_float32_in_whole_rounds_and_a_rest(ops, m, n, k):
+    x, w = rand(m, k), rand(n, k, seed=3)
+    expected = x.double() @ w.double().T
+    bound = (14 * 2.0 ** -23 + (k / 32 + 8) * 2.0 ** -24) * (x.abs().double() @ w.abs().double().T)  # as above
+    out = ops.linear_f32_tc(x, w)
+    ops.check_device_errors(torch.device(DEV))
+    assert bool(((out.double() - expected).abs() <= bound).all())
+    assert torch.equal(out, ops.linear_f32_tc(x, w, constant=True))
+
+
 @pytest.mark.parametrize("m", [1, 8, 40, 200])
 def test_linear_float32_reads_weights_that_the_kernel_before_it_wrote(ops, m):
     """A weight made by the launch just ahead in the stream, one after the other in the same memory; and the same bits from
