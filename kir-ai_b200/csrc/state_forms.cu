@@ -146,7 +146,9 @@ __global__ void rms_pair_mean_kernel(const float* __restrict__ a, const float* _
 
 // The same with 16-byte accesses, both rows kept in registers (up to four pieces a thread) and both sums in one pass through
 // shared memory: 17 us a launch at three rows of 4,096 before, under 4 now.
-__global__ void rms_pair_mean_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ wa,
+// EARLY: the weights too are asked for ahead of the sums (up to 512 threads: a block of 1,024 has no registers for them).
+template <bool EARLY>
+__global__ void __launch_bounds__(EARLY ? 512 : 1024) rms_pair_mean_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ wa,
                                          const float* __restrict__ wb, float eps, float* __restrict__ out, int width) {
     __shared__ float2 scratch[32];
     pdl_launch_dependents();
@@ -164,7 +166,7 @@ __global__ void rms_pair_mean_vec_kernel(const float* __restrict__ a, const floa
         const bool inside = c < width;
         x[n] = inside ? *reinterpret_cast<const float4*>(pa + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         y[n] = inside ? *reinterpret_cast<const float4*>(pb + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (inside) u[n] = *reinterpret_cast<const float4*>(wa + c), v[n] = *reinterpret_cast<const float4*>(wb + c);
+        if (EARLY && inside) u[n] = *reinterpret_cast<const float4*>(wa + c), v[n] = *reinterpret_cast<const float4*>(wb + c);
     }
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -181,6 +183,7 @@ __global__ void rms_pair_mean_vec_kernel(const float* __restrict__ a, const floa
     for (int n = 0; n < 4; ++n) {
         const int c = (n * blockDim.x + threadIdx.x) * 4;
         if (c >= width) break;
+        if (!EARLY) u[n] = *reinterpret_cast<const float4*>(wa + c), v[n] = *reinterpret_cast<const float4*>(wb + c);
         *reinterpret_cast<float4*>(out + (long)blockIdx.x * width + c) =
             make_float4(0.5f * (x[n].x * ra * u[n].x + y[n].x * rb * v[n].x), 0.5f * (x[n].y * ra * u[n].y + y[n].y * rb * v[n].y),
                         0.5f * (x[n].z * ra * u[n].z + y[n].z * rb * v[n].z), 0.5f * (x[n].w * ra * u[n].w + y[n].w * rb * v[n].w));
@@ -193,7 +196,7 @@ KIRAI_EXPORT int kirai_rms_pair_mean(const float* a, const float* b, const float
     if (width <= 0) return KIRAI_ERR_BAD_SIZE;
     if (width % 4 == 0 && width <= 16384 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)wa | (uintptr_t)wb | (uintptr_t)out) & 15) == 0) {
         const int wide = width <= 4096 ? 256 : (width <= 8192 ? 512 : 1024);
-        return launch_pdl(rms_pair_mean_vec_kernel, dim3(rows), dim3(wide), 0, stream, 1u, a, b, wa, wb, eps, out, width);
+        return launch_pdl(wide <= 512 ? rms_pair_mean_vec_kernel<true> : rms_pair_mean_vec_kernel<false>, dim3(rows), dim3(wide), 0, stream, 1u, a, b, wa, wb, eps, out, width);
     }
     const int threads = width >= 1024 ? 256 : 128;
     return launch_pdl(rms_pair_mean_kernel, dim3(rows), dim3(threads), 0, stream, 1u, a, b, wa, wb, eps, out, width);
