@@ -199,16 +199,44 @@ __device__ __forceinline__ void st_cluster_f32(uint32_t address, float value) {
 __device__ __forceinline__ float silu_mul(float gate, float up) {
     return __fdividef(gate * up, 1.0f + __expf(-gate));
 }
-// act(gate) * up.  The tanh form of gelu, 0.5 z (1 + tanh(y)) with y = sqrt(2 / pi) (z + 0.044715 z^3), is
-// z * sigmoid(2 y): the same one exponential and one division as silu, with another argument.
-__device__ __forceinline__ float gate_mul(const Epilogue& ep, float gate, float up) {
+// act(gate) * up for several values at once.  The tanh form of gelu, 0.5 z (1 + tanh(y)) with y = sqrt(2 / pi) (z + 0.044715 z^3), is
+// z * sigmoid(2 y): the same one exponential and one division as silu, with another argument.  The activation is looked up once
+// and not for each value: a branch between two values keeps their exponentials and divisions, some 100 cycles of latency each, from
+// overlapping, and made the epilogue of a tile of 64 tokens take 6 us (a chunk of 16 tokens 1.2 us).
+template <int COUNT>
+__device__ __forceinline__ void gate_mul_all(const Epilogue& ep, const float (&gate)[COUNT], const float (&up)[COUNT], float (&out)[COUNT]) {
     if (ep.gate_act == 2) {
-        const float g = fminf(gate, ep.gate_limit);
-        const float u = fminf(fmaxf(up, -ep.gate_limit), ep.gate_limit);
-        return __fdividef(g * (u + 1.0f), 1.0f + __expf(-ep.gate_slope * g));
+        const float limit = ep.gate_limit, slope = ep.gate_slope;
+#pragma unroll
+        for (int j = 0; j < COUNT; ++j) {
+            const float g = fminf(gate[j], limit);
+            const float u = fminf(fmaxf(up[j], -limit), limit);
+            out[j] = __fdividef(g * (u + 1.0f), 1.0f + __expf(-slope * g));
+        }
+    } else if (ep.gate_act == 1) {
+#pragma unroll
+        for (int j = 0; j < COUNT; ++j) {
+            const float t = 1.5957691216057308f * fmaf(0.044715f * gate[j] * gate[j], gate[j], gate[j]);
+            out[j] = __fdividef(gate[j] * up[j], 1.0f + __expf(-t));
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < COUNT; ++j) out[j] = silu_mul(gate[j], up[j]);
     }
-    const float t = ep.gate_act == 1 ? 1.5957691216057308f * fmaf(0.044715f * gate * gate, gate, gate) : gate;
-    return __fdividef(gate * up, 1.0f + __expf(-t));
+}
+// The swapped kernel's share of it: a thread holds one weight row's values of 16 tokens, gate rows in lanes without bit 3 and their
+// up rows eight lanes on.  A pair of lanes shares the tokens, the first eight to the gate's lane, so that each value is worked out
+// once: out[j] is token 8 (lane >> 3 & 1) + j.
+__device__ __forceinline__ void gate_mul_pair(const Epilogue& ep, const float (&v)[16], int lane, float (&out)[8]) {
+    const bool upper = lane & 8;
+    float gate[8], up[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float other = __shfl_xor_sync(0xffffffffu, upper ? v[j] : v[8 + j], 8);
+        gate[j] = upper ? other : v[j];
+        up[j] = upper ? v[8 + j] : other;
+    }
+    gate_mul_all<8>(ep, gate, up, out);
 }
 
 // SWAP false: X = A (rows m), Y = W (rows n), C[m, n].  SWAP true: X = W, Y = A.
@@ -556,11 +584,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 // (every product has read the ring: it is free)
                 if (EPI == 1) {
                     // this lane holds weight row x_row: rows 16k..16k+7 are gate rows, 16k+8..16k+15 their up rows
+                    float out[8];
+                    gate_mul_pair(ep, v, lane, out);
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float out = gate_mul(ep, v[j], __shfl_xor_sync(0xffffffffu, v[j], 8));
-                        if ((lane & 8) == 0) stage[(c0 - h0 + j) * 132 + (tile_row >> 4) * 8 + (tile_row & 7)] = out;
-                    }
+                    for (int j = 0; j < 8; ++j) stage[(c0 - h0 + (lane & 8) + j) * 132 + (tile_row >> 4) * 8 + (tile_row & 7)] = out[j];
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) stage[(c0 - h0 + j) * 132 + tile_row] = v[j];
@@ -588,13 +615,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             }
             if (EPI == 1 && SWAP) {
                 // this lane holds weight row x_row: rows 16k..16k+7 are gate rows, 16k+8..16k+15 their up rows
-                float out[16];
+                float out[8];
+                gate_mul_pair(ep, v, lane, out);
+                if (x_row < x_rows) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) out[j] = gate_mul(ep, v[j], __shfl_xor_sync(0xffffffffu, v[j], 8));
-                if ((lane & 8) == 0 && x_row < x_rows) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const int y = y0 + c0 + j;
+                    for (int j = 0; j < 8; ++j) {
+                        const int y = y0 + c0 + (lane & 8) + j;
                         if (y < y_rows) C[(size_t)y * ldc + (x_row >> 4) * 8 + (x_row & 7)] = from_f32<OutT>(out[j]);
                     }
                 }
@@ -604,18 +630,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             if (EPI == 1) {
                 // columns y0 + c0 .. + 15 are 8 gate rows then their 8 up rows: 8 outputs at (y0 + c0) / 2
                 OutT* dst = C + (size_t)x_row * ldc + ((y0 + c0) >> 1);
+                float gate[8], up[8], out[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) gate[j] = v[j], up[j] = v[j + 8];
+                gate_mul_all<8>(ep, gate, up, out);
                 if (y0 + c0 + 16 <= y_rows && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
                     uint32_t packed[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        __nv_bfloat162 pair = __floats2bfloat162_rn(gate_mul(ep, v[2 * j], v[2 * j + 8]), gate_mul(ep, v[2 * j + 1], v[2 * j + 9]));
+                        __nv_bfloat162 pair = __floats2bfloat162_rn(out[2 * j], out[2 * j + 1]);
                         packed[j] = *reinterpret_cast<uint32_t*>(&pair);
                     }
                     *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
                 } else {
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        if (y0 + c0 + j + 8 < y_rows) dst[j] = from_f32<OutT>(gate_mul(ep, v[j], v[j + 8]));
+                        if (y0 + c0 + j + 8 < y_rows) dst[j] = from_f32<OutT>(out[j]);
                 }
             } else if (SWAP) {
 #pragma unroll
@@ -1107,9 +1137,11 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_x, const 
                     uint32_t r[16];
                     tmem_load_32x16(tmem_acc + (uint32_t)c0, r);
                     tmem_load_wait();
-                    if (EPI == 1) {
+                    if constexpr (EPI == 1) {
+                        float gate[8], up[8];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] = gate_mul(ep, __uint_as_float(r[j]) * my_scale, __uint_as_float(r[j + 8]) * my_scale);
+                        for (int j = 0; j < 8; ++j) gate[j] = __uint_as_float(r[j]) * my_scale, up[j] = __uint_as_float(r[j + 8]) * my_scale;
+                        gate_mul_all<8>(ep, gate, up, v);
                     } else {
 #pragma unroll
                         for (int j = 0; j < PER; ++j) {
