@@ -412,8 +412,10 @@ __device__ __forceinline__ void prefetch_state_rows(const float* mine, int lane,
 // heads of 128 x 64: 16.2 and 13.3 us (the matrix memory, 16 heads of 128 x 256: 16.8 and 15.7).
 // xbc [T, inner + 2 G N] (float32): x, then B, then C, after convolution and silu; dt_raw (float32, row stride
 // dt_stride): the step sizes before softplus; y [T, inner] (float32) = S^T C + D x.
+// Registers are kept to 40 where a column's threads hold 16 rows each: at 74 an SM took three blocks of the 768 that three requests
+// make, and the second round of blocks waited a second time for everything that one waits for.
 template <int REGS, bool WIDE>
-__global__ void __launch_bounds__(256) ssm_walk_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, long dt_stride,
+__global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, long dt_stride,
                                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                                 float* __restrict__ state, long state_len, long ssm_off, const int* __restrict__ query_start,
                                 const int* __restrict__ slots, float* __restrict__ y, int heads, int groups, int N, int P,
@@ -423,6 +425,7 @@ __global__ void __launch_bounds__(256) ssm_walk_kernel(const float* __restrict__
     const int columns = blockDim.x / split;
     const int p = blockIdx.z * columns + (WIDE ? threadIdx.x % columns : threadIdx.x / split), s = WIDE ? threadIdx.x / columns : threadIdx.x % split;
     __shared__ float part[WIDE ? 2 : 1][WIDE ? 256 : 1];
+    __shared__ float bc_s[WIDE ? 2 : 1][WIDE ? 512 : 1];  // a token's B and C, up to 256 columns each
     const long first = query_start[request];
     const int count = (int)(query_start[request + 1] - first);
     const int slot = slots[request];
@@ -450,12 +453,26 @@ __global__ void __launch_bounds__(256) ssm_walk_kernel(const float* __restrict__
         const float* Cv = Bv + groups * N;
         const float take = dt * x;
         float acc = 0.0f;
+        if constexpr (WIDE) {
+            float* const bc = bc_s[t & 1];
+            for (int n = threadIdx.x; n < 2 * N; n += blockDim.x) bc[n] = n < N ? Bv[n] : Cv[n - N];
+            __syncthreads();
 #pragma unroll
-        for (int i = 0; i < REGS; ++i) {
-            const int n = s + i * split;
-            if (n < N) {
-                S[i] = fmaf(decay, S[i], take * Bv[n]);
-                acc = fmaf(S[i], Cv[n], acc);
+            for (int i = 0; i < REGS; ++i) {
+                const int n = s + i * split;
+                if (n < N) {
+                    S[i] = fmaf(decay, S[i], take * bc[n]);
+                    acc = fmaf(S[i], bc[N + n], acc);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < REGS; ++i) {
+                const int n = s + i * split;
+                if (n < N) {
+                    S[i] = fmaf(decay, S[i], take * Bv[n]);
+                    acc = fmaf(S[i], Cv[n], acc);
+                }
             }
         }
         if (WIDE) {
@@ -469,6 +486,7 @@ __global__ void __launch_bounds__(256) ssm_walk_kernel(const float* __restrict__
         if (live && s == 0) y[row * inner + head * P + p] = fmaf(skip, x, acc);
     }
     if (live) {
+        if (WIDE) asm volatile("" : "+l"(mine));  // (the rows' addresses are worked out again here instead of being held in 32 registers)
 #pragma unroll
         for (int i = 0; i < REGS; ++i) {
             const int n = s + i * split;
@@ -504,7 +522,7 @@ KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_s
     int split, threads, chunks;
     const int regs = walk_shape(N, P, &split, &threads, &chunks);
     if (!regs) return KIRAI_ERR_BAD_SIZE;
-    const bool wide = (threads / split) % 32 == 0;
+    const bool wide = (threads / split) % 32 == 0 && N <= 256;  // (a token's B and C lie in shared memory)
 #define KIRAI_SSM(R)                                                                                                         \
     return launch_pdl(wide ? ssm_walk_kernel<R, true> : ssm_walk_kernel<R, false>, dim3(requests, heads, chunks), dim3(threads), 0, stream, 1u, xbc, dt_raw, dt_stride, \
                       dt_bias, a_log, d_skip, state, state_len, ssm_off, query_start, slots, y, heads, groups, N, P, split,  \
@@ -522,8 +540,9 @@ KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_s
 // once more and stores them, after every block of the walk has read the old ones.
 // rows (float32, row stride): q [H d], k [H d], v [H dv], then the input gates' [H] and the forget gates' [H]
 // pre-activations.  state [slots, state_len]: S [H, d, dv], then n [H, d], then m [H].  o [T, H dv] (float32).
+// Registers are kept to 80 (16 rows a thread), for three blocks on an SM: 384 blocks of three requests in one round.
 template <int REGS, bool WIDE>
-__global__ void __launch_bounds__(256) matrix_memory_walk_kernel(const float* __restrict__ rows, long row_stride, const float* __restrict__ in_bias,
+__global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 3 : 0) matrix_memory_walk_kernel(const float* __restrict__ rows, long row_stride, const float* __restrict__ in_bias,
                                           const float* __restrict__ keep_bias, float cap, float q_scale, float* __restrict__ state,
                                           long state_len, const int* __restrict__ query_start, const int* __restrict__ slots,
                                           float* __restrict__ o, int heads, int d, int dv, int split, int num_slots) {
