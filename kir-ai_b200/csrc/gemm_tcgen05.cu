@@ -61,35 +61,39 @@ using namespace sm100;
 // free once its products are done: the cluster meets once before anything is sent (LATE), every CTA keeps the chunks it
 // owns in tensor memory (see `scatter` in the kernel), and the staged stores go through the rest of the ring 64 tokens
 // at a time.  One CTA per SM with six stages and up to three splits where the launch fits the SMs, else three stages,
-// two CTAs per SM and no split.  Tiles of 64 tokens take the same way where the launch fits the SMs (eight stages,
-// up to four splits), and slots beside a ring of four otherwise.
+// two CTAs per SM and no split.  Tiles of 32 and 64 tokens have room beside the ring for the chunks that a CTA receives (32 KB at
+// most, not a slot for every CTA's whole tile), so that their clusters meet once and not twice: the four products of a 4B layer at
+// 64 tokens 57.5 to 56.4 us, of an 8B layer at 37 tokens 76.1 to 75.1 (64 tokens: a ring of seven stages; eight, with every byte of
+// shared memory, 56.9).
 template <int BN, bool DEEP = false, bool STREAM = (BN <= 64)>
 struct GemmSmem {
     static constexpr bool streaming = STREAM;
-    static constexpr bool late_slots = STREAM && (BN > 64 || (BN == 64 && DEEP));  // (tiles of 256 tokens: one CTA per SM and four stages, DEEP or not)
+    static constexpr bool late_slots = STREAM && BN > 64;  // (tiles of 256 tokens: one CTA per SM and four stages, DEEP or not)
     static constexpr int x_bytes = GEMM_BM * GEMM_BK * 2;
     static constexpr int y_bytes = BN * GEMM_BK * 2;
     static constexpr int stage_bytes = x_bytes + y_bytes;
-    static constexpr int max_splits = !STREAM ? 1 : (BN <= 64 ? 4 : (DEEP || BN > 128 ? 3 : 1));  // BN <= 64: up to 128 KB of slots beside the ring
-    static constexpr int slot_bytes = BN * GEMM_BM * 4;  // one 32-bit partial tile
+    static constexpr int max_splits = !STREAM ? 1 : (BN <= 64 ? 4 : (DEEP || BN > 128 ? 3 : 1));
+    static constexpr int slot_bytes = BN * GEMM_BM * 4;  // one 32-bit partial tile (tiles of 16 tokens)
     static constexpr int stages = !STREAM ? (200 * 1024 / stage_bytes)
-                                          : (BN > 128 ? 4 : (BN > 64 ? (DEEP ? 6 : 3) : (DEEP ? (BN <= 16 ? 10 : (BN <= 32 ? 7 : 8)) : 4)));
+                                          : (BN > 128 ? 4 : (BN > 64 ? (DEEP ? 6 : 3) : (DEEP ? (BN <= 16 ? 10 : (BN <= 32 ? 9 : 7)) : 4)));
     static constexpr int barrier_bytes = 2048;  // barriers [0, 256), row scales [256, 256 + 4 BN) (BN <= 256)
     static constexpr int stage_tokens = BN < 64 ? BN : 64;  // tokens that the staged stores take through shared memory at a time
     // (from 1024 on, tiles of up to 64 tokens: the list of chosen experts)
     static_assert(!streaming || (2 * stages + 1) * 8 + 4 <= 256, "the streaming kernel's barriers must end before the row scales");
-    static_assert(!DEEP || BN <= 32 || late_slots, "a long ring beside slots is for the smallest tiles");
-    // LATE: what a CTA receives (from each other CTA the 16-token chunks that it owns, 8 KB each) and the staged tokens
-    // lie in its ring; the most is received with two splits (half the tile from one sender) or with max_splits
+    // what a CTA receives: from each other CTA of its cluster the 16-token chunks that it owns, 8 KB each (LATE: it lies in its
+    // ring, the staged tokens behind it)
     static constexpr int chunks = BN / 16;
-    static constexpr int most_received = (((chunks + 1) / 2) > (max_splits - 1) * ((chunks + max_splits - 1) / max_splits)
-                                              ? (chunks + 1) / 2 : (max_splits - 1) * ((chunks + max_splits - 1) / max_splits)) * 16 * GEMM_BM * 4;
+    static constexpr int received(int splits) { return (splits - 1) * ((chunks + splits - 1) / splits) * 16 * GEMM_BM * 4; }
+    static constexpr int larger(int a, int b) { return a > b ? a : b; }
+    static constexpr int most_received = larger(max_splits >= 2 ? received(2) : 0, larger(max_splits >= 3 ? received(3) : 0, max_splits >= 4 ? received(4) : 0));
+    static constexpr int slots_bytes(int splits) { return BN >= 32 ? most_received : splits * slot_bytes; }
     static_assert(!late_slots || max_splits == 1 || most_received + stage_tokens * 132 * 4 <= stages * stage_bytes,
                   "the other CTAs' partial chunks and the staged tokens lie in the ring");
     static constexpr int ctas_per_sm = streaming && !DEEP && BN <= 128 ? 2 : 1;
     static constexpr int total(int splits) {  // + slack to align the base to 1024 bytes
-        return stages * stage_bytes + barrier_bytes + (splits > 1 && !late_slots ? splits * slot_bytes : 0) + 1024;
+        return stages * stage_bytes + barrier_bytes + (splits > 1 && !late_slots ? slots_bytes(splits) : 0) + 1024;
     }
+    static_assert(!streaming || stages * stage_bytes + barrier_bytes + (late_slots ? 0 : slots_bytes(max_splits)) + 1024 <= 227 * 1024, "shared memory of an SM");
 };
 
 template <int BN>
@@ -183,6 +187,8 @@ __device__ __forceinline__ void named_barrier_128() { asm volatile("bar.sync 1, 
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The address, in the cluster's shared window, that `local` has in CTA `rank`; and a store to it.
 __device__ __forceinline__ uint32_t cluster_address(uint32_t local, uint32_t rank) {
     uint32_t remote;
@@ -255,6 +261,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     constexpr bool CHOSEN = sizeof...(Chosen) > 0;
     static_assert(!CHOSEN || (SWAP && BN <= 64 && EPI == 0), "the list lies behind the row scales of up to 64 tokens");
     constexpr int STAGES = Smem::stages;
+    constexpr bool ANNOUNCED = !Smem::late_slots && BN >= 64;
     constexpr bool LATE = Smem::late_slots;  // what other CTAs send lies in the receiver's ring (see GemmSmem)
     // Tiles of 32 tokens and more, split along K: every CTA of the cluster sums and stores a share of the tile's
     // 16-token chunks (chunk c belongs to CTA c % splits) instead of the first CTA all of it.  A CTA sends the chunks
@@ -347,6 +354,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     __syncthreads();
     tc_fence_after();
     if constexpr (CHOSEN) pdl_launch_dependents();
+    if (ANNOUNCED && splits > 1) cluster_arrive();
     const uint32_t tmem_base = *tmem_slot;
     float res[16];  // EPI 2: the stream's values under this thread's 16 outputs
     float norm_w = 0.0f;
@@ -370,7 +378,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             const int x_first = SWAP ? 0 : 1, y_first = SWAP ? 1 : 0;  // which operand is the weights
             // tiled weights (SWAP only): this tile's boxes lie one after the other
             const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)x_tile * total_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
-            // this CTA's i-th block of K, counted from kb_begin: the i-th, but for the blocks of experts that are left out
+            // this CTA's i-th block of K, counted from kb_begin: the CTAs of a launch begin at blocks spread over the range and come
+            // round, so that they do not all ask L2 for the same block of the tokens' rows at the same time (gate/up of the 4B
+            // shape alone, 64 tokens 26.0 to 24.1 us, 16 tokens 20.7 to 19.3; of the 8B shape's 192 tiles 38.1 to 37.4 and 32.8 to 32.6).
+            // Of chosen experts: the i-th, but for the blocks that are left out.
+            const int turn = CHOSEN ? 0 : (int)((long)blockIdx.x * num_kb / gridDim.x);
             auto block = [&](int i) {
                 if constexpr (CHOSEN) {
                     const ChosenExperts& ce = chosen_of(chosen...);
@@ -378,8 +390,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                         const int at = kb_begin + i, unit = ce.unit, own = chosen_s[0] * unit;
                         return (at < own ? chosen_s[1 + at / unit] * unit + at % unit : ce.experts * unit + at - own) - kb_begin;
                     }
+                    return i;
                 }
-                return i;
+                const int at = i + turn;
+                return at < num_kb ? at : at - num_kb;
             };
             auto load_x = [&](uint32_t dst, uint32_t full, int i) {
                 if (SWAP && boxes) bulk_load_1d(dst, boxes + (size_t)i * GEMM_BOX_BYTES, GEMM_BOX_BYTES, full);
@@ -467,8 +481,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         if (tile_row == 0) gemm_stamp(ep, 3);
     }
     // LATE: the receivers' rings take what is sent, so nothing is sent before every CTA of the cluster has seen its
-    // last product finish (all threads arrive here, the epilogue warps after their wait for the accumulator)
-    if (splits > 1 && LATE) cluster_sync_all();
+    // last product finish (all threads arrive here, the epilogue warps after their wait for the accumulator).  Else it is enough
+    // that every CTA of the cluster has begun, which it said long ago.  (Tiles of up to 32 tokens leave that out: a cluster's CTAs
+    // begin together, and the pair of barriers cost a layer of the 8B shape's products 0.7 of 65 us at one token.)
+    if (LATE && splits > 1) cluster_sync_all();
+    if (ANNOUNCED && splits > 1) cluster_wait();
     if (warp >= 2 && scatter) {
         // every chunk of 16 tokens that another CTA owns goes to that CTA: its slot [sender][chunk / splits], the senders
         // in rank order without the owner itself, 16 x 128 floats column-major (lanes side by side)
