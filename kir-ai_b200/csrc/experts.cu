@@ -614,22 +614,40 @@ __global__ void terms_norm_add_kernel(float* __restrict__ resid, const FeedForwa
     const float same = same_weight(f, token);
     float4* dst = reinterpret_cast<float4*>(resid + base);
     const float4* w4 = reinterpret_cast<const float4*>(norm_weight);
-    float4 kept[VEC], stream[VEC], w[VEC];
+    float4 kept[VEC], stream[VEC], w[VEC], shared[VEC];
     float acc = 0.0f;
+    // (all rows are asked for before any is used: which of them there are is looked up once and not between a thread's pieces)
 #pragma unroll
     for (int n = 0; n < VEC; ++n) {
         const int i = threadIdx.x + n * blockDim.x;
         kept[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < quads) stream[n] = dst[i], w[n] = w4[i];
+    }
+    if (f.routed) {
+#pragma unroll
+        for (int n = 0; n < VEC; ++n) {
+            const int i = threadIdx.x + n * blockDim.x;
+            if (i < quads) kept[n] = load4(f.routed + base + 4 * (size_t)i);
+        }
+    }
+    if (f.shared) {
+#pragma unroll
+        for (int n = 0; n < VEC; ++n) {
+            const int i = threadIdx.x + n * blockDim.x;
+            if (i < quads) shared[n] = load4(f.shared + base + 4 * (size_t)i);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < VEC; ++n) {
+        const int i = threadIdx.x + n * blockDim.x;
         if (i < quads) {
-            stream[n] = dst[i], w[n] = w4[i];
-            if (f.routed) kept[n] = load4(f.routed + base + 4 * (size_t)i);
             if (f.sorted) {
                 for (int j = 0; j < f.top; ++j) {
                     const int slot = f.slot_of[(size_t)token * f.top + j];
                     if (slot >= 0) add_scaled4(kept[n], f.weights[(size_t)token * f.top + j], load4(f.sorted + (size_t)slot * hidden + 4 * (size_t)i));
                 }
             }
-            if (f.shared) add_scaled4(kept[n], share, load4(f.shared + base + 4 * (size_t)i));
+            if (f.shared) add_scaled4(kept[n], share, shared[n]);
             if (same != 0.0f) add_scaled4(kept[n], same, stream[n]);
             acc += (kept[n].x * kept[n].x + kept[n].y * kept[n].y) + (kept[n].z * kept[n].z + kept[n].w * kept[n].w);
         }
