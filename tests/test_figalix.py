@@ -1093,3 +1093,10 @@ def test_sums_under_a_tanh_and_pairs_of_normed_rows_from_aligned_rows(rows, widt
         got = ops.rms_pair_mean(placed(d1, shift), placed(d2, shift), placed(w, shift), placed(b, shift), 1e-6).double().cpu()
         unit = lambda x: x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-6)  # noqa: E731
         assert float((got - 0.5 * (unit(d1) * w.double() + unit(d2) * b.double())).abs().max()) <= 16.0 * 2.0 ** -19
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,groups,state,vdim", [(2, 2, 132, 96), (1, 1, 256, 64), (1, 1, 260, 64)])
+def test_walks_up_to_and_beyond_the_columns_that_shared_memory_holds(heads, groups, state, vdim):
+    """A block's threads hold whole runs of 32 columns here; up to 256 rows of a state B and C come through shared memory."""
+    test_state_space_runs_in_chunks_as_token_by_token(heads, groups, state, vdim)
