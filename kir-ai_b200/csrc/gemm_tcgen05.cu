@@ -380,9 +380,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)x_tile * total_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
             // this CTA's i-th block of K, counted from kb_begin: the CTAs of a launch begin at blocks spread over the range and come
             // round, so that they do not all ask L2 for the same block of the tokens' rows at the same time (gate/up of the 4B
-            // shape alone, 64 tokens 26.0 to 24.1 us, 16 tokens 20.7 to 19.3; of the 8B shape's 192 tiles 38.1 to 37.4 and 32.8 to 32.6).
-            // Of chosen experts: the i-th, but for the blocks that are left out.
-            const int turn = CHOSEN ? 0 : (int)((long)blockIdx.x * num_kb / gridDim.x);
+            // shape, 64 tokens 21.9 to 19.9 us, 16 tokens 19.5 to 18.2; of the 8B shape, 37 tokens 33.5 to 32.6, 8 tokens 31.1 both ways).
+            // CTAs that share K between them begin at different blocks as it is, and lost 0.1 to 0.5 us by it.  Of chosen experts: the i-th, but for the blocks that are left out.
+            const int turn = CHOSEN || splits > 1 ? 0 : (int)((long)blockIdx.x * num_kb / gridDim.x);
             auto block = [&](int i) {
                 if constexpr (CHOSEN) {
                     const ChosenExperts& ce = chosen_of(chosen...);
