@@ -549,7 +549,7 @@ int launch(const void* q, const void* cache, void* out, const int* block_table, 
         if (!tmap::bf16_2d_sw128(&kv_map, cache, rows, head_dim, head_dim, piece_rows, 64)) return KIRAI_ERR_BAD_ALIGN;
     }
     auto kernel = attention_prefill_tc_kernel<D>;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::total);
+    cudaError_t err = allow_shared((const void*)kernel, Smem::total);
     if (err != cudaSuccess) return (int)err;
     dim3 grid(kv_heads, (unsigned)(((long)max_query_len * group + TA_ROWS - 1) / TA_ROWS), requests);
     if (grid.y > 65535) return KIRAI_ERR_BAD_SIZE;

@@ -203,12 +203,28 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 #include <cstdlib>
+#include <map>
+#include <utility>
 static inline bool pdl_enabled() {
     static const bool enabled = [] {
         const char* value = std::getenv("KIRAI_PDL");
         return !(value && value[0] == '0');
     }();
     return enabled;
+}
+
+// Raises `kernel`'s limit on dynamic shared memory to `bytes`, asking the runtime only where this thread has not done so on this
+// device (a limit that stands is no smaller than the kernel's other launches want).
+static inline cudaError_t allow_shared(const void* kernel, int bytes) {
+    static thread_local std::map<std::pair<const void*, int>, int> granted;
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    int& known = granted[std::make_pair(kernel, device)];
+    if (bytes <= known) return cudaSuccess;
+    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (err == cudaSuccess) known = bytes;
+    return err;
 }
 
 // Launches `kernel` with programmatic stream serialization (and, if cluster_z > 1, as clusters of

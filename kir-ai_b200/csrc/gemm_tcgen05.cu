@@ -1322,7 +1322,7 @@ static int launch_persistent_tile(int width, const void* A, const void* W, bool 
     auto kernel = gemm_tcgen05_persistent_kernel<MT, OutT, EPI>;
     const int smem_bytes = stages * (MT * GEMM_BOX_BYTES + width * GEMM_BK * 2) + GEMM_BARRIER_BYTES + 1024 +  // + slack to align the ring
                            (EPI == 2 ? 4 * 32 * 32 * 4 : 0);                                                   // + the epilogue's staging buffers
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+    cudaError_t err = allow_shared((const void*)kernel, smem_bytes);
     if (err != cudaSuccess) return (int)err;
     return launch_pdl(kernel, dim3(grid), dim3(64 + 128 * MT), (size_t)smem_bytes, stream, 1u, map_a, map_w,
                       tiled ? (const uint8_t*)W : (const uint8_t*)nullptr, (OutT*)C, M, N, K, ldc, width, stages, ep, error_flag);
@@ -1415,7 +1415,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
             if (busy * used <= sm_count() && deep_rings()) {
                 using Deep = GemmSmem<BN, true, true>;
                 auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, true, Chosen...>;
-                cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Deep::total(Deep::max_splits));
+                cudaError_t err = allow_shared((const void*)kernel, Deep::total(Deep::max_splits));
                 if (err != cudaSuccess) return (int)err;
                 if (used > 1 && splits > 1 && busy > max_resident_clusters(kernel, Deep::total(used), used)) continue;
                 return launch_pdl(kernel, grid, dim3(GEMM_THREADS), (size_t)Deep::total(used), stream, (unsigned)used, map_x,
@@ -1424,7 +1424,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
         }
         if (used > Smem::max_splits) continue;  // (tiles of 128 tokens split only with the long ring)
         auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, false, Chosen...>;
-        cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::total(Smem::max_splits));
+        cudaError_t err = allow_shared((const void*)kernel, Smem::total(Smem::max_splits));
         if (err != cudaSuccess) return (int)err;
         // launches of more CTAs than SMs run in waves anyway; only a launch meant to be one wave is fitted
         if (used > 1 && splits > 1 && clusters * used <= 2L * sm_count() &&
