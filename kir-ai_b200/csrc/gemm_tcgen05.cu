@@ -382,6 +382,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             // round, so that they do not all ask L2 for the same block of the tokens' rows at the same time (gate/up of the 4B
             // shape, 64 tokens 21.9 to 19.9 us, 16 tokens 19.5 to 18.2; of the 8B shape, 37 tokens 33.5 to 32.6, 8 tokens 31.1 both ways).
             // CTAs that share K between them begin at different blocks as it is, and lost 0.1 to 0.5 us by it.  Of chosen experts: the i-th, but for the blocks that are left out.
+            // A launch reads every box once, and gigabytes of them go by between two uses: they leave L2 first, so that the step's
+            // rows, states, norm weights and lately written keys stay (steps of the 8B shape: one request 24.18 to 23.92 ms, eight
+            // 28.9 to 28.46; 64 requests of the 4B shape's layers 11.33 to 11.12; three of the Damilix shape 16.4 to 15.97).  The
+            // many-token kernel, whose tiles share boxes through L2, lost by it (32.7 to 33.2 ms for 8,064 tokens of the 32B shape).
+            const uint64_t evict_first = evict_first_policy();
             const int turn = CHOSEN || splits > 1 ? 0 : (int)((long)blockIdx.x * num_kb / gridDim.x);
             auto block = [&](int i) {
                 if constexpr (CHOSEN) {
@@ -396,7 +401,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 return at < num_kb ? at : at - num_kb;
             };
             auto load_x = [&](uint32_t dst, uint32_t full, int i) {
-                if (SWAP && boxes) bulk_load_1d(dst, boxes + (size_t)i * GEMM_BOX_BYTES, GEMM_BOX_BYTES, full);
+                if (SWAP && boxes) bulk_load_1d_once(dst, boxes + (size_t)i * GEMM_BOX_BYTES, GEMM_BOX_BYTES, full, evict_first);
                 else tma_load_2d(dst, &map_x, full, (kb_begin + i) * GEMM_BK, x0);
             };
             const int head = num_kb < STAGES ? num_kb : STAGES;

@@ -92,6 +92,18 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst, const void* src, uint
                  : "memory");
 }
 
+// The same for bytes that are read once: they are the first to leave L2 again.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+    return policy;
+}
+__device__ __forceinline__ void bulk_load_1d_once(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t evict_first) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar), "l"(evict_first)
+                 : "memory");
+}
+
 // ------------------------------------------------------------- tensor memory
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t columns) {  // whole warp; columns: power of 2 >= 32
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(columns) : "memory");
