@@ -9,8 +9,9 @@
 // warps, too few to hide the barriers of a tile); the operands of four columns come from
 // shared memory as 16-byte loads (12 wavefronts for 64 FMAs a lane, so that the FMA pipe and not shared memory sets the
 // pace), and `fma.rn.f32x2` halves the instructions.  Bound by the FMA pipe: the 4B shape's layer (32 heads of 128, 8 kv
-// heads) at 515 tokens is 2.2 GFLOP, 30 us at 72 TFLOP/s; measured 130 us (plain kernel: 1,139), the heaviest row tile's nine key tiles one after
-// another setting the end.  Weights overlay the key tile, so that a CTA takes 101 KB and
+// heads) at 515 tokens is 2.2 GFLOP, 30 us at 72 TFLOP/s; measured 116 us inside a prompt (152 with four warps a CTA and the
+// longest rows of the rest beside the longest; plain kernel: 1,139), the heaviest row tile's nine key tiles one after another setting
+// the end.  Weights overlay the key tile, so that a CTA takes 101 KB and
 // two fit an SM; the value tile is fetched while the scores are made, and a key tile's fetch hides behind the other CTA.
 //
 // Decode kernel (one token per request): a CTA takes a (request, kv head) and up to eight query heads of its group; each

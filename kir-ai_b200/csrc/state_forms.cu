@@ -409,11 +409,12 @@ __device__ __forceinline__ void prefetch_state_rows(const float* mine, int lane,
 // WIDE (a block has whole runs of 32 columns): the threads of a warp have adjacent columns of the same rows, so that the state is
 // read and written in whole lines and B and C are the same address for a warp; a column's threads meet in shared memory.
 // Otherwise they lie side by side in a warp, which touches 16 bytes of each row, and meet by shuffles.  Three requests, 128
-// heads of 128 x 64: 16.2 and 13.3 us (the matrix memory, 16 heads of 128 x 256: 16.8 and 15.7).
+// heads of 128 x 64: 16.2 and 13.3 us inside a step (the matrix memory, 16 heads of 128 x 256: 16.8 and 15.7), before registers were
+// held down as below.
 // xbc [T, inner + 2 G N] (float32): x, then B, then C, after convolution and silu; dt_raw (float32, row stride
 // dt_stride): the step sizes before softplus; y [T, inner] (float32) = S^T C + D x.
 // Registers are kept to 40 where a column's threads hold 16 rows each: at 74 an SM took three blocks of the 768 that three requests
-// make, and the second round of blocks waited a second time for everything that one waits for.
+// make, and the second round of blocks waited a second time for everything that one waits for (11.7 to 9.6 us a launch).
 template <int REGS, bool WIDE>
 __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, long dt_stride,
                                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
@@ -540,7 +541,8 @@ KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_s
 // once more and stores them, after every block of the walk has read the old ones.
 // rows (float32, row stride): q [H d], k [H d], v [H dv], then the input gates' [H] and the forget gates' [H]
 // pre-activations.  state [slots, state_len]: S [H, d, dv], then n [H, d], then m [H].  o [T, H dv] (float32).
-// Registers are kept to 80 (16 rows a thread), for three blocks on an SM: 384 blocks of three requests in one round.
+// Registers are kept to 80 (16 rows a thread), for three blocks on an SM: 384 blocks of three requests in one round (15.0 to 12.4 us
+// with the normaliser's kernel).
 template <int REGS, bool WIDE>
 __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 3 : 0) matrix_memory_walk_kernel(const float* __restrict__ rows, long row_stride, const float* __restrict__ in_bias,
                                           const float* __restrict__ keep_bias, float cap, float q_scale, float* __restrict__ state,
