@@ -347,9 +347,7 @@ class NativeScheduler(Scheduler):
             assert self.waiting[0] is request
             self.waiting.popleft()
             request.pages = self._tables.adopt(request.request_id, request.key, slots[i])
-            for tensor in self.cache.state.values():  # a fresh state slot, as CacheManager.open leaves it
-                if tensor is not None:
-                    tensor[request.pages.slot].zero_()
+            self.cache.clear_states(request.pages.slot)  # as CacheManager.open leaves it
             request.state = RUNNING
             self.running.append(request)
         chosen = [Scheduled(self._by_key[keys[i]], first[i], count[i], bool(sample[i])) for i in range(runs)]
