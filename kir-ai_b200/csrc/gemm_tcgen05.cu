@@ -46,17 +46,17 @@ using namespace sm100;
 #define GEMM_BARRIER_BYTES 2048                 // persistent kernel: barriers behind the ring
 #define GEMM_MAX_STAGES 12                      // persistent kernel: the longest ring
 
-// Shared memory of one CTA: the ring of stages, the barriers, then (only with split-K) one slot
-// per CTA of the cluster for the partial tiles.  The swapped, weight-streaming case (BN <= 64)
-// keeps the ring small enough for two CTAs per SM, so that every SM streams weights even when
-// there are fewer tiles than two waves (but see DEEP below); the many-token case takes as many stages as fit.
+// Shared memory of one CTA of the weight-streaming kernel: the ring of stages, the barriers, then (only with split-K) room
+// for the partial tiles of the cluster's other CTAs.  Tiles of up to 64 tokens
+// keep the ring small enough for two CTAs per SM, so that every SM streams weights even when
+// there are fewer tiles than two waves (but see DEEP below).
 // DEEP (weight-streaming case, BN <= 32): a launch with no more CTAs than SMs gains nothing from a second CTA per
 // SM; its CTAs take a longer ring instead, because 4 stages of 16 KB in each of 128 CTAs are 8 MB in flight, fewer
 // than the memory system needs to run at its rate (about 1.5 us of latency x 6.4 TB/s).  Ten stages for up to 16
 // tokens (the 96 CTAs of the 8B shape's q, k, v product then stream at the memory's rate: 7 stages 9.5 us, 10 stages 8.5).
 // Tried on top of this and taken out: the partial tiles of a cluster row by row, sent with 16-byte stores (no faster:
 // what the first CTA waits for at the end of a split product is the slowest of its cluster, not the stores).
-// STREAM (the swapped, weight-streaming kernel) with BN = 128 (65 to 128 tokens): a partial tile is 64 KB, so slots
+// BN = 128 (65 to 128 tokens): a partial tile is 64 KB, so slots
 // for the other CTAs' partial results do not fit beside a ring.  They lie IN the receiving CTA's ring instead, which is
 // free once its products are done: the cluster meets once before anything is sent (LATE), every CTA keeps the chunks it
 // owns in tensor memory (see `scatter` in the kernel), and the staged stores go through the rest of the ring 64 tokens
@@ -65,21 +65,19 @@ using namespace sm100;
 // most, not a slot for every CTA's whole tile), so that their clusters meet once and not twice: the four products of a 4B layer at
 // 64 tokens 57.5 to 56.4 us, of an 8B layer at 37 tokens 76.1 to 75.1 (64 tokens: a ring of seven stages; eight, with every byte of
 // shared memory, 56.9).
-template <int BN, bool DEEP = false, bool STREAM = (BN <= 64)>
+template <int BN, bool DEEP>
 struct GemmSmem {
-    static constexpr bool streaming = STREAM;
-    static constexpr bool late_slots = STREAM && BN > 64;  // (tiles of 256 tokens: one CTA per SM and four stages, DEEP or not)
+    static constexpr bool late_slots = BN > 64;  // (tiles of 256 tokens: one CTA per SM and four stages, DEEP or not)
     static constexpr int x_bytes = GEMM_BM * GEMM_BK * 2;
     static constexpr int y_bytes = BN * GEMM_BK * 2;
     static constexpr int stage_bytes = x_bytes + y_bytes;
-    static constexpr int max_splits = !STREAM ? 1 : (BN <= 64 ? 4 : (DEEP || BN > 128 ? 3 : 1));
+    static constexpr int max_splits = BN <= 64 ? 4 : (DEEP || BN > 128 ? 3 : 1);
     static constexpr int slot_bytes = BN * GEMM_BM * 4;  // one 32-bit partial tile (tiles of 16 tokens)
-    static constexpr int stages = !STREAM ? (200 * 1024 / stage_bytes)
-                                          : (BN > 128 ? 4 : (BN > 64 ? (DEEP ? 6 : 3) : (DEEP ? (BN <= 16 ? 10 : (BN <= 32 ? 9 : 7)) : 4)));
+    static constexpr int stages = BN > 128 ? 4 : (BN > 64 ? (DEEP ? 6 : 3) : (DEEP ? (BN <= 16 ? 10 : (BN <= 32 ? 9 : 7)) : 4));
     static constexpr int barrier_bytes = 2048;  // barriers [0, 256), row scales [256, 256 + 4 BN) (BN <= 256)
     static constexpr int stage_tokens = BN < 64 ? BN : 64;  // tokens that the staged stores take through shared memory at a time
     // (from 1024 on, tiles of up to 64 tokens: the list of chosen experts)
-    static_assert(!streaming || (2 * stages + 1) * 8 + 4 <= 256, "the streaming kernel's barriers must end before the row scales");
+    static_assert((2 * stages + 1) * 8 + 4 <= 256, "the streaming kernel's barriers must end before the row scales");
     // what a CTA receives: from each other CTA of its cluster the 16-token chunks that it owns, 8 KB each (LATE: it lies in its
     // ring, the staged tokens behind it)
     static constexpr int chunks = BN / 16;
@@ -89,11 +87,11 @@ struct GemmSmem {
     static constexpr int slots_bytes(int splits) { return BN >= 32 ? most_received : splits * slot_bytes; }
     static_assert(!late_slots || max_splits == 1 || most_received + stage_tokens * 132 * 4 <= stages * stage_bytes,
                   "the other CTAs' partial chunks and the staged tokens lie in the ring");
-    static constexpr int ctas_per_sm = streaming && !DEEP && BN <= 128 ? 2 : 1;
+    static constexpr int ctas_per_sm = !DEEP && BN <= 128 ? 2 : 1;
     static constexpr int total(int splits) {  // + slack to align the base to 1024 bytes
         return stages * stage_bytes + barrier_bytes + (splits > 1 && !late_slots ? slots_bytes(splits) : 0) + 1024;
     }
-    static_assert(!streaming || stages * stage_bytes + barrier_bytes + (late_slots ? 0 : slots_bytes(max_splits)) + 1024 <= 227 * 1024, "shared memory of an SM");
+    static_assert(stages * stage_bytes + barrier_bytes + (late_slots ? 0 : slots_bytes(max_splits)) + 1024 <= 227 * 1024, "shared memory of an SM");
 };
 
 template <int BN>
@@ -253,11 +251,11 @@ __device__ __forceinline__ void gate_mul_pair(const Epilogue& ep, const float (&
 // rows, ...) and stores silu(gate) * up, [M, N / 2].
 // Chosen: nothing, or ChosenExperts.
 template <int BN, bool SWAP, typename OutT, int EPI, bool DEEP, typename... Chosen>
-__global__ void __launch_bounds__(GEMM_THREADS, GemmSmem<BN, DEEP, true>::ctas_per_sm)
+__global__ void __launch_bounds__(GEMM_THREADS, GemmSmem<BN, DEEP>::ctas_per_sm)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const uint8_t* __restrict__ w_tiled, OutT* __restrict__ C, int M, int N, int K, long ldc,
                     int k_blocks_per_split, int splits, Epilogue ep, int* __restrict__ error_flag, Chosen... chosen) {
-    using Smem = GemmSmem<BN, DEEP, true>;
+    using Smem = GemmSmem<BN, DEEP>;
     constexpr bool CHOSEN = sizeof...(Chosen) > 0;
     static_assert(!CHOSEN || (SWAP && BN <= 64 && EPI == 0), "the list lies behind the row scales of up to 64 tokens");
     constexpr int STAGES = Smem::stages;
@@ -1382,7 +1380,7 @@ static long max_resident_clusters(Kernel kernel, int smem_bytes, int cluster_z) 
 template <int BN, bool SWAP, typename OutT, int EPI, typename... Chosen>
 static int launch_config(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
                          int splits, const Epilogue& ep, int* error_flag, cudaStream_t stream, const Chosen&... chosen) {
-    using Smem = GemmSmem<BN, false, true>;
+    using Smem = GemmSmem<BN, false>;
     CUtensorMap map_x, map_y;
     const void* x_ptr = SWAP ? W : A;
     const void* y_ptr = SWAP ? A : W;
@@ -1395,7 +1393,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
     const int total_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
     if (splits < 1) splits = 1;
     int max_splits = Smem::max_splits;
-    if constexpr (BN == 128) max_splits = GemmSmem<BN, true, true>::max_splits;  // (tiles of 128 tokens split only with the long ring)
+    if constexpr (BN == 128) max_splits = GemmSmem<BN, true>::max_splits;  // (tiles of 128 tokens split only with the long ring)
     if (splits > max_splits) splits = max_splits;  // slots in the first CTA's shared memory
     if (splits > total_k_blocks) splits = total_k_blocks;
     const uint8_t* boxes = tiled ? (const uint8_t*)W : (const uint8_t*)nullptr;
@@ -1418,7 +1416,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
                 if (expected > 0) busy = expected * grid.y;
             }
             if (busy * used <= sm_count() && deep_rings()) {
-                using Deep = GemmSmem<BN, true, true>;
+                using Deep = GemmSmem<BN, true>;
                 auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, true, Chosen...>;
                 cudaError_t err = allow_shared((const void*)kernel, Deep::total(Deep::max_splits));
                 if (err != cudaSuccess) return (int)err;
