@@ -55,6 +55,8 @@ struct TcAttnSmem {
     static_assert((4 * TA_STAGES + 5) * 8 + 4 <= barrier_bytes, "the barriers and the tensor-memory slot must fit their region");
     static constexpr int table_entries = 1024;
     static constexpr int total = q_bytes + ring_bytes + barrier_bytes + table_entries * 4 + 1024;
+    static_assert(alone_with_all_columns(total), "a CTA with all of the tensor memory shares no SM with this one");
+    static_assert(TaTmem<D>::cols < 512 || total >= ALL_COLUMNS_SHARED, "all columns");
 };
 
 // [rows][64 bf16] panels with the TMA 128-byte swizzle: chunk c of row r at chunk c ^ (r & 7).
@@ -142,7 +144,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
                             const int* __restrict__ context_len, int q_heads, int kv_heads, int head_dim,
                             long q_row_stride, int page_size, int box_rows, int piece_rows, int table_width, int num_pages,
                             int window, ScoreForm form, int* __restrict__ error_flag) {
-    pdl_launch_dependents();
     using Smem = TcAttnSmem<D>;
     constexpr int PANELS = Smem::panels;
     const float scale_log2 = form.cap_log2 != 0.0f ? 1.0f : form.scale_log2;  // capped scores are in the exponent's units already
@@ -215,6 +216,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const bf
     if (warp == 1) {
         tmem_alloc(smem_addr(tmem_slot), TaTmem<D>::cols);
         tmem_relinquish();
+        pdl_launch_dependents();  // only now: a product's CTA that shares the SM must find its tensor memory after this one
     }
     // Q tile: row r is token (row0 + r) / group, head kv_head * group + (row0 + r) % group; ten pieces of 16 bytes of a thread
     // are asked for before the first is stored (one at a time, with a division each, they were a third of a short prompt's launch)
@@ -583,6 +585,11 @@ static int attention_prefill_tc_entry(const void* q, const void* cache, void* ou
                            head_dim, q_row_stride, page_size, table_width, num_pages, window, scale, softcap, error_flag, stream, sinks);
     return launch<256>(q, cache, out, block_table, query_start, context_len, requests, max_query_len, q_heads, kv_heads,
                        head_dim, q_row_stride, page_size, table_width, num_pages, window, scale, softcap, error_flag, stream, sinks);
+}
+
+// Bytes of dynamic shared memory of a CTA.
+KIRAI_EXPORT int kirai_attention_prefill_tc_shared(int head_dim) {
+    return head_dim <= 64 ? TcAttnSmem<64>::total : head_dim <= 128 ? TcAttnSmem<128>::total : TcAttnSmem<256>::total;
 }
 
 KIRAI_EXPORT int kirai_attention_prefill_tc_bf16(const void* q, const void* cache, void* out, const int* block_table,

@@ -101,6 +101,7 @@ struct ChainSmem {
     static_assert(4 * BN * 4 <= 1024, "four warps' sums of squares must fit");
     static constexpr int total = stages * stage_bytes + barrier_bytes + 1024;  // + slack to align the base to 1024 bytes
     static constexpr int tmem_columns = 2 * BN < 32 ? 32 : 2 * BN;
+    static_assert(alone_with_all_columns(total), "a CTA with all of the tensor memory shares no SM with this one");
 };
 
 __device__ __forceinline__ int ld_acquire(const int* address) {

@@ -48,6 +48,8 @@ struct Shape {
     static_assert(ring >= BN * TILE_N * 4, "the ring takes a tile's sums");
     static_assert(2 * BN + 2 * 48 <= columns, "tensor memory: two blocks of partial sums and of planes");
     static_assert(total * ctas <= 227 * 1024, "shared memory of an SM");
+    static_assert(alone_with_all_columns(total), "a CTA with all of the tensor memory shares no SM with this one");
+    static_assert(columns < 512 || total >= ALL_COLUMNS_SHARED, "all columns");
 };
 
 __device__ __forceinline__ void tmem_store_32x8(uint32_t taddr, const uint32_t (&r)[8]) {

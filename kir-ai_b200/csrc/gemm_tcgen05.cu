@@ -92,6 +92,7 @@ struct GemmSmem {
         return stages * stage_bytes + barrier_bytes + (splits > 1 && !late_slots ? slots_bytes(splits) : 0) + 1024;
     }
     static_assert(stages * stage_bytes + barrier_bytes + (late_slots ? 0 : slots_bytes(max_splits)) + 1024 <= 227 * 1024, "shared memory of an SM");
+    static_assert(alone_with_all_columns(stages * stage_bytes + barrier_bytes + 1024), "a CTA of the persistent kernel shares no SM with this one");
 };
 
 template <int BN>
@@ -1281,6 +1282,15 @@ static int persistent_stages(int row_tiles, int width) {
     const int stages = 200 * 1024 / (row_tiles * GEMM_BOX_BYTES + width * GEMM_BK * 2);
     return stages < GEMM_MAX_STAGES ? stages : GEMM_MAX_STAGES;
 }
+// Dynamic shared memory of a CTA, the residual-and-norm epilogue's buffers aside: the ring, the barriers and slack to align the
+// ring, but no less than what keeps other kernels' tensor memory off an SM whose 512 columns this one has (some widths' rings
+// are as small as 156 KB, which left room for a CTA of prompt attention over heads of up to 64 columns).
+static int persistent_shared(int row_tiles, int width) {
+    const int ring = persistent_stages(row_tiles, width) * (row_tiles * GEMM_BOX_BYTES + width * GEMM_BK * 2);
+    const int bytes = ring + GEMM_BARRIER_BYTES + 1024;
+    return bytes > ALL_COLUMNS_SHARED ? bytes : ALL_COLUMNS_SHARED;
+}
+KIRAI_EXPORT int kirai_gemm_bf16_many_shared(int row_tiles, int width) { return persistent_shared(row_tiles, width); }
 static PersistentTile persistent_tile(int M, int N, int K, int epi, bool grouped, size_t out_bytes) {
     if (epi == 2 || grouped) return PersistentTile{1, N <= 128 ? 128 : 256};
     const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -1323,8 +1333,7 @@ static int launch_persistent_tile(int width, const void* A, const void* W, bool 
     const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
     const int stages = persistent_stages(MT, width);
     auto kernel = gemm_tcgen05_persistent_kernel<MT, OutT, EPI>;
-    const int smem_bytes = stages * (MT * GEMM_BOX_BYTES + width * GEMM_BK * 2) + GEMM_BARRIER_BYTES + 1024 +  // + slack to align the ring
-                           (EPI == 2 ? 4 * 32 * 32 * 4 : 0);                                                   // + the epilogue's staging buffers
+    const int smem_bytes = persistent_shared(MT, width) + (EPI == 2 ? 4 * 32 * 32 * 4 : 0);  // + the epilogue's staging buffers
     cudaError_t err = allow_shared((const void*)kernel, smem_bytes);
     if (err != cudaSuccess) return (int)err;
     return launch_pdl(kernel, dim3(grid), dim3(64 + 128 * MT), (size_t)smem_bytes, stream, 1u, map_a, map_w,

@@ -105,6 +105,19 @@ __device__ __forceinline__ void bulk_load_1d_once(uint32_t dst, const void* src,
 }
 
 // ------------------------------------------------------------- tensor memory
+// `tmem_alloc` waits until the columns are free, without a limit, and a kernel may hold columns while it waits for the kernels
+// ahead of it in its stream.  So that no two of them wait for each other:
+//  * a kernel that takes its columns after pdl_wait() lets the next kernel start only once it has them: a CTA of the next one
+//    that came first would keep the columns and wait for the end of this one, which would wait for the columns;
+//  * a CTA that takes all 512 columns asks for at least ALL_COLUMNS_SHARED bytes of shared memory, beside which no other CTA that
+//    uses tensor memory fits an SM (`alone_with_all_columns`, asserted by each of these kernels with its smallest size).
+// The other kernels take their columns ahead of pdl_wait(), and those of any of their CTAs that fit an SM together are at most 512
+// (32 columns with 75 KB, 64 and 128 with 99, 256 with 83 or 195).
+constexpr int SM_SHARED = 228 * 1024, CTA_SHARED_RESERVED = 1024;  // bytes of an SM, and what the system takes for each of its CTAs
+constexpr int ALL_COLUMNS_SHARED = 192 * 1024;
+constexpr bool alone_with_all_columns(int dynamic_bytes) {
+    return dynamic_bytes + CTA_SHARED_RESERVED + ALL_COLUMNS_SHARED + CTA_SHARED_RESERVED > SM_SHARED;
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t columns) {  // whole warp; columns: power of 2 >= 32
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(columns) : "memory");
 }
