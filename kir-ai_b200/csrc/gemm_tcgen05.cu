@@ -186,8 +186,6 @@ __device__ __forceinline__ void named_barrier_128() { asm volatile("bar.sync 1, 
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // The address, in the cluster's shared window, that `local` has in CTA `rank`; and a store to it.
 __device__ __forceinline__ uint32_t cluster_address(uint32_t local, uint32_t rank) {
     uint32_t remote;
@@ -260,7 +258,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     constexpr bool CHOSEN = sizeof...(Chosen) > 0;
     static_assert(!CHOSEN || (SWAP && BN <= 64 && EPI == 0), "the list lies behind the row scales of up to 64 tokens");
     constexpr int STAGES = Smem::stages;
-    constexpr bool ANNOUNCED = !Smem::late_slots && BN >= 64;
     constexpr bool LATE = Smem::late_slots;  // what other CTAs send lies in the receiver's ring (see GemmSmem)
     // Tiles of 32 tokens and more, split along K: every CTA of the cluster sums and stores a share of the tile's
     // 16-token chunks (chunk c belongs to CTA c % splits) instead of the first CTA all of it.  A CTA sends the chunks
@@ -353,7 +350,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     __syncthreads();
     tc_fence_after();
     if constexpr (CHOSEN) pdl_launch_dependents();
-    if (ANNOUNCED && splits > 1) cluster_arrive();
+    if (!LATE && splits > 1) cluster_say_begun();
     const uint32_t tmem_base = *tmem_slot;
     float res[16];  // EPI 2: the stream's values under this thread's 16 outputs
     float norm_w = 0.0f;
@@ -486,10 +483,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
     // LATE: the receivers' rings take what is sent, so nothing is sent before every CTA of the cluster has seen its
     // last product finish (all threads arrive here, the epilogue warps after their wait for the accumulator).  Else it is enough
-    // that every CTA of the cluster has begun, which it said long ago.  (Tiles of up to 32 tokens leave that out: a cluster's CTAs
-    // begin together, and the pair of barriers cost a layer of the 8B shape's products 0.7 of 65 us at one token.)
-    if (LATE && splits > 1) cluster_sync_all();
-    if (ANNOUNCED && splits > 1) cluster_wait();
+    // that every CTA of the cluster has begun, which it said long ago.
+    if (splits > 1) {
+        __syncwarp();  // (a warp's load or MMA thread comes from a branch of its own)
+        if (LATE) cluster_sync_all();
+        else cluster_wait_begun();
+    }
     if (warp >= 2 && scatter) {
         // every chunk of 16 tokens that another CTA owns goes to that CTA: its slot [sender][chunk / splits], the senders
         // in rank order without the owner itself, 16 x 128 floats column-major (lanes side by side)

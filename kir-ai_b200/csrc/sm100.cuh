@@ -174,6 +174,13 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
+// ------------------------------------------------------------------ clusters
+// Shared memory of another CTA of the cluster may be touched only once that CTA runs.  Every thread of the cluster says so as soon as
+// its CTA is set up (nothing is released: what a CTA writes for others is ordered by a later meeting) and waits for the others
+// right before the first store to one of them, long after they have said it.
+__device__ __forceinline__ void cluster_say_begun() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_begun() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // 32 consecutive 32-bit columns of this thread's lane (warp w of a warpgroup reads lanes 32 (w % 4) ..).
 __device__ __forceinline__ void tmem_load_32x32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(

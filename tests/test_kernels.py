@@ -260,6 +260,21 @@ def test_linear_tcgen05_against_plain(ops, m, n, k, out_dtype):
     ops.check_device_errors(torch.device(DEV))
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 128, 200])
+@pytest.mark.parametrize("splits", [2, 3, 4])
+def test_split_products_of_one_block_a_cta(ops, m, splits):
+    """The shortest way from a CTA's start to its first store into another CTA's shared memory: every one must have begun by then.
+    The same bits each time, and the sums of 64 * splits products."""
+    x, w = rand(m, 64 * splits, dtype=torch.bfloat16), rand(640, 64 * splits, dtype=torch.bfloat16, seed=3)
+    tiled = ops.tile_weight(w)
+    out = ops.linear_tcgen05(x, tiled, torch.float32, splits=splits)
+    expected, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((out.double() - expected).abs() <= 64 * splits * 2.0 ** -24 * size).all())  # 32-bit sums in any order
+    for _ in range(20):
+        assert torch.equal(ops.linear_tcgen05(x, tiled, torch.float32, splits=splits), out)
+    ops.check_device_errors(torch.device(DEV))
+
+
 # tiles of the many-token kernel that the rule picks on 148 SMs: 128 and 256 rows (with a last tile of one half, or of a part of
 # one), widths that cut weight boxes, columns beyond the last whole tile or box, a K that ends inside a block
 @pytest.mark.parametrize("m,n,k", [(300, 2560, 64), (300, 6144, 72), (640, 2568, 136), (1100, 2560, 264), (1408, 4104, 1096),
