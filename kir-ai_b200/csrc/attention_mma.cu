@@ -750,7 +750,8 @@ __device__ __forceinline__ void append_new_token(const DecodeArgs& args, const f
 // CTA's first work: the tiles that earlier steps filled are requested before griddepcontrol.wait, the rest after.
 // t_begin and t_end count the tiles that the query walks (`runs`: a window that keeps the sequence's first `keep` keys
 // walks those keys' tiles and then the window's; without kept keys walked tile v is key tile runs.first + v).
-template <int D, bool HEADS, int W = DecodeTile<D>::WARPS>
+// CLUSTER: dst_partial may lie in another CTA's shared memory, and this CTA has said that it runs (cluster_say_begun).
+template <int D, bool HEADS, int W = DecodeTile<D>::WARPS, bool CLUSTER = false>
 __device__ __forceinline__ int decode_attend_range(const CUtensorMap& kv_map, const DecodeArgs& args, uint8_t* smem, int req,
                                                    int kv_head, int pos, int key_lo, int last_tile, int t_begin, int t_end,
                                                    int k_base, bool first, bf16* __restrict__ out,
@@ -984,6 +985,7 @@ __device__ __forceinline__ int decode_attend_range(const CUtensorMap& kv_map, co
     }
     }
     __syncthreads();
+    if constexpr (CLUSTER) sm100::cluster_wait_begun();
     for (int id = tid; id < group * head_dim; id += DC_WARPS * 32) {
         const int row = id / head_dim, col = id % head_dim;
         float m_all = -INFINITY;
@@ -1094,6 +1096,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, DecodeArgs a
     if (threadIdx.x == 0) sm100::tma_prefetch_descriptor(&kv_map);
     decode_init_barriers<D, W>(smem);
     if (PAIR) {
+        sm100::cluster_say_begun();
         const int stride = args.head_dim + 2;
         float* own = reinterpret_cast<float*>(smem + Smem::q_bytes + Smem::merge_bytes);  // this CTA's rows, behind its warps' merge buffer
         float* slots = reinterpret_cast<float*>(smem + Smem::pair_offset);  // in the first CTA: the other CTAs' rows, [rank - 1][group][stride]
@@ -1104,8 +1107,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, DecodeArgs a
             asm volatile("mapa.u64 %0, %1, %2;" : "=l"(mapped) : "l"((unsigned long long)(uintptr_t)(slots + (size_t)(split - 1) * group * stride)), "r"(0u));
             dst = reinterpret_cast<float*>((uintptr_t)mapped);
         }
-        decode_attend_range<D, HEADS>(kv_map, args, smem, req, kv_head, pos, key_lo, last_tile, t_begin, t_end, 0, true, out,
-                                      dst, (long)stride, runs, keep);
+        decode_attend_range<D, HEADS, W, true>(kv_map, args, smem, req, kv_head, pos, key_lo, last_tile, t_begin, t_end, 0, true, out,
+                                               dst, (long)stride, runs, keep);
         // the rows are in place in the first CTA (release), which may read them after the meeting (acquire)
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (split == 0) {

@@ -823,6 +823,26 @@ def test_decode_attention_cut_into_any_number_of_ranges(ops, q_heads, kv_heads, 
     ops.check_device_errors(q.device)
 
 
+@pytest.mark.parametrize("q_heads,kv_heads,head_dim", [(8, 2, 128), (32, 2, 64), (6, 6, 48)])
+def test_decode_attention_with_more_ranges_than_keys(ops, q_heads, kv_heads, head_dim):
+    """Clusters of two to five CTAs of which some have no keys and come to their stores into the first CTA's shared memory at once."""
+    dtype, page_size, lengths = torch.bfloat16, 16, [1, 15, 17, 40]
+    cache, table, keys, values = paged_setup(dtype, lengths, kv_heads, head_dim, page_size, seed=31)
+    for r, length in enumerate(lengths):
+        ops.kv_write(keys[r].to(DEV).contiguous(), values[r].to(DEV).contiguous(), cache, table,
+                     torch.full((length,), r, dtype=torch.int32, device=DEV), torch.arange(length, dtype=torch.int32, device=DEV))
+    q = rand(len(lengths), q_heads, head_dim, dtype=dtype, seed=32)
+    ctx = torch.tensor(lengths, dtype=torch.int32, device=DEV)
+    one = ops.attention_decode(q, cache, table, ctx, None, head_dim ** -0.5, 1).float()
+    for splits in (2, 3, 4, 5):
+        got = ops.attention_decode(q, cache, table, ctx, None, head_dim ** -0.5, splits)
+        # one rounding of the result and the weights to bfloat16 (2^-9 each) on values of up to about 4, as above
+        assert float((got.float() - one).abs().max()) <= 1e-2, splits
+        for _ in range(10):
+            assert torch.equal(ops.attention_decode(q, cache, table, ctx, None, head_dim ** -0.5, splits), got), splits
+    ops.check_device_errors(q.device)
+
+
 @pytest.mark.parametrize("m,inter,k,splits", [(1, 128, 64, 0), (5, 200, 136, 0), (16, 1000, 512, 3), (64, 1536, 1032, 8),
                                               (65, 264, 192, 0), (128, 1536, 1032, 0), (100, 6144, 1024, 3), (250, 1536, 2048, 2),
                                               (300, 1000, 520, 0), (1024, 768, 256, 0)])
