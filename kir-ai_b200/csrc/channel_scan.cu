@@ -696,23 +696,22 @@ KIRAI_EXPORT int kirai_channel_chunks(const float* rows, long stride, const floa
     a.cols = choose_cols((long)(share ? units : requests) * heads, d, dv, share != nullptr);
     if (a.cols <= 0) return KIRAI_ERR_UNSUPPORTED;
     const int runs = cols_pitch(a.cols) / 16, pieces = (dv + a.cols - 1) / a.cols;
-    static long granted_prepare = 0, granted[3][5] = {};  // (one device a process)
     const long prepare_bytes = prepare_floats(d, rank) * 4;
-    status = grant_shared(channel_prepare_kernel, prepare_bytes, &granted_prepare);
+    status = (int)allow_shared((const void*)channel_prepare_kernel, (int)prepare_bytes);
     if (status == 0)
         status = launch_pdl(channel_prepare_kernel, dim3(units, heads), dim3(THREADS), (size_t)prepare_bytes, stream, 1u, a);
     if (status != 0) return status;
     if (!share) {
         auto chain = KIRAI_BY_RUNS(runs, channel_chain_kernel);
         const long bytes = product_floats(d, a.cols, CHAIN) * 4;
-        status = grant_shared(chain, bytes, &granted[0][runs]);
+        status = (int)allow_shared((const void*)chain, (int)bytes);
         return status != 0 ? status : launch_pdl(chain, dim3(requests, heads, pieces), dim3(THREADS), (size_t)bytes, stream, 1u, a);
     }
     auto own = KIRAI_BY_RUNS(runs, channel_share_kernel);
     auto out = KIRAI_BY_RUNS(runs, channel_out_kernel);
     const long own_bytes = product_floats(d, a.cols, SHARE) * 4, bytes = product_floats(d, a.cols, READ) * 4;
-    status = grant_shared(own, own_bytes, &granted[1][runs]);
-    if (status == 0) status = grant_shared(out, bytes, &granted[2][runs]);
+    status = (int)allow_shared((const void*)own, (int)own_bytes);
+    if (status == 0) status = (int)allow_shared((const void*)out, (int)bytes);
     if (status == 0) status = launch_pdl(own, dim3(units, heads, pieces), dim3(THREADS), (size_t)own_bytes, stream, 1u, a);
     if (status == 0)
         status = launch_pdl(channel_carry_kernel, dim3(requests, heads, (unsigned)(((long)d * dv + 255) / 256)), dim3(256), 0, stream, 1u, a);

@@ -70,14 +70,6 @@ __device__ __forceinline__ int first_chunk(const int* __restrict__ query_start, 
     return before;
 }
 
-template <typename Kernel>
-int grant_shared(Kernel kernel, long bytes, long* granted) {
-    if (bytes <= *granted) return 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return launch_status();
-    *granted = bytes;
-    return 0;
-}
-
 #define KIRAI_BY_RUNS(runs, name) ((runs) == 1 ? name<1> : (runs) == 2 ? name<2> : (runs) == 3 ? name<3> : name<4>)
 
 }  // namespace

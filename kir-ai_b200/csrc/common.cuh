@@ -204,6 +204,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 
 #include <cstdlib>
 #include <map>
+#include <mutex>
 #include <utility>
 static inline bool pdl_enabled() {
     static const bool enabled = [] {
@@ -213,18 +214,26 @@ static inline bool pdl_enabled() {
     return enabled;
 }
 
-// Raises `kernel`'s limit on dynamic shared memory to `bytes`, asking the runtime only where this thread has not done so on this
-// device (a limit that stands is no smaller than the kernel's other launches want).
+// Raises `kernel`'s limit on dynamic shared memory on the current device to `bytes`, and never lowers it: the limit is one for all
+// threads of the process, whose launches of a kernel may want different sizes.  The runtime is asked only where the known limit is
+// too low (every launch of a kernel is in one source file, which keeps the limits of its kernels).
 static inline cudaError_t allow_shared(const void* kernel, int bytes) {
-    static thread_local std::map<std::pair<const void*, int>, int> granted;
+    static std::mutex mutex;
+    static std::map<std::pair<const void*, int>, int> granted;
     int device = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess) return err;
-    int& known = granted[std::make_pair(kernel, device)];
-    if (bytes <= known) return cudaSuccess;
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (err == cudaSuccess) known = bytes;
-    return err;
+    try {
+        std::lock_guard<std::mutex> lock(mutex);
+        int& known = granted[std::make_pair(kernel, device)];
+        if (bytes <= known) return cudaSuccess;
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (err == cudaSuccess) known = bytes;
+        else cudaGetLastError();  // (a refusal leaves no error behind)
+        return err;
+    } catch (...) {  // (no room for the entry; nothing may be thrown through a C entry point)
+        return cudaErrorMemoryAllocation;
+    }
 }
 
 // Launches `kernel` with programmatic stream serialization (and, if cluster_z > 1, as clusters of

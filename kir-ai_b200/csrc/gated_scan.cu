@@ -541,7 +541,7 @@ int real_gated_step_launch(const StepArgs& a, int gates_bf16, void* out, cudaStr
     auto kernel = gates_bf16 ? (vec ? step_kernel<O, bf16, true>(a.taps) : step_kernel<O, bf16, false>(a.taps))
                              : (vec ? step_kernel<O, float, true>(a.taps) : step_kernel<O, float, false>(a.taps));
     if (smem > 48 * 1024) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t err = allow_shared((const void*)kernel, (int)smem);
         if (err != cudaSuccess) return (int)err;
     }
     return launch_pdl_clusters(kernel, dim3(cuts, blocks), dim3(256), smem, stream, dim3(cuts, 1, 1), a, (O*)out);

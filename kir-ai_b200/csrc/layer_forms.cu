@@ -541,7 +541,7 @@ static int qkv_wide_norm_write_launch(const float* qkv, long qkv_stride, const f
                        (uintptr_t)k_weight | (uintptr_t)q_out | (uintptr_t)cache) & 15) == 0;
     auto kernel = vec ? qkv_wide_norm_write_kernel<T, true> : qkv_wide_norm_write_kernel<T, false>;
     if (smem > 48 * 1024) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t err = allow_shared((const void*)kernel, (int)smem);
         if (err != cudaSuccess) return (int)err;
     }
     const int cols = (q_heads + kv_heads) * dk;

@@ -209,7 +209,7 @@ static int add_layernorm_launch(float* resid, const void* delta, const float* de
     const size_t smem = (size_t)hidden * sizeof(float);
     auto kernel = add_layernorm_kernel<T, O>;
     if (smem > 48 * 1024) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t err = allow_shared((const void*)kernel, (int)smem);
         if (err != cudaSuccess) return (int)err;
     }
     const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);

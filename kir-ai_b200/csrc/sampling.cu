@@ -725,7 +725,7 @@ KIRAI_EXPORT int kirai_sample_rows(const float* logits, float* probs_scratch, co
     int per = 0;
     if (sample_rows_over_a_cluster(rows, vocab, &per)) {
         const size_t slice_bytes = (size_t)per * sizeof(float);
-        cudaError_t err = cudaFuncSetAttribute(sample_rows_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slice_bytes);
+        cudaError_t err = allow_shared((const void*)sample_rows_cluster_kernel, (int)slice_bytes);
         if (err != cudaSuccess) return (int)err;
         return launch_pdl_clusters(sample_rows_cluster_kernel, dim3(SC_CTAS, rows), dim3(SC_THREADS), slice_bytes, stream,
                                    dim3(SC_CTAS, 1, 1), logits, temperature, top_p, draw, out, vocab, per, error_flag);

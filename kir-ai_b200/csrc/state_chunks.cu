@@ -752,14 +752,12 @@ int chunk_scan_launch(ChunkScan a, int requests, int units, ChunkSide side, cuda
     if (a.cols <= 0) return KIRAI_ERR_UNSUPPORTED;
     const int runs = cols_pitch(a.cols) / 16;
     const int pieces = (a.dv + a.cols - 1) / a.cols;
-    static long granted[3][5] = {};  // (one device a process)
     if (units > 0 && rows_in_quads(a, side)) {
         const int wide = (a.dv + COLS - 1) / COLS;
         const long local_bytes = 4 * (local_rows_floats(a.d) > scores_floats(a.d) ? local_rows_floats(a.d) : scores_floats(a.d));
         const long out_bytes = 4 * out_rows_floats(a.d);
-        static long granted_rows[2] = {};
-        int status = grant_shared(chunk_local_rows_kernel, local_bytes, &granted_rows[0]);
-        if (status == 0) status = grant_shared(chunk_out_rows_kernel, out_bytes, &granted_rows[1]);
+        int status = (int)allow_shared((const void*)chunk_local_rows_kernel, (int)local_bytes);
+        if (status == 0) status = (int)allow_shared((const void*)chunk_out_rows_kernel, (int)out_bytes);
         if (status == 0)
             status = launch_pdl(chunk_local_rows_kernel, dim3(units, a.heads, wide + 1), dim3(THREADS), (size_t)local_bytes, stream, 1u, a, side,
                                 requests, wide);
@@ -774,8 +772,8 @@ int chunk_scan_launch(ChunkScan a, int requests, int units, ChunkSide side, cuda
     if (units > 0) {
         auto local = KIRAI_BY_RUNS(runs, chunk_local_kernel);
         auto out = KIRAI_BY_RUNS(runs, chunk_out_kernel);
-        int status = grant_shared(local, bytes, &granted[1][runs]);
-        if (status == 0) status = grant_shared(out, bytes, &granted[2][runs]);
+        int status = (int)allow_shared((const void*)local, (int)bytes);
+        if (status == 0) status = (int)allow_shared((const void*)out, (int)bytes);
         if (status == 0)
             status = launch_pdl(local, dim3(units, a.heads, pieces), dim3(THREADS), (size_t)bytes, stream, 1u, a, side, requests);
         const long entries = (long)a.d * a.dv + (a.memory ? a.d : 0);
@@ -787,7 +785,7 @@ int chunk_scan_launch(ChunkScan a, int requests, int units, ChunkSide side, cuda
         return status;
     }
     auto kernel = KIRAI_BY_RUNS(runs, chunk_scan_kernel);
-    int status = grant_shared(kernel, bytes, &granted[0][runs]);
+    int status = (int)allow_shared((const void*)kernel, (int)bytes);
     if (status != 0) return status;
     status = launch_pdl(kernel, dim3(requests, a.heads, pieces), dim3(THREADS), (size_t)bytes, stream, 1u, a);
     if (status != 0 || !a.memory) return status;

@@ -199,7 +199,7 @@ int streams_norm_launch(const StreamArgs& a, void* out, int rows, cudaStream_t s
     if (smem > 200 * 1024) return KIRAI_ERR_BAD_SIZE;
     auto kernel = streams_norm_kernel<T>;
     if (smem > 48 * 1024) {
-        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t err = allow_shared((const void*)kernel, (int)smem);
         if (err != cudaSuccess) return (int)err;
     }
     return launch_pdl(kernel, dim3(rows), dim3(threads), smem, stream, 1u, a, (T*)out);

@@ -306,6 +306,28 @@ def test_many_token_products_take_the_tiles_tested_above(ops):
     assert {rows for rows, _ in tiles} == {1, 2} and len({width for _, width in tiles}) >= 6 and any(width % 128 for _, width in tiles)
 
 
+def test_threads_whose_products_want_different_shared_memory(ops):
+    """One kernel, two sizes: the smaller one, launched first by another thread, must not take from the larger one what it was
+    granted before (a limit belongs to the kernel, not to a thread)."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    rows = (1153, 2048)  # tiles of 256 x 144 and 256 x 240 on 148 SMs
+    tiles = [divmod(ops.library().kirai_gemm_bf16_many_tile(m, 4096, 4096, 0), 1000) for m in rows]
+    sizes = [ops.library().kirai_gemm_bf16_many_shared(*tile) for tile in tiles]
+    assert tiles[0][0] == tiles[1][0] and sizes[0] > sizes[1]
+    w = ops.tile_weight(rand(4096, 4096, dtype=torch.bfloat16, scale=0.1))
+    x = [rand(m, 4096, dtype=torch.bfloat16, scale=0.5) for m in rows]
+    begin = lambda: torch.ones(1, device=DEV).add_(1)  # noqa: E731  (a launch of torch's, which gives the thread its device)
+    with ThreadPoolExecutor(1, initializer=begin) as first, ThreadPoolExecutor(1, initializer=begin) as second:
+        wanted = first.submit(ops.linear_tcgen05, x[0], w).result()
+        second.submit(ops.linear_tcgen05, x[1], w).result()
+        assert torch.equal(first.submit(ops.linear_tcgen05, x[0], w).result(), wanted)
+        # and at the same time
+        runs = [pool.submit(lambda i=i: [ops.linear_tcgen05(x[i], w) for _ in range(50)][-1]) for i, pool in enumerate((first, second))]
+        assert torch.equal(runs[0].result(), wanted) and runs[1].result().shape == (rows[1], 4096)
+    ops.check_device_errors(torch.device(DEV))
+
+
 def test_linear_refuses_rows_that_tma_cannot_read(ops):
     x, w = rand(4, 70, dtype=torch.bfloat16), rand(32, 70, dtype=torch.bfloat16)
     with pytest.raises(ops.KernelError):
