@@ -406,7 +406,7 @@ __device__ __forceinline__ void prefetch_state_rows(const float* mine, int lane,
 
 // ------------------------------------------------------------------ state-space walk
 // Block (request, head); thread (p, s): column p of the head's state [N, P], rows s, s + SPLIT, ...
-// WIDE (a block has whole runs of 32 columns): the threads of a warp have adjacent columns of the same rows, so that the state is
+// WIDE (a block has whole runs of 32 columns, with 256 threads up to eight a column: states of up to WALK_WIDE_ROWS rows): the threads of a warp have adjacent columns of the same rows, so that the state is
 // read and written in whole lines and B and C are the same address for a warp; a column's threads meet in shared memory.
 // Otherwise they lie side by side in a warp, which touches 16 bytes of each row, and meet by shuffles.  Three requests, 128
 // heads of 128 x 64: 16.2 and 13.3 us inside a step (the matrix memory, 16 heads of 128 x 256: 16.8 and 15.7), before registers were
@@ -415,6 +415,7 @@ __device__ __forceinline__ void prefetch_state_rows(const float* mine, int lane,
 // dt_stride): the step sizes before softplus; y [T, inner] (float32) = S^T C + D x.
 // Registers are kept to 40 where a column's threads hold 16 rows each: at 74 an SM took three blocks of the 768 that three requests
 // make, and the second round of blocks waited a second time for everything that one waits for (11.7 to 9.6 us a launch).
+#define WALK_WIDE_ROWS 128
 template <int REGS, bool WIDE>
 __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, long dt_stride,
                                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
@@ -426,7 +427,7 @@ __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kern
     const int columns = blockDim.x / split;
     const int p = blockIdx.z * columns + (WIDE ? threadIdx.x % columns : threadIdx.x / split), s = WIDE ? threadIdx.x / columns : threadIdx.x % split;
     __shared__ float part[WIDE ? 2 : 1][WIDE ? 256 : 1];
-    __shared__ float bc_s[WIDE ? 2 : 1][WIDE ? 512 : 1];  // a token's B and C, up to 256 columns each
+    __shared__ float bc_s[WIDE ? 2 : 1][WIDE ? 2 * WALK_WIDE_ROWS : 1];  // a token's B and C
     const long first = query_start[request];
     const int count = (int)(query_start[request + 1] - first);
     const int slot = slots[request];
@@ -523,7 +524,7 @@ KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_s
     int split, threads, chunks;
     const int regs = walk_shape(N, P, &split, &threads, &chunks);
     if (!regs) return KIRAI_ERR_BAD_SIZE;
-    const bool wide = (threads / split) % 32 == 0 && N <= 256;  // (a token's B and C lie in shared memory)
+    const bool wide = (threads / split) % 32 == 0 && N <= WALK_WIDE_ROWS;
 #define KIRAI_SSM(R)                                                                                                         \
     return launch_pdl(wide ? ssm_walk_kernel<R, true> : ssm_walk_kernel<R, false>, dim3(requests, heads, chunks), dim3(threads), 0, stream, 1u, xbc, dt_raw, dt_stride, \
                       dt_bias, a_log, d_skip, state, state_len, ssm_off, query_start, slots, y, heads, groups, N, P, split,  \

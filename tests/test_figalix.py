@@ -1096,7 +1096,9 @@ def test_sums_under_a_tanh_and_pairs_of_normed_rows_from_aligned_rows(rows, widt
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("heads,groups,state,vdim", [(2, 2, 132, 96), (1, 1, 256, 64), (1, 1, 260, 64)])
-def test_walks_up_to_and_beyond_the_columns_that_shared_memory_holds(heads, groups, state, vdim):
-    """A block's threads hold whole runs of 32 columns here; up to 256 rows of a state B and C come through shared memory."""
+@pytest.mark.parametrize("heads,groups,state,vdim", [(2, 2, 128, 96), (1, 1, 100, 33), (1, 1, 16, 64), (1, 1, 4, 40), (2, 2, 132, 96), (1, 1, 256, 64),
+                                                     (1, 1, 260, 64)])
+def test_walks_up_to_and_beyond_the_rows_that_shared_memory_holds(heads, groups, state, vdim):
+    """Up to 128 rows of a state a block's threads hold whole runs of 32 columns (the first four; 8 threads a column, 8 with columns
+    beyond the last, 1, and 1 with 4 rows) and B and C come through shared memory; from 129 rows on they hold 16 columns or 8."""
     test_state_space_runs_in_chunks_as_token_by_token(heads, groups, state, vdim)
