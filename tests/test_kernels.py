@@ -1025,6 +1025,29 @@ def test_32_bit_attention_tiles_against_64_bit_arithmetic(ops, q_heads, kv_heads
             assert float((got.double() - rows)[finite].abs().max()) <= bound, (r, float((got.double() - rows)[finite].abs().max()))
 
 
+# 32 and 8 heads: 8 CTAs for each 16 tokens.  On 148 SMs: one CTA an SM at most, two from 149 CTAs on (the order of whose second ones is
+# turned), the last launch of two an SM, and one more
+@pytest.mark.parametrize("tokens,before,q_heads,kv_heads,window", [(288, 0, 32, 8, None), (300, 0, 32, 8, None), (405, 0, 32, 8, None), (405, 333, 32, 8, 100),
+                                                                   (592, 17, 32, 8, None), (593, 0, 32, 8, None), (1000, 0, 12, 3, None)])
+def test_32_bit_attention_of_one_request_in_every_order_of_its_tiles(ops, tokens, before, q_heads, kv_heads, window):
+    length, head_dim, page_size = tokens + before, 128, 16
+    cache, table, keys, values = paged_setup(torch.float32, [length], kv_heads, head_dim, page_size, seed=5)
+    ops.kv_write(keys[0].to(DEV).contiguous(), values[0].to(DEV).contiguous(), cache, table, torch.zeros(length, dtype=torch.int32, device=DEV),
+                 torch.arange(length, dtype=torch.int32, device=DEV))
+    q = rand(tokens, q_heads, head_dim, seed=6)
+    start, context = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ([0, tokens], [length]))
+    out = torch.full((tokens, q_heads * head_dim), float("nan"), device=DEV)
+    ops.attention_f32_prefill(q, cache, table, start, context, tokens, window, head_dim ** -0.5, out=out)
+    ops.check_device_errors(torch.device(DEV))
+    k, v = (x[0].double().to(DEV).repeat_interleave(q_heads // kv_heads, dim=1) for x in (keys, values))
+    i, j = torch.arange(before, length, device=DEV)[:, None], torch.arange(length, device=DEV)[None, :]
+    seen = (j <= i) & ((i - j < window) if window else True)
+    scores = torch.einsum("thd,jhd->htj", q.double(), k) * head_dim ** -0.5
+    expected = torch.einsum("htj,jhd->thd", torch.softmax(scores.masked_fill(~seen, -math.inf), dim=-1), v)
+    # every row written, and within the bound derived above
+    assert float((out.view(tokens, q_heads, head_dim).double() - expected).abs().max()) <= 3e-5
+
+
 def test_32_bit_attention_reports_a_missing_page(ops):
     cache, table, keys, values = paged_setup(torch.float32, [40], 1, 32, 8)
     q = rand(40, 2, 32)
