@@ -21,6 +21,8 @@
 //
 // Values that are not finite: the cuts of an infinity are not numbers, so a sum that is not finite is worked out again by
 // its thread as the chain of FMAs that the plain kernel computes.
+#include <algorithm>
+
 #include "sm100.cuh"
 #include "tensor_map.cuh"
 
@@ -357,13 +359,22 @@ int launch_tc(const float* A, const float* W, const bf16* planes, float* C, int 
 // round of CTAs takes 8 us and, per 32 values of K, 0.66 us (32 rows, two CTAs on an SM or one), 0.58 or 0.90 us (64 rows,
 // one or two), 0.70 us (128 rows) or 0.88 us (192 rows); fewer CTAs run at once where they come in clusters of 3, 4 or 8.
 // A split has to save a twentieth.  (Of all cuts, swept over 4 weight sizes and 9 to 800 rows, this takes the fastest.)
+// The times and the clusters that run at once are those of 148 SMs; with another number a round is as many CTAs as that holds.
+static int sm_count() {
+    static const int count = [] {
+        int device = 0, value = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 148;
+        return value;
+    }();
+    return count;
+}
 struct Cut {
     int bn, splits;
     float us;  // by the times above
 };
 static constexpr int cut_rows[4] = {32, 64, 128, 192};
 static constexpr float cut_block_us[4] = {0.66f, 0.58f, 0.70f, 0.88f};
-static Cut choose_cut(int M, int N, int K) {
+static Cut choose_cut(int M, int N, int K, int sms) {
     constexpr int cuts[5] = {1, 2, 3, 4, 8}, at_once[5] = {148, 148, 120, 132, 112};
     constexpr const int* bns = cut_rows;
     constexpr const float* block_us = cut_block_us;
@@ -378,7 +389,7 @@ static Cut choose_cut(int M, int N, int K) {
         for (int c = 0; c < 5; ++c) {
             const int s = cuts[c];
             if (s > 1 && blocks / s < 4) break;
-            const long ctas = tiles * s, room = bns[b] <= 64 ? 2 * at_once[c] : at_once[c];
+            const long ctas = tiles * s, fit = std::max(1L, (long)at_once[c] * sms / 148), room = bns[b] <= 64 ? 2 * fit : fit;
             const long rounds = (ctas + room - 1) / room;
             const float us = bns[b] == 64 && ctas > 128 ? 0.90f : block_us[b];
             const float total = (float)rounds * (8.0f + us * (float)((blocks + s - 1) / s)) * (s > 1 ? 1.05f : 1.0f);
@@ -395,21 +406,25 @@ static Cut choose_cut(int M, int N, int K) {
 // 12), the columns of the whole rounds are one launch and the rest a second one with a cut of its own, finer along K, which
 // starts as the first one's CTAs end.  How many columns (a multiple of TILE_N) the first launch takes and its rows a tile;
 // 0 where one launch is as good to a twentieth.
-static int whole_rounds(int M, int N, int K, float single_us, int* bn) {
+static int whole_rounds(int M, int N, int K, int sms, float single_us, int* bn) {
     const int blocks = (K + BLOCK_K - 1) / BLOCK_K;
     const long columns = (N + TILE_N - 1) / TILE_N;
     float least = 0.95f * single_us;
     int taken = 0;
     for (int b = 0; b < 4; ++b) {
         if (b > 0 && cut_rows[b - 1] >= M) break;
-        const long row_tiles = (M + cut_rows[b] - 1) / cut_rows[b], room = cut_rows[b] <= 64 ? 296 : 148;
+        const long row_tiles = (M + cut_rows[b] - 1) / cut_rows[b], room = cut_rows[b] <= 64 ? 2L * sms : sms;
         const long rounds = columns * row_tiles / room, first = rounds * room / row_tiles;
-        if (rounds < 1 || first < 1 || first >= columns) continue;
+        if (rounds < 1 || first < 1 || first >= columns || row_tiles > 65535) continue;
         const float us = (cut_rows[b] == 64 ? 0.90f : cut_block_us[b]) * (float)blocks;
-        const float total = (float)rounds * (8.0f + us) + choose_cut(M, (int)(N - first * TILE_N), K).us;
+        const float total = (float)rounds * (8.0f + us) + choose_cut(M, (int)(N - first * TILE_N), K, sms).us;
         if (total < least) least = total, taken = (int)first * TILE_N, *bn = cut_rows[b];
     }
     return taken;
+}
+// The same for a device of `sms` SMs: the columns of the first launch (0: one launch takes them all), `rows` its rows a tile.
+KIRAI_EXPORT int kirai_gemm_f32_tc_first_columns(int M, int N, int K, int sms, int* rows) {
+    return whole_rounds(M, N, K, sms, choose_cut(M, N, K, sms).us, rows);
 }
 
 static int launch_cut(const Cut& cut, const float* A, const float* W, bf16* planes, float* C, int M, int N, int K, long lda, long ldc, int pitch,
@@ -438,9 +453,10 @@ KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || (long)3 * M > 0x7fffffffL || splits < 0 || splits > 8) return KIRAI_ERR_BAD_SIZE;
     if (K % 4 != 0 || lda % 4 != 0 || (((uintptr_t)A_ | (uintptr_t)W_ | (uintptr_t)planes_) & 15) != 0) return KIRAI_ERR_BAD_ALIGN;
-    const Cut cut = bn == 0 ? choose_cut(M, N, K) : Cut{bn, splits > 0 ? splits : 1, 0.0f};
+    const int sms = sm_count();
+    const Cut cut = bn == 0 ? choose_cut(M, N, K, sms) : Cut{bn, splits > 0 ? splits : 1, 0.0f};
     int first_bn = 0;
-    const int first = bn == 0 && splits == 0 ? whole_rounds(M, N, K, cut.us, &first_bn) : 0;
+    const int first = bn == 0 && splits == 0 ? whole_rounds(M, N, K, sms, cut.us, &first_bn) : 0;
     const int pitch = (K + 7) / 8 * 8;
     const long quads = (long)M * (K / 4);
     const long cut_blocks = (quads + 255) / 256;
@@ -453,7 +469,7 @@ KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_
     if (first > 0) {
         const int done = launch_cut(Cut{first_bn, 1, 0.0f}, A, W, planes, C, M, first, K, lda, ldc, pitch, constant, error_flag, stream);
         if (done != 0) return done;
-        return launch_cut(choose_cut(M, N - first, K), A, W + (size_t)first * K, planes, C + first, M, N - first, K, lda, ldc, pitch, constant,
+        return launch_cut(choose_cut(M, N - first, K, sms), A, W + (size_t)first * K, planes, C + first, M, N - first, K, lda, ldc, pitch, constant,
                           error_flag, stream);
     }
     return launch_cut(cut, A, W, planes, C, M, N, K, lda, ldc, pitch, constant, error_flag, stream);

@@ -1,0 +1,31 @@
+"""Rules by which launches are cut, asked on the host for devices of any size."""
+import ctypes
+
+import pytest
+
+
+@pytest.fixture(scope="module")
+def lib():
+    import kirai_b200  # noqa: F401
+    from kirai_b200.csrc import ops
+
+    return ops.library()
+
+
+@pytest.mark.parametrize("sms", [108, 132, 148, 160])
+def test_32_bit_products_fill_whole_rounds_of_the_device_that_runs_them(lib, sms):
+    cut = 0
+    a_little_more = 128 * (2 * sms // 3 + 3)  # columns that make two rounds and about nine CTAs of three tiles of 192 rows
+    for m, n, k in [(576, a_little_more, 2560), (515, 19456, 516), (515, 19456, 2560), (576, 6460, 1028), (128, 19200, 700), (30, 38404, 260), (800, 24576, 4096), (9, 151936, 2560)]:
+        rows = ctypes.c_int(0)
+        first = lib.kirai_gemm_f32_tc_first_columns(m, n, k, sms, ctypes.byref(rows))
+        if first == 0:
+            continue
+        cut += 1
+        assert first % 128 == 0 and 0 < first < n and rows.value in (32, 64, 128, 192)
+        tiles, room = -(-m // rows.value), sms * (2 if rows.value <= 64 else 1)
+        ctas = first // 128 * tiles
+        assert ctas % room == 0 or room - ctas % room < tiles  # the last round lacks less than a column of tiles
+    assert cut
+    if sms == 148:  # 456 CTAs of 192 rows: three rounds, and 4 columns of tiles to the second launch
+        assert (lib.kirai_gemm_f32_tc_first_columns(515, 19456, 2560, sms, ctypes.byref(rows)), rows.value) == (148 * 128, 192)
