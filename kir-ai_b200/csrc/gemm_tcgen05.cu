@@ -242,21 +242,21 @@ __device__ __forceinline__ void gate_mul_pair(const Epilogue& ep, const float (&
     gate_mul_all<8>(ep, gate, up, out);
 }
 
-// SWAP false: X = A (rows m), Y = W (rows n), C[m, n].  SWAP true: X = W, Y = A.
+// X = W, Y = A: the weights' rows fill the MMA.
 // Split-K: the CTAs of a cluster (1, 1, splits) cover one tile; each stores its 32-bit partial
 // tile into its slot in the shared memory of the cluster's first CTA (distributed shared memory),
 // which adds the slots in rank order and stores the result: no partial sum goes to global memory.
 // EPI 0 stores C.  EPI 1 expects W's rows interleaved in eights (8 gate rows, the 8 matching up
 // rows, ...) and stores silu(gate) * up, [M, N / 2].
 // Chosen: nothing, or ChosenExperts.
-template <int BN, bool SWAP, typename OutT, int EPI, bool DEEP, typename... Chosen>
+template <int BN, typename OutT, int EPI, bool DEEP, typename... Chosen>
 __global__ void __launch_bounds__(GEMM_THREADS, GemmSmem<BN, DEEP>::ctas_per_sm)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
                     const uint8_t* __restrict__ w_tiled, OutT* __restrict__ C, int M, int N, int K, long ldc,
                     int k_blocks_per_split, int splits, Epilogue ep, int* __restrict__ error_flag, Chosen... chosen) {
     using Smem = GemmSmem<BN, DEEP>;
     constexpr bool CHOSEN = sizeof...(Chosen) > 0;
-    static_assert(!CHOSEN || (SWAP && BN <= 64 && EPI == 0), "the list lies behind the row scales of up to 64 tokens");
+    static_assert(!CHOSEN || (BN <= 64 && EPI == 0), "the list lies behind the row scales of up to 64 tokens");
     constexpr int STAGES = Smem::stages;
     constexpr bool LATE = Smem::late_slots;  // what other CTAs send lies in the receiver's ring (see GemmSmem)
     // Tiles of 32 tokens and more, split along K: every CTA of the cluster sums and stores a share of the tile's
@@ -265,7 +265,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     // order, which is the order in which the first CTA added whole tiles, so the sums are the same bits.  (With the
     // first CTA doing everything, a product of 64 tokens spent 3.7 us sending, 3.6 us adding and 4 us storing after
     // its last MMA; the o projection of the 8B shape took 18 us at 64 tokens and 8 us at 16.)
-    const bool scatter = SWAP && BN >= 32 && splits > 1;
+    const bool scatter = BN >= 32 && splits > 1;
     constexpr int CHUNKS = BN / 16;
     const int owned_chunks = scatter ? (CHUNKS + splits - 1) / splits : CHUNKS;  // the most that one CTA owns
     const int first_c0 = scatter ? 16 * (int)blockIdx.z : 0;  // this CTA's first chunk of tokens (none if beyond the tile)
@@ -354,12 +354,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
     float res[16];  // EPI 2: the stream's values under this thread's 16 outputs
     float norm_w = 0.0f;
-    // Staged stores (SWAP): a thread holds one output column of 16 tokens, so storing from that layout takes 16 to 32
+    // Staged stores: a thread holds one output column of 16 tokens, so storing from that layout takes 16 to 32
     // narrow store instructions a thread, which measured 0.4 to 2.6 us at the end of a launch (longest when the next
     // kernel's CTAs already stream beside it).  Where rows are 16-byte aligned the values go through shared memory
     // (the idle ring; 132 floats to a token) and every thread stores 16 adjacent columns of one token in 16-byte pieces.
     const bool c_aligned = ((uintptr_t)C & 15) == 0 && (ldc * (long)sizeof(OutT)) % 16 == 0;
-    const bool staged = SWAP && c_aligned &&
+    const bool staged = c_aligned &&
                         (EPI == 2 ? (N % 8 == 0 && (((uintptr_t)ep.residual | (uintptr_t)ep.norm_weight) & 15) == 0)
                                   : (EPI == 1 ? N % 16 == 0 : N % 8 == 0));
     float4 res4[4], norm4[4];  // EPI 2, staged: the stream's values and the norm's weights under this thread's 16 columns of token y0 + tile_row / 8
@@ -369,10 +369,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
     if (warp == 0) {
         if (elect_one()) {
-            // The weights do not depend on the kernel before this one: with SWAP the X operand (weights)
-            // of the first ring of stages is fetched at once, and only the activations wait for it.
-            const int x_first = SWAP ? 0 : 1, y_first = SWAP ? 1 : 0;  // which operand is the weights
-            // tiled weights (SWAP only): this tile's boxes lie one after the other
+            // The weights do not depend on the kernel before this one: those of the first ring of stages
+            // are fetched at once, and only the activations wait for it.
+            // tiled weights: this tile's boxes lie one after the other
             const uint8_t* boxes = w_tiled ? w_tiled + ((size_t)x_tile * total_k_blocks + kb_begin) * GEMM_BOX_BYTES : nullptr;
             // this CTA's i-th block of K, counted from kb_begin: the CTAs of a launch begin at blocks spread over the range and come
             // round, so that they do not all ask L2 for the same block of the tokens' rows at the same time (gate/up of the 4B
@@ -397,7 +396,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 return at < num_kb ? at : at - num_kb;
             };
             auto load_x = [&](uint32_t dst, uint32_t full, int i) {
-                if (SWAP && boxes) bulk_load_1d_once(dst, boxes + (size_t)i * GEMM_BOX_BYTES, GEMM_BOX_BYTES, full, evict_first);
+                if (boxes) bulk_load_1d_once(dst, boxes + (size_t)i * GEMM_BOX_BYTES, GEMM_BOX_BYTES, full, evict_first);
                 else tma_load_2d(dst, &map_x, full, (kb_begin + i) * GEMM_BK, x0);
             };
             const int head = num_kb < STAGES ? num_kb : STAGES;
@@ -405,18 +404,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 const uint32_t full = smem_addr(&full_bar[i]);
                 mbar_expect_tx(full, Smem::stage_bytes);
                 const uint32_t dst = smem_addr(smem + i * Smem::stage_bytes);
-                const int at = block(i), k = (kb_begin + at) * GEMM_BK;
-                if (x_first == 0) load_x(dst, full, at);
-                if (y_first == 0) tma_load_2d(dst + Smem::x_bytes, &map_y, full, k, y0);
+                load_x(dst, full, block(i));
             }
             pdl_wait();  // what the kernel before wrote (the activations) is complete and visible
             gemm_stamp(ep, 1);
             for (int i = 0; i < head; ++i) {
                 const uint32_t full = smem_addr(&full_bar[i]);
                 const uint32_t dst = smem_addr(smem + i * Smem::stage_bytes);
-                const int at = block(i), k = (kb_begin + at) * GEMM_BK;
-                if (x_first == 1) load_x(dst, full, at);
-                if (y_first == 1) tma_load_2d(dst + Smem::x_bytes, &map_y, full, k, y0);
+                tma_load_2d(dst + Smem::x_bytes, &map_y, full, (kb_begin + block(i)) * GEMM_BK, y0);
             }
             for (int i = head; i < num_kb; ++i) {
                 const int s = i % STAGES;
@@ -455,7 +450,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     } else {
         pdl_wait();  // the output buffer may still be read by the kernel before this one
         // what the epilogue reads from global memory is fetched while the products run
-        if ((rank == 0 || scatter) && SWAP) {
+        if (rank == 0 || scatter) {
             if (ep.row_sumsq) {
                 // the scales of this tile's tokens, computed once by the first BN threads
                 for (int t = tile_row; t < BN; t += GEMM_BM) scale_s[t] = (y0 + t < M) ? row_scale_of(ep, y0 + t, M) : 0.0f;
@@ -533,9 +528,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
     if (warp >= 2 && (rank == 0 || scatter)) {
         const int x_row = x0 + tile_row;  // row of X that this thread holds
-        const int x_rows = SWAP ? N : M;
-        const int y_rows = SWAP ? M : N;
-        const float my_scale = (!SWAP && ep.row_sumsq && x_row < M) ? row_scale_of(ep, x_row, M) : 1.0f;
+        const int x_rows = N, y_rows = M;
         // The staged stores take Smem::stage_tokens tokens at a time through shared memory: all of a tile of up to 64
         // tokens through the idle ring; of 128 tokens two halves; LATE: through what the received chunks leave of it.
         constexpr int HALF = Smem::stage_tokens;
@@ -547,7 +540,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         for (int c0 = h0; c0 < h0 + HALF; c0 += 16) {
             if (y0 + c0 >= y_rows) break;  // uniform across the warp
             if (scatter && (uint32_t)(c0 >> 4) % (uint32_t)splits != rank) continue;  // another CTA's chunk
-            if (EPI == 2 && SWAP && c0 != first_c0) load_residual_column<BN>(ep, x_row, y0, c0, M, N, res);
+            if (EPI == 2 && c0 != first_c0) load_residual_column<BN>(ep, x_row, y0, c0, M, N, res);
             float v[16];
             if (scatter) {
                 // the partial chunks in rank order: the other CTAs' from the slots, this CTA's own from tensor memory
@@ -592,7 +585,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             }
             if (ep.row_sumsq) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] *= SWAP ? scale_s[c0 + j] : my_scale;
+                for (int j = 0; j < 16; ++j) v[j] *= scale_s[c0 + j];
             }
             if (EPI == 3) {
                 // (v holds the whole sum over K here, also where the cluster split it)
@@ -600,7 +593,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 for (int j = 0; j < 16; ++j) v[j] = v[j] > 0.0f ? v[j] * v[j] : 0.0f;
             }
             if (tile_row == 0) gemm_stamp(ep, 6);
-            if (SWAP && staged) {
+            if (staged) {
                 // (every product has read the ring: it is free)
                 if (EPI == 1) {
                     // this lane holds weight row x_row: rows 16k..16k+7 are gate rows, 16k+8..16k+15 their up rows
@@ -614,7 +607,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 }
                 continue;
             }
-            if (EPI == 2 && SWAP) {
+            if (EPI == 2) {
                 // this lane holds output column x_row of tokens y0 + c0 .. + 15.  The squares of the sums go to shared
                 // memory (the ring is idle: every product has read it), token by token, 132 floats to a token; they
                 // are added up after the loop.  (Sixteen warp reductions here, one after the other, took 2 us.)
@@ -633,7 +626,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 }
                 continue;
             }
-            if (EPI == 1 && SWAP) {
+            if (EPI == 1) {
                 // this lane holds weight row x_row: rows 16k..16k+7 are gate rows, 16k+8..16k+15 their up rows
                 float out[8];
                 gate_mul_pair(ep, v, lane, out);
@@ -647,58 +640,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 continue;
             }
             if (x_row >= x_rows) continue;
-            if (EPI == 1) {
-                // columns y0 + c0 .. + 15 are 8 gate rows then their 8 up rows: 8 outputs at (y0 + c0) / 2
-                OutT* dst = C + (size_t)x_row * ldc + ((y0 + c0) >> 1);
-                float gate[8], up[8], out[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) gate[j] = v[j], up[j] = v[j + 8];
-                gate_mul_all<8>(ep, gate, up, out);
-                if (y0 + c0 + 16 <= y_rows && sizeof(OutT) == 2 && (((uintptr_t)dst & 15) == 0)) {
-                    uint32_t packed[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        __nv_bfloat162 pair = __floats2bfloat162_rn(out[2 * j], out[2 * j + 1]);
-                        packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-                    }
-                    *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (y0 + c0 + j + 8 < y_rows) dst[j] = from_f32<OutT>(out[j]);
-                }
-            } else if (SWAP) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int y = y0 + c0 + j;
-                    if (y < y_rows) C[(size_t)y * ldc + x_row] = from_f32<OutT>(v[j]);
-                }
-            } else {
-                OutT* dst = C + (size_t)x_row * ldc + y0 + c0;
-                const bool full = (y0 + c0 + 16 <= y_rows) && (((uintptr_t)dst & 15) == 0);
-                if (full && sizeof(OutT) == 2) {
-                    uint32_t packed[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                        packed[j] = *reinterpret_cast<uint32_t*>(&pair);
-                    }
-                    uint4* out = reinterpret_cast<uint4*>(dst);
-                    out[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    out[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                } else if (full && sizeof(OutT) == 4) {
-                    float4* out = reinterpret_cast<float4*>(dst);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) out[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (y0 + c0 + j < y_rows) dst[j] = from_f32<OutT>(v[j]);
-                }
+            for (int j = 0; j < 16; ++j) {
+                const int y = y0 + c0 + j;
+                if (y < y_rows) C[(size_t)y * ldc + x_row] = from_f32<OutT>(v[j]);
             }
         }
         if (tile_row == 0) gemm_stamp(ep, 7);
-        if (SWAP && staged) {
+        if (staged) {
             named_barrier_128();
             const int part = tile_row & 7;
 #pragma unroll 1
@@ -775,7 +724,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             if (h0 + HALF < BN) named_barrier_128();  // the next half is staged where this one was read
         }
         }  // halves
-        if (EPI == 2 && SWAP && !staged) {
+        if (EPI == 2 && !staged) {
             // this tile's share of each token's sum of squares: eight lanes add a token's 128 squares, sixteen each
             // (rotated so that the 32 lanes of a warp read 32 banks), in a fixed order.  (Tiles of up to 64 tokens only:
             // the launch gives wider tiles to this kernel only where the staged stores apply.)
@@ -1385,19 +1334,15 @@ static long max_resident_clusters(Kernel kernel, int smem_bytes, int cluster_z) 
     return answer;
 }
 
-template <int BN, bool SWAP, typename OutT, int EPI, typename... Chosen>
+template <int BN, typename OutT, int EPI, typename... Chosen>
 static int launch_config(const void* A, const void* W, bool tiled, void* C, int M, int N, int K, long lda, long ldc,
                          int splits, const Epilogue& ep, int* error_flag, cudaStream_t stream, const Chosen&... chosen) {
     using Smem = GemmSmem<BN, false>;
     CUtensorMap map_x, map_y;
-    const void* x_ptr = SWAP ? W : A;
-    const void* y_ptr = SWAP ? A : W;
-    const uint64_t x_rows = SWAP ? N : M, y_rows = SWAP ? M : N;
-    const uint64_t x_stride = SWAP ? K : lda, y_stride = SWAP ? lda : K;
-    if (tiled && (!SWAP || ((uintptr_t)W & 15))) return KIRAI_ERR_BAD_ALIGN;
-    if (!tmap::bf16_2d_sw128(&map_y, y_ptr, y_rows, K, y_stride, BN, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
+    if (tiled && ((uintptr_t)W & 15)) return KIRAI_ERR_BAD_ALIGN;
+    if (!tmap::bf16_2d_sw128(&map_y, A, M, K, lda, BN, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
     if (tiled) map_x = map_y;  // not read: the boxes are fetched by address
-    else if (!tmap::bf16_2d_sw128(&map_x, x_ptr, x_rows, K, x_stride, GEMM_BM, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
+    else if (!tmap::bf16_2d_sw128(&map_x, W, N, K, K, GEMM_BM, GEMM_BK)) return KIRAI_ERR_BAD_ALIGN;
     const int total_k_blocks = (K + GEMM_BK - 1) / GEMM_BK;
     if (splits < 1) splits = 1;
     int max_splits = Smem::max_splits;
@@ -1412,7 +1357,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
     for (;; --splits) {
         const int per_split = (total_k_blocks + splits - 1) / splits;
         const int used = (total_k_blocks + per_split - 1) / per_split;
-        dim3 grid((unsigned)((x_rows + GEMM_BM - 1) / GEMM_BM), (unsigned)((y_rows + BN - 1) / BN), (unsigned)used);
+        dim3 grid((unsigned)((N + GEMM_BM - 1) / GEMM_BM), (unsigned)((M + BN - 1) / BN), (unsigned)used);
         if (grid.y > 65535) return KIRAI_ERR_BAD_SIZE;
         const long clusters = (long)grid.x * grid.y;
         if constexpr (BN <= 128) {  // (tiles of 256 tokens have one configuration: four stages, one CTA per SM)
@@ -1425,7 +1370,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
             }
             if (busy * used <= sm_count() && deep_rings()) {
                 using Deep = GemmSmem<BN, true>;
-                auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, true, Chosen...>;
+                auto kernel = gemm_tcgen05_kernel<BN, OutT, EPI, true, Chosen...>;
                 cudaError_t err = allow_shared((const void*)kernel, Deep::total(Deep::max_splits));
                 if (err != cudaSuccess) return (int)err;
                 if (used > 1 && splits > 1 && busy > max_resident_clusters(kernel, Deep::total(used), used)) continue;
@@ -1434,7 +1379,7 @@ static int launch_config(const void* A, const void* W, bool tiled, void* C, int 
             }
         }
         if (used > Smem::max_splits) continue;  // (tiles of 128 tokens split only with the long ring)
-        auto kernel = gemm_tcgen05_kernel<BN, SWAP, OutT, EPI, false, Chosen...>;
+        auto kernel = gemm_tcgen05_kernel<BN, OutT, EPI, false, Chosen...>;
         cudaError_t err = allow_shared((const void*)kernel, Smem::total(Smem::max_splits));
         if (err != cudaSuccess) return (int)err;
         // launches of more CTAs than SMs run in waves anyway; only a launch meant to be one wave is fitted
@@ -1480,20 +1425,20 @@ static int gemm_dispatch(const void* A, const void* W, bool tiled, void* C, int 
     if (K % 8 != 0 || lda % 8 != 0) return KIRAI_ERR_BAD_ALIGN;  // TMA needs 16-byte row strides
     if (EPI == 1 && N % 16 != 0) return KIRAI_ERR_BAD_SIZE;      // whole groups of 8 gate + 8 up rows
     if (splits <= 0) splits = M <= 256 ? choose_splits(M, N, K) : 1;
-#define KIRAI_GEMM_CASE(BN, SWAP) \
-    return launch_config<BN, SWAP, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, splits, ep, error_flag, stream)
-    if (M <= 16) KIRAI_GEMM_CASE(16, true);
-    if (M <= 32) KIRAI_GEMM_CASE(32, true);
-    if (M <= 64) KIRAI_GEMM_CASE(64, true);
+#define KIRAI_GEMM_CASE(BN) \
+    return launch_config<BN, OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, splits, ep, error_flag, stream)
+    if (M <= 16) KIRAI_GEMM_CASE(16);
+    if (M <= 32) KIRAI_GEMM_CASE(32);
+    if (M <= 64) KIRAI_GEMM_CASE(64);
     // 65 to 128 tokens: still bound by the weight stream, which the many-token kernel below leaves to 16 to 96 CTAs
     // (230 us for the four products of an 8B layer against 66 us at 64 tokens).  The weight-streaming kernel takes
     // them where its staged stores apply (they do for every 16-byte aligned output).
-    if (M <= 128 && streams_wide_tiles(C, ldc, sizeof(OutT), N, EPI, ep)) KIRAI_GEMM_CASE(128, true);
+    if (M <= 128 && streams_wide_tiles(C, ldc, sizeof(OutT), N, EPI, ep)) KIRAI_GEMM_CASE(128);
     // 129 to 256 tokens: tiles of 256 tokens fill an SM each, so only launches of no more tiles than SMs (the 8B shape's
     // gate/up product, 192 tiles, ran as two waves: 99 us against 59 us in the many-token kernel; its down product, 32
     // tiles split three ways, 38 against 67)
     const bool one_wave = (N + GEMM_BM - 1) / GEMM_BM <= sm_count();
-    if (M <= 256 && one_wave && streams_wide_tiles(C, ldc, sizeof(OutT), N, EPI, ep)) KIRAI_GEMM_CASE(256, true);
+    if (M <= 256 && one_wave && streams_wide_tiles(C, ldc, sizeof(OutT), N, EPI, ep)) KIRAI_GEMM_CASE(256);
     if (M <= 256 && EPI == 2 && N % 8 == 0 && (M <= 128 || one_wave)) return KIRAI_ERR_BAD_ALIGN;  // see kirai_gemm_bf16_residual_parts
 #undef KIRAI_GEMM_CASE
     return launch_persistent<OutT, EPI>(A, W, tiled, C, M, N, K, lda, ldc, ep, error_flag, stream);
@@ -1571,8 +1516,8 @@ KIRAI_EXPORT int kirai_gemm_bf16_chosen(const void* A, const void* W, int tiled,
     if (!columns) chosen.expected_tiles = expected_tiles < 1 ? 1 : (expected_tiles < pieces ? expected_tiles : pieces);
     const int splits = choose_splits(M, columns ? N : chosen.expected_tiles * GEMM_BM, K);
 #define KIRAI_CHOSEN(BN)                                                                                                                      \
-    return form == 0 ? launch_config<BN, true, bf16, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream, chosen) \
-                     : launch_config<BN, true, float, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream, chosen)
+    return form == 0 ? launch_config<BN, bf16, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream, chosen) \
+                     : launch_config<BN, float, 0>(A, W, tiled != 0, C, M, N, K, lda, ldc, splits, ep, error_flag, stream, chosen)
     if (M <= 16) KIRAI_CHOSEN(16);
     if (M <= 32) KIRAI_CHOSEN(32);
     KIRAI_CHOSEN(64);
