@@ -1219,8 +1219,12 @@ static int sm_count() {
 // partly empty a quarter less for what is empty (the others get its share of L2 and power), and a tile of 256 rows its epilogue
 // on top, during which its accumulators are not free: 1,000 columns where a row goes to registers before it is stored, 3,000 where the
 // activation is worked out or 32-bit values are stored first.  128 x 256, which many full rounds run best, is left for
-// 6 % or more, and widths that cut the weights' boxes in pieces count 1.5 % more.  Fitted to 44 shapes (4B, 8B and 32B layers, 300 to
-// 2,048 tokens), each timed at 24 tiles: what it picks is 0.5 % slower than the best on average, 9 % at most.
+// 8 % or more (where this count gives 6 to 8 % less it was the faster one in 9 of 14 products, by up to 9 %), and widths that cut the weights' boxes in
+// pieces count 1.5 % more.  Fitted to 44 shapes (4B, 8B and 32B layers, 300 to
+// 2,048 tokens), each timed at 24 tiles, and compared with 128 x 256 alone at 388 products of other decoders' layers and heads, 129 to 2,048
+// tokens: 0.84 of its time on average, 1.016 at most.  Tiles of 256 rows begin at 128 columns: 33 products of 33 that took 96 or 112
+// by the same count were slower than in 128 x 256, by 4 to 13 % (4,096 x 4,096 at 900 to 1,012 tokens 30.5 us in 148 tiles of 256 x 112,
+// 27.0 in 128 of 128 x 256).
 // Grouped products, whose tiles without rows are known on the device alone, and the residual-and-norm epilogue, whose
 // callers count its column tiles, keep 128 x 256.
 struct PersistentTile {
@@ -1247,13 +1251,13 @@ static PersistentTile persistent_tile(int M, int N, int K, int epi, bool grouped
     double least = 0.0;
     for (int row_tiles = 1; row_tiles <= 2; ++row_tiles) {
         const long m_tiles = (M + row_tiles * GEMM_BM - 1) / (row_tiles * GEMM_BM);
-        for (int width = 256; width >= (row_tiles == 1 ? 48 : 96); width -= 16) {
+        for (int width = 256; width >= (row_tiles == 1 ? 48 : 128); width -= 16) {
             const long tiles = m_tiles * ((N + width - 1) / width), whole = (tiles + sms - 1) / sms;
             const double rounds = whole == 1 ? 1.0 : 0.25 * tiles / sms + 0.75 * whole;
             const double block = row_tiles == 1 ? width + 80.0 : 1.95 * (width + 32.0);
             const double exposed = row_tiles == 1 ? 0.0 : (epi == 1 || out_bytes == 4 ? 3000.0 : 1000.0);
             double cost = rounds * (k_blocks * block + exposed);
-            if (row_tiles == 1 && width == 256) cost *= 0.94;
+            if (row_tiles == 1 && width == 256) cost *= 0.92;
             if (width % 64 != 0) cost *= 1.015;
             if (least == 0.0 || cost < least) least = cost, best = PersistentTile{row_tiles, width};
         }
