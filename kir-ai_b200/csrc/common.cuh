@@ -46,6 +46,10 @@ __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat1
 // for weights and states this way while the kernel before them still runs: between two uses in a decode step gigabytes of
 // other weights have gone through L2, and a first load from memory costs about a microsecond.
 #define PREFETCH_ROWS 148  // a kernel with a block per row asks ahead up to so many rows; with more, blocks that start later find the lines
+// Whether a kernel with a block per row holds in registers all that the row needs before its sums are made (EARLY), in place of
+// reading it afterwards: that takes a third more registers, and from a few blocks an SM on, of 512 threads from two on, fewer
+// blocks beside each other cost more than a row's second wait.  (Measured: see the kernels.)
+static inline bool reads_early(long rows, int width) { return rows <= PREFETCH_ROWS || (rows <= 5 * PREFETCH_ROWS && width <= 4096); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ float warp_sum(float v) {

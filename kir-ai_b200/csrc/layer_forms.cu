@@ -103,8 +103,9 @@ __global__ void norm_add_kernel(float* __restrict__ resid, const float* __restri
 }
 
 // The same with 16-byte loads, the row of y kept in registers between the statistics and the add (width a multiple
-// of 4, at most 4 * VEC * blockDim values).
-template <int VEC>
+// of 4, at most 4 * VEC * blockDim values).  EARLY (see reads_early; 70 registers in place of 32): 3 rows of 4,096 3.03 to 2.20 us, 700
+// rows 6.89 to 5.48; not EARLY: 700 rows of 8,192 9.3 us in place of 11.2, 2,048 rows of 2,560 8.2 in place of 9.4, of 8,192 37.0 in place of 42.7.
+template <int VEC, bool EARLY>
 __global__ void norm_add_vec_kernel(float* __restrict__ resid, const float* __restrict__ y, const float* __restrict__ weight,
                                     bf16* __restrict__ copy, int hidden, float eps) {
     pdl_launch_dependents();
@@ -125,7 +126,8 @@ __global__ void norm_add_vec_kernel(float* __restrict__ resid, const float* __re
 #pragma unroll
     for (int n = 0; n < VEC; ++n) {
         const int i = threadIdx.x + n * blockDim.x;
-        if (i < quads) kept[n] = src[i], stream[n] = dst[i], w[n] = w4[i];
+        if (i < quads) kept[n] = src[i];
+        if (EARLY && i < quads) stream[n] = dst[i], w[n] = w4[i];
     }
 #pragma unroll
     for (int n = 0; n < VEC; ++n) {
@@ -143,6 +145,7 @@ __global__ void norm_add_vec_kernel(float* __restrict__ resid, const float* __re
     for (int n = 0; n < VEC; ++n) {
         const int i = threadIdx.x + n * blockDim.x;
         if (i < quads) {
+            if (!EARLY) stream[n] = dst[i], w[n] = w4[i];
             float4 r = stream[n];
             r.x += kept[n].x * scale * w[n].x;
             r.y += kept[n].y * scale * w[n].y;
@@ -167,7 +170,7 @@ KIRAI_EXPORT int kirai_norm_add(float* resid, const float* y, const float* weigh
     const bool aligned = hidden % 4 == 0 && (((uintptr_t)resid | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)copy) & 15) == 0;
     if (aligned && hidden <= 4 * 4 * 512) {
         const int threads = hidden <= 4 * 4 * 128 ? 128 : (hidden <= 4 * 4 * 256 ? 256 : 512);
-        return launch_pdl(norm_add_vec_kernel<4>, dim3(rows), dim3(threads), 0, stream, 1u, resid, y, weight, (bf16*)copy, hidden, eps);
+        return launch_pdl(reads_early(rows, hidden) ? norm_add_vec_kernel<4, true> : norm_add_vec_kernel<4, false>, dim3(rows), dim3(threads), 0, stream, 1u, resid, y, weight, (bf16*)copy, hidden, eps);
     }
     const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
     return launch_pdl(norm_add_kernel, dim3(rows), dim3(threads), 0, stream, 1u, resid, y, weight, (bf16*)copy, hidden, eps);

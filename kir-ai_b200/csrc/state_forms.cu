@@ -146,7 +146,9 @@ __global__ void rms_pair_mean_kernel(const float* __restrict__ a, const float* _
 
 // The same with 16-byte accesses, both rows kept in registers (up to four pieces a thread) and both sums in one pass through
 // shared memory: 17 us a launch at three rows of 4,096 before, under 4 now.
-// EARLY: the weights too are asked for ahead of the sums (up to 512 threads: a block of 1,024 has no registers for them).
+// EARLY: the weights too are asked for ahead of the sums (84 registers in place of 58, up to 512 threads: a block of 1,024 has no
+// registers for them): 3 rows of 4,096 2.86 to 2.36 us, 700 rows 6.8 to 6.1; not EARLY (see reads_early; short rows from 149 on too): 700 rows of 256
+// 3.5 us in place of 4.1, 149 rows of 8,192 4.2 in place of 4.9, 2,048 rows of 256, 4,096 and 8,192 5.9, 14.7 and 32.1 in place of 8.6, 21.1 and 48.6.
 template <bool EARLY>
 __global__ void __launch_bounds__(EARLY ? 512 : 1024) rms_pair_mean_vec_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ wa,
                                          const float* __restrict__ wb, float eps, float* __restrict__ out, int width) {
@@ -196,7 +198,8 @@ KIRAI_EXPORT int kirai_rms_pair_mean(const float* a, const float* b, const float
     if (width <= 0) return KIRAI_ERR_BAD_SIZE;
     if (width % 4 == 0 && width <= 16384 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)wa | (uintptr_t)wb | (uintptr_t)out) & 15) == 0) {
         const int wide = width <= 4096 ? 256 : (width <= 8192 ? 512 : 1024);
-        return launch_pdl(wide <= 512 ? rms_pair_mean_vec_kernel<true> : rms_pair_mean_vec_kernel<false>, dim3(rows), dim3(wide), 0, stream, 1u, a, b, wa, wb, eps, out, width);
+        const bool early = width <= 8192 && reads_early(rows, width) && (rows <= PREFETCH_ROWS || width > 2048);
+        return launch_pdl(early ? rms_pair_mean_vec_kernel<true> : rms_pair_mean_vec_kernel<false>, dim3(rows), dim3(wide), 0, stream, 1u, a, b, wa, wb, eps, out, width);
     }
     const int threads = width >= 1024 ? 256 : 128;
     return launch_pdl(rms_pair_mean_kernel, dim3(rows), dim3(threads), 0, stream, 1u, a, b, wa, wb, eps, out, width);

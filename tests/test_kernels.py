@@ -1235,3 +1235,40 @@ def test_the_error_word_leaves_a_step_beside_its_tokens(ops):
     flag.zero_()
     ops.decode_advance(results[:3], sampled, positions, lengths)
     assert results.tolist() == [5, 9, 2, 3] and positions.tolist() == [6, 7, 8] and lengths.tolist() == [7, 8, 9]
+
+
+@pytest.mark.parametrize("width", [256, 2048, 2052, 4096, 4100, 8192])
+@pytest.mark.parametrize("rows", [148, 149, 740, 741])
+def test_row_kernels_on_both_sides_of_where_they_read_early(ops, rows, width):
+    """Up to 148 rows, and up to 740 of at most 4,096 columns, a block asks for the whole row at once, then for its parts in turn: the
+    same arithmetic, so the same bits as the first rows give alone, and the formulas."""
+    stream, y, other = (rand(rows, width, seed=i) for i in (1, 2, 3))
+    w, w2 = rand(width, seed=4), rand(width, seed=5)
+    gates = torch.rand(rows, 3, generator=torch.Generator().manual_seed(6)).to(DEV)
+    unit = lambda x, eps: x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + eps)  # noqa: E731
+
+    def added(n):
+        resid = stream[:n].clone()
+        copy = ops.norm_add(resid, y[:n].contiguous(), w, 1e-6, torch.bfloat16)
+        return resid, copy
+
+    def terms(n):
+        resid = stream[:n].clone()
+        slots = torch.arange(2 * n, dtype=torch.int32, device=DEV).view(n, 2)
+        sorted_rows = torch.cat([y[:n, None], other[:n, None]], dim=1).reshape(2 * n, width).bfloat16()
+        copy = ops.terms_norm_add(resid, y[:n].contiguous(), (sorted_rows, slots, gates[:n, 1:].contiguous()), other[:n].contiguous(), gates[:n].contiguous(), 0, (1, 1),
+                                  w, 1e-6, torch.bfloat16)
+        return resid, copy
+
+    def mean(n):
+        return (ops.rms_pair_mean(y[:n].contiguous(), other[:n].contiguous(), w, w2, 1e-6),)
+
+    for run in (added, terms, mean):
+        for whole, few in zip(run(rows), run(5)):
+            assert torch.equal(whole[:5], few)
+    sums = y.double() + gates[:, :1].double() * other.double() + gates[:, 1:2].double() * stream.double()
+    sums += gates[:, 1:2].double() * y.bfloat16().double() + gates[:, 2:].double() * other.bfloat16().double()
+    # a dozen 32-bit operations on values of up to about 30, and sums of up to 8,192 squares in a tree
+    for got, want in ((added(rows)[0], stream.double() + unit(y, 1e-6) * w.double()), (terms(rows)[0], stream.double() + unit(sums, 1e-6) * w.double()),
+                      (mean(rows)[0], 0.5 * (unit(y, 1e-6) * w.double() + unit(other, 1e-6) * w2.double()))):
+        assert float((got.double() - want).abs().max()) <= 32 * 16.0 * 2.0 ** -24
