@@ -416,11 +416,17 @@ __device__ __forceinline__ void prefetch_state_rows(const float* mine, int lane,
 // held down as below.
 // xbc [T, inner + 2 G N] (float32): x, then B, then C, after convolution and silu; dt_raw (float32, row stride
 // dt_stride): the step sizes before softplus; y [T, inner] (float32) = S^T C + D x.
-// Registers are kept to 40 where a column's threads hold 16 rows each: at 74 an SM took three blocks of the 768 that three requests
-// make, and the second round of blocks waited a second time for everything that one waits for (11.7 to 9.6 us a launch).
+// SHARED (WIDE, 16 rows a thread, more than one thread a column): a token's B and C come through shared memory, and registers are kept to
+// 40: at 75 an SM took three blocks of the 768 that three requests make, and the second round of blocks waited a second time for
+// everything that one waits for (11.7 to 9.6 us a launch).  Alone, three requests of 128 heads of 128 x 64 12.0 to 10.0 us, 32 113 to 73.
+// Where more than one block an SM but no second round of three is launched, and where a thread has a column to itself, the loads from
+// global memory, many of them in flight, are the faster way: 8 requests of 24 heads of 100 x 48 6.3 us in place of 7.3, of 32 of 64 x 64
+// 5.7 in place of 6.1, 5 tokens of 16 heads of 16 x 64 7.5 in place of 11.5.
+// FEW (not WIDE): up to 128 registers for loads in flight, two blocks an SM, where that makes no more rounds than the three blocks of
+// 73 registers do: three requests of 16 heads of 256 x 64 10.8 to 8.7 us, but 32 of 8 heads of 300 x 64 55 to 61.
 #define WALK_WIDE_ROWS 128
-template <int REGS, bool WIDE>
-__global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, long dt_stride,
+template <int REGS, bool WIDE, bool SHARED, bool FEW = false>
+__global__ void __launch_bounds__(256, SHARED ? 6 : FEW ? 2 : 0) ssm_walk_kernel(const float* __restrict__ xbc, const float* __restrict__ dt_raw, long dt_stride,
                                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ d_skip,
                                 float* __restrict__ state, long state_len, long ssm_off, const int* __restrict__ query_start,
                                 const int* __restrict__ slots, float* __restrict__ y, int heads, int groups, int N, int P,
@@ -430,7 +436,7 @@ __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kern
     const int columns = blockDim.x / split;
     const int p = blockIdx.z * columns + (WIDE ? threadIdx.x % columns : threadIdx.x / split), s = WIDE ? threadIdx.x / columns : threadIdx.x % split;
     __shared__ float part[WIDE ? 2 : 1][WIDE ? 256 : 1];
-    __shared__ float bc_s[WIDE ? 2 : 1][WIDE ? 2 * WALK_WIDE_ROWS : 1];  // a token's B and C
+    __shared__ float bc_s[SHARED ? 2 : 1][SHARED ? 2 * WALK_WIDE_ROWS : 1];  // a token's B and C
     const long first = query_start[request];
     const int count = (int)(query_start[request + 1] - first);
     const int slot = slots[request];
@@ -438,10 +444,11 @@ __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kern
     const int inner = heads * P, channels = inner + 2 * groups * N;
     const float decay_rate = -expf(a_log[head]), skip = d_skip[head], bias = dt_bias[head];
     const bool live = p < P;
-    float* mine = state + slot * state_len + ssm_off + ((long)head * N) * P + p;
-    if (WIDE && slot >= 0 && slot < num_slots) prefetch_state_rows<REGS>(mine, threadIdx.x & 31, p, s, split, N, P);
+    if (WIDE && slot >= 0 && slot < num_slots)
+        prefetch_state_rows<REGS>(state + slot * state_len + ssm_off + ((long)head * N) * P + p, threadIdx.x & 31, p, s, split, N, P);
     pdl_wait();
     if (slot < 0 || slot >= num_slots) return;
+    float* mine = state + slot * state_len + ssm_off + ((long)head * N) * P + p;
     float S[REGS];
 #pragma unroll
     for (int i = 0; i < REGS; ++i) {
@@ -458,7 +465,7 @@ __global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 6 : 0) ssm_walk_kern
         const float* Cv = Bv + groups * N;
         const float take = dt * x;
         float acc = 0.0f;
-        if constexpr (WIDE) {
+        if constexpr (SHARED) {
             float* const bc = bc_s[t & 1];
             for (int n = threadIdx.x; n < 2 * N; n += blockDim.x) bc[n] = n < N ? Bv[n] : Cv[n - N];
             __syncthreads();
@@ -517,6 +524,15 @@ static int walk_shape(int rows, int cols, int* split, int* threads, int* chunks)
     return per <= 4 ? 4 : per <= 16 ? 16 : per <= 64 ? 64 : 0;
 }
 
+static int walk_sms() {
+    static const int count = [] {
+        int device = 0, value = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&value, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 148;
+        return value;
+    }();
+    return count;
+}
+
 KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_stride, const float* dt_bias, const float* a_log,
                                 const float* d_skip, float* state, long state_len, long ssm_off, const int* query_start,
                                 const int* slots, float* y, int requests, int heads, int groups, int N, int P, int num_slots,
@@ -528,14 +544,15 @@ KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_s
     const int regs = walk_shape(N, P, &split, &threads, &chunks);
     if (!regs) return KIRAI_ERR_BAD_SIZE;
     const bool wide = (threads / split) % 32 == 0 && N <= WALK_WIDE_ROWS;
-#define KIRAI_SSM(R)                                                                                                         \
-    return launch_pdl(wide ? ssm_walk_kernel<R, true> : ssm_walk_kernel<R, false>, dim3(requests, heads, chunks), dim3(threads), 0, stream, 1u, xbc, dt_raw, dt_stride, \
-                      dt_bias, a_log, d_skip, state, state_len, ssm_off, query_start, slots, y, heads, groups, N, P, split,  \
-                      num_slots)
-    if (regs == 4) KIRAI_SSM(4);
-    if (regs == 16) KIRAI_SSM(16);
-    KIRAI_SSM(64);
-#undef KIRAI_SSM
+    const long blocks = (long)requests * heads * chunks, two = 2L * walk_sms(), three = 3L * walk_sms();
+    const bool shared = wide && split > 1 && (blocks <= walk_sms() || blocks > three);
+    const bool few = (blocks + two - 1) / two <= (blocks + three - 1) / three;
+    auto kernel = regs == 4 ? (wide ? ssm_walk_kernel<4, true, false> : ssm_walk_kernel<4, false, false>)
+                : regs == 64 ? ssm_walk_kernel<64, false, false>
+                : shared ? ssm_walk_kernel<16, true, true> : wide ? ssm_walk_kernel<16, true, false>
+                : few ? ssm_walk_kernel<16, false, false, true> : ssm_walk_kernel<16, false, false>;
+    return launch_pdl(kernel, dim3(requests, heads, chunks), dim3(threads), 0, stream, 1u, xbc, dt_raw, dt_stride, dt_bias, a_log, d_skip,
+                      state, state_len, ssm_off, query_start, slots, y, heads, groups, N, P, split, num_slots);
 }
 
 // ------------------------------------------------------------------ matrix-memory walk
@@ -545,10 +562,11 @@ KIRAI_EXPORT int kirai_ssm_walk(const float* xbc, const float* dt_raw, long dt_s
 // once more and stores them, after every block of the walk has read the old ones.
 // rows (float32, row stride): q [H d], k [H d], v [H dv], then the input gates' [H] and the forget gates' [H]
 // pre-activations.  state [slots, state_len]: S [H, d, dv], then n [H, d], then m [H].  o [T, H dv] (float32).
-// Registers are kept to 80 (16 rows a thread), for three blocks on an SM: 384 blocks of three requests in one round (15.0 to 12.4 us
-// with the normaliser's kernel).
-template <int REGS, bool WIDE>
-__global__ void __launch_bounds__(256, WIDE && REGS == 16 ? 3 : 0) matrix_memory_walk_kernel(const float* __restrict__ rows, long row_stride, const float* __restrict__ in_bias,
+// TIGHT (WIDE, 16 rows a thread): registers are kept to 80, for three blocks on an SM, so that 384 blocks of three requests are one round
+// (15.0 to 12.4 us inside a step with the normaliser's kernel, alone 15.6 to 12.6).  With fewer loads in flight a round takes up to 1.36 times as long, so
+// it is for launches that save more rounds than that (one request 9.4 us, TIGHT 11.3; five tokens 28.4 and 38.7; 4 heads of 64 x 64 7.5 and 8.3).
+template <int REGS, bool WIDE, bool TIGHT>
+__global__ void __launch_bounds__(256, TIGHT ? 3 : 0) matrix_memory_walk_kernel(const float* __restrict__ rows, long row_stride, const float* __restrict__ in_bias,
                                           const float* __restrict__ keep_bias, float cap, float q_scale, float* __restrict__ state,
                                           long state_len, const int* __restrict__ query_start, const int* __restrict__ slots,
                                           float* __restrict__ o, int heads, int d, int dv, int split, int num_slots) {
@@ -671,16 +689,14 @@ KIRAI_EXPORT int kirai_matrix_memory_walk(const float* rows, long row_stride, co
     int split, threads, chunks;
     const int regs = walk_shape(d, dv, &split, &threads, &chunks);
     if (!regs) return KIRAI_ERR_BAD_SIZE;
-    int status;
     const bool wide = (threads / split) % 32 == 0;
-#define KIRAI_MM(R)                                                                                                            \
-    status = launch_pdl(wide ? matrix_memory_walk_kernel<R, true> : matrix_memory_walk_kernel<R, false>, dim3(requests, heads, chunks), dim3(threads), 0, stream, 1u, rows,       \
-                        row_stride, in_bias, keep_bias, cap, q_scale, state, state_len, query_start, slots, o, heads, d, dv,   \
-                        split, num_slots)
-    if (regs == 4) KIRAI_MM(4);
-    else if (regs == 16) KIRAI_MM(16);
-    else KIRAI_MM(64);
-#undef KIRAI_MM
+    const long blocks = (long)requests * heads * chunks, two = 2L * walk_sms(), three = 3L * walk_sms();
+    const bool tight = 1.36 * (double)((blocks + three - 1) / three) < (double)((blocks + two - 1) / two);
+    auto kernel = regs == 4 ? (wide ? matrix_memory_walk_kernel<4, true, false> : matrix_memory_walk_kernel<4, false, false>)
+                : regs == 64 ? matrix_memory_walk_kernel<64, false, false>
+                : !wide ? matrix_memory_walk_kernel<16, false, false> : tight ? matrix_memory_walk_kernel<16, true, true> : matrix_memory_walk_kernel<16, true, false>;
+    const int status = launch_pdl(kernel, dim3(requests, heads, chunks), dim3(threads), 0, stream, 1u, rows, row_stride, in_bias, keep_bias, cap, q_scale,
+                                  state, state_len, query_start, slots, o, heads, d, dv, split, num_slots);
     if (status != 0) return status;
     const int norm_threads = d >= 256 ? 256 : ((d + 31) / 32) * 32;
     return launch_pdl(matrix_memory_norm_kernel, dim3(requests, heads), dim3(norm_threads), 0, stream, 1u, rows, row_stride, in_bias,

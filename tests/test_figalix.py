@@ -1102,3 +1102,39 @@ def test_walks_up_to_and_beyond_the_rows_that_shared_memory_holds(heads, groups,
     """Up to 128 rows of a state a block's threads hold whole runs of 32 columns (the first four; 8 threads a column, 8 with columns
     beyond the last, 1, and 1 with 4 rows) and B and C come through shared memory; from 129 rows on they hold 16 columns or 8."""
     test_state_space_runs_in_chunks_as_token_by_token(heads, groups, state, vdim)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [49, 74, 75, 148, 149, 222, 223])
+@pytest.mark.parametrize("rows", [16, 24, 64, 100, 128])
+def test_walks_of_many_blocks_give_the_bits_of_a_few(heads, rows):
+    """How many blocks a launch has decides how its registers are held down and whether B and C come through shared memory: 2
+    requests of 49 heads (98 blocks, an SM each), up to 444 (three an SM) and beyond.  The first head alone gives the same bits."""
+    from types import SimpleNamespace
+    from kirai_b200.csrc import ops
+
+    gen = torch.Generator().manual_seed(heads + rows)
+    cols, lens = 64, [3, 1]
+    T, batch = sum(lens), SimpleNamespace(query_start=torch.tensor([0, 3, 4], dtype=torch.int32, device="cuda:0"), slots=torch.tensor([1, 0], dtype=torch.int32, device="cuda:0"),
+                                          num_requests=2, max_query_len=3)
+    draw = lambda *shape: torch.randn(*shape, generator=gen).to("cuda:0")  # noqa: E731
+    x, bc, dt, state = draw(T, heads, cols), draw(T, 2 * rows), draw(T, heads), draw(2, heads, rows * cols)
+    bias, a_log, skip = draw(heads), draw(heads), draw(heads)
+
+    def ssm(n):
+        st = state[:, :n].reshape(2, -1).clone()
+        y = ops.ssm_walk(torch.cat([x[:, :n].reshape(T, -1), bc], dim=1).contiguous(), dt[:, :n].contiguous(), bias[:n].contiguous(), a_log[:n].contiguous(),
+                         skip[:n].contiguous(), st, 0, batch, n, 1, rows, cols, walk_limit=100)
+        return y.view(T, n, cols)[:, 0], st.view(2, n, -1)[:, 0]
+
+    q, k, gates, norm = draw(T, heads, rows), draw(T, heads, rows), draw(T, 2, heads), draw(2, heads, rows)
+
+    def memory(n):
+        st = torch.cat([state[:, :n].reshape(2, -1), norm[:, :n].reshape(2, -1), bias[:n].expand(2, n)], dim=1).contiguous()
+        parts = [t[:, :n].reshape(T, -1) for t in (q, k, x)] + [gates[:, :, :n].reshape(T, -1)]
+        o = ops.matrix_memory_walk(torch.cat(parts, dim=1).contiguous(), None, None, 8.0, rows ** -0.5, st, batch, n, rows, cols, walk_limit=100)
+        return o.view(T, n, cols)[:, 0], st[:, : n * rows * cols].view(2, n, -1)[:, 0]
+
+    for walk in (ssm, memory):
+        for many, few in zip(walk(heads), walk(1)):
+            assert torch.equal(many, few), walk.__name__
