@@ -405,11 +405,13 @@ static Cut choose_cut(int M, int N, int K, int sms) {
 // Where a product's tiles fill a few rounds and a little of one more (456 CTAs of 192 rows on 148 SMs: four rounds, the last with
 // 12), the columns of the whole rounds are one launch and the rest a second one with a cut of its own, finer along K, which
 // starts as the first one's CTAs end.  How many columns (a multiple of TILE_N) the first launch takes and its rows a tile;
-// 0 where one launch is as good to a twentieth.
-static int whole_rounds(int M, int N, int K, int sms, float single_us, int* bn) {
+// 0 where one launch is as good to a twentieth.  A single launch of several rounds of 128 rows counts 0.63 us a block here (measured: 640 rows of 6,144 x
+// 2,560 111 us, counted 128 by the time above, and 119 as two launches; of 19,456 x 2,560 360 us, counted 384, and 379 as two).
+static int whole_rounds(int M, int N, int K, int sms, const Cut& single, int* bn) {
     const int blocks = (K + BLOCK_K - 1) / BLOCK_K;
     const long columns = (N + TILE_N - 1) / TILE_N;
-    float least = 0.95f * single_us;
+    const bool counted_high = single.bn == 128 && single.splits == 1;
+    float least = 0.95f * single.us * (counted_high ? (8.0f + 0.63f * (float)blocks) / (8.0f + cut_block_us[2] * (float)blocks) : 1.0f);
     int taken = 0;
     for (int b = 0; b < 4; ++b) {
         if (b > 0 && cut_rows[b - 1] >= M) break;
@@ -424,7 +426,7 @@ static int whole_rounds(int M, int N, int K, int sms, float single_us, int* bn) 
 }
 // The same for a device of `sms` SMs: the columns of the first launch (0: one launch takes them all), `rows` its rows a tile.
 KIRAI_EXPORT int kirai_gemm_f32_tc_first_columns(int M, int N, int K, int sms, int* rows) {
-    return whole_rounds(M, N, K, sms, choose_cut(M, N, K, sms).us, rows);
+    return whole_rounds(M, N, K, sms, choose_cut(M, N, K, sms), rows);
 }
 
 static int launch_cut(const Cut& cut, const float* A, const float* W, bf16* planes, float* C, int M, int N, int K, long lda, long ldc, int pitch,
@@ -456,7 +458,7 @@ KIRAI_EXPORT int kirai_gemm_f32_tc(const void* A_, const void* W_, void* planes_
     const int sms = sm_count();
     const Cut cut = bn == 0 ? choose_cut(M, N, K, sms) : Cut{bn, splits > 0 ? splits : 1, 0.0f};
     int first_bn = 0;
-    const int first = bn == 0 && splits == 0 ? whole_rounds(M, N, K, sms, cut.us, &first_bn) : 0;
+    const int first = bn == 0 && splits == 0 ? whole_rounds(M, N, K, sms, cut, &first_bn) : 0;
     const int pitch = (K + 7) / 8 * 8;
     const long quads = (long)M * (K / 4);
     const long cut_blocks = (quads + 255) / 256;

@@ -29,6 +29,9 @@ def test_32_bit_products_fill_whole_rounds_of_the_device_that_runs_them(lib, sms
     assert cut
     if sms == 148:  # 456 CTAs of 192 rows: three rounds, and 4 columns of tiles to the second launch
         assert (lib.kirai_gemm_f32_tc_first_columns(515, 19456, 2560, sms, ctypes.byref(rows)), rows.value) == (148 * 128, 192)
+        # measured as two launches 119 and 379 us, as one 111 and 360
+        for n in (6144, 19456):
+            assert lib.kirai_gemm_f32_tc_first_columns(640, n, 2560, sms, ctypes.byref(rows)) == 0
 
 
 def test_tiles_of_many_token_products_are_those_that_measured_faster(lib):
