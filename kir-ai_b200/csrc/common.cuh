@@ -45,6 +45,7 @@ __device__ __forceinline__ bf16 from_f32<bf16>(float v) { return __float2bfloat1
 // the line: L2 is where every SM's loads and stores meet, so a later load finds what was written last.  Kernels of few rows ask
 // for weights and states this way while the kernel before them still runs: between two uses in a decode step gigabytes of
 // other weights have gone through L2, and a first load from memory costs about a microsecond.
+#define PREFETCH_TURNS 8   // of blocks that would all ask for the same lines, so many do (add_dyt, 148 rows of 4,096: 2.3 us, 2.6 where all asked)
 #define PREFETCH_ROWS 148  // a kernel with a block per row asks ahead up to so many rows; with more, blocks that start later find the lines
 // Whether a kernel with a block per row holds in registers all that the row needs before its sums are made (EARLY), in place of
 // reading it afterwards: that takes a third more registers, and from a few blocks an SM on, of 512 threads from two on, fewer

@@ -183,7 +183,9 @@ router_gates_few_kernel(const T* __restrict__ x, long x_stride, const float* __r
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* row = x + (size_t)token * x_stride;
     const float* w = router + (size_t)e * hidden;
-    for (int i = threadIdx.x * 32; i < hidden; i += ROUTER_WARPS * 32 * 32) prefetch_l2(w + i);
+    if (token < PREFETCH_TURNS) {
+        for (int i = threadIdx.x * 32; i < hidden; i += ROUTER_WARPS * 32 * 32) prefetch_l2(w + i);
+    }
     pdl_wait();
     float* out = gates + (size_t)token * (experts + rule.extra);
     float dot = 0.0f;

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256) add_dyt_vec_kernel(float* __restrict__ re
                                                           const int* __restrict__ row_index, int width) {
     pdl_launch_dependents();
     const int c = (blockIdx.y * 256 + threadIdx.x) * 4;
-    if (gridDim.x <= PREFETCH_ROWS && (threadIdx.x & 7) == 0 && c < width) prefetch_l2(w + c), prefetch_l2(b + c);
+    if (gridDim.x <= PREFETCH_ROWS && blockIdx.x < PREFETCH_TURNS && (threadIdx.x & 7) == 0 && c < width) prefetch_l2(w + c), prefetch_l2(b + c);
     pdl_wait();
     if (c >= width) return;
     const float a = alpha[0];
